@@ -390,17 +390,14 @@ enum FinOp {
 };
 
 // The scalar update OP of group g from its reduced tile partials tot, by
-// one thread.  owner = false leaves the per-group arrays (diagT, upperT,
-// vnorm) untouched: the persistent step kernel applies the step updates in
-// every block that holds a tile of the group (same inputs, same result) and
-// lets one block write them.
+// one thread.
 template <int OP>
 __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double tot1, int it,
                                           int MI, double tol, int mpass,
                                           double *__restrict__ diagT,
                                           double *__restrict__ upperT,
                                           double *__restrict__ vnorm,
-                                          int *__restrict__ any_active, bool owner);
+                                          int *__restrict__ any_active);
 
 // One block per group: reduce the group's tile partials in a fixed order
 // (thread-strided sequential sums, then the block tree of LZ_THREADS
@@ -446,8 +443,7 @@ __device__ void fin_body(GState &s, int g, const double *__restrict__ part, int 
     }
   }
   if (threadIdx.x != 0) return;
-  fin_apply<OP>(s, g, tot[0], tot[1], it, MI, tol, mpass, diagT, upperT, vnorm, any_active,
-                true);
+  fin_apply<OP>(s, g, tot[0], tot[1], it, MI, tol, mpass, diagT, upperT, vnorm, any_active);
 }
 
 template <int OP>
@@ -456,7 +452,7 @@ __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double 
                                           double *__restrict__ diagT,
                                           double *__restrict__ upperT,
                                           double *__restrict__ vnorm,
-                                          int *__restrict__ any_active, bool owner) {
+                                          int *__restrict__ any_active) {
   const double tot[2] = {tot0, tot1};
   double dn = (double)s.n;
   if (OP == FIN_IV_MEAN || OP == FIN_INIT_MEAN || OP == FIN_PMEAN || OP == FIN_RITZ_MEAN) {
@@ -468,7 +464,7 @@ __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double 
     double rnorm = __dsqrt_rn(rtr);
     s.rnorm = rnorm;
     s.rtol = __dmul_rn(rnorm, tol);
-    if (owner) vnorm[(ll)g * (MI + 1)] = rnorm;
+    vnorm[(ll)g * (MI + 1)] = rnorm;
     s.rtz2 = 1.0;
     s.rtz1 = rtr;
     s.beta = 0.0;
@@ -484,8 +480,7 @@ __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double 
     double pap = tot[0], pap_old = s.pap;
     s.pap = pap;
     s.alpha = __ddiv_rn(s.rtz1, pap);
-    if (!owner) {
-    } else if (it == 0) {
+    if (it == 0) {
       diagT[(ll)g * MI] = __ddiv_rn(pap, s.rtz1);
     } else {
       double bb = __dmul_rn(s.beta, s.beta);
@@ -496,7 +491,7 @@ __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double 
   } else if (OP == FIN_RTR) {
     double rtr = tot[0];
     double rnorm = __dsqrt_rn(rtr);
-    if (owner) vnorm[(ll)g * (MI + 1) + it + 1] = rnorm;
+    vnorm[(ll)g * (MI + 1) + it + 1] = rnorm;
     s.rnorm = rnorm;
     s.iters = it + 1;
     if (rnorm < s.rtol) {
@@ -510,7 +505,7 @@ __device__ __forceinline__ void fin_apply(GState &s, int g, double tot0, double 
     s.beta = __ddiv_rn(s.rtz1, s.rtz2);
     // the off-diagonal that the next step's FIN_PAP enters (the same
     // expression on the same values), known now for the Ritz residual bound
-    if (owner && it + 1 < MI)
+    if (it + 1 < MI)
       upperT[(ll)g * MI + it] =
           __ddiv_rn(__dmul_rn(-s.beta, s.pap), __dsqrt_rn(__dmul_rn(s.rtz2, s.rtz1)));
   } else if (OP == FIN_PASS_END) {
@@ -1434,216 +1429,6 @@ k_spmv_tma(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
   if (fuse) fused_fin<FIN_PAP>(gs, g, part, fa, sh);
 }
 
-// ---------------------------------------------------------------------------
-// Persistent segmented step kernel: every Lanczos step of a pass
-// (src/fiedler.c:458-504) for all groups of the level in one cooperative
-// launch, in place of the six launches per step (P update, its
-// finalisation, SpMV, finalisation, R update, finalisation).  Block b owns
-// tiles b, b + G, b + 2G, ... (G blocks, all resident: a cooperative launch
-// refuses a grid that does not fit).  A step is three phases separated by
-// grid barriers; each phase runs the same tile body as the stand-alone
-// kernel (pr_tile, spmv_tile) and writes the same tile partials, into a
-// partial array of its own.  After a barrier every block reduces, for each
-// of its tiles whose group runs, the group's partials in the order of k_fin
-// (256 virtual threads: strided sequential sums, warp trees, the warps in
-// order) and applies the scalar update to its own copy of the group state
-// in shared memory; the block holding the group's first tile writes the
-// per-group arrays and, at the end, the state.  Results are bitwise those of
-// the launch-per-kernel pass.  Each barrier wait gives up after about one
-// second (globaltimer), sets err and returns; a block that sees err set
-// returns at its next barrier, so the kernel always ends.
-// ---------------------------------------------------------------------------
-constexpr int PS_THREADS = LZ_THREADS;  // the finalisation order is k_fin's
-constexpr int PS_SLOTS = 32;            // tiles per block at most
-
-struct StepArgs {
-  const ll *tbeg, *tend;
-  const int *tgrp;
-  GState *gs;
-  void *p, *w, *V;
-  ll VS;
-  const unsigned *ell;
-  const ll *slice_off;
-  const int *slice_w;
-  double *part;  // 3 T: the P, SpMV and R tile partials
-  double *diagT, *upperT, *vnorm;
-  unsigned *bar;  // barrier arrivals (zero at launch)
-  int *run_cnt;   // per step: groups still running after it (zero at launch)
-  int *err;       // 2: a barrier wait gave up
-  int T, MI;
-  double tol;
-};
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__global__ void k_ps_reset(unsigned *__restrict__ bar, int *__restrict__ run_cnt, int MI) {
-  pdl_entry();
-  if (threadIdx.x == 0) bar[0] = 0u;
-  for (int i = threadIdx.x; i < MI; i += blockDim.x) run_cnt[i] = 0;
-}
-
-// Grid barrier number k (targets k G arrivals).  False when it gave up or
-// another block did.
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *err) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    int ok = 1;
-    const unsigned long long t0 = global_ns();
-    for (unsigned n = 0;; n++) {
-      if (ld_acquire_u32(bar) >= target) break;
-      if (*(volatile int *)err) {
-        ok = 0;
-        break;
-      }
-      if ((n & 63) == 63 && (global_ns() - t0 > 1000000000ull || n > (1u << 26))) {
-        atomicExch(err, 2);  // about one second, or 2^26 polls of at least 64 ns
-        ok = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    __threadfence();
-    ok_s = ok;
-  }
-  __syncthreads();
-  __threadfence();  // every thread: later loads see the other blocks' writes
-  return ok_s != 0;
-}
-
-// The step finalisation OP for every slot of the block whose group runs, in
-// k_fin's reduction order (256 threads: strided sequential sums, warp trees,
-// the warps in order).  A group of more than 256 tiles is reduced by the
-// whole block with k_fin's own code (eight loads in flight per thread); a
-// smaller one by one warp that stands in for the 256 threads (each holds at
-// most one partial), all of its loads issued before the trees.
-template <int OP>
-__device__ __forceinline__ void step_fin(GState *st, const int *sg, int nslot,
-                                         const double *__restrict__ part, const StepArgs &a,
-                                         int it, double *sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = 0; k < nslot; k++) {  // big groups: the whole block
-    GState &s = st[k];
-    if (!s.run || s.ntiles <= PS_THREADS) continue;  // block-uniform
-    double acc = 0.0;
-    for (int q = threadIdx.x; q < s.ntiles; q += 8 * PS_THREADS) {  // as fin_body
-      double x[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++)
-        x[u] = q + u * PS_THREADS < s.ntiles ? __ldcg(&part[s.tile0 + q + u * PS_THREADS]) : 0.0;
-#pragma unroll
-      for (int u = 0; u < 8; u++)
-        if (q + u * PS_THREADS < s.ntiles) acc = __dadd_rn(acc, x[u]);
-    }
-    const double tot = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-      const int t = blockIdx.x + k * gridDim.x;
-      fin_apply<OP>(s, sg[k], tot, 0.0, it, a.MI, a.tol, 0, a.diagT, a.upperT, a.vnorm, nullptr,
-                    t == s.tile0);
-    }
-    __syncthreads();
-  }
-  for (int k = warp; k < nslot; k += PS_THREADS / 32) {  // small groups: a warp each
-    GState &s = st[k];
-    if (!s.run || s.ntiles > PS_THREADS) continue;  // warp-uniform
-    double x[PS_THREADS / 32];
-#pragma unroll
-    for (int u = 0; u < PS_THREADS / 32; u++) {
-      const int q = lane + 32 * u;
-      x[u] = q < s.ntiles ? __dadd_rn(0.0, __ldcg(&part[s.tile0 + q])) : 0.0;
-    }
-    double tot = 0.0;
-#pragma unroll
-    for (int u = 0; u < PS_THREADS / 32; u++) {
-      const double ws = warp_tree_sum(x[u]);
-      if (lane == 0) tot = __dadd_rn(tot, ws);
-    }
-    if (lane == 0) {
-      const int t = blockIdx.x + k * gridDim.x;
-      fin_apply<OP>(s, sg[k], tot, 0.0, it, a.MI, a.tol, 0, a.diagT, a.upperT, a.vnorm, nullptr,
-                    t == s.tile0);
-    }
-  }
-}
-
-template <typename VT>
-__global__ void __launch_bounds__(PS_THREADS, 8) k_steps(StepArgs a) {
-  __shared__ GState st[PS_SLOTS];
-  __shared__ int sg[PS_SLOTS];
-  __shared__ double cs[LZ_TILE / 32 + 2];
-  __shared__ float2 cs2[LZ_TILE / 32 + 2];
-  __shared__ double wlut[16];
-  __shared__ double sh[32];
-  const int G = gridDim.x;
-  const int nslot = (a.T - (int)blockIdx.x + G - 1) / G;  // tiles blockIdx.x + k G < T
-  VT *p = static_cast<VT *>(a.p), *w = static_cast<VT *>(a.w), *V = static_cast<VT *>(a.V);
-  double *partP = a.part, *partS = a.part + a.T, *partR = a.part + 2 * (ll)a.T;
-  for (int k = threadIdx.x; k < nslot; k += PS_THREADS) {
-    sg[k] = a.tgrp[blockIdx.x + k * G];
-    st[k] = a.gs[sg[k]];
-  }
-  if (threadIdx.x < 16) wlut[threadIdx.x] = (double)threadIdx.x;
-  __syncthreads();
-  unsigned nbar = 0;
-  for (int it = 0; it < a.MI; it++) {
-    // p = r (step 0) or beta (p - c) + r; partials of sum p
-    for (int k = 0; k < nslot; k++) {
-      if (!st[k].run) continue;  // block-uniform
-      const int t = blockIdx.x + k * G;
-      pr_tile<VT, TM_P, 1>(a.tbeg[t], a.tend[t], (VT)st[k].c, (VT)st[k].beta, (VT)st[k].alpha,
-                           it, p, w, V, a.VS, cs, cs2, partP, t);
-      __syncthreads();
-    }
-    if (!grid_barrier(a.bar, ++nbar * (unsigned)G, a.err)) return;
-    if (it > 0 && ld_acquire_u32(reinterpret_cast<const unsigned *>(a.run_cnt) + it - 1) == 0)
-      break;  // no group of the level runs (the same value in every block)
-    step_fin<FIN_PMEAN>(st, sg, nslot, partP, a, it, sh);
-    __syncthreads();
-    // w = L p; partials of sum w (p - c)
-    for (int k = 0; k < nslot; k++) {
-      if (!st[k].run) continue;
-      const int t = blockIdx.x + k * G;
-      spmv_tile<VT>(a.tbeg[t], a.tend[t], (VT)st[k].c, a.ell, a.slice_off, a.slice_w, p, w, wlut,
-                    cs, cs2, partS, t);
-      __syncthreads();
-    }
-    if (!grid_barrier(a.bar, ++nbar * (unsigned)G, a.err)) return;
-    step_fin<FIN_PAP>(st, sg, nslot, partS, a, it, sh);
-    __syncthreads();
-    // V[it+1] = V[it] - alpha w; partials of sum V[it+1]^2
-    for (int k = 0; k < nslot; k++) {
-      if (!st[k].run) continue;
-      const int t = blockIdx.x + k * G;
-      pr_tile<VT, TM_R, 1>(a.tbeg[t], a.tend[t], (VT)st[k].c, (VT)st[k].beta, (VT)st[k].alpha,
-                           it, p, w, V, a.VS, cs, cs2, partR, t);
-      __syncthreads();
-    }
-    if (!grid_barrier(a.bar, ++nbar * (unsigned)G, a.err)) return;
-    step_fin<FIN_RTR>(st, sg, nslot, partR, a, it, sh);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int running = 0;
-      for (int k = 0; k < nslot; k++)
-        if (blockIdx.x + k * G == st[k].tile0 && st[k].run) running++;
-      if (running) atomicAdd(&a.run_cnt[it], running);
-    }
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < nslot; k += PS_THREADS)
-    if ((int)blockIdx.x + k * G == st[k].tile0) a.gs[sg[k]] = st[k];
-}
-
 // Ritz vector f_i = sum_j coef_j V_j[i] (j < iters, src/fiedler.c:520-535)
 // and the tile partial of sum f, R rows per lane (16-byte loads of each
 // basis row).  FP32: compensated dot (Ogita, Rump and Oishi's Dot2) with each
@@ -1999,7 +1784,7 @@ __device__ __forceinline__ double warp_max_d(double v) {
 // bracket of relative width rel
 __device__ double eig_index(const double *d, const double *e2, int n, int k, double lo,
                             double hi, double rel = 2.2e-16) {
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31;
   double a = lo, b = hi;
   for (int round = 0; round < 24; round++) {
     double w = __dsub_rn(b, a);
@@ -2085,47 +1870,20 @@ __global__ void k_tri_eig(GState *__restrict__ gs, int ngroups,
 // T_k (k = it + 1) the tridiagonal matrix of the pass so far, theta its
 // smallest eigenvalue and y the normalised eigenvector, the Lanczos relation
 // L V_k = V_k T_k + b_k v_(k+1) e_k^T gives |L V_k y - theta V_k y| = |b_k y_k|
-// for an orthonormal basis, b_k = upperT[it] being the off-diagonal that
-// step it + 1 enters (FIN_RTR of step it writes it).  theta by multisection
-// to a relative 1e-10; y_k from the bottom twist of T_k - theta I: the
+// for an orthonormal basis, b_k being the off-diagonal that step it + 1
+// enters.  theta by multisection to a relative 1e-10 (from [0.99 th0, th0]
+// when th0 > 0, the last check's Ritz value: the smallest Ritz value never
+// grows with the steps of a pass; both ends are checked by Sturm counts, else
+// Gershgorin's interval); y_k from the bottom twist of T_k - theta I: the
 // pivots d_i of its LDL^T factorisation (positive below the last for the
 // smallest eigenvalue) and z_(k-1) = 1, z_i = -e_i z_(i+1) / d_i,
-// y_k = 1 / |z|.  Writes the bound to bound_out[g MI + it] (when given) and,
-// when it is below stop_below, asks to end the group's pass (stopreq).
-// It runs on a second stream beside the next steps: it reads only entries
-// of T that step it completed (each written with the same value wherever it
-// is written), whether the group ran step it, and its own fields of the
-// group state, so its answer does not depend on how far the other stream
-// has got; k_apply_stop turns the request into run = 0 at a fixed step after
-// joining the streams.  To spend little of the FP64 pipe, a group whose
-// last bound was above 30 stop_below is computed again only `span` steps
-// after it, and the multisection starts from [0.99 theta', theta'], theta'
-// the last check's Ritz value (the smallest Ritz value never grows with the
-// steps of a pass; both ends are checked by Sturm counts, else Gershgorin's
-// interval).  One warp per group; a group whose T_k has an eigenvalue below
-// 0 is left alone.
-__global__ void k_ritz_bound(GState *__restrict__ gs, int ngroups,
-                             const double *__restrict__ diagT, const double *__restrict__ upperT,
-                             int MI, int it, double stop_below, int span,
-                             double *__restrict__ bound_out) {
-  pdl_entry();
-  extern __shared__ double rb_sm[];
-  const int g = blockIdx.x, lane = threadIdx.x;
-  if (g >= ngroups) return;
-  GState &st = gs[g];
-  if (!st.active || *(volatile const int *)&st.iters < it + 1) return;  // step it not run
-  if (!bound_out && st.rb_it >= 0 && st.rb_bound > 30.0 * stop_below && it - st.rb_it < span)
-    return;  // far from stopping: not yet
-  const int n = it + 1;
-  double *D0 = rb_sm, *E0 = D0 + MI, *e2 = E0 + MI;
-  for (int i = lane; i < n; i += 32) {
-    D0[i] = diagT[(ll)g * MI + i];
-    if (i < n - 1) {
-      const double ev = upperT[(ll)g * MI + i];
-      E0[i] = ev;
-      e2[i] = __dmul_rn(ev, ev);
-    }
-  }
+// y_k = 1 / |z|.  One warp; D0 / E0 the diagonals of T_k, e2 and dv scratch
+// of n values each.  Returns the bound and theta (0 when T_k has an
+// eigenvalue below 0; the bound is then 1e300) on lane 0.
+__device__ __noinline__ double ritz_bound_warp(const double *D0, const double *E0, double *e2, double *dv,
+                                  int n, double bk, double th0, double &theta_out) {
+  const int lane = threadIdx.x & 31;
+  for (int i = lane; i < n - 1; i += 32) e2[i] = __dmul_rn(E0[i], E0[i]);
   __syncwarp();
   double glo = 1e300, ghi = -1e300;
   for (int i = lane; i < n; i += 32) {
@@ -2138,7 +1896,6 @@ __global__ void k_ritz_bound(GState *__restrict__ gs, int ngroups,
   const double pad = fmax(1e-300, 2.2e-16 * fmax(fabs(glo), fabs(ghi))) * 4.0;
   glo -= pad, ghi += pad;
   // lane 0: eigenvalues below 0; lanes 1, 2: the warm bracket's ends
-  const double th0 = st.rb_theta;
   const double xq = lane == 1 ? 0.99 * th0 : th0;
   const int cq = (lane == 0 || (th0 > 0.0 && lane < 3)) ? sturm_count(D0, e2, n, lane ? xq : 0.0)
                                                           : 0;
@@ -2150,11 +1907,9 @@ __global__ void k_ritz_bound(GState *__restrict__ gs, int ngroups,
       pd ? (warm ? eig_index(D0, e2, n, 0, 0.99 * th0, th0, 1e-10)
                  : eig_index(D0, e2, n, 0, glo, ghi, 1e-10))
          : 0.0;
-  if (lane != 0) return;
   double bound = 1e300;
-  if (pd) {
+  if (pd && lane == 0) {
     // pivots of T_k - theta I, then z from the bottom (scaled to stay finite)
-    double *dv = e2 + MI;
     double d = __dsub_rn(D0[0], theta);
     dv[0] = d;
     for (int i = 1; i < n; i++) {
@@ -2175,11 +1930,50 @@ __global__ void k_ritz_bound(GState *__restrict__ gs, int ngroups,
       ss = fma(z, z, ss);
     }
     const double yk = fast_div(fabs(zl), __dsqrt_rn(ss));
-    bound = __dmul_rn(fabs(upperT[(ll)g * MI + it]), yk);
+    bound = __dmul_rn(fabs(bk), yk);
   }
+  theta_out = pd ? theta : 0.0;
+  return bound;
+}
+
+// The bound of every running group after step it (launch-per-kernel passes;
+// the team kernel calls ritz_bound_warp itself).  Writes it to
+// bound_out[g MI + it] (when given) and, when it is below stop_below, asks to
+// end the group's pass (stopreq).  It runs on a second stream beside the next
+// steps: it reads only entries of T that step it completed (each written with
+// the same value wherever it is written), whether the group ran step it, and
+// its own fields of the group state, so its answer does not depend on how far
+// the other stream has got; k_apply_stop turns the request into run = 0 at a
+// fixed step after joining the streams.  To spend little of the FP64 pipe, a
+// group whose last bound was above 30 stop_below is computed again only
+// `span` steps after it.  One warp per group; a group whose T_k has an
+// eigenvalue below 0 is left alone.
+__global__ void k_ritz_bound(GState *__restrict__ gs, int ngroups,
+                             const double *__restrict__ diagT, const double *__restrict__ upperT,
+                             int MI, int it, double stop_below, int span,
+                             double *__restrict__ bound_out) {
+  pdl_entry();
+  extern __shared__ double rb_sm[];
+  const int g = blockIdx.x, lane = threadIdx.x;
+  if (g >= ngroups) return;
+  GState &st = gs[g];
+  if (!st.active || *(volatile const int *)&st.iters < it + 1) return;  // step it not run
+  if (!bound_out && st.rb_it >= 0 && st.rb_bound > 30.0 * stop_below && it - st.rb_it < span)
+    return;  // far from stopping: not yet
+  const int n = it + 1;
+  double *D0 = rb_sm, *E0 = D0 + MI, *e2 = E0 + MI;
+  for (int i = lane; i < n; i += 32) {
+    D0[i] = diagT[(ll)g * MI + i];
+    if (i < n - 1) E0[i] = upperT[(ll)g * MI + i];
+  }
+  __syncwarp();
+  double theta;
+  const double bound =
+      ritz_bound_warp(D0, E0, e2, e2 + MI, n, upperT[(ll)g * MI + it], st.rb_theta, theta);
+  if (lane != 0) return;
   if (bound_out) bound_out[(ll)g * MI + it] = bound;
   st.rb_it = it;
-  st.rb_theta = pd ? theta : 0.0;
+  st.rb_theta = theta;
   st.rb_bound = bound;
   if (bound < stop_below) st.stopreq = 1;
 }
@@ -2194,6 +1988,923 @@ __global__ void k_apply_stop(GState *__restrict__ gs, int ngroups) {
     st.run = 0;
     st.stopreq = 0;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Team step kernel: every Lanczos step of a pass (src/fiedler.c:458-504) for
+// all groups of the level in one cooperative launch, in place of the six
+// launches per step (P update, its finalisation, SpMV, finalisation, R
+// update, finalisation).  A group belongs to a team of one or more blocks
+// (one block per SM); each block of a team owns a contiguous run of the
+// group's tiles and keeps their rows of p and w (and r when it fits) in shared
+// memory for the whole pass; only p, for the other blocks, and the Krylov row
+// go to HBM.  A team works through a list of groups; teams never wait for
+// each other.
+//
+// The block's rows of the matrix are encoded once per level (k_team_encode)
+// with 16-bit entries that index shared memory: the block's own rows, then
+// its halo (the sorted list of the other rows its entries name), whose values
+// it fetches once per step.  So an entry takes 2 bytes instead of 4 and a
+// gather is a shared-memory load: the 32 gathers of a warp touch about eight
+// cache lines, and the L1 lookups of those, not HBM, bounded the SpMV.  The
+// encoded rows stay in shared memory too when they fit, else they stream
+// from L2 a slice ahead.
+//
+// The three places of a step where a team has to agree (p complete, p.Lp,
+// |r|^2) exchange the tile partials through 16-byte slots that hold the value
+// and a tag (pass epoch, step): a block polls the slots of its group until
+// every tag has arrived, so the partials travel with the flag and no separate
+// counter is needed.  Every block then reduces them in k_fin's order and
+// applies the same scalar update.  Tile partials keep the chunk trees of
+// pr_tile / spmv_tile; the trees of several chunks are folded into one
+// (merge2: the lanes a tree no longer needs carry the next chunk), because
+// GB300's FP64 pipe takes 16 cycles per warp instruction whatever the number
+// of useful lanes.  For the same reason an FP64 product enters a sum without
+// its rounding error (s + (x y - s) rounds back to s).  Results are bitwise
+// those of the launch-per-kernel pass.
+//
+// The early pass exit's Ritz residual bound runs on an extra warp of the
+// team's first block beside the next steps; its stop request travels in the
+// tag of that block's first |r|^2 slot of the step before it takes effect.
+// Every wait gives up after about one second, sets err and returns; a block
+// that sees err set returns at its next wait, so the kernel always ends.
+//
+// Bound by the FP64 pipe with FP64 vectors (59k of 110k cycles of a step at
+// 4096 rows per block are the SpMV's DFMAs) and by instruction issue with
+// FP32 ones.  Partitions before and after, launch-per-kernel steps against
+// these: 4K hexes 9.2 -> 5.7 ms, 65K 56.7 -> 40.6, a 61K quad mesh 125 -> 79,
+// 1M in FP64 217 -> 183.
+// ---------------------------------------------------------------------------
+constexpr int TS_NW = 19;               // worker warps (plus the checker)
+constexpr int TS_THREADS = (TS_NW + 1) * 32;
+constexpr int TS_TILES = 32;            // tiles per block at most (512 rows or more each)
+constexpr int TS_SMEM = 212 * 1024;     // dynamic shared memory at most
+constexpr int TS_LOCAL = 1 << 14;       // places of p in a block (14-bit index)
+constexpr int TS_REP = 8;               // copies of the slots
+constexpr int TS_HALO = 6400;           // halo rows at most
+constexpr ll TS_GROUP = 1280 * 1024;    // rows of a group at most (the encoder's bitmap)
+template <typename VT>
+__host__ __device__ constexpr int ts_cap() {  // own rows at most
+  return sizeof(VT) == 8 ? 8192 : 11264;
+}
+// Place of own row i in the shared p: every 32 rows are followed by a gap of
+// one vector, so that rows a multiple of 32 apart (the other side of a block
+// of a spatial order) lie in different banks.
+template <typename VT>
+__host__ __device__ constexpr int ts_place(int i) {
+  return i + (i >> 5) * (sizeof(VT) == 8 ? 2 : 4);
+}
+constexpr unsigned TS_STOP = 1u << 31;
+
+// A double in two 8-byte words, 32 bits of it and the tag in each: a word is
+// read whole or not at all, so the value is complete when both tags match.
+struct __align__(16) TeamSlot {
+  unsigned long long lo, hi;
+};
+
+struct TeamArgs {
+  const ll *tbeg, *tend;
+  GState *gs;
+  void *pbuf[2], *V;
+  ll VS;
+  const ll *slice_off;
+  const int *slice_w;
+  const int4 *blk;    // per block: first entry of its group list, entries, rank, team size
+  const int *item0;   // per block: its first item (an item: a block's rows of one group)
+  const int *glist;
+  const unsigned *enc;  // encoded rows, halo lists (TS_HALO each) and their lengths, per item
+  const int *halo, *nhalo;
+  int max_w;
+  TeamSlot *slot;     // the P, SpMV and R tile partials: 3 x TS_REP x T
+  const unsigned long long *epoch;
+  double *diagT, *upperT, *vnorm;
+  int *err;           // 2: a wait gave up
+  int T, MI;
+  int rows_cap;       // own rows of shared memory per vector
+  int halo_cap;       // halo rows
+  int enc_cap;        // words of shared memory for the encoded rows (0: they stream)
+  int r_in;           // r in shared memory too
+  // early pass exit (stop_below <= 0: off)
+  double stop_below;
+  int e_min, e_stride, e_delay, e_span;
+};
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__global__ void k_team_epoch(unsigned long long *__restrict__ epoch) {
+  pdl_entry();
+  epoch[0] += 1ull;
+}
+__device__ __forceinline__ void slot_put(TeamSlot *s, double v, unsigned tag, bool rel) {
+  const unsigned long long t = (unsigned long long)tag << 32;
+  const unsigned long long lo = t | (unsigned)__double2loint(v),
+                           hi = t | (unsigned)__double2hiint(v);
+  if (rel) __threadfence();  // (the block's earlier writes, ordered by its barrier)
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(s), "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void slot_get(const TeamSlot *s, unsigned long long &lo,
+                                         unsigned long long &hi) {
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(s)
+               : "memory");
+}
+__device__ __forceinline__ bool slot_has(unsigned long long lo, unsigned long long hi,
+                                         unsigned tag) {
+  return ((unsigned)(lo >> 32) & ~TS_STOP) == tag && ((unsigned)(hi >> 32) & ~TS_STOP) == tag;
+}
+template <int ID>
+__device__ __forceinline__ void bar_n(int n) {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(n) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void bar_arrive_n(int n) {
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(n) : "memory");
+}
+
+// One chunk's partial sum per lane: FP64 value, or compensated FP32 pair.
+template <typename VT>
+struct Fold;
+template <>
+struct Fold<double> {
+  using T = double;
+  __device__ static __forceinline__ T zero() { return 0.0; }
+  __device__ static __forceinline__ void acc(T &a, double x) { a = __dadd_rn(a, x); }
+  __device__ static __forceinline__ void first(T &a, double x) { a = x; }
+  // x y: the error of the product would be rounded away again
+  __device__ static __forceinline__ void acc_prod(T &a, double x, double y) {
+    a = __dadd_rn(a, __dmul_rn(x, y));
+  }
+  __device__ static __forceinline__ void first_prod(T &a, double x, double y) {
+    a = __dmul_rn(x, y);
+  }
+  __device__ static __forceinline__ T join(T a, T b) { return __dadd_rn(a, b); }
+  __device__ static __forceinline__ T shfl_down(T a, int o) {
+    return __shfl_down_sync(0xffffffffu, a, o);
+  }
+  __device__ static __forceinline__ T shfl_xor(T a, int o) {
+    return __shfl_xor_sync(0xffffffffu, a, o);
+  }
+  __device__ static __forceinline__ double value(T a) { return a; }
+};
+template <>
+struct Fold<float> {
+  using T = float2;
+  __device__ static __forceinline__ T zero() { return make_float2(0.f, 0.f); }
+  __device__ static __forceinline__ void acc(T &a, float x) { two_sum_pair(a.x, a.y, x, 0.f); }
+  __device__ static __forceinline__ void first(T &a, float x) { a = make_float2(x, 0.f); }
+  __device__ static __forceinline__ void acc_prod(T &a, float x, float y) {
+    const float s = x * y;
+    two_sum_pair(a.x, a.y, s, (float)fma(x, y, -s));
+  }
+  __device__ static __forceinline__ void first_prod(T &a, float x, float y) {
+    const float s = x * y;
+    a = make_float2(s, (float)fma(x, y, -s));
+  }
+  __device__ static __forceinline__ T join(T a, T b) {
+    two_sum_pair(a.x, a.y, b.x, b.y);
+    return a;
+  }
+  __device__ static __forceinline__ T shfl_down(T a, int o) {
+    return make_float2(__shfl_down_sync(0xffffffffu, a.x, o), __shfl_down_sync(0xffffffffu, a.y, o));
+  }
+  __device__ static __forceinline__ T shfl_xor(T a, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+  }
+  __device__ static __forceinline__ double value(T a) { return (double)a.x + (double)a.y; }
+};
+
+// Two trees in one: the lanes without bit `off` take a's next sums, the
+// others b's (TwoSum and + give the same bits for either order).
+template <typename VT>
+__device__ __forceinline__ typename Fold<VT>::T merge2(typename Fold<VT>::T a,
+                                                       typename Fold<VT>::T b, int off) {
+  using F = Fold<VT>;
+  const bool up = (threadIdx.x & off) != 0;
+  const typename F::T keep = up ? b : a, send = up ? a : b;
+  return F::join(keep, F::shfl_xor(send, off));
+}
+// M chunk trees (offsets 16 .. 1); chunk m's sum ends on lane fold_lane(m)
+template <typename VT, int M>
+__device__ __forceinline__ typename Fold<VT>::T fold_chunks(const typename Fold<VT>::T *v) {
+  using F = Fold<VT>;
+  typename F::T t;
+  if (M == 2) {
+    t = merge2<VT>(v[0], v[1 % M], 16);
+    t = F::join(t, F::shfl_down(t, 8));
+  } else {  // 4
+    t = merge2<VT>(merge2<VT>(v[0], v[1 % M], 16), merge2<VT>(v[2 % M], v[3 % M], 16), 8);
+  }
+  t = F::join(t, F::shfl_down(t, 4));
+  t = F::join(t, F::shfl_down(t, 2));
+  return F::join(t, F::shfl_down(t, 1));
+}
+// one tree of n values (zero on the other lanes: their levels are skipped)
+template <typename VT>
+__device__ __forceinline__ typename Fold<VT>::T fold_one(typename Fold<VT>::T t, int n) {
+  using F = Fold<VT>;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < n) t = F::join(t, F::shfl_down(t, o));  // warp-uniform
+  return t;
+}
+__device__ __forceinline__ int fold_lane(int m) { return ((m & 1) << 4) | ((m >> 1) << 3); }
+
+// The group's sum of its tile partials by one warp, in k_fin's order: x[u]
+// sums the tiles of k_fin's thread 32 u + l (strided by 256), a tree per 32
+// threads, then the eight in order (the trees of unused threads are zero).
+// The partials come from the block's own table (solo) or from the slots,
+// polled until they carry `tag`.  Returns the sum on every lane; flags: 1 a
+// tag carried the stop request, 2 a wait gave up.
+__device__ __noinline__ double team_sum(const double *own, const TeamSlot *slot, int nt,
+                                        unsigned tag, bool acq, int *err, int *flags) {
+  const int lane = threadIdx.x & 31;
+  int fl = 0;
+  double x[8];
+#pragma unroll
+  for (int u = 0; u < 8; u++) x[u] = 0.0;
+  if (own) {
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (lane + 32 * u < nt) x[u] = own[lane + 32 * u];
+  } else {
+    for (int base = 0; base < nt; base += 256) {
+      unsigned long long lo[8], hi[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        lo[u] = hi[u] = (unsigned long long)(base + lane + 32 * u < nt ? ~tag : tag) << 32;
+      // every round asks for all the slots still missing at once (a round
+      // takes one L2 latency, whatever their number)
+      unsigned long long t0 = 0;
+      for (unsigned n = 1;; n++) {
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (!slot_has(lo[u], hi[u], tag)) slot_get(slot + base + lane + 32 * u, lo[u], hi[u]);
+        bool missing = false;
+#pragma unroll
+        for (int u = 0; u < 8; u++) missing = missing || !slot_has(lo[u], hi[u], tag);
+        if (!__any_sync(0xffffffffu, missing)) break;
+        if ((n & 255) == 0) {  // warp-uniform
+          const unsigned long long t1 = global_ns();
+          if (t0 == 0) t0 = t1;
+          if (t1 - t0 > 1000000000ull || n > (1u << 26)) {
+            if (missing) atomicExch(err, 2);
+            fl |= 2;
+          }
+          if (*(volatile int *)err) fl |= 2;
+          if (__any_sync(0xffffffffu, fl & 2)) break;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        if (lo[u] >> 63) fl |= slot_has(lo[u], hi[u], tag) ? 1 : 0;
+        const double v = __hiloint2double((int)(unsigned)hi[u], (int)(unsigned)lo[u]);
+        if (base + lane + 32 * u < nt) x[u] = base ? __dadd_rn(x[u], v) : v;
+      }
+    }
+    if (acq) __threadfence();  // what the others wrote before is visible from here on
+  }
+  *flags = __reduce_or_sync(0xffffffffu, fl);
+  double tot;
+  if (nt <= 32) {
+    tot = fold_one<double>(x[0], nt);
+  } else if (nt <= 64) {
+    const double t = fold_chunks<double, 2>(x);
+    tot = __dadd_rn(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 16));
+  } else {
+    const double t = fold_chunks<double, 4>(x);
+    tot = __shfl_sync(0xffffffffu, t, 0);
+#pragma unroll
+    for (int u = 1; u < 4; u++) tot = __dadd_rn(tot, __shfl_sync(0xffffffffu, t, fold_lane(u)));
+    if (nt > 128) {
+      const double t2 = fold_chunks<double, 4>(x + 4);
+#pragma unroll
+      for (int u = 0; u < 4; u++) tot = __dadd_rn(tot, __shfl_sync(0xffffffffu, t2, fold_lane(u)));
+    }
+  }
+  return __shfl_sync(0xffffffffu, tot, 0);
+}
+
+// The partials of the block's tiles from their chunk sums (nc chunks per tile,
+// nf in all), a warp per tile, into the own table (solo) or the slots.
+template <typename VT>
+__device__ __forceinline__ void team_publish(bool solo, double *own, TeamSlot *slot, int T,
+                                             const typename Fold<VT>::T *cs, int nc, int nf,
+                                             int tn, unsigned tag, bool rel) {
+  using F = Fold<VT>;
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < tn; t += TS_NW) {
+    const int n = min(nc, nf - t * nc);
+    typename F::T s = lane < n ? cs[t * nc + lane] : F::zero();
+    for (int q = lane + 32; q < n; q += 32) s = F::join(s, cs[t * nc + q]);
+    s = fold_one<VT>(s, n);
+    if (solo) {
+      if (lane == 0) own[t] = F::value(s);
+    } else {  // a lane per copy
+      const double v = __shfl_sync(0xffffffffu, F::value(s), 0);
+      if (lane < TS_REP) slot_put(slot + (ll)lane * T + t, v, tag, rel);
+    }
+  }
+}
+
+// small non-negative integer (< 2^20) as a double, by integer instructions
+__device__ __forceinline__ double small_u2d(unsigned d) {
+  const int e = 31 - __clz((int)d);
+  const unsigned hi = d ? ((unsigned)(1023 + e) << 20) | ((d << (20 - e)) & 0xFFFFFu) : 0u;
+  return __hiloint2double((int)hi, 0);
+}
+
+// Where the encoded rows of a block start that owns the slices from sl on
+// (first ELL word `word`) and the tiles from `tile` on.  Two entries a word:
+// a slice of width w takes (w + 1) / 2 rows of 32 words, slice q of the block
+// starting at half its ELL offset plus 32 q.  A slice that two blocks share
+// is encoded by both, so every tile leaves room for one widest slice more.
+__device__ __forceinline__ ll enc_base(ll word, ll sl, int tile, int max_w) {
+  return word + 32 * sl + (ll)tile * (max_w + 1) * 32;
+}
+
+// One block per item: the halo list and the encoded rows.  The halo is marked
+// in a bitmap over the group's rows, so that it comes out sorted (neighbouring
+// halo rows are fetched together) and a row's place in it is a prefix count.
+// A word holds two entries: places in the shared p (ts_place(own row - B0), or
+// p_cap + place in the halo) in bits 0-13 and 18-31, weight codes in bits
+// 14-15 and 16-17 (0, 1, 2, 3 for the weights 0, 1, 2, 4).  bad:
+// another weight, or a halo of more than halo_cap rows (the level then keeps
+// the launch-per-kernel steps).
+constexpr int TE_THREADS = 1024;
+template <typename VT>
+__global__ void __launch_bounds__(TE_THREADS)
+k_team_encode(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
+              const GState *__restrict__ gs, const unsigned *__restrict__ ell,
+              const ll *__restrict__ slice_off, const int *__restrict__ slice_w,
+              const int4 *__restrict__ blk, const int *__restrict__ item0,
+              const int *__restrict__ glist, const int2 *__restrict__ items, int p_cap,
+              int halo_cap, int max_w, unsigned *__restrict__ enc, int *__restrict__ halo,
+              int *__restrict__ nhalo, int *__restrict__ bad) {
+  constexpr int CH = 32 * VecOf<VT>::R;
+  extern __shared__ __align__(16) unsigned te_smem[];
+  __shared__ int wsum[32];
+  const int item = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int2 who = items[item];  // block, entry of its list
+  const int4 me = blk[who.x];
+  const GState &st = gs[glist[me.x + who.y]];
+  const int nt = st.ntiles, rank = me.z, size = me.w;
+  const int ta = (int)((ll)nt * rank / size), tz = (int)((ll)nt * (rank + 1) / size);
+  const ll b0 = tbeg[st.tile0 + ta], e1 = tend[st.tile0 + tz - 1], B0 = b0 / CH * CH;
+  const ll g0 = st.start;
+  const int nword = size > 1 ? (int)((st.n + 31) >> 5) : 0, nblk = (nword + 3) >> 2;
+  unsigned *bits = te_smem;
+  unsigned short *pre = reinterpret_cast<unsigned short *>(bits + ((nword + 3) & ~3));
+  for (int k = threadIdx.x; k < ((nword + 3) & ~3); k += TE_THREADS) bits[k] = 0u;
+  __syncthreads();
+  const ll sl0 = b0 >> 5;
+  const int ns = (int)(((e1 - 1) >> 5) - sl0) + 1;
+  if (size > 1) {
+    for (int q = warp; q < ns; q += TE_THREADS / 32) {
+      const ll i = (sl0 + q) * 32 + lane;
+      const unsigned *ep = ell + slice_off[sl0 + q] + lane;
+      const int wd = (i >= b0 && i < e1) ? slice_w[sl0 + q] : 0;
+      for (int k = 0; k < wd; k++) {
+        const int j = (int)(ep[(ll)k * 32] & 0x0FFFFFFFu);
+        if (j < b0 || j >= e1) atomicOr(&bits[(j - g0) >> 5], 1u << ((j - g0) & 31));
+      }
+    }
+    __syncthreads();
+    // prefix counts per four words: a run of blocks per thread
+    const int per = (nblk + TE_THREADS - 1) / TE_THREADS, q0 = threadIdx.x * per;
+    auto count4 = [&](int q) {
+      return __popc(bits[4 * q]) + __popc(bits[4 * q + 1]) + __popc(bits[4 * q + 2]) +
+             __popc(bits[4 * q + 3]);
+    };
+    int c = 0;
+    for (int q = q0; q < min(q0 + per, nblk); q++) c += count4(q);
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < TE_THREADS / 32; w++) {
+      if (w < warp) before += wsum[w];
+      total += wsum[w];
+    }
+    if (total > halo_cap) {  // block-uniform
+      if (threadIdx.x == 0) atomicOr(bad, 1);
+      return;
+    }
+    if (threadIdx.x == 0) nhalo[item] = total;
+    int run = before + inc - c;
+    int *out = halo + (ll)item * TS_HALO;
+    for (int q = q0; q < min(q0 + per, nblk); q++) {
+      pre[q] = (unsigned short)run;
+      for (int w = 4 * q; w < 4 * q + 4; w++)
+        for (unsigned m = bits[w]; m; m &= m - 1)
+          out[run++] = (int)(g0 + (ll)w * 32 + __ffs(m) - 1);
+    }
+    __syncthreads();
+  }
+  unsigned *eo = enc + enc_base(slice_off[sl0], sl0, st.tile0 + ta, max_w);
+  int mine = 0;
+  for (int q = warp; q < ns; q += TE_THREADS / 32) {
+    const ll i = (sl0 + q) * 32 + lane;
+    const ll so = slice_off[sl0 + q];
+    const unsigned *ep = ell + so + lane;
+    const int wd = slice_w[sl0 + q];
+    const bool valid = i >= b0 && i < e1;
+    const unsigned self = valid ? (unsigned)ts_place<VT>((int)(i - B0)) : 0u;  // weight 0
+    // (slices start at half their ELL word, rounded up per slice)
+    unsigned *op = eo + ((so - slice_off[sl0]) >> 1) + 32 * q + lane;
+    for (int k = 0; k < wd; k += 2) {
+      unsigned w2 = 0;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        unsigned loc = self, code = 0;
+        if (valid && k + h < wd) {
+          const unsigned x = ep[(ll)(k + h) * 32];
+          const unsigned wt = x >> 28;
+          const int j = (int)(x & 0x0FFFFFFFu);
+          if (wt != 0) {
+            code = wt == 4u ? 3u : wt;
+            if (wt > 4u || wt == 3u) mine = 1;
+            if (j >= b0 && j < e1) {
+              loc = (unsigned)ts_place<VT>((int)(j - B0));
+            } else {
+              const int r = (int)(j - g0), w = r >> 5;
+              int before = pre[w >> 2];
+              for (int z = w & ~3; z < w; z++) before += __popc(bits[z]);
+              loc = (unsigned)(p_cap + before + __popc(bits[w] & ((1u << (r & 31)) - 1u)));
+            }
+          }
+        }
+        w2 |= h ? (code << 16) | (loc << 18) : loc | (code << 14);
+      }
+      op[(k >> 1) * 32] = w2;
+    }
+  }
+  if (__any_sync(0xffffffffu, mine) && lane == 0) atomicOr(bad, 1);
+}
+
+// Two entries of a row: y += w p_j (FP64, and the weights summed) or
+// y += w (p_i - p_j) (FP32: a weight-0 entry names the row itself, so its
+// difference is 0 whatever its weight), in spmv_tile's operations.
+template <typename VT>
+struct RowSum {
+  VT s = (VT)0;
+  unsigned d = 0;
+  __device__ __forceinline__ void add(unsigned c, VT pi, VT pj) {
+    if (sizeof(VT) == 4) {
+      s = (VT)fmaf(__int_as_float((int)(c * 0x00800000u + 0x3F000000u)), (float)pi - (float)pj,
+                   (float)s);
+    } else {
+      s = (VT)fma(__hiloint2double(c ? (int)((1022u + c) << 20) : 0, 0), (double)pj, (double)s);
+      d += (1u << c) >> 1;
+    }
+  }
+  __device__ __forceinline__ VT done(VT pi) const {
+    if (sizeof(VT) == 4) return s;
+    return (VT)fma(small_u2d(d), (double)pi, -(double)s);
+  }
+};
+// NWORD words (two entries each) of a row, the gathers first
+template <typename VT, int NWORD>
+__device__ __forceinline__ void row_words(RowSum<VT> &r, const unsigned *w, VT pi, const VT *sp) {
+  VT a[NWORD], b[NWORD];
+#pragma unroll
+  for (int u = 0; u < NWORD; u++) {
+    a[u] = sp[w[u] & 0x3FFFu];
+    b[u] = sp[w[u] >> 18];
+  }
+#pragma unroll
+  for (int u = 0; u < NWORD; u++) {
+    r.add((w[u] >> 14) & 3u, pi, a[u]);
+    r.add((w[u] >> 16) & 3u, pi, b[u]);
+  }
+}
+
+template <typename VT>
+__global__ void __launch_bounds__(TS_THREADS, 1) k_team_steps(TeamArgs a) {
+  constexpr int NW = TS_NW, WT = NW * 32;
+  using Vec = VecOf<VT>;
+  using VV = typename Vec::T;
+  constexpr int R = Vec::R, CH = 32 * R;
+  constexpr int MAXS = ts_cap<VT>() / 32 + TS_TILES + 2;
+  using F = Fold<VT>;
+  using FT = typename F::T;
+  extern __shared__ __align__(16) unsigned char ts_smem[];
+  __shared__ GState st;
+  __shared__ FT cs[MAXS];                   // chunk sums
+  __shared__ int soff[MAXS + 1];            // the block's encoded slices: first word
+  // chunk f of 32 rows: its index / 32, first and last valid lane (6 bits each)
+  __shared__ int desc[MAXS];
+  __shared__ double own[TS_TILES];          // solo: the tile partials
+  __shared__ double cdiag[MAX_MITER], cup[MAX_MITER], cwork[2 * MAX_MITER];
+  __shared__ double s_old[3];               // values the table needs after FIN_PAP's update
+  __shared__ double s_tot;
+  __shared__ int s_fail, s_cmd[2], s_reply, s_run, s_done, s_stopnow;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int4 me = a.blk[blockIdx.x];
+  if (me.y <= 0) return;
+  const int rank = me.z, size = me.w;
+  const bool solo = size == 1, lead = rank == 0;
+  const bool early = a.stop_below > 0.0 && lead;
+  if (warp == NW) {  // the checker: Ritz residual bounds of the team's running group
+    if (!early) return;
+    int rb_it = -1, turn = 0;
+    double rb_theta = 0.0, rb_bound = 1e300;
+    for (;;) {
+      bar_n<2>(64);
+      const int cmd = s_cmd[turn];
+      turn ^= 1;
+      if (cmd == 0) return;
+      if (cmd == 1) {  // a new group
+        rb_it = -1, rb_theta = 0.0, rb_bound = 1e300;
+        continue;
+      }
+      const int it = cmd - 2;
+      int ask = 0;
+      if (!(rb_it >= 0 && rb_bound > 30.0 * a.stop_below && it - rb_it < a.e_span)) {
+        double theta;
+        const double b = ritz_bound_warp(cdiag, cup, cwork, cwork + MAX_MITER, it + 1, cup[it],
+                                         rb_theta, theta);
+        rb_bound = __shfl_sync(0xffffffffu, b, 0);
+        rb_it = it, rb_theta = theta;
+        ask = rb_bound < a.stop_below;
+      }
+      if (lane == 0) s_reply = ask;
+      __syncwarp();
+      bar_arrive_n<3>(64);
+    }
+  }
+  VT *sp = reinterpret_cast<VT *>(ts_smem);  // own rows of p (ts_place), then the halo
+  const int p_cap = ts_place<VT>(a.rows_cap);
+  VT *sw = sp + p_cap + a.halo_cap, *sr = sw + a.rows_cap;
+  int *shl = reinterpret_cast<int *>(sr + (a.r_in ? a.rows_cap : 0));
+  unsigned *senc = reinterpret_cast<unsigned *>(shl + a.halo_cap);
+  VT *V = static_cast<VT *>(a.V);
+  int turn = 0;  // command slot (the last worker warp sends the commands)
+  auto command = [&](int c) {
+    if (lane == 0) s_cmd[turn] = c;
+    turn ^= 1;
+    __syncwarp();
+    bar_n<2>(64);
+  };
+  const unsigned epoch = (unsigned)(a.epoch[0] & 0x7FFFFFull) << 8;
+  for (int gi = 0; gi < me.y; gi++) {
+    const int g = a.glist[me.x + gi];
+    bar_n<1>(WT);  // the previous group is done with the shared state
+    if (threadIdx.x == 0) {
+      st = a.gs[g];
+      s_fail = 0;
+    }
+    bar_n<1>(WT);
+    if (!st.run) continue;
+    const int nt = st.ntiles, tile0 = st.tile0;
+    const int ta = (int)((ll)nt * rank / size), tn = (int)((ll)nt * (rank + 1) / size) - ta;
+    const ll b0 = a.tbeg[tile0 + ta], e1 = a.tend[tile0 + ta + tn - 1];
+    const ll B0 = b0 / CH * CH;  // row of index 0 of the shared vectors
+    // own tiles: t covers the indices [lb + t tr, min(lb + (t + 1) tr, le))
+    const int lb = (int)(b0 - B0), le = (int)(e1 - B0);
+    const int tr = tn > 1 ? (int)(a.tbeg[tile0 + ta + 1] - b0) : le - lb;
+    // chunks per tile and in all (a tile starts anywhere inside its first chunk)
+    const int ncv = (lb % CH + tr + CH - 1) / CH, nc32 = (lb % 32 + tr + 31) / 32;
+    const int ll0 = lb + (tn - 1) * tr;
+    const int nfv = (tn - 1) * ncv + (ll0 % CH + (le - ll0) + CH - 1) / CH;
+    const int nf32 = (tn - 1) * nc32 + (ll0 % 32 + (le - ll0) + 31) / 32;
+    // chunk f lies in tile f / nc (exact: f < 2^10, nc < 2^9)
+    const unsigned mgv = (1u << 20) / (unsigned)ncv + 1;
+    // each block polls one of TS_REP copies of the slots: every block of a
+    // team reads all of them, and one copy is a hot spot in L2 (125 blocks and
+    // tiles: 2.5 us per exchange; 128 blocks, 512 tiles: 5.5 us)
+    TeamSlot *const pub = a.slot + tile0 + ta;
+    const ll srow = (ll)TS_REP * a.T;
+    const TeamSlot *slotP = a.slot + (ll)(rank & (TS_REP - 1)) * a.T + tile0, *slotS = slotP + srow,
+                   *slotR = slotS + srow;
+    // the block's slices of the matrix, its halo, and r_0
+    const ll sl0 = b0 >> 5;
+    const int ns = (int)(((e1 - 1) >> 5) - sl0) + 1;
+    const ll eo = a.slice_off[sl0];
+    const int item = a.item0[blockIdx.x] + gi;
+    const unsigned *enc = a.enc + enc_base(eo, sl0, tile0 + ta, a.max_w);
+    for (int k = threadIdx.x; k < ns; k += WT)
+      soff[k] = (int)((a.slice_off[sl0 + k] - eo) >> 1) + 32 * k;
+    if (threadIdx.x == 0)
+      soff[ns] = (int)((a.slice_off[sl0 + ns - 1] - eo) >> 1) + 32 * (ns - 1) +
+                 a.slice_w[sl0 + ns - 1] * 16 + 32;
+    for (int f = threadIdx.x; f < nf32; f += WT) {
+      const int t = f / nc32, tb = lb + t * tr, te = min(tb + tr, le);
+      const int sl = (tb >> 5) + (f - t * nc32);
+      desc[f] = sl << 12 | max(tb - sl * 32, 0) << 6 | min(te - sl * 32, 32);
+    }
+    const int nh = solo ? 0 : a.nhalo[item];
+    for (int k = threadIdx.x; k < nh; k += WT) shl[k] = a.halo[(ll)item * TS_HALO + k];
+    if (a.r_in)
+      for (int i = lb + threadIdx.x; i < le; i += WT) sr[i] = V[B0 + i];
+    if (early && warp == NW - 1) command(1);
+    bar_n<1>(WT);
+    if (a.enc_cap)
+      for (int k = threadIdx.x; k < soff[ns]; k += WT) senc[k] = enc[k];
+    bar_n<1>(WT);
+    int pending = -1;  // step of the bound check under way
+    for (int it = 0;; it++) {
+      const unsigned tag = epoch | (unsigned)(it + 1);
+      VT *pg = static_cast<VT *>(a.pbuf[it & 1]) + B0;
+      const VT *rp = a.r_in ? sr : V + (ll)it * a.VS + B0;
+      const double *mine = solo ? own : nullptr;
+      int flags = 0;
+      // ---- p = r (step 0) or beta (p - c) + r; sum p
+      {
+        const VT c = (VT)st.c, beta = (VT)st.beta;
+        for (int f0 = 2 * warp; f0 < nfv; f0 += 2 * NW) {
+          FT acc[2];
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            const int f = f0 + m, t = (int)((unsigned)f * mgv >> 20);
+            acc[m] = F::zero();
+            if (f >= nfv) continue;  // warp-uniform
+            const int tb = lb + t * tr, te = min(tb + tr, le);
+            const int i0 = (tb / CH + (f - t * ncv)) * CH + lane * R;
+            if (i0 >= tb && i0 + R <= te) {
+              VT x[R], y[R], o[R];
+              Vec::get(*reinterpret_cast<const VV *>(rp + i0), x);
+              if (it > 0) Vec::get(*reinterpret_cast<const VV *>(sp + ts_place<VT>(i0)), y);
+#pragma unroll
+              for (int k = 0; k < R; k++) o[k] = it == 0 ? x[k] : (VT)fma(beta, y[k] - c, x[k]);
+              *reinterpret_cast<VV *>(sp + ts_place<VT>(i0)) = Vec::make(o);
+              if (!solo) *reinterpret_cast<VV *>(pg + i0) = Vec::make(o);
+              F::first(acc[m], o[0]);
+#pragma unroll
+              for (int k = 1; k < R; k++) F::acc(acc[m], o[k]);
+            } else {
+#pragma unroll
+              for (int k = 0; k < R; k++)
+                if (i0 + k >= tb && i0 + k < te) {
+                  const VT xv = rp[i0 + k];
+                  VT &pv = sp[ts_place<VT>(i0 + k)];
+                  const VT ov = it == 0 ? xv : (VT)fma(beta, pv - c, xv);
+                  pv = ov;
+                  if (!solo) pg[i0 + k] = ov;
+                  F::acc(acc[m], ov);
+                }
+            }
+          }
+          const FT t = fold_chunks<VT, 2>(acc);
+          if (lane == 0) cs[f0] = t;
+          if (lane == 16 && f0 + 1 < nfv) cs[f0 + 1] = t;
+        }
+      }
+      bar_n<1>(WT);
+      team_publish<VT>(solo, own, pub, a.T, cs, ncv, nfv, tn, tag, true);
+      if (solo) bar_n<1>(WT);
+      double tot = 0.0;
+      if (warp == 0) {
+        tot = team_sum(mine, slotP, nt, tag, true, a.err, &flags);
+        if (lane == 0) {
+          if (flags & 2) s_fail = 1;
+          s_tot = tot;
+        }
+      }
+      bar_n<1>(WT);  // every block's p is visible
+      if (s_fail) break;
+      // (the mean of p is first needed after the products)
+      if (warp == NW - 1 && lane == 0) st.c = __ddiv_rn(s_tot, (double)st.n);
+      if (nh > 0) {
+        for (int k = threadIdx.x; k < nh; k += WT) sp[p_cap + k] = (pg - B0)[shl[k]];
+        bar_n<1>(WT);
+      }
+      // ---- w = L p
+      const int sl_b = lb >> 5;
+      auto where = [&](int f, int &i, bool &valid, int &so, int &nw) {
+        const int d = desc[f], sl = d >> 12;
+        i = sl * 32 + lane;
+        valid = lane >= ((d >> 6) & 63) && lane < (d & 63);
+        so = soff[sl - sl_b];
+        nw = (((soff[sl - sl_b + 1] - so) >> 4) - 1) >> 1;  // (w + 1) / 2
+      };
+      if (a.enc_cap) {
+        for (int f = warp; f < nf32; f += NW) {
+          int i, so, nw;
+          bool valid;
+          where(f, i, valid, so, nw);
+          const unsigned *ep = senc + so + lane;
+          const VT pi = valid ? sp[ts_place<VT>(i)] : (VT)0;
+          RowSum<VT> r;
+          int k = 0;
+#pragma unroll 1
+          for (; k + 4 <= nw; k += 4) {
+            unsigned w4[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) w4[u] = ep[(k + u) * 32];
+            row_words<VT, 4>(r, w4, pi, sp);
+          }
+#pragma unroll 1
+          for (; k < nw; k++) {
+            const unsigned w1 = ep[k * 32];
+            row_words<VT, 1>(r, &w1, pi, sp);
+          }
+          if (valid) sw[i] = r.done(pi);
+        }
+      } else {
+        // the words of a slice (16 of them ahead) are loaded while the
+        // previous slice is multiplied
+        unsigned nx[16];
+        const int nwc = (a.max_w + 1) / 2;
+        auto fetch = [&](int f) {
+          int i, so, nw;
+          bool valid;
+          where(f, i, valid, so, nw);
+          const unsigned *ep = enc + so + lane;
+          // (a slice narrower than the level's widest: what follows it too)
+          if (nwc <= 4) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) nx[u] = __ldcs(ep + u * 32);
+          } else if (nwc <= 8) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) nx[u] = __ldcs(ep + u * 32);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 16; u++) nx[u] = __ldcs(ep + u * 32);
+          }
+        };
+        if (warp < nf32) fetch(warp);
+        for (int f = warp; f < nf32; f += NW) {
+          int i, so, nw;
+          bool valid;
+          where(f, i, valid, so, nw);
+          unsigned w[16];
+#pragma unroll
+          for (int u = 0; u < 16; u++) w[u] = nx[u];
+          if (f + NW < nf32) fetch(f + NW);
+          const VT pi = valid ? sp[ts_place<VT>(i)] : (VT)0;
+          RowSum<VT> r;
+#pragma unroll
+          for (int u = 0; u < 16; u += 4) {
+            if (u + 4 <= nw) {
+              row_words<VT, 4>(r, w + u, pi, sp);
+            } else {
+              if (u < nw) row_words<VT, 1>(r, w + u, pi, sp);
+              if (u + 1 < nw) row_words<VT, 1>(r, w + u + 1, pi, sp);
+              if (u + 2 < nw) row_words<VT, 1>(r, w + u + 2, pi, sp);
+            }
+          }
+#pragma unroll 1
+          for (int k = 16; k < nw; k++) {  // rows of more than 32 entries
+            const unsigned w1 = __ldcs(enc + so + lane + k * 32);
+            row_words<VT, 1>(r, &w1, pi, sp);
+          }
+          if (valid) sw[i] = r.done(pi);
+        }
+      }
+      bar_n<1>(WT);
+      // ---- sum w (p - c)
+      {
+        const VT c = (VT)st.c;
+        for (int f0 = 4 * warp; f0 < nf32; f0 += 4 * NW) {
+          FT acc[4];
+#pragma unroll
+          for (int m = 0; m < 4; m++) {
+            const int f = f0 + m;
+            acc[m] = F::zero();
+            if (f >= nf32) continue;
+            const int d = desc[f], i = (d >> 12) * 32 + lane;
+            if (lane >= ((d >> 6) & 63) && lane < (d & 63)) F::first_prod(acc[m], sw[i], sp[ts_place<VT>(i)] - c);
+          }
+          const FT t = fold_chunks<VT, 4>(acc);
+          if ((lane & 7) == 0) {
+            const int m = (lane >> 4) | ((lane >> 2) & 2);
+            if (f0 + m < nf32) cs[f0 + m] = t;
+          }
+        }
+      }
+      bar_n<1>(WT);
+      team_publish<VT>(solo, own, pub + srow, a.T, cs, nc32, nf32, tn, tag, false);
+      if (solo) bar_n<1>(WT);
+      if (warp == 0) {
+        const double pap =
+            team_sum(mine, slotS, nt, tag, false, a.err, &flags);
+        if (lane == 0) {
+          s_old[0] = st.pap, s_old[1] = st.rtz1, s_old[2] = st.beta;
+          st.pap = pap;
+          st.alpha = __ddiv_rn(st.rtz1, pap);
+          if (flags & 2) s_fail = 1;
+        }
+      }
+      bar_n<1>(WT);
+      if (s_fail) break;
+      // ---- r = r - alpha w, a row of V too; sum r^2.  The first block's last
+      // worker warp enters the step's diagonal of T beside it.
+      if (lead && warp == NW - 1 && lane == 0) {
+        const double d =
+            it == 0 ? __ddiv_rn(st.pap, s_old[1])
+                    : __ddiv_rn(__dadd_rn(__dmul_rn(__dmul_rn(s_old[2], s_old[2]), s_old[0]), st.pap),
+                                s_old[1]);
+        a.diagT[(ll)g * a.MI + it] = d;
+        cdiag[it] = d;
+      }
+      {
+        const VT alpha = (VT)st.alpha;
+        VT *vn = V + (ll)(it + 1) * a.VS + B0;
+        for (int f0 = 2 * warp; f0 < nfv; f0 += 2 * NW) {
+          FT acc[2];
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            const int f = f0 + m, t = (int)((unsigned)f * mgv >> 20);
+            acc[m] = F::zero();
+            if (f >= nfv) continue;
+            const int tb = lb + t * tr, te = min(tb + tr, le);
+            const int i0 = (tb / CH + (f - t * ncv)) * CH + lane * R;
+            if (i0 >= tb && i0 + R <= te) {
+              VT x[R], y[R], o[R];
+              Vec::get(*reinterpret_cast<const VV *>(rp + i0), x);
+              Vec::get(*reinterpret_cast<const VV *>(sw + i0), y);
+#pragma unroll
+              for (int k = 0; k < R; k++) o[k] = (VT)fma(-alpha, y[k], x[k]);
+              if (a.r_in) *reinterpret_cast<VV *>(sr + i0) = Vec::make(o);
+              *reinterpret_cast<VV *>(vn + i0) = Vec::make(o);
+              F::first_prod(acc[m], o[0], o[0]);
+#pragma unroll
+              for (int k = 1; k < R; k++) F::acc_prod(acc[m], o[k], o[k]);
+            } else {
+#pragma unroll
+              for (int k = 0; k < R; k++)
+                if (i0 + k >= tb && i0 + k < te) {
+                  const VT ov = (VT)fma(-alpha, sw[i0 + k], rp[i0 + k]);
+                  if (a.r_in) sr[i0 + k] = ov;
+                  vn[i0 + k] = ov;
+                  F::acc_prod(acc[m], ov, ov);
+                }
+            }
+          }
+          const FT t = fold_chunks<VT, 2>(acc);
+          if (lane == 0) cs[f0] = t;
+          if (lane == 16 && f0 + 1 < nfv) cs[f0 + 1] = t;
+        }
+      }
+      // a bound check whose request takes effect before the next step
+      const bool join = pending >= 0 && it + 1 == pending + a.e_delay;
+      if (join) {
+        pending = -1;
+        if (warp == 0) {
+          bar_n<3>(64);
+          if (lane == 0) s_stopnow = s_reply;
+        }
+      }
+      bar_n<1>(WT);
+      const bool ask = join && s_stopnow != 0;
+      team_publish<VT>(solo, own, pub + 2 * srow, a.T, cs, ncv, nfv, tn, ask ? tag | TS_STOP : tag,
+                       false);
+      if (solo) bar_n<1>(WT);
+      if (warp < 2) {  // warp 0: beta; warp 1: the norm and the stopping tests
+        const double rtr =
+            team_sum(mine, slotR, nt, tag, false, a.err, &flags);
+        if (lane == 0) {
+          if (flags & 2) s_fail = 1;
+          if (warp == 0) {
+            st.rtz2 = st.rtz1;
+            st.rtz1 = rtr;
+            st.beta = __ddiv_rn(rtr, st.rtz2);
+          } else {
+            const double rnorm = __dsqrt_rn(rtr);
+            st.rnorm = rnorm;
+            st.iters = it + 1;
+            s_done = rnorm < st.rtol;
+            s_run = !(rnorm < st.rtol || it + 1 >= st.miter || (flags & 1) || ask);
+            if (lead) a.vnorm[(ll)g * (a.MI + 1) + it + 1] = rnorm;
+          }
+        }
+      }
+      bar_n<1>(WT);
+      if (s_fail) break;
+      const bool check = early && s_run && it + 1 >= a.e_min &&
+                         (it + 1 - a.e_min) % a.e_stride == 0 && it + a.e_delay < a.MI;
+      if (lead && warp == NW - 1) {
+        // the off-diagonal that the next step enters (FIN_PAP computes the
+        // same expression on the same values)
+        if (lane == 0 && it + 1 < a.MI) {
+          const double u = __ddiv_rn(__dmul_rn(-st.beta, st.pap),
+                                     __dsqrt_rn(__dmul_rn(st.rtz2, st.rtz1)));
+          a.upperT[(ll)g * a.MI + it] = u;
+          cup[it] = u;
+        }
+        if (check) command(it + 2);
+      }
+      if (check) pending = it;
+      if (!s_run) break;
+    }
+    if (pending >= 0 && warp == 0) bar_n<3>(64);  // the check under way ends first
+    if (s_fail) break;
+    if (lead && threadIdx.x == 32) {
+      st.run = 0;
+      if (s_done) st.done = 1;
+      st.stopreq = 0;
+      a.gs[g] = st;
+    }
+  }
+  if (early && warp == NW - 1) command(0);
 }
 
 __global__ void k_set_active(GState *__restrict__ gs, int ngroups) {
@@ -2266,13 +2977,19 @@ struct Lanczos {
   DBuf<long long> loop_ctr;      // device restart loop: passes, SpMV steps
   bool reorth = false;           // reorthogonalise every residual (opt-in)
   DBuf<double> part2, hro;       //   its tile partials and coefficients
-  // persistent step kernel (k_steps): with PARRSB_GPU_PERSIST=1, unless per-
-  // kernel timing, reorthogonalisation or a fused finalisation is asked for,
-  // and when the level's tiles fit its resident grid
-  bool persist = false;
-  int ps_grid = 0;               //   its blocks
-  DBuf<unsigned> ps_bar;         //   barrier arrivals
-  DBuf<int> ps_run;              //   groups still running after each step
+  // team step kernel (k_team_steps): the steps of a pass in one launch
+  bool team = false;
+  int ts_grid = 0;                           // its blocks
+  int ts_rows = 0, ts_halo = 0, ts_enc = 0, ts_r = 0;  // shared memory: TeamArgs' caps and r_in
+  std::vector<int4> ts_blk;                  // per block: group list, rank, team size
+  std::vector<int> ts_list, ts_item0;
+  std::vector<int2> ts_items;                // per item: block, entry of its list
+  DBuf<int4> d_blk;
+  DBuf<int> d_list, d_item0, d_halo, d_nhalo, d_bad;
+  DBuf<int2> d_items;
+  DBuf<unsigned> d_enc;
+  DBuf<TeamSlot> slots;
+  DBuf<unsigned long long> ts_epoch;
   DBuf<ll> fq;                   // fixed-point f of the residual check (FP32)
   DBuf<unsigned> gmax, tmax;     //   each group's and tile's largest |f| (IEEE bits)
   bool resid_stop = false;       // restarts decided by the FP64 eigen-residual
@@ -2498,12 +3215,12 @@ struct Lanczos {
     tile<TM_INIT_R, GATE_ACTIVE>();
     fin<FIN_INIT_RTR, GATE_ACTIVE>(0, tol);
     mark(4 * MI + 1);
-    if (persist) {
-      steps_persistent(lv, tol);
+    if (team) {
+      team_steps(lv);
       *spmv_launches += MI;
     }
     int pending = -1;  // step of the bound check whose stop requests are due
-    for (int it = 0; it < (persist ? 0 : MI); it++) {
+    for (int it = 0; it < (team ? 0 : MI); it++) {
       if (pending >= 0 && it == pending + early_delay) {  // join, then apply the requests
         CK(cudaEventRecord(ev_join, side));
         CK(cudaStreamWaitEvent(st, ev_join, 0));
@@ -2598,28 +3315,33 @@ struct Lanczos {
 
   // kernels of the steps of one pass
   long long step_kernels() const {
-    if (persist) return 2;
+    if (team) return 2;
     return (long long)MI * ((pr_fused && !reorth) ? 3 : 5) + (sp_fused ? 0 : MI) +
            (reorth ? 3ll * MI : 0) + bound_launches();
   }
 
-  // all steps of the pass in one cooperative launch (k_steps)
-  void steps_persistent(const Level &lv, double tol) {
+  // all steps of the pass in one cooperative launch (k_team_steps)
+  void team_steps(const Level &lv) {
     cudaStream_t st = ctx().stream;
-    // (a kernel, not memset nodes, in front of the cooperative launch)
-    k_ps_reset<<<1, 128, 0, st>>>(ps_bar.p, ps_run.p, MI);
-    CK_LAUNCH();
-    StepArgs sa;
-    sa.tbeg = tbeg.p, sa.tend = tend.p, sa.tgrp = tgrp.p, sa.gs = gs.p;
-    sa.p = p.p, sa.w = w.p, sa.V = V.p, sa.VS = VS;
-    sa.ell = lv.ell.p, sa.slice_off = lv.slice_off.p, sa.slice_w = lv.slice_w.p;
-    sa.part = part.p;
-    sa.diagT = diagT.p, sa.upperT = upperT.p, sa.vnorm = vnorm.p;
-    sa.bar = ps_bar.p, sa.run_cnt = ps_run.p, sa.err = err.p;
-    sa.T = T, sa.MI = MI, sa.tol = tol;
+    // (a kernel, not a memset node, in front of the cooperative launch)
+    launch_pdl(k_team_epoch, 1, 1, 0, st, ts_epoch.p);
+    TeamArgs ta;
+    ta.tbeg = tbeg.p, ta.tend = tend.p, ta.gs = gs.p;
+    ta.pbuf[0] = p.p, ta.pbuf[1] = w.p, ta.V = V.p, ta.VS = VS;
+    ta.slice_off = lv.slice_off.p, ta.slice_w = lv.slice_w.p;
+    ta.blk = d_blk.p, ta.item0 = d_item0.p, ta.glist = d_list.p;
+    ta.enc = d_enc.p, ta.halo = d_halo.p, ta.nhalo = d_nhalo.p, ta.max_w = lv.max_w;
+    ta.slot = slots.p, ta.epoch = ts_epoch.p;
+    ta.diagT = diagT.p, ta.upperT = upperT.p, ta.vnorm = vnorm.p;
+    ta.err = err.p, ta.T = T, ta.MI = MI;
+    ta.rows_cap = ts_rows, ta.halo_cap = ts_halo, ta.enc_cap = ts_enc, ta.r_in = ts_r;
+    ta.stop_below = early * resid_tol;
+    ta.e_min = early_min, ta.e_stride = early_stride, ta.e_delay = early_delay;
+    ta.e_span = 3 * early_stride;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ps_grid);
-    cfg.blockDim = dim3(PS_THREADS);
+    cfg.gridDim = dim3((unsigned)ts_grid);
+    cfg.blockDim = dim3(TS_THREADS);
+    cfg.dynamicSmemBytes = team_smem();
     cfg.stream = st;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;
@@ -2627,24 +3349,220 @@ struct Lanczos {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     ctx().kernel_launches++;
-    CK(cudaLaunchKernelEx(&cfg, k_steps<VT>, sa));
+    CK(cudaLaunchKernelEx(&cfg, k_team_steps<VT>, ta));
+  }
+  size_t team_smem() const {
+    return (size_t)(ts_place<VT>(ts_rows) + ts_rows * (ts_r ? 2 : 1) + ts_halo) * sizeof(VT) +
+           (size_t)ts_halo * sizeof(int) + (size_t)ts_enc * sizeof(unsigned);
   }
 
-  // whether this level runs its steps in k_steps, and with how many blocks
-  bool want_persist() {
+  // Assigns the level's groups to teams of blocks (G in all, one per SM).  A
+  // group whose rows fit the share of one block goes to a single block, which
+  // takes such groups one after the other (largest first, to the least loaded
+  // block); a larger one gets a team of its own, with as few rows per block as
+  // the blocks allow.  Where that needs more blocks than there are, the large
+  // groups share teams of equal size.  False: some group does not fit.
+  bool plan_teams(int G) {
+    constexpr ll CAP = ts_cap<VT>();
+    // what a step of a group costs beside its rows, in rows (team_pays)
+    constexpr ll BASE = sizeof(VT) == 8 ? 700 : 2700;
+    ts_blk.assign(G, make_int4(0, 0, 0, 1));
+    ts_list.clear();
+    ll total = 0, biggest = 0;
+    for (const GState &s : hgs) total += s.n, biggest = std::max(biggest, s.n);
+    if (biggest > TS_GROUP) return false;
+    auto tiles_at = [&](const GState &s, ll rows) {  // tiles per block at `rows` rows
+      return (int)std::max<ll>(1, std::min<ll>(rows / std::min(tile_rows(s.n), s.n), TS_TILES));
+    };
+    auto team_of = [&](const GState &s, ll rows) {
+      const int k = tiles_at(s, rows);
+      return (s.ntiles + k - 1) / k;
+    };
+    std::vector<int> order(A), small, big;
+    for (int g = 0; g < A; g++) order[g] = g;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return hgs[x].n > hgs[y].n; });
+    auto split = [&](ll rows, ll &blocks, ll &rest) {
+      small.clear(), big.clear();
+      blocks = rest = 0;
+      for (int g : order) {
+        const int s = team_of(hgs[g], rows);
+        if (s > 1)
+          big.push_back(g), blocks += s;
+        else
+          small.push_back(g), rest += hgs[g].n + BASE;
+      }
+    };
+    ll blocks = 0, rest = 0, rows = std::max<ll>(512, total / G);
+    bool own = false;
+    for (;;) {
+      rows = std::min(rows, CAP);
+      split(rows, blocks, rest);
+      const ll bins = G - blocks;
+      own = blocks <= G &&
+            (rest == 0 || (bins > 0 && (rest <= bins * (rows + BASE) || rows == CAP)));
+      if (own || rows == CAP) break;
+      rows += std::max<ll>(64, rows / 16);
+    }
+    int used = 0;
+    if (own) {
+      for (int g : big) {
+        const int s = team_of(hgs[g], rows);
+        for (int r = 0; r < s; r++)
+          ts_blk[used + r] = make_int4((int)ts_list.size(), 1, r, s);
+        ts_list.push_back(g);
+        used += s;
+      }
+    } else {
+      split(CAP, blocks, rest);
+      if (!big.empty()) {
+        int s = 1;
+        ll load = 0;
+        for (int g : big) s = std::max(s, team_of(hgs[g], CAP)), load += hgs[g].n + BASE;
+        if (s > G - (rest ? 1 : 0)) return false;
+        int nt = (int)std::max<ll>(1, (ll)llround((double)G * load / (double)(load + rest)) / s);
+        while (rest && nt > 1 && nt * s >= G) nt--;
+        nt = std::min(nt, (int)big.size());
+        std::vector<std::vector<int>> lists(nt);
+        std::vector<ll> w(nt, 0);
+        for (int g : big) {
+          const int t = (int)(std::min_element(w.begin(), w.end()) - w.begin());
+          lists[t].push_back(g);
+          w[t] += hgs[g].n;
+        }
+        for (int t = 0; t < nt; t++) {
+          for (int r = 0; r < s; r++)
+            ts_blk[used + r] = make_int4((int)ts_list.size(), (int)lists[t].size(), r, s);
+          ts_list.insert(ts_list.end(), lists[t].begin(), lists[t].end());
+          used += s;
+        }
+      }
+    }
+    if (!small.empty()) {
+      const int nb = std::min<int>(G - used, (int)small.size());
+      if (nb <= 0) return false;
+      std::vector<std::vector<int>> lists(nb);
+      std::vector<std::pair<ll, int>> heap;  // (load, block), least loaded first
+      for (int b = 0; b < nb; b++) heap.push_back({0, b});
+      auto later = [](const std::pair<ll, int> &x, const std::pair<ll, int> &y) { return x > y; };
+      for (int g : small) {
+        std::pop_heap(heap.begin(), heap.end(), later);
+        lists[heap.back().second].push_back(g);
+        heap.back().first += hgs[g].n + BASE;
+        std::push_heap(heap.begin(), heap.end(), later);
+      }
+      for (int b = 0; b < nb; b++) {
+        ts_blk[used + b] = make_int4((int)ts_list.size(), (int)lists[b].size(), 0, 1);
+        ts_list.insert(ts_list.end(), lists[b].begin(), lists[b].end());
+      }
+      used += nb;
+    }
+    ts_grid = used;
+    ts_blk.resize(used);
+    // the items, and the rows per block
+    ts_items.clear();
+    ts_item0.clear();
+    for (int b = 0; b < used; b++) {
+      ts_item0.push_back((int)ts_items.size());
+      for (int q = 0; q < ts_blk[b].y; q++) ts_items.push_back(make_int2(b, q));
+    }
+    ll most = 0;
+    for (const int4 &b : ts_blk)
+      for (int q = 0; q < b.y; q++) {
+        const GState &s = hgs[ts_list[b.x + q]];
+        const ll k = ((ll)s.ntiles + b.w - 1) / b.w;
+        if (k > TS_TILES || s.ntiles < b.w) return false;
+        most = std::max(most, std::min(k * tile_rows(s.n), s.n));
+      }
+    if (most > CAP) return false;
+    constexpr ll CH = 32 * VecOf<VT>::R;
+    ts_rows = (int)((most + 2 * CH) / CH * CH);
+    return true;
+  }
+
+  // Microseconds of a step in k_team_steps (the busiest block, all groups of
+  // its list) and in the launch-per-kernel pass, fitted to hex meshes on a
+  // GB300 (rows per block 512-8192, 64K-8M rows in all).  Measured, FP64, team
+  // against launches: 65K rows 16 / 28 us, 524K in 8 groups 57 / 82, 1M in one
+  // group 118 / 141; FP32: 65K 12 / 23, 524K 24 / 44, 1M in 16 groups 35 / 52;
+  // 1M in one group 54 / 52 and 8M in 512 groups 230 / 255 (lists of 7 groups
+  // a team) are not worth it, hence the margin.
+  bool team_pays() const {
+    const bool f64 = sizeof(VT) == 8;
+    double worst = 0.0, rows = 0.0;
+    for (const GState &s : hgs) rows += (double)s.n;
+    for (const int4 &b : ts_blk) {
+      double t = 0.0;
+      for (int q = 0; q < b.y; q++) {
+        const GState &s = hgs[ts_list[b.x + q]];
+        const ll k = ((ll)s.ntiles + b.w - 1) / b.w;
+        t += 7.3 + (f64 ? 0.0106 : 0.00266) * (double)std::min(k * tile_rows(s.n), s.n) +
+             (b.w > 1 ? 0.03 * s.ntiles : 0.0);
+      }
+      worst = std::max(worst, t * (b.y > 1 && b.w > 1 ? 1.35 : 1.2));
+    }
+    return worst < (f64 ? 24.0 + 112e-6 * rows : 22.0 + 29e-6 * rows);
+  }
+
+  // whether this level runs its steps in k_team_steps (PARRSB_GPU_PERSIST=0:
+  // never, 1: wherever its groups fit)
+  bool want_team(const Level &lv) {
     const char *e = getenv("PARRSB_GPU_PERSIST");
-    if (!e || atoi(e) == 0) return false;  // opt-in
-    if (reorth || pr_fused || sp_fused || !ev.empty() || T <= 0) return false;
+    if (e && atoi(e) == 0) return false;
+    const bool force = e && atoi(e) != 0;
+    if (reorth || pr_fused || sp_fused || bound_log || !ev.empty() || T <= 0) return false;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<VT>, PS_THREADS, 0));
-    const ll cap = (ll)sms * per_sm;
-    if (cap <= 0) return false;
-    ps_grid = (int)std::min<ll>(T, cap);
-    if ((T + ps_grid - 1) / ps_grid > PS_SLOTS) return false;
-    ps_bar.ensure(1);
-    ps_run.ensure((size_t)MI);
+    ensure_smem_limit(k_team_steps<VT>, TS_SMEM);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_team_steps<VT>, TS_THREADS,
+                                                     TS_SMEM));
+    if (per_sm < 1 || !plan_teams(sms) || !(force || team_pays())) return false;
+    // shared memory: p and w, the halo, then the encoded rows, then r as they fit
+    const bool halos = ts_blk[0].w > 1;  // (teams of several blocks come first)
+    // (a compact run of r rows of a 3D mesh has about 1.5 r^(2/3) x 6 halo rows)
+    ts_halo = halos ? std::min({TS_HALO, TS_LOCAL - ts_place<VT>(ts_rows), 3 * ts_rows}) : 0;
+    ts_enc = ts_r = 0;
+    if (ts_halo < 0 || ts_place<VT>(ts_rows) > TS_LOCAL || team_smem() > TS_SMEM) return false;
+    const ll words = ((ll)ts_rows / 32 + 2) * ((lv.max_w + 1) / 2 + 1) * 32;
+    ts_r = 1;
+    if (team_smem() > TS_SMEM) ts_r = 0;
+    if (ts_r && team_smem() + words * sizeof(unsigned) <= TS_SMEM) ts_enc = (int)words;
+    int multi = 0;  // items with a halo: those of the teams of several blocks
+    for (const int2 &it : ts_items) multi += ts_blk[it.x].w > 1;
+    ll biggest = 0;
+    for (const GState &s : hgs) biggest = std::max(biggest, s.n);
+    const size_t bm = halos ? (size_t)((biggest + 127) / 128) * (16 + 2) + 64 : 64;
+    if (bm > (size_t)TS_SMEM) return false;
+    cudaStream_t st = ctx().stream;
+    d_blk.ensure(ts_blk.size()), d_list.ensure(ts_list.size());
+    d_item0.ensure(ts_item0.size()), d_items.ensure(ts_items.size());
+    h2d(d_blk.p, ts_blk.data(), ts_blk.size());
+    h2d(d_list.p, ts_list.data(), ts_list.size());
+    h2d(d_item0.p, ts_item0.data(), ts_item0.size());
+    h2d(d_items.p, ts_items.data(), ts_items.size());
+    d_nhalo.ensure(ts_items.size());
+    d_halo.ensure((size_t)std::max(multi, 1) * TS_HALO);
+    d_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
+                 (size_t)(T + 1) * (size_t)(lv.max_w + 1) * 32 + 128);
+    d_bad.ensure(1);
+    CK(cudaMemsetAsync(d_bad.p, 0, sizeof(int), st));
+    ensure_smem_limit(k_team_encode<VT>, TS_SMEM);
+    k_team_encode<VT><<<(unsigned)ts_items.size(), TE_THREADS, bm, st>>>(
+        tbeg.p, tend.p, gs.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, d_blk.p, d_item0.p, d_list.p,
+        d_items.p, ts_place<VT>(ts_rows), ts_halo, lv.max_w, d_enc.p, d_halo.p, d_nhalo.p,
+        d_bad.p);
+    CK_LAUNCH();
+    int bad = 0;
+    d2h(&bad, d_bad.p, 1);
+    sync();
+    if (bad) return false;
+    slots.ensure((size_t)3 * TS_REP * T);
+    CK(cudaMemsetAsync(slots.p, 0, (size_t)3 * TS_REP * T * sizeof(TeamSlot), ctx().stream));
+    if (!ts_epoch.p) {
+      ts_epoch.alloc(1);
+      CK(cudaMemsetAsync(ts_epoch.p, 0, sizeof(unsigned long long), ctx().stream));
+    }
     return true;
   }
 
@@ -2740,8 +3658,7 @@ struct Lanczos {
       const char *v = getenv("PARRSB_GPU_PASS_LOG");
       return v ? atoi(v) : 0;
     }();
-    // early pass exit (residual-stop mode only; the persistent step kernel
-    // takes no checks): after steps 3, 6, 9, ... a group whose Ritz residual
+    // early pass exit (residual-stop mode only): after steps 3, 6, 9, ... a group whose Ritz residual
     // bound is below 0.7 rsb_tol ends its pass three steps later (the check
     // runs beside the next two); the FP64 residual of its Ritz vector still
     // decides whether it restarts.
@@ -2802,8 +3719,8 @@ struct Lanczos {
     }();
     // sticky fallbacks after a graph could not be built (any thread, any device)
     static std::atomic<bool> device_loop_broken{false};
-    static std::atomic<bool> persist_broken{false};  // a graph with k_steps failed once
-    persist = !persist_broken && want_persist();
+    static std::atomic<bool> team_broken{false};  // a graph with k_team_steps failed once
+    team = !team_broken && want_team(lv);
     for (int attempt = 0;
          attempt < 2 && !exec && use_graph && ev.empty() && device_loop_env && !device_loop_broken;
          attempt++) try {
@@ -2846,10 +3763,10 @@ struct Lanczos {
       if (exec) cudaGraphExecDestroy(exec);
       if (graph) cudaGraphDestroy(graph);
       exec = nullptr, graph = nullptr;
-      if (persist) {  // try again with the launch-per-kernel steps
-        persist_broken = true;
-        persist = false;
-        fprintf(stderr, "parrsb_gb300: persistent step kernel unavailable in graphs (%s)\n",
+      if (team) {  // try again with the launch-per-kernel steps
+        team_broken = true;
+        team = false;
+        fprintf(stderr, "parrsb_gb300: team step kernel unavailable in graphs (%s)\n",
                 cudaGetErrorString(e.err));
         continue;
       }
@@ -2888,7 +3805,7 @@ struct Lanczos {
       ctx().stats.lanczos_host_ms[1] +=
           std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
     } catch (const CudaError &e) {
-      if (!persist) throw;
+      if (!team) throw;
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
         cudaGraph_t g2 = nullptr;
@@ -2899,9 +3816,9 @@ struct Lanczos {
       if (exec) cudaGraphExecDestroy(exec);
       if (graph) cudaGraphDestroy(graph);
       exec = nullptr, graph = nullptr;
-      persist_broken = true;
-      persist = false;
-      fprintf(stderr, "parrsb_gb300: persistent step kernel unavailable in graphs (%s)\n",
+      team_broken = true;
+      team = false;
+      fprintf(stderr, "parrsb_gb300: team step kernel unavailable in graphs (%s)\n",
               cudaGetErrorString(e.err));
     }
     const long long per_pass_kernels =
@@ -3358,6 +4275,7 @@ void build_level(const Graph &g, const int *perm, const int *inv, const int *grp
   CK_LAUNCH();
   ll total = exclusive_scan_ll(slots.p, lv.slice_off.p, nslice);
   h2d(lv.slice_off.p + nslice, &total, 1);  // end of the last slice
+  lv.words = total;
   lv.ell.ensure((size_t)total + 32);
   k_ell_fill<<<grid_for(N, 256), 256, 0, st>>>(perm, inv, grp, g.rowptr.p, g.col.p, g.w.p, N,
                                                lv.slice_off.p, lv.slice_w.p, lv.ell.p);
@@ -3833,6 +4751,7 @@ bool coarse_predict_level(const Level &lv, const int *perm, const int *grp, cons
   CK_LAUNCH();
   const ll total = exclusive_scan_ll(slots.p, lvc.slice_off.p, nslice);
   h2d(lvc.slice_off.p + nslice, &total, 1);
+  lvc.words = total;
   lvc.ell.ensure((size_t)total + 32);
   k_coarse_rows<true><<<cb, 256, 0, st>>>(lv.ell.p, lv.slice_off.p, lv.slice_w.p, cmap.p,
                                           agg_off.p, vals.p, Nc, rowlen.p, lvc.slice_off.p,

@@ -27,6 +27,7 @@ struct Level {
   DBuf<unsigned> ell;
   DBuf<ll> slice_off;
   DBuf<int> slice_w;
+  ll words = 0;  // ELL words of all slices
   ll nnz = 0;    // restricted nonzeros of the active rows
   ll rows = 0;   // active rows
   int max_w = 0; // widest slice
