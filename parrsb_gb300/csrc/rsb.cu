@@ -1706,67 +1706,97 @@ __device__ __forceinline__ int sturm_count(const double *d, const double *e2, in
   return cnt;
 }
 
-// y / x with a single-precision reciprocal refined by two Newton steps
-__device__ __forceinline__ double fast_div(double y, double x) {
-  double ax = fabs(x);
-  double r;
-  if (ax > 1e-30 && ax < 1e30) {
-    r = (double)__frcp_rn((float)x);
+// A dependent FP64 instruction takes 64 cycles on GB300 (measured, one warp:
+// multiply, add, FMA alike; a division 574), so the serial loops below keep
+// comparisons and zero tests on the bit pattern (magnitudes of doubles order
+// as their bits do) and take everything that does not depend on the chain out
+// of it, onto the other lanes.
+__device__ __forceinline__ long long mag_bits(double x) {
+  return __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll;
+}
+// 1 / x from a single-precision reciprocal refined by two Newton steps
+__device__ __forceinline__ double fast_rcp(double x) {
+  const long long ax = mag_bits(x);
+  if (ax > 0x39B4484BFEEBC2A0ll && ax < 0x46293E5939A08CEAll) {  // 1e-30 < |x| < 1e30
+    double r = (double)__frcp_rn((float)x);
     r = fma(r, fma(-x, r, 1.0), r);
-    r = fma(r, fma(-x, r, 1.0), r);
-  } else {
-    r = __ddiv_rn(1.0, x);
+    return fma(r, fma(-x, r, 1.0), r);
   }
-  double q = __dmul_rn(y, r);
-  return fma(r, fma(-x, q, y), q);  // one correction of the quotient
+  return __ddiv_rn(1.0, x);
+}
+// y / x, r = fast_rcp(x): one correction of the quotient
+__device__ __forceinline__ double div_rcp(double y, double x, double r) {
+  const double q = __dmul_rn(y, r);
+  return fma(r, fma(-x, q, y), q);
+}
+__device__ __forceinline__ double fast_div(double y, double x) {
+  return div_rcp(y, x, fast_rcp(x));
 }
 
-__device__ void tri_solve_pivot(int n, const double *a0, const double *e, double lam,
-                                double *x, double *a, double *b, double *c, double *c2,
-                                int *piv, double tiny) {
-  // factor (T - lam I) = P L U with U having two super-diagonals (dgttrf)
-  for (int i = 0; i < n; i++) a[i] = __dsub_rn(a0[i], lam);
-  for (int i = 0; i < n - 1; i++) b[i] = e[i], c[i] = e[i], c2[i] = 0.0;
+// T - lam I = P L U with U having two super-diagonals (dgttrf), by lane 0 of
+// the warp: a, c, c2 the diagonals of U, b the multipliers.  L^-1 P is applied
+// to x (all ones) in the same loop.
+__device__ void tri_factor(int n, const double *a0, const double *e, double lam, double *x,
+                           double *a, double *b, double *c, double *c2, int *piv, double tiny) {
+  // the rows of T - lam I enter one ahead of the elimination
+  double ai = __dsub_rn(a0[0], lam), ci = n > 1 ? e[0] : 0.0, xi = 1.0;
   for (int i = 0; i < n - 1; i++) {
-    if (fabs(a[i]) >= fabs(b[i])) {
+    const double bi = e[i], an = __dsub_rn(a0[i + 1], lam);  // row i + 1
+    const double cn = i < n - 2 ? e[i + 1] : 0.0;
+    if (mag_bits(ai) >= mag_bits(bi)) {
       piv[i] = 0;
-      if (a[i] == 0.0) a[i] = tiny;
-      double fact = fast_div(b[i], a[i]);
-      b[i] = fact;
-      a[i + 1] = fma(-fact, c[i], a[i + 1]);
-      c2[i] = 0.0;
+      if (mag_bits(ai) == 0) ai = tiny;
+      const double fact = fast_div(bi, ai);
+      a[i] = ai, b[i] = fact, c[i] = ci, c2[i] = 0.0;
+      ai = fma(-fact, ci, an);
+      ci = cn;
+      x[i] = xi;
+      xi = fma(-fact, xi, 1.0);
     } else {
       piv[i] = 1;
-      double fact = fast_div(a[i], b[i]);
-      a[i] = b[i];
-      b[i] = fact;
-      double t = c[i];
-      c[i] = a[i + 1];
-      a[i + 1] = fma(-fact, a[i + 1], t);
-      if (i < n - 2) {
-        c2[i] = c[i + 1];
-        c[i + 1] = __dmul_rn(-fact, c[i + 1]);
-      } else {
-        c2[i] = 0.0;
-      }
+      const double fact = fast_div(ai, bi);
+      a[i] = bi, b[i] = fact, c[i] = an;
+      ai = fma(-fact, an, ci);
+      c2[i] = i < n - 2 ? cn : 0.0;
+      ci = i < n - 2 ? __dmul_rn(-fact, cn) : 0.0;
+      x[i] = 1.0;
+      xi = fma(-fact, 1.0, xi);
     }
   }
-  if (n > 0 && a[n - 1] == 0.0) a[n - 1] = tiny;
-  for (int i = 0; i < n - 1; i++) {  // L with row interchanges
+  if (mag_bits(ai) == 0) ai = tiny;
+  a[n - 1] = ai;
+  x[n - 1] = xi;
+}
+// L^-1 P applied to x again (the second sweep), by lane 0
+__device__ void tri_forward(int n, const double *b, const int *piv, double *x) {
+  double xi = x[0];
+  for (int i = 0; i < n - 1; i++) {
+    const double xn = x[i + 1];
     if (piv[i]) {
-      double t = x[i];
-      x[i] = x[i + 1];
-      x[i + 1] = fma(-b[i], x[i], t);
+      x[i] = xn;
+      xi = fma(-b[i], xn, xi);
     } else {
-      x[i + 1] = fma(-b[i], x[i], x[i + 1]);
+      x[i] = xi;
+      xi = fma(-b[i], xi, xn);
     }
   }
-  for (int i = n - 1; i >= 0; i--) {  // U
+  x[n - 1] = xi;
+}
+// U x = x, then the norm of x; lane 0; r = 1 / a (fast_rcp)
+__device__ double tri_back(int n, const double *a, const double *r, const double *c,
+                           const double *c2, double *x) {
+  double x1 = 0.0, x2 = 0.0;
+  for (int i = n - 1; i >= 0; i--) {
     double v = x[i];
-    if (i + 1 < n) v = fma(-c[i], x[i + 1], v);
-    if (i + 2 < n) v = fma(-c2[i], x[i + 2], v);
-    x[i] = fast_div(v, a[i]);
+    if (i + 1 < n) v = fma(-c[i], x1, v);
+    if (i + 2 < n) v = fma(-c2[i], x2, v);
+    x2 = x1;
+    x1 = div_rcp(v, a[i], r[i]);
+    x[i] = x1;
   }
+  double nrm = 0.0;
+  for (int i = 0; i < n; i++) nrm = fma(x[i], x[i], nrm);
+  return nrm;
 }
 
 __device__ __forceinline__ double warp_min_d(double v) {
@@ -1849,17 +1879,26 @@ __global__ void k_tri_eig(GState *__restrict__ gs, int ngroups,
     double lp = eig_index(D0, e2, n, c0, glo, ghi);
     lam = fabs(lp) < fabs(ln) ? lp : ln;
   }
-  if (lane == 0) {
-    double tnorm = fmax(fabs(glo), fabs(ghi));
-    double tiny = fmax(tnorm, 1e-300) * 1e-16;
-    for (int i = 0; i < n; i++) x[i] = 1.0;
-    for (int sweep = 0; sweep < 2; sweep++) {
-      tri_solve_pivot(n, D0, E0, lam, x, a, b, c, c2, piv, tiny);
-      double nrm = 0.0;
-      for (int i = 0; i < n; i++) nrm = fma(x[i], x[i], nrm);
-      double inv = nrm > 0.0 ? fast_div(1.0, __dsqrt_rn(nrm)) : 0.0;
-      for (int i = 0; i < n; i++) x[i] = __dmul_rn(x[i], inv);
+  // inverse iteration: the factors of T - lam I serve both sweeps, and lane 0
+  // has its chains of dependent FP64 instructions to itself (the reciprocals
+  // of U's diagonal and the scaling run on all lanes)
+  const double tnorm = fmax(fabs(glo), fabs(ghi));
+  const double tiny = fmax(tnorm, 1e-300) * 1e-16;
+  if (lane == 0) tri_factor(n, D0, E0, lam, x, a, b, c, c2, piv, tiny);
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) e2[i] = fast_rcp(a[i]);
+  __syncwarp();
+  for (int sweep = 0; sweep < 2; sweep++) {
+    double inv = 0.0;
+    if (lane == 0) {
+      if (sweep) tri_forward(n, b, piv, x);
+      const double nrm = tri_back(n, a, e2, c, c2, x);
+      inv = nrm > 0.0 ? fast_div(1.0, __dsqrt_rn(nrm)) : 0.0;
     }
+    inv = __shfl_sync(0xffffffffu, inv, 0);
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) x[i] = __dmul_rn(x[i], inv);
+    __syncwarp();
   }
   __syncwarp();
   for (int j = lane; j < n; j += 32)
@@ -1908,29 +1947,39 @@ __device__ __noinline__ double ritz_bound_warp(const double *D0, const double *E
                  : eig_index(D0, e2, n, 0, glo, ghi, 1e-10))
          : 0.0;
   double bound = 1e300;
-  if (pd && lane == 0) {
+  if (pd) {
     // pivots of T_k - theta I, then z from the bottom (scaled to stay finite)
-    double d = __dsub_rn(D0[0], theta);
-    dv[0] = d;
-    for (int i = 1; i < n; i++) {
-      d = __dsub_rn(__dsub_rn(D0[i], theta), fast_div(e2[i - 1], d));
-      dv[i] = d;
-    }
-    double z = 1.0, zl = 1.0, ss = 1.0;  // current z_i, z_(k-1), sum of squares
-    for (int i = n - 2; i >= 0; i--) {
-      z = fast_div(__dmul_rn(-E0[i], z), dv[i]);
-      if (!(fabs(z) < 1e150)) {
-        if (!isfinite(z)) {  // a zero pivot: the pair is exact to working precision
-          zl = 0.0;
-          ss = 1.0;
-          break;
-        }
-        z = __dmul_rn(z, 1e-150), zl = __dmul_rn(zl, 1e-150), ss = __dmul_rn(ss, 1e-300);
+    for (int i = lane; i < n; i += 32) dv[i] = __dsub_rn(D0[i], theta);
+    __syncwarp();
+    if (lane == 0) {
+      double d = dv[0];
+      for (int i = 1; i < n; i++) {
+        d = __dsub_rn(dv[i], fast_div(e2[i - 1], d));
+        dv[i] = d;
       }
-      ss = fma(z, z, ss);
     }
-    const double yk = fast_div(fabs(zl), __dsqrt_rn(ss));
-    bound = __dmul_rn(fabs(bk), yk);
+    __syncwarp();
+    for (int i = lane; i < n - 1; i += 32) e2[i] = fast_rcp(dv[i]);
+    __syncwarp();
+    if (lane == 0) {
+      double z = 1.0, zl = 1.0, ss = 1.0;  // current z_i, z_(k-1), sum of squares
+      for (int i = n - 2; i >= 0; i--) {
+        z = div_rcp(__dmul_rn(-E0[i], z), dv[i], e2[i]);
+        const long long az = mag_bits(z);
+        if (az >= 0x5F138D352E5096AFll) {  // not |z| < 1e150
+          if (az >= 0x7FF0000000000000ll) {  // a zero pivot: the pair is exact to working precision
+            zl = 0.0;
+            ss = 1.0;
+            break;
+          }
+          z = __dmul_rn(z, 1e-150), zl = __dmul_rn(zl, 1e-150), ss = __dmul_rn(ss, 1e-300);
+        }
+        ss = fma(z, z, ss);
+      }
+      const double yk = fast_div(fabs(zl), __dsqrt_rn(ss));
+      bound = __dmul_rn(fabs(bk), yk);
+    }
+    __syncwarp();
   }
   theta_out = pd ? theta : 0.0;
   return bound;
