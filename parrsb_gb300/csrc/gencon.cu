@@ -19,8 +19,6 @@ namespace prsb {
 namespace {
 
 __constant__ int c_pre_to_sym[8] = {0, 1, 3, 2, 4, 5, 7, 6};
-__constant__ int c_nbr[8][3] = {{1, 2, 4}, {0, 3, 5}, {0, 3, 6}, {1, 2, 7},
-                                {0, 5, 6}, {1, 4, 7}, {2, 4, 7}, {3, 5, 6}};
 // faces in symmetric corner order (0-based), src/con-periodic.c:8-10
 __constant__ int c_face_mask3[6] = {
     (1 << 0) | (1 << 4) | (1 << 6) | (1 << 2), (1 << 1) | (1 << 3) | (1 << 7) | (1 << 5),
@@ -32,47 +30,88 @@ __device__ __forceinline__ double dsq(double a, double b) {
   return __dmul_rn(t, t);
 }
 
-// Points in symmetric order and their min squared neighbour distance.
-__global__ void k_points(const double *__restrict__ coord, ll nel, int ndim,
-                         double *__restrict__ x0, double *__restrict__ x1,
-                         double *__restrict__ x2, double *__restrict__ dx) {
-  ll e = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  int nv = ndim == 2 ? 4 : 8;
-  double px[8][3];
-  const double *c = coord + e * nv * ndim;
-  for (int k = 0; k < nv; k++) {
-    int j = c_pre_to_sym[k];
-    px[k][0] = c[j * ndim + 0];
-    px[k][1] = c[j * ndim + 1];
-    px[k][2] = ndim == 3 ? c[j * ndim + 2] : 0.0;
-  }
-  for (int k = 0; k < nv; k++) {
-    ll p = e * nv + k;
-    x0[p] = px[k][0];
-    x1[p] = px[k][1];
-    x2[p] = px[k][2];
-    double m = 1.7976931348623157e308;
-    for (int q = 0; q < ndim; q++) {
-      int nb = c_nbr[k][q];
-      double d = __dadd_rn(dsq(px[k][0], px[nb][0]), dsq(px[k][1], px[nb][1]));
-      if (ndim == 3) d = __dadd_rn(d, dsq(px[k][2], px[nb][2]));
-      m = (m < d) ? m : d;
+__device__ __forceinline__ bool nan_bits(double x) {
+  return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll;
+}
+// m < d ? m : d for squares (never negative: their bits order as they do)
+// without the FP64 pipe's comparison
+__device__ __forceinline__ double min_sq(double m, double d) {
+  const bool lt = __double_as_longlong(m) < __double_as_longlong(d);
+  return lt && !nan_bits(m) && !nan_bits(d) ? m : d;
+}
+
+// Points in symmetric order and their min squared neighbour distance.  A CTA
+// stages its elements' corners in shared memory (coalesced loads and stores:
+// 0.46 -> 0.26 ms per million hexes) and a thread takes an element: each of
+// the 12 edges (4 in 2D) is measured once for its two corners, since the FP64
+// pipe bounds the kernel ((a - b)^2 and (b - a)^2 are the same bits).
+constexpr int GP_ELEMS = 128;
+template <int NDIM>
+__global__ void __launch_bounds__(GP_ELEMS)
+k_points(const double *__restrict__ coord, ll nel, double *__restrict__ x0,
+         double *__restrict__ x1, double *__restrict__ x2, double *__restrict__ dx) {
+  constexpr int NV = NDIM == 2 ? 4 : 8, ROW = NV * NDIM;
+  constexpr int PAD = ROW + 1;  // an element's row in shared memory
+  extern __shared__ double gp[];
+  const ll e0 = (ll)blockIdx.x * GP_ELEMS;
+  const int ne = (int)(nel - e0 < GP_ELEMS ? nel - e0 : GP_ELEMS);
+  for (int k = threadIdx.x; k < ne * ROW; k += GP_ELEMS)
+    gp[(k / ROW) * PAD + k % ROW] = coord[e0 * ROW + k];
+  __syncthreads();
+  double m[NV];
+  if ((int)threadIdx.x < ne) {
+    const double *c = gp + threadIdx.x * PAD;
+    double px[NV][NDIM];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      constexpr int sym[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+#pragma unroll
+      for (int q = 0; q < NDIM; q++) px[k][q] = c[sym[k] * NDIM + q];
+      m[k] = 1.7976931348623157e308;
     }
-    dx[p] = m;
+    // edge by edge; a corner meets its neighbours in increasing order
+    auto edge = [&](int a, int b) {
+      double d = __dadd_rn(dsq(px[a][0], px[b][0]), dsq(px[a][1], px[b][1]));
+      if (NDIM == 3) d = __dadd_rn(d, dsq(px[a][NDIM - 1], px[b][NDIM - 1]));
+      m[a] = min_sq(m[a], d);
+      m[b] = min_sq(m[b], d);
+    };
+    edge(0, 1), edge(0, 2);
+    if (NDIM == 3) edge(0, NV - 4);
+    edge(1, 3);
+    if (NDIM == 3) edge(1, NV - 3);
+    edge(2, 3);
+    if (NDIM == 3)
+      edge(2, NV - 2), edge(3, NV - 1), edge(NV - 4, NV - 3), edge(NV - 4, NV - 2),
+          edge(NV - 3, NV - 1), edge(NV - 2, NV - 1);
+  }
+  __syncthreads();
+  // out through shared memory: the distances, then each coordinate in place
+  double *out[4] = {x0, x1, x2, dx};
+  for (int q = 0; q < 4; q++) {
+    if (q == 3) {
+      __syncthreads();
+      if ((int)threadIdx.x < ne)
+#pragma unroll
+        for (int k = 0; k < NV; k++) gp[threadIdx.x * PAD + k] = m[k];
+      __syncthreads();
+    }
+    for (int k = threadIdx.x; k < ne * NV; k += GP_ELEMS) {
+      const int e = k / NV, v = k % NV;
+      double val;
+      if (q == 3)
+        val = gp[e * PAD + v];
+      else
+        val = q < NDIM ? gp[e * PAD + c_pre_to_sym[v] * NDIM + q] : 0.0;
+      out[q][e0 * NV + k] = val;
+    }
   }
 }
 
-__global__ void k_gc_keys(const int *__restrict__ ord, const double *__restrict__ x,
-                          const ll *__restrict__ segid, ll np,
-                          u64 *__restrict__ keys, int *__restrict__ vals,
-                          int *__restrict__ seg_of_pt) {
+__global__ void k_gc_keys(const int *__restrict__ ord, const double *__restrict__ x, ll np,
+                          u64 *__restrict__ keys) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= np) return;
-  int p = ord[i];
-  keys[i] = ordered_key(x[p]);
-  vals[i] = p;
-  if (seg_of_pt) seg_of_pt[p] = (int)segid[i];
+  if (i < np) keys[i] = ordered_key(x[ord[i]]);
 }
 
 __global__ void k_iota(int *__restrict__ a, ll n) {
@@ -80,50 +119,181 @@ __global__ void k_iota(int *__restrict__ a, ll n) {
   if (i < n) a[i] = (int)i;
 }
 
-// flag[j] |= gap between sorted neighbours j-1, j along coordinate x.
-__global__ void k_gaps(const int *__restrict__ ord, const double *__restrict__ x,
+__device__ __forceinline__ double key_value(u64 k) {
+  return __longlong_as_double((ll)((k >> 63) ? (k ^ 0x8000000000000000ull) : ~k));
+}
+
+// whether a gap separates sorted neighbours at squared distance d with the
+// smallest neighbour distances da, db
+__device__ __forceinline__ bool gap_between(double d, double da, double db, double tol2) {
+  return d > __dmul_rn(da < db ? da : db, tol2);
+}
+
+// flag[j] |= gap between sorted neighbours j-1, j along the coordinate that
+// was sorted last (its values are the keys).  A warp's lane takes its left
+// neighbour's point from the lane beside it, so dx is gathered once.
+__global__ void k_gaps(const int *__restrict__ ord, const u64 *__restrict__ keys,
                        const double *__restrict__ dx, ll np, double tol2,
                        int first_pass, int *__restrict__ flag) {
-  ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  double x = 0.0, w = 0.0;
+  if (j < np) x = key_value(keys[j]), w = dx[ord[j]];
+  double xl = __shfl_up_sync(0xffffffffu, x, 1), wl = __shfl_up_sync(0xffffffffu, w, 1);
   if (j >= np) return;
+  if (lane == 0 && j > 0) xl = key_value(keys[j - 1]), wl = dx[ord[j - 1]];
   if (j == 0) {
     flag[0] = 1;
     return;
   }
-  int pj = ord[j], pk = ord[j - 1];
-  double d = dsq(x[pj], x[pk]);
-  double m = __dmul_rn(dx[pj] < dx[pk] ? dx[pj] : dx[pk], tol2);
-  int f = d > m ? 1 : 0;
+  const int f = gap_between(dsq(x, xl), w, wl, tol2) ? 1 : 0;
   if (first_pass)
     flag[j] = f;
   else if (f)
     flag[j] = 1;
 }
 
-// segid = inclusive prefix of flags minus one, from the exclusive scan.
-__global__ void k_segid(const int *__restrict__ flag, ll *__restrict__ scan, ll np) {
-  ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < np) scan[i] = scan[i] + flag[i] - 1;
+// After the first round of sorts: when every two neighbours inside a segment
+// are in order along every axis, the later rounds move nothing, and what is
+// left of them is the gaps along each axis between neighbours: they enter flag
+// here and the rounds are skipped.  (The copies of a vertex usually carry the
+// same bits, so its segment is in order along every axis.)  unsettled: some
+// pair is out of order; flag2 is then ignored.
+__global__ void k_gc_settle(const int *__restrict__ ord, const double *__restrict__ x0,
+                            const double *__restrict__ x1, const double *__restrict__ x2,
+                            const double *__restrict__ dx, const int *__restrict__ flag, ll np,
+                            int ndim, double tol2, int *__restrict__ flag2,
+                            int *__restrict__ unsettled) {
+  const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  double v[4] = {0.0, 0.0, 0.0, 0.0}, l[4];
+  auto load = [&](ll i, double *o) {
+    const int p = ord[i];
+    o[0] = x0[p], o[1] = x1[p], o[2] = ndim == 3 ? x2[p] : 0.0, o[3] = dx[p];
+  };
+  if (j < np) load(j, v);
+#pragma unroll
+  for (int q = 0; q < 4; q++) l[q] = __shfl_up_sync(0xffffffffu, v[q], 1);
+  bool bad = false;
+  if (j < np) {
+    if (lane == 0 && j > 0) load(j - 1, l);
+    int f = flag[j];
+    if (!f) {
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        if (q >= ndim) break;
+        if (ordered_key(l[q]) > ordered_key(v[q])) bad = true;
+        // (equal coordinates have no gap unless the distance is not a number)
+        if (__double_as_longlong(l[q]) != __double_as_longlong(v[q]) || nan_bits(v[q]))
+          if (gap_between(dsq(v[q], l[q]), v[3], l[3], tol2)) f = 1;
+      }
+    }
+    flag2[j] = f;
+  }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) *unsettled = 1;
 }
 
-__global__ void k_ids(const int *__restrict__ ord, const ll *__restrict__ segid,
-                      ll np, ll *__restrict__ ids) {
-  ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < np) ids[ord[i]] = segid[i];
+// Segment of every position from the start flags (flag[0] is set): tile sums,
+// their scan by one block, and the tiles again.  The segments' starts come
+// out with it; the longest one needs them (k_max_len).
+constexpr int GS_THREADS = 256, GS_ITEMS = 16, GS_TILE = GS_THREADS * GS_ITEMS;
+__device__ __forceinline__ int gs_block_excl(int v, int *total) {
+  __shared__ int ws[GS_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) ws[warp] = x;
+  __syncthreads();
+  int before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < GS_THREADS / 32; w++) {
+    if (w < warp) before += ws[w];
+    all += ws[w];
+  }
+  __syncthreads();
+  *total = all;
+  return before + x - v;
+}
+// the flags of a warp's GS_ITEMS words of 32 positions, and their number
+__device__ __forceinline__ int gs_words(const int *__restrict__ flag, ll i0, ll np, u32 *w) {
+  int c = 0;
+#pragma unroll
+  for (int r = 0; r < GS_ITEMS; r++) {
+    const ll i = i0 + r * 32 + (threadIdx.x & 31);
+    w[r] = __ballot_sync(0xffffffffu, i < np && flag[i] != 0);
+    c += __popc(w[r]);
+  }
+  return c;
+}
+__global__ void __launch_bounds__(GS_THREADS)
+k_gs_sums(const int *__restrict__ flag, ll np, int *__restrict__ bsum) {
+  u32 w[GS_ITEMS];
+  const ll i0 = (ll)blockIdx.x * GS_TILE + (threadIdx.x >> 5) * (32 * GS_ITEMS);
+  const int c = gs_words(flag, i0, np, w);
+  int total;
+  gs_block_excl((threadIdx.x & 31) == 0 ? c : 0, &total);
+  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(GS_THREADS)
+k_gs_scan(int *__restrict__ bsum, int nb, int *__restrict__ out) {
+  int run = 0;
+  for (int b = 0; b < nb; b += GS_THREADS) {
+    const int i = b + threadIdx.x;
+    const int v = i < nb ? bsum[i] : 0;
+    int total;
+    const int ex = gs_block_excl(v, &total);
+    if (i < nb) bsum[i] = run + ex;
+    run += total;
+  }
+  if (threadIdx.x == 0) out[0] = run, out[1] = 0;  // segments; longest one (k_max_len)
+}
+__global__ void __launch_bounds__(GS_THREADS)
+k_gs_write(const int *__restrict__ flag, ll np, const int *__restrict__ bsum,
+           int *__restrict__ seg, int *__restrict__ seg_start) {
+  u32 w[GS_ITEMS];
+  const int lane = threadIdx.x & 31;
+  const ll i0 = (ll)blockIdx.x * GS_TILE + (threadIdx.x >> 5) * (32 * GS_ITEMS);
+  const int c = gs_words(flag, i0, np, w);
+  int total;
+  const int before = gs_block_excl(lane == 0 ? c : 0, &total);
+  int run = bsum[blockIdx.x] + __shfl_sync(0xffffffffu, before, 0);
+#pragma unroll
+  for (int r = 0; r < GS_ITEMS; r++) {
+    const ll i = i0 + r * 32 + lane;
+    const int s = run + __popc(w[r] & (0xFFFFFFFFu >> (31 - lane))) - 1;
+    run += __popc(w[r]);
+    if (i >= np) continue;
+    seg[i] = s;
+    if ((w[r] >> lane) & 1u) seg_start[s] = (int)i;
+  }
+}
+__global__ void k_max_len(const int *__restrict__ seg_start, int *__restrict__ nseg_max, ll np) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = nseg_max[0];
+  int len = 0;
+  if (i < n) len = (int)((i + 1 < n ? seg_start[i + 1] : np) - seg_start[i]);
+  len = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
+  if ((threadIdx.x & 31) == 0 && len > nseg_max[1]) atomicMax(&nseg_max[1], len);
 }
 
-__global__ void k_seg_starts(const int *__restrict__ flag, const ll *__restrict__ segid,
-                             ll np, ll nseg, ll *__restrict__ seg_start) {
+__global__ void k_ids(const int *__restrict__ ord, const int *__restrict__ seg,
+                      ll np, ll *__restrict__ ids, int *__restrict__ ids32) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < np && flag[i]) seg_start[segid[i]] = i;
-  if (i == np - 1) seg_start[nseg] = np;
+  if (i >= np) return;
+  const int p = ord[i], s = seg[i];
+  ids[p] = s;
+  ids32[p] = s;
 }
 
-__global__ void k_element_check(const ll *__restrict__ ids, ll nel, int nv,
+__global__ void k_element_check(const int *__restrict__ ids, ll nel, int nv,
                                 int *__restrict__ err) {
   ll e = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
-  ll g[8];
+  int g[8];
   for (int k = 0; k < nv; k++) g[k] = ids[e * nv + k];
   for (int a = 0; a < nv; a++)
     for (int b = a + 1; b < nv; b++)
@@ -136,39 +306,68 @@ __global__ void k_element_check(const ll *__restrict__ ids, ll nel, int nv,
 // face_check: an element e that contains exactly 3 of the 4 corners of a
 // face of element i is an error.  Candidates e are the elements sharing a
 // vertex with i (the points of i's vertex segments); e is examined once, at
-// the lowest corner of i that it contains.
-__global__ void k_face_check(const ll *__restrict__ ids, const int *__restrict__ ord,
-                             const ll *__restrict__ seg_start, ll nseg, ll nel,
-                             int *__restrict__ err) {
-  ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nel) return;
-  const int nv = 8;
-  ll gi[8];
-  for (int k = 0; k < nv; k++) gi[k] = ids[i * nv + k];
-  for (int k = 0; k < nv; k++) {
-    ll s = gi[k];
-    ll b = seg_start[s], e = seg_start[s + 1];
-    for (ll q = b; q < e; q++) {
-      ll el = ord[q] / nv;
-      unsigned mask = 0;
-      for (int a = 0; a < nv; a++) {
-        ll ga = ids[el * nv + a];
-        for (int c = 0; c < nv; c++)
-          if (ga == gi[c]) mask |= 1u << c;
-      }
-      if ((__ffs(mask) - 1) != k) continue;  // seen at a lower corner
-      for (int f = 0; f < 6; f++)
-        if (__popc(mask & c_face_mask3[f]) == 3) {
-          atomicOr(err, 1);
-          return;
-        }
+// the lowest corner of i that it contains.  A thread per element and corner
+// (32-bit ids, a sector per candidate): 1.17 -> 0.52 ms per million hexes
+// against a thread per element on 64-bit ids.
+__global__ void __launch_bounds__(256)
+k_face_check(const int *__restrict__ ids, const int *__restrict__ ord,
+             const int *__restrict__ seg_start, int nseg, ll np, int *__restrict__ err) {
+  const ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= np) return;
+  const int k = (int)(p & 7);
+  int gi[8];
+  const int4 *row = reinterpret_cast<const int4 *>(ids + (p & ~7ll));
+  const int4 a = row[0], b = row[1];
+  gi[0] = a.x, gi[1] = a.y, gi[2] = a.z, gi[3] = a.w;
+  gi[4] = b.x, gi[5] = b.y, gi[6] = b.z, gi[7] = b.w;
+  const int s = ids[p];
+  const int q1 = s + 1 < nseg ? seg_start[s + 1] : (int)np;
+  for (int q = seg_start[s]; q < q1; q++) {
+    const ll el = ord[q] >> 3;
+    if (el == (p >> 3)) continue;  // (holds all four corners of every face)
+    const int4 *er = reinterpret_cast<const int4 *>(ids + el * 8);
+    const int4 c = er[0], d = er[1];
+    const int g[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+    unsigned mask = 0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      bool in = false;
+#pragma unroll
+      for (int v = 0; v < 8; v++) in = in || g[v] == gi[u];
+      mask |= in ? 1u << u : 0u;
     }
+    if ((__ffs(mask) - 1) != k) continue;  // seen at a lower corner
+    for (int f = 0; f < 6; f++)
+      if (__popc(mask & c_face_mask3[f]) == 3) {
+        atomicOr(err, 1);
+        return;
+      }
   }
 }
 
 __global__ void k_plus_one(const ll *__restrict__ ids, ll n, long long *__restrict__ out) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = ids[i] + 1;
+}
+
+// segments of the positions from the start flags: seg, seg_start, their
+// number and the longest one
+void segments_of(GenconWs &ws, const int *flag, ll np, ll *nseg, ll *longest) {
+  cudaStream_t st = ctx().stream;
+  const int nb = (int)((np + GS_TILE - 1) / GS_TILE);
+  ws.bsum.ensure((size_t)nb);
+  k_gs_sums<<<nb, GS_THREADS, 0, st>>>(flag, np, ws.bsum.p);
+  CK_LAUNCH();
+  k_gs_scan<<<1, GS_THREADS, 0, st>>>(ws.bsum.p, nb, ws.nseg_max.p);
+  CK_LAUNCH();
+  k_gs_write<<<nb, GS_THREADS, 0, st>>>(flag, np, ws.bsum.p, ws.seg.p, ws.seg_start.p);
+  CK_LAUNCH();
+  k_max_len<<<grid_for(np, 256), 256, 0, st>>>(ws.seg_start.p, ws.nseg_max.p, np);
+  CK_LAUNCH();
+  int h[2];
+  d2h(h, ws.nseg_max.p, 2);
+  sync();
+  *nseg = h[0], *longest = h[1];
 }
 
 }  // namespace
@@ -182,69 +381,81 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     if (nseg_out) *nseg_out = 0;
     return PARRSB_OK;
   }
+  if (np > 0x7FFFFFFFll) throw ArgError{PARRSB_ERR_UNSUPPORTED, "more than 2^31 corners"};
   for (int d = 0; d < 3; d++) ws.x[d].ensure((size_t)np);
   ws.dx.ensure((size_t)np);
   ws.keys.ensure((size_t)np);
   ws.ord.ensure((size_t)np);
   ws.flag.ensure((size_t)np);
-  ws.segid.ensure((size_t)np + 1);
-  ws.seg_of_pt.ensure((size_t)np);
+  ws.flag2.ensure((size_t)np);
+  ws.seg.ensure((size_t)np);
+  ws.seg_start.ensure((size_t)np);
+  ws.nseg_max.ensure(2);
   ws.ids.ensure((size_t)np);
-  ws.vals.ensure((size_t)np);
-  k_points<<<grid_for(nel, 128), 128, 0, st>>>(d_coord, nel, ndim, ws.x[0].p, ws.x[1].p,
-                                               ws.x[2].p, ws.dx.p);
-  CK_LAUNCH();
+  ws.ids32.ensure((size_t)np);
+  {
+    const size_t smem = (size_t)GP_ELEMS * (nv * ndim + 1) * sizeof(double);
+    const unsigned nb = grid_for(nel, GP_ELEMS);
+    if (ndim == 2)
+      k_points<2><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.x[0].p, ws.x[1].p, ws.x[2].p,
+                                              ws.dx.p);
+    else
+      k_points<3><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.x[0].p, ws.x[1].p, ws.x[2].p,
+                                              ws.dx.p);
+    CK_LAUNCH();
+  }
   k_iota<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, np);
   CK_LAUNCH();
   double tol2 = tol * tol;
-  ll nseg = 1;
+  ll nseg = 1, longest = np;
+  DBuf<int> err(2);
+  CK(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), st));
   for (int t = 0; t < ndim; t++) {
-    for (int d = 0; d < ndim; d++) {
-      bool first = (t == 0 && d == 0);
-      k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[d].p, ws.segid.p, np,
-                                                   ws.keys.p, ws.vals.p,
-                                                   first ? nullptr : ws.seg_of_pt.p);
+    if (t == 1) {
+      // nothing left to sort: the later rounds' gaps at once
+      k_gc_settle<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[0].p, ws.x[1].p, ws.x[2].p,
+                                                     ws.dx.p, ws.flag.p, np, ndim, tol2,
+                                                     ws.flag2.p, err.p + 1);
       CK_LAUNCH();
-      seg_sort_pairs(ws.keys, ws.vals, np, first ? nullptr : ws.seg_of_pt.p, nseg,
-                     ws.sort);
-      std::swap(ws.ord.p, ws.vals.p);
-      std::swap(ws.ord.n, ws.vals.n);
-      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[d].p, ws.dx.p, np, tol2,
+      int unsettled = 0;
+      d2h(&unsettled, err.p + 1, 1);
+      sync();
+      if (!unsettled) {
+        std::swap(ws.flag, ws.flag2);
+        segments_of(ws, ws.flag.p, np, &nseg, &longest);
+        break;
+      }
+    }
+    for (int d = 0; d < ndim; d++) {
+      const bool first = t == 0 && d == 0;
+      if (!first && longest <= 1) continue;  // no two points left to compare
+      k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[d].p, np, ws.keys.p);
+      CK_LAUNCH();
+      sort_by_value(ws.keys, ws.ord, np, first ? nullptr : ws.seg.p, nseg, longest, ws.sort);
+      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.keys.p, ws.dx.p, np, tol2,
                                                 first ? 1 : 0, ws.flag.p);
       CK_LAUNCH();
-      ll total = exclusive_scan_int_to_ll(ws.flag.p, ws.segid.p, np);
-      k_segid<<<grid_for(np, 256), 256, 0, st>>>(ws.flag.p, ws.segid.p, np);
-      CK_LAUNCH();
-      nseg = total;
+      segments_of(ws, ws.flag.p, np, &nseg, &longest);
     }
   }
   if (nseg_out) *nseg_out = nseg;
-  k_ids<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.segid.p, np, ws.ids.p);
+  k_ids<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.seg.p, np, ws.ids.p, ws.ids32.p);
   CK_LAUNCH();
   if (d_ids_out)
     CK(cudaMemcpyAsync(d_ids_out, ws.ids.p, np * sizeof(ll), cudaMemcpyDeviceToDevice, st));
-  DBuf<int> err(1);
-  CK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
   {
     StageTimer tm(PARRSB_STAGE_CHECK);
-    k_element_check<<<grid_for(nel, 256), 256, 0, st>>>(ws.ids.p, nel, nv, err.p);
+    k_element_check<<<grid_for(nel, 256), 256, 0, st>>>(ws.ids32.p, nel, nv, err.p);
     CK_LAUNCH();
+    if (ndim == 3) {  // in 2D an edge has two corners: a count of 3 is impossible
+      k_face_check<<<grid_for(np, 256), 256, 0, st>>>(ws.ids32.p, ws.ord.p, ws.seg_start.p,
+                                                      (int)nseg, np, err.p);
+      CK_LAUNCH();
+    }
     int h_err = 0;
     d2h(&h_err, err.p, 1);
     sync();
     if (h_err) return 1;
-    if (ndim == 3) {  // in 2D an edge has two corners: a count of 3 is impossible
-      DBuf<ll> seg_start((size_t)nseg + 1);
-      k_seg_starts<<<grid_for(np, 256), 256, 0, st>>>(ws.flag.p, ws.segid.p, np, nseg,
-                                                      seg_start.p);
-      CK_LAUNCH();
-      k_face_check<<<grid_for(nel, 128), 128, 0, st>>>(ws.ids.p, ws.ord.p, seg_start.p,
-                                                       nseg, nel, err.p);
-      CK_LAUNCH();
-      d2h(&h_err, err.p, 1);
-      sync();
-      if (h_err) return 1;
-    }
   }
   if (d_vtx) {
     k_plus_one<<<grid_for(np, 256), 256, 0, st>>>(ws.ids.p, np, d_vtx);

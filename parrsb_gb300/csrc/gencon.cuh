@@ -9,8 +9,11 @@ struct GenconWs {
   SortWs sort;
   DBuf<double> x[3], dx;
   DBuf<u64> keys;
-  DBuf<int> ord, vals, flag, seg_of_pt;
-  DBuf<ll> segid, ids;
+  DBuf<int> ord, flag, flag2;
+  DBuf<int> seg, seg_start, bsum;  // segment of every position, first position of each
+  DBuf<int> nseg_max;              // number of segments, longest one
+  DBuf<ll> ids;
+  DBuf<int> ids32;
 };
 
 // Device-resident gencon.  d_coord: nel*nv*ndim corner coordinates in

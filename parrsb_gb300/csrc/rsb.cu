@@ -4058,7 +4058,8 @@ __global__ void k_fied_keys(const double *__restrict__ f_pos, const int *__restr
                             ll N, u64 *__restrict__ keys, int *__restrict__ vals) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  keys[i] = grp[i] >= 0 ? ordered_key(f_pos[i]) : 0ull;
+  // (positions outside the groups keep their order: one value, that of 0.0)
+  keys[i] = grp[i] >= 0 ? ordered_key(f_pos[i]) : 0x8000000000000000ull;
   vals[i] = (int)i;
 }
 
@@ -5083,7 +5084,9 @@ static void rsb_impl(const long long *d_vtx, const double *cent, ll N, int nv, i
       StageTimer tm(PARRSB_STAGE_SORT);
       k_fied_keys<<<grid_for(N, 256), 256, 0, st>>>(f_pos.p, grp.p, N, keys.p, vals.p);
       CK_LAUNCH();
-      seg_sort_pairs(keys, vals, N, segpos.p, (ll)groups.size(), sws);
+      ll longest = 1;
+      for (ll n : all_n) longest = std::max(longest, n);
+      sort_by_value(keys, vals, N, segpos.p, (ll)groups.size(), longest, sws);
       k_gather_perm<<<grid_for(N, 256), 256, 0, st>>>(vals.p, perm.p, f_pos.p, N, perm2.p,
                                                       f_tmp.p);
       CK_LAUNCH();

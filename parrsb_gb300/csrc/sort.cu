@@ -14,6 +14,8 @@
 // digit order and writes each digit's run with consecutive addresses.  One
 // up-front kernel builds the global digit histograms of every pass; passes
 // whose digit is constant over all items are skipped.
+#include <algorithm>
+
 #include "sort.cuh"
 
 namespace prsb {
@@ -249,6 +251,462 @@ k_scatter(const u64 *__restrict__ kin, const int *__restrict__ vin,
   }
 }
 
+// ---------------------------------------------------------------------------
+// Sort of doubles inside contiguous segments (sort_by_value).  The segments
+// tile the positions, so they never move and need no digit passes of their
+// own; what remains depends on the longest one:
+//   up to RANK_MAX      every item counts the items of its segment before it
+//   up to LOCAL_MAX     a CTA sorts whole segments in shared memory (bitonic,
+//                       ties by position, which makes it stable)
+//   longer              four radix passes over 32-bit keys (segment, then the
+//                       value in fixed point over the range of all values),
+//                       half the bytes and half the passes of the 64-bit keys;
+//                       the few items that share a 32-bit key are then put
+//                       right by their full keys (k_fix_runs), long runs (a
+//                       value that many items share, and one beside it) by a
+//                       CTA each.  Runs too long or too many for that (many
+//                       values that differ in their last bits only) take the
+//                       full radix sort.
+// ---------------------------------------------------------------------------
+constexpr int RANK_MAX = 32;
+constexpr int RANK_THREADS = 512;
+constexpr int LOCAL_MAX = 8192;
+constexpr int FIX_MAX = 32;  // items of a run that one thread puts right
+constexpr int RUN_LIST = 1024;  // longer runs that CTAs put right
+
+// keys[i], vals[i] of the segments of at most RANK_MAX items, out of place.
+// The CTA sees its positions and RANK_MAX more on both sides.
+__global__ void __launch_bounds__(RANK_THREADS)
+k_seg_rank(const u64 *__restrict__ keys, const int *__restrict__ vals,
+           const int *__restrict__ seg, ll n, u64 *__restrict__ kout, int *__restrict__ vout) {
+  constexpr int W = RANK_THREADS + 2 * RANK_MAX;
+  __shared__ u64 sk[W];
+  __shared__ int ss[W];
+  const ll base = (ll)blockIdx.x * RANK_THREADS - RANK_MAX;
+  for (int k = threadIdx.x; k < W; k += RANK_THREADS) {
+    const ll i = base + k;
+    const bool in = i >= 0 && i < n;
+    sk[k] = in ? keys[i] : 0ull;
+    ss[k] = in ? seg[i] : -1 - (i < 0 ? 0 : 1);
+  }
+  __syncthreads();
+  const int me = threadIdx.x + RANK_MAX;
+  const ll i = base + me;
+  if (i >= n) return;
+  const u64 key = sk[me];
+  const int s = ss[me];
+  int before = 0, j = me - 1;
+  for (; j >= 0 && ss[j] == s; j--) before += sk[j] <= key;
+  const int first = j + 1;
+  for (j = me + 1; j < W && ss[j] == s; j++) before += sk[j] < key;
+  const ll to = base + first + before;
+  kout[to] = key;
+  vout[to] = vals[i];
+}
+
+// Segments of at most W / 2 items: CTA b sorts those that start in
+// [b W / 2, (b + 1) W / 2), in place.  Bitonic network over (segment, key,
+// place); H = W / 2.
+// (one item of padding per eight, against bank conflicts)
+__host__ __device__ constexpr int lo_at(int i) { return i + (i >> 3); }
+constexpr size_t local_smem(int w) { return (size_t)lo_at(w) * 12; }
+struct LoItem {
+  u64 k;
+  u32 p;  // segment above bit 16, place below (ties by place)
+};
+__device__ __forceinline__ void lo_exchange(LoItem &a, LoItem &b, bool up) {
+  const u32 ga = a.p >> 16, gb = b.p >> 16;
+  const bool gt = ga != gb ? ga > gb : (a.k != b.k ? a.k > b.k : a.p > b.p);
+  if (gt == up) {
+    const LoItem t = a;
+    a = b;
+    b = t;
+  }
+}
+// K strides of the network, st, st / 2, ..., at once: a thread keeps the 2^K
+// items they connect in registers, so a pass over shared memory does three
+// steps instead of one (32 segments of 8192 items: 116 -> 96 us)
+template <int THREADS, int K>
+__device__ __forceinline__ void lo_steps(u64 *sk, u32 *sp, int p2, int size, int st) {
+  const int lo = st >> (K - 1);
+  for (int u = threadIdx.x; u < p2 >> K; u += THREADS) {
+    const int low = u & (lo - 1), base = ((u - low) << K) + low;
+    const bool up = (base & size) == 0;
+    LoItem v[1 << K];
+#pragma unroll
+    for (int j = 0; j < 1 << K; j++) {
+      const int i = lo_at(base + j * lo);
+      v[j].k = sk[i], v[j].p = sp[i];
+    }
+#pragma unroll
+    for (int b = K - 1; b >= 0; b--)
+#pragma unroll
+      for (int j = 0; j < 1 << K; j++)
+        if (!(j & (1 << b))) lo_exchange(v[j], v[j | (1 << b)], up);
+#pragma unroll
+    for (int j = 0; j < 1 << K; j++) {
+      const int i = lo_at(base + j * lo);
+      sk[i] = v[j].k, sp[i] = v[j].p;
+    }
+  }
+  __syncthreads();
+}
+// p2 (a power of two) items in shared memory, by the whole CTA
+template <int THREADS>
+__device__ __forceinline__ void bitonic_sort(u64 *sk, u32 *sp, int p2) {
+  for (int size = 2; size <= p2; size <<= 1) {
+    int st = size >> 1;
+    for (; st >= 4; st >>= 3) lo_steps<THREADS, 3>(sk, sp, p2, size, st);
+    if (st == 2)
+      lo_steps<THREADS, 2>(sk, sp, p2, size, st);
+    else if (st == 1)
+      lo_steps<THREADS, 1>(sk, sp, p2, size, st);
+  }
+}
+// the sorted items out: keys from sk, values moved from their old places
+template <int W, int THREADS>
+__device__ __forceinline__ void local_store(const u64 *sk, const u32 *sp, int m,
+                                            u64 *__restrict__ keys, int *__restrict__ vals) {
+  int v[W / THREADS];
+#pragma unroll
+  for (int r = 0; r < W / THREADS; r++) {
+    const int k = threadIdx.x + r * THREADS;
+    v[r] = k < m ? vals[sp[lo_at(k)] & 0xFFFFu] : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < W / THREADS; r++) {
+    const int k = threadIdx.x + r * THREADS;
+    if (k < m) keys[k] = sk[lo_at(k)], vals[k] = v[r];
+  }
+}
+template <int W, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+k_seg_local(u64 *__restrict__ keys, int *__restrict__ vals, const int *__restrict__ seg, ll n) {
+  constexpr int H = W / 2;
+  extern __shared__ __align__(16) unsigned char lo_smem[];
+  u64 *sk = reinterpret_cast<u64 *>(lo_smem);
+  u32 *sp = reinterpret_cast<u32 *>(sk + lo_at(W));
+  __shared__ int s_lo, s_hi;
+  const ll b0 = (ll)blockIdx.x * H;
+  if (threadIdx.x == 0) s_lo = 1 << 30, s_hi = 1 << 30;
+  __syncthreads();
+  // the first start at or after b0, and at or after b0 + H (else the end)
+  for (int k = threadIdx.x; k <= W; k += THREADS) {
+    const ll i = b0 + k;
+    if (i > n) break;
+    if (i == n || i == 0 || (seg ? seg[i] != seg[i - 1] : false)) {
+      if (k < H) atomicMin(&s_lo, k);
+      if (k >= H || i == n) atomicMin(&s_hi, k);
+    }
+  }
+  __syncthreads();
+  const int lo = s_lo, hi = s_hi;
+  const int m = hi - lo;
+  if (lo >= H || m <= 1 || m > W) return;
+  const ll i0 = b0 + lo;
+  const int seg0 = seg ? seg[i0] : 0;
+  int p2 = 2;
+  while (p2 < m) p2 <<= 1;
+  for (int k = threadIdx.x; k < p2; k += THREADS) {
+    sk[lo_at(k)] = k < m ? keys[i0 + k] : ~0ull;
+    sp[lo_at(k)] = k < m ? (u32)(seg ? seg[i0 + k] - seg0 : 0) << 16 | (u32)k : 0xFFFF0000u | (u32)k;
+  }
+  __syncthreads();
+  bitonic_sort<THREADS>(sk, sp, p2);
+  local_store<W, THREADS>(sk, sp, m, keys + i0, vals + i0);
+}
+
+__global__ void k_range_init(u64 *__restrict__ range) {
+  range[0] = ~0ull, range[1] = 0ull, range[2] = 0ull, range[3] = 0ull;
+}
+__global__ void k_key_range(const u64 *__restrict__ keys, ll n, u64 *__restrict__ range) {
+  u64 mn = ~0ull, mx = 0ull;
+  const ll stride = (ll)gridDim.x * blockDim.x;
+  for (ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const u64 k = keys[i];
+    mn = k < mn ? k : mn;
+    mx = k > mx ? k : mx;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const u64 a = __shfl_xor_sync(0xffffffffu, mn, o), b = __shfl_xor_sync(0xffffffffu, mx, o);
+    mn = a < mn ? a : mn;
+    mx = b > mx ? b : mx;
+  }
+  __shared__ u64 smn[32], smx[32];
+  if ((threadIdx.x & 31) == 0) smn[threadIdx.x >> 5] = mn, smx[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+      mn = smn[w] < mn ? smn[w] : mn;
+      mx = smx[w] > mx ? smx[w] : mx;
+    }
+    atomicMin(&range[0], mn);
+    atomicMax(&range[1], mx);
+  }
+}
+
+// 62-bit fixed point of the double behind an ordered key, the unit 2^(em - 1084)
+// (truncated towards zero: non-decreasing in the value)
+__device__ __forceinline__ int key_exp(u64 k) {
+  const u64 b = (k >> 63) ? (k ^ 0x8000000000000000ull) : ~k;
+  return (int)((b >> 52) & 0x7FF);
+}
+__device__ __forceinline__ ll key_fixed(u64 k, int em) {
+  const bool neg = (k >> 63) == 0;
+  const u64 b = neg ? ~k : k ^ 0x8000000000000000ull;
+  const int e = (int)((b >> 52) & 0x7FF);
+  u64 m = b & 0xFFFFFFFFFFFFFull;
+  if (e) m |= 1ull << 52;
+  const int sh = em - (e ? e : 1);  // >= 0
+  m = sh < 63 ? (m << 9) >> sh : 0ull;
+  return neg ? -(ll)m : (ll)m;
+}
+
+// q[i] = segment (top sb bits), value over the range (32 - sb bits)
+__global__ void k_quant(const u64 *__restrict__ keys, const int *__restrict__ seg, ll n, int sb,
+                        const u64 *__restrict__ range, u32 *__restrict__ q,
+                        int *__restrict__ idx) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const u64 k0 = range[0], k1 = range[1];
+  const int em = max(1, max(key_exp(k0), key_exp(k1)));
+  const ll f0 = key_fixed(k0, em);
+  const u64 r = (u64)(key_fixed(k1, em) - f0);
+  const int s = max(0, 64 - __clzll((ll)r) - (32 - sb));
+  const u32 v = (u32)((u64)(key_fixed(keys[i], em) - f0) >> s);
+  q[i] = v | (seg && sb ? (u32)seg[i] << (32 - sb) : 0u);
+  idx[i] = (int)i;
+}
+
+__global__ void __launch_bounds__(SORT_THREADS)
+k_tile_hist32(const u32 *__restrict__ q, ll n, int shift, u32 *__restrict__ counts, int ntiles) {
+  __shared__ u32 h[NWARP][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < NWARP * 256; i += blockDim.x) (&h[0][0])[i] = 0;
+  __syncthreads();
+  const ll base = (ll)blockIdx.x * TILE + warp * (32 * ITEMS_PER_THREAD);
+  u32 d[ITEMS_PER_THREAD];
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++) {
+    const ll i = base + r * 32 + lane;
+    d[r] = i < n ? (q[i] >> shift) & 255u : 256u;
+  }
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++)
+    if (d[r] < 256) atomicAdd(&h[warp][d[r]], 1u);
+  __syncthreads();
+  for (int dd = threadIdx.x; dd < 256; dd += blockDim.x) {
+    u32 s = 0;
+#pragma unroll
+    for (int w = 0; w < NWARP; w++) s += h[w][dd];
+    counts[(ll)dd * ntiles + blockIdx.x] = s;
+  }
+}
+
+// k_scatter for 32-bit keys: a pair is one 8-byte word in shared memory
+__global__ void __launch_bounds__(SORT_THREADS)
+k_scatter32(const u32 *__restrict__ kin, const int *__restrict__ vin, u32 *__restrict__ kout,
+            int *__restrict__ vout, ll n, int shift, const u32 *__restrict__ counts,
+            const u32 *__restrict__ totals, int ntiles) {
+  __shared__ u32 wcnt[NWARP][256];
+  __shared__ u32 gbase[256];  // global place of a digit's first item of this tile, minus its local one
+  __shared__ u32 tl[256];
+  __shared__ u32 ws[8], ws2[8];
+  extern __shared__ __align__(16) unsigned char sc_smem[];
+  uint2 *st = reinterpret_cast<uint2 *>(sc_smem);  // TILE
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < NWARP * 256; i += blockDim.x) (&wcnt[0][0])[i] = 0;
+  u32 dbase = 0;
+  {
+    const u32 v = threadIdx.x < 256 ? totals[threadIdx.x] : 0u;
+    u32 x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (threadIdx.x < 256 && lane == 31) ws[warp] = x;
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      u32 off = 0;
+      for (int w = 0; w < warp; w++) off += ws[w];
+      dbase = off + x - v + counts[(ll)threadIdx.x * ntiles + blockIdx.x];
+    }
+  }
+  u32 key[ITEMS_PER_THREAD], rank[ITEMS_PER_THREAD];
+  int val[ITEMS_PER_THREAD];
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const ll base = (ll)blockIdx.x * TILE + warp * (32 * ITEMS_PER_THREAD);
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++) {
+    const ll i = base + r * 32 + lane;
+    key[r] = i < n ? kin[i] : 0u;
+    val[r] = i < n ? vin[i] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++) {
+    const bool valid = base + r * 32 + lane < n;
+    const u32 d = valid ? (key[r] >> shift) & 255u : 256u;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    u32 before = 0;
+    if (valid) before = wcnt[warp][d];
+    __syncwarp();
+    rank[r] = before + __popc(peers & lt_mask);
+    if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = before + __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  {
+    u32 run = 0;
+    if (threadIdx.x < 256) {
+      const int d = threadIdx.x;
+#pragma unroll
+      for (int w = 0; w < NWARP; w++) {
+        const u32 t = wcnt[w][d];
+        wcnt[w][d] = run;
+        run += t;
+      }
+    }
+    u32 x = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (threadIdx.x < 256 && lane == 31) ws2[warp] = x;
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      u32 off = 0;
+      for (int w = 0; w < warp; w++) off += ws2[w];
+      const u32 t0 = off + x - run;
+      tl[threadIdx.x] = t0;
+      gbase[threadIdx.x] = dbase - t0;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++)
+    if (base + r * 32 + lane < n) {
+      const u32 d = (key[r] >> shift) & 255u;
+      st[tl[d] + wcnt[warp][d] + rank[r]] = make_uint2(key[r], (u32)val[r]);
+    }
+  __syncthreads();
+  const ll t0 = (ll)blockIdx.x * TILE;
+  const int tn = (int)(n - t0 < TILE ? n - t0 : TILE);
+  for (int t = threadIdx.x; t < tn; t += blockDim.x) {
+    const uint2 kv = st[t];
+    const u32 pos = gbase[(kv.x >> shift) & 255u] + (u32)t;
+    kout[pos] = kv.x;
+    vout[pos] = (int)kv.y;
+  }
+}
+
+__global__ void k_gather_kv(const int *__restrict__ idx, const u64 *__restrict__ keys,
+                            const int *__restrict__ vals, ll n, u64 *__restrict__ kout,
+                            int *__restrict__ vout) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int j = idx[i];
+  kout[i] = keys[j];
+  vout[i] = vals[j];
+}
+
+__global__ void k_gather_val(const int *__restrict__ idx, const int *__restrict__ in, ll n,
+                             int *__restrict__ out) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = in[idx[i]];
+}
+__global__ void k_iota_pos(int *__restrict__ a, ll n) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) a[i] = (int)i;
+}
+
+// Runs of equal 32-bit keys into the order of their full keys: the thread of a
+// run's first item sorts a run of at most FIX_MAX by insertion (stable); of a
+// longer one every pair of neighbours is checked, and a run that is not in
+// order is listed once (mark, zero before the launch) for k_sort_run.
+// range[2]: a run cannot be listed; range[3]: runs listed.
+__device__ __forceinline__ ll run_bound(const u32 *__restrict__ q, ll n, u64 v) {
+  ll lo = 0, hi = n;  // first position with q >= v
+  while (lo < hi) {
+    const ll mid = (lo + hi) >> 1;
+    if ((u64)q[mid] < v)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+__device__ __forceinline__ void list_run(const u32 *__restrict__ q, ll n, u32 qi,
+                                         u64 *__restrict__ range, int *__restrict__ mark,
+                                         int2 *__restrict__ runs) {
+  if (*(volatile u64 *)&range[2]) return;
+  const ll b = run_bound(q, n, qi);
+  if (atomicExch(&mark[b], 1)) return;
+  const ll e = run_bound(q, n, (u64)qi + 1);
+  const u64 at = e - b <= LOCAL_MAX ? atomicAdd(&range[3], 1ull) : (u64)RUN_LIST;
+  if (at < RUN_LIST)
+    runs[at] = make_int2((int)b, (int)(e - b));
+  else
+    range[2] = 1ull;
+}
+__global__ void k_fix_runs(const u32 *__restrict__ q, ll n, u64 *__restrict__ keys,
+                           int *__restrict__ vals, u64 *__restrict__ range,
+                           int *__restrict__ mark, int2 *__restrict__ runs) {
+  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const u32 qi = q[i];
+  if (i > 0 && q[i - 1] == qi) {
+    if (i >= FIX_MAX && q[i - FIX_MAX] == qi && keys[i] < keys[i - 1])
+      list_run(q, n, qi, range, mark, runs);
+    return;
+  }
+  int len = 1;
+  bool sorted = true;
+  u64 prev = keys[i];
+  while (len <= FIX_MAX && i + len < n && q[i + len] == qi) {
+    const u64 k = keys[i + len];
+    sorted = sorted && prev <= k;
+    prev = k;
+    len++;
+  }
+  if (sorted) return;
+  if (len > FIX_MAX) {
+    list_run(q, n, qi, range, mark, runs);
+    return;
+  }
+  for (int a = 1; a < len; a++) {
+    const u64 k = keys[i + a];
+    const int v = vals[i + a];
+    int b = a;
+    while (b > 0 && keys[i + b - 1] > k) {
+      keys[i + b] = keys[i + b - 1];
+      vals[i + b] = vals[i + b - 1];
+      b--;
+    }
+    keys[i + b] = k;
+    vals[i + b] = v;
+  }
+}
+// one CTA per listed run
+__global__ void __launch_bounds__(1024)
+k_sort_run(const int2 *__restrict__ runs, u64 *__restrict__ keys, int *__restrict__ vals) {
+  extern __shared__ __align__(16) unsigned char lo_smem[];
+  u64 *sk = reinterpret_cast<u64 *>(lo_smem);
+  u32 *sp = reinterpret_cast<u32 *>(sk + lo_at(LOCAL_MAX));
+  const int2 r = runs[blockIdx.x];
+  int p2 = 2;
+  while (p2 < r.y) p2 <<= 1;
+  for (int k = threadIdx.x; k < p2; k += 1024) {
+    sk[lo_at(k)] = k < r.y ? keys[r.x + k] : ~0ull;
+    sp[lo_at(k)] = k < r.y ? (u32)k : 0xFFFF0000u | (u32)k;
+  }
+  __syncthreads();
+  bitonic_sort<1024>(sk, sp, p2);
+  local_store<LOCAL_MAX, 1024>(sk, sp, r.y, keys + r.x, vals + r.x);
+}
+
 int bits_for(ll nseg) {
   int b = 0;
   while (nseg > 1 && ((ll)1 << b) < nseg) b++;
@@ -310,6 +768,100 @@ void seg_sort_pairs(DBuf<u64> &keys, DBuf<int> &vals, ll n,
     std::swap(vals.p, ws.vtmp.p);
     std::swap(vals.n, ws.vtmp.n);
   }
+}
+
+void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos, ll nseg,
+                   ll max_len, SortWs &ws) {
+  if (n <= 1 || max_len <= 1) return;
+  cudaStream_t st = ctx().stream;
+  if (!seg_of_pos) nseg = 1;
+  if (seg_of_pos && max_len <= RANK_MAX) {
+    ws.ktmp.ensure((size_t)n);
+    ws.vtmp.ensure((size_t)n);
+    k_seg_rank<<<grid_for(n, RANK_THREADS), RANK_THREADS, 0, st>>>(keys.p, vals.p, seg_of_pos, n,
+                                                                   ws.ktmp.p, ws.vtmp.p);
+    CK_LAUNCH();
+    std::swap(keys, ws.ktmp);
+    std::swap(vals, ws.vtmp);
+    return;
+  }
+  if (max_len <= 1024) {
+    k_seg_local<2048, 256><<<grid_for(n, 1024), 256, local_smem(2048), st>>>(keys.p, vals.p,
+                                                                            seg_of_pos, n);
+    CK_LAUNCH();
+    return;
+  }
+  if (max_len <= LOCAL_MAX) {
+    auto kern = k_seg_local<2 * LOCAL_MAX, 1024>;
+    ensure_smem_limit(kern, (int)local_smem(2 * LOCAL_MAX));
+    kern<<<grid_for(n, LOCAL_MAX), 1024, local_smem(2 * LOCAL_MAX), st>>>(keys.p, vals.p,
+                                                                          seg_of_pos, n);
+    CK_LAUNCH();
+    return;
+  }
+  const int sb = bits_for(nseg);
+  bool full = sb > 16;  // too few bits left for the values
+  if (!full) {
+    ws.range.ensure(4);
+    ws.runs.ensure(RUN_LIST);
+    ws.q.ensure((size_t)n), ws.qtmp.ensure((size_t)n);
+    ws.idx.ensure((size_t)n), ws.idxtmp.ensure((size_t)n);
+    ws.ktmp.ensure((size_t)n), ws.vtmp.ensure((size_t)n);
+    const int ntiles = (int)((n + TILE - 1) / TILE);
+    ws.counts.ensure((size_t)256 * ntiles);
+    ws.totals.ensure(256);
+    k_range_init<<<1, 1, 0, st>>>(ws.range.p);
+    CK_LAUNCH();
+    k_key_range<<<(unsigned)std::min<ll>((n + 1023) / 1024, 152 * 4), 256, 0, st>>>(keys.p, n,
+                                                                                  ws.range.p);
+    CK_LAUNCH();
+    k_quant<<<grid_for(n, 256), 256, 0, st>>>(keys.p, seg_of_pos, n, sb, ws.range.p, ws.q.p,
+                                              ws.idx.p);
+    CK_LAUNCH();
+    ensure_smem_limit(k_scatter32, (int)(TILE * sizeof(uint2)));  // with the tables over 48 KB
+    for (int shift = 0; shift < 32; shift += 8) {
+      k_tile_hist32<<<ntiles, SORT_THREADS, 0, st>>>(ws.q.p, n, shift, ws.counts.p, ntiles);
+      CK_LAUNCH();
+      k_tile_scan<<<256, 1024, 0, st>>>(ws.counts.p, ntiles, ws.totals.p);
+      CK_LAUNCH();
+      k_scatter32<<<ntiles, SORT_THREADS, TILE * sizeof(uint2), st>>>(ws.q.p, ws.idx.p, ws.qtmp.p, ws.idxtmp.p, n,
+                                                   shift, ws.counts.p, ws.totals.p, ntiles);
+      CK_LAUNCH();
+      std::swap(ws.q, ws.qtmp);
+      std::swap(ws.idx, ws.idxtmp);
+    }
+    k_gather_kv<<<grid_for(n, 256), 256, 0, st>>>(ws.idx.p, keys.p, vals.p, n, ws.ktmp.p,
+                                                  ws.vtmp.p);
+    CK_LAUNCH();
+    CK(cudaMemsetAsync(ws.idxtmp.p, 0, (size_t)n * sizeof(int), st));
+    k_fix_runs<<<grid_for(n, 256), 256, 0, st>>>(ws.q.p, n, ws.ktmp.p, ws.vtmp.p, ws.range.p,
+                                                 ws.idxtmp.p, ws.runs.p);
+    CK_LAUNCH();
+    u64 said[2] = {0, 0};
+    d2h(said, ws.range.p + 2, 2);
+    sync();
+    full = said[0] != 0;
+    if (!full && said[1] > 0) {
+      ensure_smem_limit(k_sort_run, (int)local_smem(LOCAL_MAX));
+      k_sort_run<<<(unsigned)said[1], 1024, local_smem(LOCAL_MAX), st>>>(ws.runs.p, ws.ktmp.p,
+                                                                         ws.vtmp.p);
+      CK_LAUNCH();
+    }
+  }
+  if (!full) {
+    std::swap(keys, ws.ktmp);
+    std::swap(vals, ws.vtmp);
+    return;
+  }
+  // the full radix sort of (key, position), the segments by position
+  DBuf<int> pos((size_t)n);
+  k_iota_pos<<<grid_for(n, 256), 256, 0, st>>>(pos.p, n);
+  CK_LAUNCH();
+  seg_sort_pairs(keys, pos, n, seg_of_pos, nseg, ws);
+  ws.idx.ensure((size_t)n);
+  k_gather_val<<<grid_for(n, 256), 256, 0, st>>>(pos.p, vals.p, n, ws.idx.p);
+  CK_LAUNCH();
+  std::swap(vals, ws.idx);
 }
 
 }  // namespace prsb
