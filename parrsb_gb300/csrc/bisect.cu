@@ -14,6 +14,8 @@
 // to the CPU restatement's.  Group sums use the canonical 32-wide tile tree.
 #include <float.h>
 
+#include <algorithm>
+
 #include "bisect.cuh"
 
 #include <type_traits>
@@ -45,86 +47,141 @@ __device__ __forceinline__ bool seg_active(int p, ll n, int do_local) {
   return p > 1 || (do_local && p == 1 && n >= 2);
 }
 
-__device__ __forceinline__ ll find_seg(const ll *off, ll nseg, ll w) {
-  ll lo = 0, hi = nseg - 1;  // last s with off[s] <= w
-  while (lo < hi) {
-    ll mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= w)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
+// Two canonical shuffle trees (offsets 16 .. 1) in one: after the first step
+// the lanes of bit 4 carry the second value (a + b gives the same bits in
+// either order), so two sums take five additions of the warp instead of ten;
+// the FP64 pipe takes 16 cycles per warp instruction whatever its lanes do.
+// a's sum ends on lane 0, b's on lane 16.
+__device__ __forceinline__ double tree_pair(double a, double b) {
+  const bool up = (threadIdx.x & 16) != 0;
+  const double keep = up ? b : a, send = up ? a : b;
+  double v = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, 16));
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
+  return v;
 }
 
-// One warp per 32-item tile of a segment.  Level 0 generates values from
-// elements; later levels reduce the previous level's tile values.
-// Values are sums (canonical shuffle tree).
+// V sums per segment (even V): one block per 1024 consecutive items of a
+// segment takes two levels of the canonical 32-wide tree at once (a warp per
+// 32-item tile, then the first warp over the tiles); a segment's count shrinks
+// by 1024 per launch.  GEN_ARRAY reduces the previous launch's values.  Only
+// segments with cnt[s] > 0 take part; a segment that already has one value is
+// copied, not reduced again (the canonical tree stops at one value).
 template <int V, int GEN>
-__global__ void k_seg_tree(const int *__restrict__ perm,
-                           const double *__restrict__ cent, ll N,
-                           const ll *__restrict__ seg_start,
-                           const ll *__restrict__ seg_cnt,  // items per segment
-                           ll nseg, const ll *__restrict__ tile_off,
-                           ll ntiles, const double *__restrict__ in,
-                           const ll *__restrict__ in_off,
-                           const double *__restrict__ avg,
-                           double *__restrict__ out) {
-  ll w = ((ll)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (w >= ntiles) return;
-  ll s = find_seg(tile_off, nseg, w);
-  ll t = w - tile_off[s];
-  ll m = seg_cnt[s];
-  ll i = t * 32 + lane;
-  bool valid = i < m;
+__global__ void __launch_bounds__(1024)
+k_seg_tree(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
+           const ll *__restrict__ seg_start, const int *__restrict__ cnt, ll nseg,
+           const int *__restrict__ off, const double *__restrict__ in,
+           const int *__restrict__ in_off, const double *__restrict__ avg,
+           double *__restrict__ out) {
+  static_assert(V % 2 == 0, "sums are folded in pairs");
+  __shared__ double sv[V][32];
+  __shared__ int s_seg;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((int)blockIdx.x >= off[nseg]) return;
+  if (threadIdx.x == 0) {
+    ll lo = 0, hi = nseg - 1;  // last s with off[s] <= blockIdx.x
+    while (lo < hi) {
+      const ll mid = (lo + hi + 1) >> 1;
+      if (off[mid] <= (int)blockIdx.x)
+        lo = mid;
+      else
+        hi = mid - 1;
+    }
+    s_seg = (int)lo;
+  }
+  __syncthreads();
+  const int s = s_seg;
+  const int m = cnt[s], i = ((int)blockIdx.x - off[s]) * 1024 + (int)threadIdx.x;
   double v[V];
 #pragma unroll
   for (int q = 0; q < V; q++) v[q] = 0.0;
-  if (valid) {
+  if (i < m) {
     if (GEN == GEN_ARRAY) {
-      ll src = (in_off[s] + i) * V;
+      const ll src = ((ll)in_off[s] + i) * V;
 #pragma unroll
       for (int q = 0; q < V; q++) v[q] = in[src + q];
     } else {
-      int e = perm[seg_start[s] + i];
-      double c0 = cent[e], c1 = cent[N + e], c2 = cent[2 * N + e];
+      const int e = perm[seg_start[s] + i];
+      const double c0 = cent[e], c1 = cent[N + e], c2 = cent[2 * N + e];
       if (GEN == GEN_MEAN) {
-        v[0] = c0, v[1] = c1;
-        if (V > 2) v[V - 1] = c2;
+        v[0] = c0, v[1] = c1, v[2] = c2;
       } else {  // inertia products (00, 01, 02, 11, 12, 22)
         const double *a = avg + 3 * s;
-        double x = __dsub_rn(c0, a[0]), y = __dsub_rn(c1, a[1]),
-               z = __dsub_rn(c2, a[2]);
+        const double x = __dsub_rn(c0, a[0]), y = __dsub_rn(c1, a[1]), z = __dsub_rn(c2, a[2]);
         v[0] = __dmul_rn(x, x);
         v[1] = __dmul_rn(x, y);
-        if (V > 2) {
-          v[2] = __dmul_rn(x, z);
-          v[3] = __dmul_rn(y, y);
-          v[4] = __dmul_rn(y, z);
-          v[5] = __dmul_rn(z, z);
-        }
+        v[2] = __dmul_rn(x, z);
+        v[3] = __dmul_rn(y, y);
+        v[V - 2] = __dmul_rn(y, z);
+        v[V - 1] = __dmul_rn(z, z);
       }
     }
   }
-  // A segment whose previous level already produced a single value is
-  // copied, not reduced again (the canonical tree stops at one value).
-  bool copy_only = (GEN == GEN_ARRAY) && m == 1;
+  const int tiles = (m + 31) / 32;
+  if (GEN == GEN_ARRAY && m == 1) {  // copied
+    if (threadIdx.x == 0)
 #pragma unroll
-  for (int q = 0; q < V; q++) {
-    double r;
-    if (copy_only)
-      r = v[q];
-    else
-      r = warp_tree_sum(v[q]);
-    if (lane == 0) out[w * V + q] = r;
+      for (int q = 0; q < V; q++) out[(ll)blockIdx.x * V + q] = v[q];
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < V; q += 2) {
+    const double t = tree_pair(v[q], v[q + 1]);
+    if (lane == 0) sv[q][warp] = t;
+    if (lane == 16) sv[q + 1][warp] = t;
+  }
+  __syncthreads();
+  if (warp > 0) return;
+  const int mine = min(32, tiles - ((int)blockIdx.x - off[s]) * 32);  // tiles of this block
+#pragma unroll
+  for (int q = 0; q < V; q += 2) {
+    const double a = lane < mine ? sv[q][lane] : 0.0, b = lane < mine ? sv[q + 1][lane] : 0.0;
+    if (tiles == 1) {  // one value after the first level
+      if (lane == 0) out[(ll)blockIdx.x * V + q] = a, out[(ll)blockIdx.x * V + q + 1] = b;
+    } else {
+      const double t = tree_pair(a, b);
+      if (lane == 0) out[(ll)blockIdx.x * V + q] = t;
+      if (lane == 16) out[(ll)blockIdx.x * V + q + 1] = t;
+    }
   }
 }
 
-__global__ void k_tile_counts(const ll *__restrict__ cnt, ll nseg,
-                              ll *__restrict__ tiles) {
-  ll s = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nseg) tiles[s] = (cnt[s] + 31) / 32;
+// Tree launch l of a level reduces cnt_l[s] items of segment s (cnt_0: its
+// elements, 0 without ranks to split; then a value per block of the launch
+// before); off_l = exclusive scan of its blocks of 1024 items, off_l[nseg] all
+// of them.  All launches' tables at once, at tab + 2 l (nseg + 1).
+__global__ void __launch_bounds__(1024)
+k_tree_offsets(const ll *__restrict__ n, const int *__restrict__ p, ll nseg, int launches,
+               int *__restrict__ tab) {
+  __shared__ int ws[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int *cnt = tab + 2 * (ll)blockIdx.x * (nseg + 1), *off = cnt + nseg + 1;
+  int run = 0;
+  for (ll b = 0; b < nseg; b += 1024) {
+    const ll s = b + threadIdx.x;
+    int c = s < nseg && p[s] > 1 ? (int)n[s] : 0;
+    for (int l = 0; l < (int)blockIdx.x; l++) c = (c + 1023) / 1024;
+    if (s < nseg) cnt[s] = c;
+    const int v = (c + 1023) / 1024;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < 32; w++) {
+      if (w < warp) before += ws[w];
+      all += ws[w];
+    }
+    if (s < nseg) off[s] = run + before + x - v;
+    run += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) off[nseg] = run;
 }
 
 // RCB boxes on the dense coordinate ranks: per segment and axis the minimum
@@ -236,32 +293,42 @@ __global__ void k_rcb_axis_rank(const u32 *__restrict__ rbox, const double *__re
 }
 
 // Power iteration (fixed start vector (31, 17, 43)/50) on the first N*N
-// entries of the row-major 3x3 tensor, as power_serial reads it.
-__device__ void power_serial_dev(double *y, int N, const double *A) {
+// entries of the row-major 3x3 tensor, as power_serial reads it, by the four
+// lanes of a quad: lane j < N holds row j and y_j.  A dependent FP64
+// instruction takes 64 cycles and a division about 570, so the rows' products
+// run side by side and the two divisions of an iteration are one instruction
+// sequence: lanes 0..2 scale by 1 / |Ay| while lane 3 takes the relative
+// change of the eigenvalue.  Same operations in the same order per value as
+// the serial loop: 68 -> 45 us per level.  Every lane of the warp calls it;
+// quads that are done idle.
+__device__ double power_quad(bool active, int N, const double *A) {
+  const int j = threadIdx.x & 3, q0 = threadIdx.x & 28;
   const double start[3] = {31.0 / 50.0, 17.0 / 50.0, 43.0 / 50.0};
   double norm = 0.0;
-  for (int i = 0; i < N; i++) {
-    y[i] = start[i];
-    norm = __dadd_rn(norm, __dmul_rn(y[i], y[i]));
-  }
-  double normi = __ddiv_rn(1.0, __dsqrt_rn(norm));
-  for (int i = 0; i < N; i++) y[i] = __dmul_rn(y[i], normi);
-  double Ay[3];
-  double err = 1.0, lambda = 0.0;
+  for (int i = 0; i < N; i++) norm = __dadd_rn(norm, __dmul_rn(start[i], start[i]));
+  double y = __dmul_rn(j < N ? start[j < 3 ? j : 0] : 0.0, __ddiv_rn(1.0, __dsqrt_rn(norm)));
+  double lambda = 0.0;
+  bool run = active;
   for (int i = 0; i < 100; i++) {
-    norm = 0.0;
-    for (int j = 0; j < N; j++) {
-      Ay[j] = 0.0;
-      for (int k = 0; k < N; k++) Ay[j] = __dadd_rn(Ay[j], __dmul_rn(A[j * N + k], y[k]));
-      norm = __dadd_rn(norm, __dmul_rn(Ay[j], Ay[j]));
+    if (!__any_sync(0xffffffffu, run)) break;
+    double ay = 0.0;
+    for (int k = 0; k < N; k++) {
+      const double yk = __shfl_sync(0xffffffffu, y, q0 + k);
+      ay = __dadd_rn(ay, __dmul_rn(j < N ? A[j * N + k] : 0.0, yk));
     }
-    double sn = __dsqrt_rn(norm);
-    if (i > 0) err = __ddiv_rn(__dsub_rn(sn, lambda), lambda);
-    lambda = sn;
-    normi = __ddiv_rn(1.0, sn);
-    for (int j = 0; j < N; j++) y[j] = __dmul_rn(Ay[j], normi);
-    if (fabs(err) < 1e-12) break;
+    const double sq = __dmul_rn(ay, ay);
+    norm = 0.0;
+    for (int k = 0; k < N; k++) norm = __dadd_rn(norm, __shfl_sync(0xffffffffu, sq, q0 + k));
+    const double sn = __dsqrt_rn(norm);
+    const double d = __ddiv_rn(j == 3 ? __dsub_rn(sn, lambda) : 1.0, j == 3 ? lambda : sn);
+    const double err = i > 0 ? __shfl_sync(0xffffffffu, d, q0 + 3) : 1.0;
+    if (run) {
+      lambda = sn;
+      y = __dmul_rn(ay, d);
+      if (fabs(err) < 1e-12) run = false;
+    }
   }
+  return y;
 }
 
 // RIB axis per segment.  Group segments (p > 1) use the tree sums in
@@ -290,54 +357,51 @@ __global__ void k_rib_mean_local(const int *__restrict__ perm,
   avg[3 * s + 2] = __ddiv_rn(a2, dn);
 }
 
-__global__ void k_rib_mean_group(const double *__restrict__ sums,
+__global__ void k_rib_mean_group(const double *__restrict__ sums, const int *__restrict__ off,
                                  const ll *__restrict__ seg_n,
                                  const int *__restrict__ p, ll nseg,
                                  double *__restrict__ avg) {
   ll s = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg || p[s] <= 1) return;
   double dn = (double)seg_n[s];
-  for (int d = 0; d < 3; d++) avg[3 * s + d] = __ddiv_rn(sums[3 * s + d], dn);
+  for (int d = 0; d < 3; d++)  // (the sums of 4, the last one unused)
+    avg[3 * s + d] = __ddiv_rn(sums[4 * (ll)off[s] + d], dn);
 }
 
-__global__ void k_rib_axis(const int *__restrict__ perm,
-                           const double *__restrict__ cent, ll N,
-                           const ll *__restrict__ seg_start,
-                           const ll *__restrict__ seg_n,
-                           const int *__restrict__ p, ll nseg, int ndim,
-                           int do_local, const double *__restrict__ avg,
-                           const double *__restrict__ isums,
-                           double *__restrict__ ev, int *__restrict__ act) {
-  ll s = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  int active = seg_active(p[s], seg_n[s], do_local);
-  act[s] = active;
-  if (!active) return;
-  double I6[6];
-  if (p[s] > 1) {
-    for (int q = 0; q < 6; q++) I6[q] = isums[6 * s + q];
-  } else {
-    for (int q = 0; q < 6; q++) I6[q] = 0.0;
-    const double *a = avg + 3 * s;
-    ll st = seg_start[s], n = seg_n[s];
-    for (ll i = 0; i < n; i++) {
-      int e = perm[st + i];
-      double x = __dsub_rn(cent[e], a[0]), y = __dsub_rn(cent[N + e], a[1]),
-             z = __dsub_rn(cent[2 * N + e], a[2]);
-      I6[0] = __dadd_rn(I6[0], __dmul_rn(x, x));
-      I6[1] = __dadd_rn(I6[1], __dmul_rn(x, y));
-      I6[2] = __dadd_rn(I6[2], __dmul_rn(x, z));
-      I6[3] = __dadd_rn(I6[3], __dmul_rn(y, y));
-      I6[4] = __dadd_rn(I6[4], __dmul_rn(y, z));
-      I6[5] = __dadd_rn(I6[5], __dmul_rn(z, z));
+__global__ void __launch_bounds__(128)
+k_rib_axis(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
+           const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
+           const int *__restrict__ p, ll nseg, int ndim, int do_local,
+           const double *__restrict__ avg, const double *__restrict__ isums,
+           const int *__restrict__ off, double *__restrict__ ev, int *__restrict__ act) {
+  const ll s = ((ll)blockIdx.x * blockDim.x + threadIdx.x) >> 2;  // a quad per segment
+  const int j = threadIdx.x & 3;
+  const bool in = s < nseg;
+  const bool active = in && seg_active(p[in ? s : 0], seg_n[in ? s : 0], do_local);
+  if (in && j == 0) act[s] = active;
+  double I6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (active) {
+    if (p[s] > 1) {
+      for (int q = 0; q < 6; q++) I6[q] = isums[6 * (ll)off[s] + q];
+    } else {
+      const double *a = avg + 3 * s;
+      ll st = seg_start[s], n = seg_n[s];
+      for (ll i = 0; i < n; i++) {
+        int e = perm[st + i];
+        double x = __dsub_rn(cent[e], a[0]), y = __dsub_rn(cent[N + e], a[1]),
+               z = __dsub_rn(cent[2 * N + e], a[2]);
+        I6[0] = __dadd_rn(I6[0], __dmul_rn(x, x));
+        I6[1] = __dadd_rn(I6[1], __dmul_rn(x, y));
+        I6[2] = __dadd_rn(I6[2], __dmul_rn(x, z));
+        I6[3] = __dadd_rn(I6[3], __dmul_rn(y, y));
+        I6[4] = __dadd_rn(I6[4], __dmul_rn(y, z));
+        I6[5] = __dadd_rn(I6[5], __dmul_rn(z, z));
+      }
     }
   }
-  double I[9] = {I6[0], I6[1], I6[2], I6[1], I6[3], I6[4], I6[2], I6[4], I6[5]};
-  double y[3] = {0.0, 0.0, 0.0};
-  power_serial_dev(y, ndim, I);
-  ev[3 * s + 0] = y[0];
-  ev[3 * s + 1] = y[1];
-  ev[3 * s + 2] = ndim == 3 ? y[2] : 0.0;
+  const double I[9] = {I6[0], I6[1], I6[2], I6[1], I6[3], I6[4], I6[2], I6[4], I6[5]};
+  const double y = power_quad(active, ndim, I);
+  if (active && j < 3) ev[3 * s + j] = j < ndim ? y : 0.0;
 }
 
 template <int KIND>
@@ -346,12 +410,12 @@ __global__ void k_keys(const int *__restrict__ perm, const double *__restrict__ 
                        const int *__restrict__ axis_or_act,
                        const double *__restrict__ avg,
                        const double *__restrict__ ev, u64 *__restrict__ keys,
-                       int *__restrict__ vals, int *__restrict__ seg_of_elem) {
+                       int *__restrict__ vals) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int s = seg_of_pos[i];
   int e = perm[i];
-  u64 k = 0;
+  u64 k = 0x8000000000000000ull;  // (the key of 0.0: a segment that keeps its order)
   if (KIND == BISECT_RCB) {  // segment id above the dense rank of the coordinate
     int ax = axis_or_act[s];
     k = (u64)(unsigned)s << 32;
@@ -368,7 +432,6 @@ __global__ void k_keys(const int *__restrict__ perm, const double *__restrict__ 
   }
   keys[i] = k;
   vals[i] = e;
-  if (KIND != BISECT_RCB) seg_of_elem[e] = s;
 }
 
 __global__ void k_child_counts(const int *__restrict__ p, const ll *__restrict__ n,
@@ -908,54 +971,66 @@ k_rcb_small(int *__restrict__ perm, const u32 *__restrict__ rank,
     levels(std::false_type{});
 }
 
+// children of every segment; lc: active segments, those with more than one
+// rank, the largest active one, the largest of all
+__global__ void k_level_counts(const int *__restrict__ p, const ll *__restrict__ n, ll nseg,
+                               int do_local, int *__restrict__ cnt, unsigned *__restrict__ lc) {
+  const ll s = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned any = s < nseg ? (unsigned)n[s] : 0u;
+  const bool a = s < nseg && seg_active(p[s], n[s], do_local);
+  if (s < nseg) cnt[s] = a ? 2 : 1;
+  const unsigned na = __popc(__ballot_sync(0xffffffffu, a)),
+                 ng = __popc(__ballot_sync(0xffffffffu, s < nseg && p[s] > 1));
+  const unsigned ma = __reduce_max_sync(0xffffffffu, a ? any : 0u),
+                 mn = __reduce_max_sync(0xffffffffu, any);
+  if ((threadIdx.x & 31) == 0) {  // one atomic per warp and number
+    if (na) atomicAdd(&lc[0], na);
+    if (ng) atomicAdd(&lc[1], ng);
+    if (ma) atomicMax(&lc[2], ma);
+    if (mn) atomicMax(&lc[3], mn);
+  }
+}
+
 __global__ void k_max_active_n(const int *__restrict__ p, const ll *__restrict__ n, ll nseg,
                                int do_local, unsigned long long *__restrict__ mx) {
   ll s = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (s < nseg && seg_active(p[s], n[s], do_local)) atomicMax(mx, (unsigned long long)n[s]);
 }
 
-// Run the tile tree over every segment of `t` until one value per segment
-// is left; result in out_final (nseg * V values).
+inline int tree_launches(ll maxn) {
+  int l = 1;
+  for (; maxn > 1024; maxn = (maxn + 1023) / 1024) l++;
+  return l;
+}
+
+// Sums of V values over every segment with more than one rank (tables of
+// k_tree_offsets), in the canonical tree; the sums of segment s are at
+// off[s] V of the returned buffer.  No host wait: the launches cover the
+// largest possible number of blocks.
 template <int V, int GEN0>
-void seg_tree_reduce(const int *perm, const double *cent, ll N, SegTable &t,
-                     const double *avg, BisectWs &ws, double *out_final) {
+const double *seg_tree_reduce(const int *perm, const double *cent, ll N, SegTable &t,
+                              const double *avg, int launches, BisectWs &ws, const int **off_out) {
   cudaStream_t st = ctx().stream;
-  ll nseg = t.count;
-  DBuf<ll> cnt((size_t)nseg), off((size_t)nseg + 1), in_off((size_t)nseg + 1);
-  CK(cudaMemcpyAsync(cnt.p, t.n.p, nseg * sizeof(ll), cudaMemcpyDeviceToDevice, st));
-  const double *in = nullptr;
-  bool first = true;
+  const ll nseg = t.count;
   DBuf<double> *bufs[2] = {&ws.red_a, &ws.red_b};
-  int cur = 0;
-  for (int level = 0; level < 16; level++) {
-    DBuf<ll> tiles((size_t)nseg);
-    k_tile_counts<<<grid_for(nseg, 256), 256, 0, st>>>(cnt.p, nseg, tiles.p);
-    CK_LAUNCH();
-    ll ntiles = exclusive_scan_ll(tiles.p, off.p, nseg);
-    DBuf<double> &ob = *bufs[cur];
-    ob.ensure((size_t)ntiles * V);
-    unsigned blocks = grid_for(ntiles * 32, 256);
-    if (first)
-      k_seg_tree<V, GEN0><<<blocks, 256, 0, st>>>(perm, cent, N, t.start.p,
-                                                        cnt.p, nseg, off.p, ntiles,
-                                                        nullptr, nullptr, avg, ob.p);
+  ll items = N;
+  for (int l = 0; l < launches; l++) {
+    const int *cnt = ws.tree_tab.p + 2 * (ll)l * (nseg + 1), *off = cnt + nseg + 1;
+    const ll blocks = std::max<ll>(1, std::min<ll>(items, items / 1024 + nseg));  // at most
+    DBuf<double> &out = *bufs[l & 1];
+    out.ensure((size_t)blocks * V);
+    if (l == 0)
+      k_seg_tree<V, GEN0><<<(unsigned)blocks, 1024, 0, st>>>(perm, cent, N, t.start.p, cnt, nseg,
+                                                             off, nullptr, nullptr, avg, out.p);
     else
-      k_seg_tree<V, GEN_ARRAY><<<blocks, 256, 0, st>>>(
-          perm, cent, N, t.start.p, cnt.p, nseg, off.p, ntiles, in, in_off.p, avg,
-          ob.p);
+      k_seg_tree<V, GEN_ARRAY><<<(unsigned)blocks, 1024, 0, st>>>(
+          perm, cent, N, t.start.p, cnt, nseg, off, bufs[(l - 1) & 1]->p, off - 2 * (nseg + 1),
+          avg, out.p);
     CK_LAUNCH();
-    if (ntiles == nseg) {  // every segment has a single value
-      CK(cudaMemcpyAsync(out_final, ob.p, (size_t)nseg * V * sizeof(double),
-                         cudaMemcpyDeviceToDevice, st));
-      return;
-    }
-    in = ob.p;
-    CK(cudaMemcpyAsync(in_off.p, off.p, nseg * sizeof(ll), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(cnt.p, tiles.p, nseg * sizeof(ll), cudaMemcpyDeviceToDevice, st));
-    first = false;
-    cur ^= 1;
+    items = blocks;
+    *off_out = off;
   }
-  throw ArgError{PARRSB_ERR_CHECK, "tree reduction did not converge"};
+  return bufs[(launches - 1) & 1]->p;
 }
 
 }  // namespace
@@ -1687,8 +1762,7 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
   ws.seg_of_elem.ensure((size_t)N);
   ws.keys.ensure((size_t)N);
   ws.vals.ensure((size_t)N);
-  DBuf<int> nact_d(1);
-  DBuf<unsigned long long> maxn_d(1);
+  DBuf<unsigned> lc_d(4);  // k_level_counts
   const size_t small_smem = small_smem_bytes();
   // PARRSB_GPU_LEVEL_LOG=1: per-level times on stderr (synchronises)
   const bool level_log = getenv("PARRSB_GPU_LEVEL_LOG") != nullptr;
@@ -1714,7 +1788,7 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
     for (int a = 0; a < ndim; a++) {
       k_axis_keys<<<grid_for(N, 256), 256, 0, st>>>(cent, N, a, ws.keys.p, ws.vals.p);
       CK_LAUNCH();
-      seg_sort_pairs(ws.keys, ws.vals, N, nullptr, 1, ws.sort);
+      sort_by_value(ws.keys, ws.vals, N, nullptr, 1, N, ws.sort);
       k_rank_flags<<<grid_for(N, 256), 256, 0, st>>>(ws.keys.p, N, flag.p);
       CK_LAUNCH();
       const ll changes = exclusive_scan_int_to_ll(flag.p, excl.p, N);
@@ -1742,18 +1816,15 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
     ll nseg = t.count;
     // active segments, their largest size, and children counts
     ws.child_cnt.ensure((size_t)nseg);
-    CK(cudaMemsetAsync(nact_d.p, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(maxn_d.p, 0, sizeof(unsigned long long), st));
-    k_child_counts<<<grid_for(nseg, 256), 256, 0, st>>>(t.p.p, t.n.p, nseg, do_local,
-                                                        ws.child_cnt.p, nact_d.p);
+    CK(cudaMemsetAsync(lc_d.p, 0, 4 * sizeof(unsigned), st));
+    k_level_counts<<<grid_for(nseg, 256), 256, 0, st>>>(t.p.p, t.n.p, nseg, do_local,
+                                                        ws.child_cnt.p, lc_d.p);
     CK_LAUNCH();
-    k_max_active_n<<<grid_for(nseg, 256), 256, 0, st>>>(t.p.p, t.n.p, nseg, do_local, maxn_d.p);
-    CK_LAUNCH();
-    int nact = 0;
-    unsigned long long maxn = 0;
-    d2h(&nact, nact_d.p, 1);
-    d2h(&maxn, maxn_d.p, 1);
+    unsigned lc[4] = {0, 0, 0, 0};
+    d2h(lc, lc_d.p, 4);
     sync();
+    const int nact = (int)lc[0], ngroup = (int)lc[1];
+    const unsigned long long maxn = lc[2], maxn_any = lc[3];
     if (level_log && kind == BISECT_RCB) {  // time of the global levels so far
       CK(cudaEventRecord(lg_e1, st));
       CK(cudaEventSynchronize(lg_e1));
@@ -1816,43 +1887,53 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
       lg_mark(0);
       k_keys<BISECT_RCB><<<grid_for(N, 256), 256, 0, st>>>(
           perm.p, cent, ws.rank.p, N, ws.seg_of_pos.p, ws.axis.p, nullptr, nullptr, ws.keys.p,
-          ws.vals.p, ws.seg_of_elem.p);
+          ws.vals.p);
       CK_LAUNCH();
       lg_mark(1);
     } else {
-      DBuf<double> sums((size_t)nseg * 3), avg((size_t)nseg * 3),
-          isums((size_t)nseg * 6);
+      DBuf<double> avg((size_t)nseg * 3);
       ws.ev.ensure((size_t)nseg * 3);
-      seg_tree_reduce<3, GEN_MEAN>(perm.p, cent, N, t, nullptr, ws, sums.p);
-      k_rib_mean_group<<<grid_for(nseg, 256), 256, 0, st>>>(sums.p, t.n.p, t.p.p, nseg,
-                                                            avg.p);
-      CK_LAUNCH();
+      const int *off = nullptr;
+      const double *isums = nullptr;
+      const int launches = tree_launches((ll)maxn);
+      if (ngroup) {
+        ws.tree_tab.ensure((size_t)2 * launches * (nseg + 1));
+        k_tree_offsets<<<launches, 1024, 0, st>>>(t.n.p, t.p.p, nseg, launches, ws.tree_tab.p);
+        CK_LAUNCH();
+        const double *sums = seg_tree_reduce<4, GEN_MEAN>(perm.p, cent, N, t, nullptr, launches,
+                                                          ws, &off);
+        k_rib_mean_group<<<grid_for(nseg, 256), 256, 0, st>>>(sums, off, t.n.p, t.p.p, nseg,
+                                                              avg.p);
+        CK_LAUNCH();
+      }
       if (do_local) {
         k_rib_mean_local<<<grid_for(nseg, 128), 128, 0, st>>>(
             perm.p, cent, N, t.start.p, t.n.p, t.p.p, nseg, 1, avg.p);
         CK_LAUNCH();
       }
-      seg_tree_reduce<6, GEN_INERTIA>(perm.p, cent, N, t, avg.p, ws, isums.p);
-      k_rib_axis<<<grid_for(nseg, 128), 128, 0, st>>>(
+      if (ngroup)
+        isums = seg_tree_reduce<6, GEN_INERTIA>(perm.p, cent, N, t, avg.p, launches, ws, &off);
+      k_rib_axis<<<grid_for(4 * nseg, 128), 128, 0, st>>>(
           perm.p, cent, N, t.start.p, t.n.p, t.p.p, nseg, ndim, do_local ? 1 : 0,
-          avg.p, isums.p, ws.ev.p, ws.axis.p);
+          avg.p, isums, off, ws.ev.p, ws.axis.p);
       CK_LAUNCH();
       k_keys<BISECT_RIB><<<grid_for(N, 256), 256, 0, st>>>(
           perm.p, cent, nullptr, N, ws.seg_of_pos.p, ws.axis.p, avg.p, ws.ev.p, ws.keys.p,
-          ws.vals.p, ws.seg_of_elem.p);
+          ws.vals.p);
       CK_LAUNCH();
     }
     // RCB keys carry the segment id above the rank; RIB keys are full doubles
     if (kind == BISECT_RCB)
       seg_sort_pairs(ws.keys, ws.vals, N, nullptr, 1, ws.sort);
     else
-      seg_sort_pairs(ws.keys, ws.vals, N, ws.seg_of_elem.p, nseg, ws.sort);
+      sort_by_value(ws.keys, ws.vals, N, ws.seg_of_pos.p, nseg, (ll)maxn_any, ws.sort);
     lg_mark(2);
     std::swap(perm.p, ws.vals.p);
     std::swap(perm.n, ws.vals.n);
     // children
     ws.child_off.ensure((size_t)nseg + 1);
-    ll nchild = exclusive_scan_int_to_ll(ws.child_cnt.p, ws.child_off.p, nseg);
+    exclusive_scan_int_to_ll_async(ws.child_cnt.p, ws.child_off.p, nseg);
+    const ll nchild = nseg + nact;
     ws.t2.reserve(nchild);
     k_children<<<grid_for(nseg, 256), 256, 0, st>>>(
         t.start.p, t.n.p, t.p.p, t.r0.p, nseg, do_local, ws.child_off.p, ws.t2.start.p,

@@ -31,7 +31,8 @@ struct BisectWs {
   DBuf<int> vals;
   DBuf<int> seg_of_pos, seg_of_elem, axis;
   DBuf<double> red_a, red_b, ev;   // reduction partials, eigenvectors
-  DBuf<ll> tile_off, child_off;
+  DBuf<int> tree_tab;              // RIB sums: items and first block per segment and launch
+  DBuf<ll> child_off;
   DBuf<int> child_cnt;
   SegTable t2;
   // RCB: dense rank of every centroid coordinate per axis (3 x N) and the
