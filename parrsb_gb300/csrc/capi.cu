@@ -601,7 +601,7 @@ extern "C" int parrsb_conn_mesh(long long *vtx, double *coord, unsigned int nel,
       // periodic faces (src/con.c:261-264); without any, the consecutive
       // renumbering leaves the ids as they are
       StageTimer tm(PARRSB_STAGE_GENCON);
-      r = periodic_device(W.gc.ids.p, W.gc.x[0].p, W.gc.x[1].p, W.gc.x[2].p, nel, (int)nDim,
+      r = periodic_device(W.gc.ids.p, W.gc.pt.p, nel, (int)nDim,
                           nseg, periodicInfo, nPeriodicFaces, W.gc.sort, &nseg);
       ctx().stats.gencon_segments = nseg;
       if (r != PARRSB_OK) {

@@ -12,6 +12,8 @@
 // Every segmented sort is stable (the reference's per-segment heapsort,
 // src/con-unique-vertices.c:6-58, is replaced by the canonical stable order;
 // both give the same ids unless a split decision sits on an exact tie).
+#include <cmath>
+
 #include "gencon.cuh"
 
 namespace prsb {
@@ -40,7 +42,9 @@ __device__ __forceinline__ double min_sq(double m, double d) {
   return lt && !nan_bits(m) && !nan_bits(d) ? m : d;
 }
 
-// Points in symmetric order and their min squared neighbour distance.  A CTA
+// Points in symmetric order: coordinates and min squared neighbour distance,
+// one 32-byte sector a point (what a later pass gathers comes with one access,
+// whichever fields it needs).  A CTA
 // stages its elements' corners in shared memory (coalesced loads and stores:
 // 0.46 -> 0.26 ms per million hexes) and a thread takes an element: each of
 // the 12 edges (4 in 2D) is measured once for its two corners, since the FP64
@@ -48,8 +52,7 @@ __device__ __forceinline__ double min_sq(double m, double d) {
 constexpr int GP_ELEMS = 128;
 template <int NDIM>
 __global__ void __launch_bounds__(GP_ELEMS)
-k_points(const double *__restrict__ coord, ll nel, double *__restrict__ x0,
-         double *__restrict__ x1, double *__restrict__ x2, double *__restrict__ dx) {
+k_points(const double *__restrict__ coord, ll nel, double4_32a *__restrict__ pt) {
   constexpr int NV = NDIM == 2 ? 4 : 8, ROW = NV * NDIM;
   constexpr int PAD = ROW + 1;  // an element's row in shared memory
   extern __shared__ double gp[];
@@ -86,32 +89,24 @@ k_points(const double *__restrict__ coord, ll nel, double *__restrict__ x0,
           edge(NV - 3, NV - 1), edge(NV - 2, NV - 1);
   }
   __syncthreads();
-  // out through shared memory: the distances, then each coordinate in place
-  double *out[4] = {x0, x1, x2, dx};
-  for (int q = 0; q < 4; q++) {
-    if (q == 3) {
-      __syncthreads();
-      if ((int)threadIdx.x < ne)
+  // the distances to shared memory, then whole points in order
+  double *sm = gp + GP_ELEMS * PAD;
+  if ((int)threadIdx.x < ne)
 #pragma unroll
-        for (int k = 0; k < NV; k++) gp[threadIdx.x * PAD + k] = m[k];
-      __syncthreads();
-    }
-    for (int k = threadIdx.x; k < ne * NV; k += GP_ELEMS) {
-      const int e = k / NV, v = k % NV;
-      double val;
-      if (q == 3)
-        val = gp[e * PAD + v];
-      else
-        val = q < NDIM ? gp[e * PAD + c_pre_to_sym[v] * NDIM + q] : 0.0;
-      out[q][e0 * NV + k] = val;
-    }
+    for (int k = 0; k < NV; k++) sm[threadIdx.x * (NV + 1) + k] = m[k];
+  __syncthreads();
+  for (int k = threadIdx.x; k < ne * NV; k += GP_ELEMS) {
+    const int e = k / NV, v = k % NV;
+    const double *c = gp + e * PAD + c_pre_to_sym[v] * NDIM;
+    pt[e0 * NV + k] = make_double4_32a(c[0], c[1], NDIM == 3 ? c[NDIM - 1] : 0.0, sm[e * (NV + 1) + v]);
   }
 }
 
+// x: coordinate d of the points
 __global__ void k_gc_keys(const int *__restrict__ ord, const double *__restrict__ x, ll np,
                           u64 *__restrict__ keys) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < np) keys[i] = ordered_key(x[ord[i]]);
+  if (i < np) keys[i] = ordered_key(x[4 * (ll)ord[i]]);
 }
 
 __global__ void k_iota(int *__restrict__ a, ll n) {
@@ -123,30 +118,66 @@ __device__ __forceinline__ double key_value(u64 k) {
   return __longlong_as_double((ll)((k >> 63) ? (k ^ 0x8000000000000000ull) : ~k));
 }
 
-// whether a gap separates sorted neighbours at squared distance d with the
-// smallest neighbour distances da, db
-__device__ __forceinline__ bool gap_between(double d, double da, double db, double tol2) {
-  return d > __dmul_rn(da < db ? da : db, tol2);
+// |x| to 23 bits, truncated, without the FP64 pipe (a conversion would use it);
+// below the normal range 0, above it infinity, not a number as it is
+__device__ __forceinline__ float rough(double x) {
+  const u64 b = (u64)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  const int e = (int)(b >> 52) - 896;
+  const u32 f = (u32)(b >> 29) - (896u << 23);
+  if (b > 0x7FF0000000000000ull) return __int_as_float(0x7FC00000);
+  return e <= 0 ? 0.0f : e >= 255 ? __int_as_float(0x7F800000) : __int_as_float((int)f);
+}
+// bounds of a non-negative value from its rough one (an error of 2^-18
+// covers the truncations and roundings on both sides)
+__device__ __forceinline__ float rough_lo(float f) {
+  return f < 1e-30f ? 0.0f : fminf(f, 3.0e38f) * (1.0f - 0x1p-18f);
+}
+__device__ __forceinline__ float rough_hi(float f) { return fmaxf(f, 1e-30f) * (1.0f + 0x1p-18f); }
+
+struct Tol2 {
+  double x;      // tol^2
+  float lo, hi;  // around it
+};
+Tol2 tol2_of(double tol) {
+  const double x = tol * tol;
+  const float f = (float)x;
+  return {x, std::nextafterf(f, -1.0f), std::nextafterf(f, INFINITY)};
+}
+
+// whether a gap separates sorted neighbours x, xl with the smallest neighbour
+// distances da, db: (x - xl)^2 > min(da, db) tol^2.  In FP64 that is five
+// instructions of 64 cycles on a sub-partition's pipe; only the difference is
+// taken there, and single precision with error bounds decides unless the two
+// sides agree to 2^-17 (settling 8M points: 321 -> 213 us)
+__device__ __forceinline__ bool gap_between(double x, double xl, double da, double db,
+                                            const Tol2 &tol) {
+  const double d = __dsub_rn(x, xl), m = min_sq(da, db);
+  const float df = rough(d), q = __fmul_rn(df, df), mf = rough(m);
+  if (q == q && mf == mf) {
+    if (rough_lo(q) > __fmul_ru(rough_hi(mf), tol.hi)) return true;
+    if (rough_hi(q) <= __fmul_rd(rough_lo(mf), tol.lo)) return false;
+  }
+  return __dmul_rn(d, d) > __dmul_rn(m, tol.x);
 }
 
 // flag[j] |= gap between sorted neighbours j-1, j along the coordinate that
 // was sorted last (its values are the keys).  A warp's lane takes its left
 // neighbour's point from the lane beside it, so dx is gathered once.
 __global__ void k_gaps(const int *__restrict__ ord, const u64 *__restrict__ keys,
-                       const double *__restrict__ dx, ll np, double tol2,
+                       const double4_32a *__restrict__ pt, ll np, Tol2 tol2,
                        int first_pass, int *__restrict__ flag) {
   const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   double x = 0.0, w = 0.0;
-  if (j < np) x = key_value(keys[j]), w = dx[ord[j]];
+  if (j < np) x = key_value(keys[j]), w = pt[ord[j]].w;
   double xl = __shfl_up_sync(0xffffffffu, x, 1), wl = __shfl_up_sync(0xffffffffu, w, 1);
   if (j >= np) return;
-  if (lane == 0 && j > 0) xl = key_value(keys[j - 1]), wl = dx[ord[j - 1]];
+  if (lane == 0 && j > 0) xl = key_value(keys[j - 1]), wl = pt[ord[j - 1]].w;
   if (j == 0) {
     flag[0] = 1;
     return;
   }
-  const int f = gap_between(dsq(x, xl), w, wl, tol2) ? 1 : 0;
+  const int f = gap_between(x, xl, w, wl, tol2) ? 1 : 0;
   if (first_pass)
     flag[j] = f;
   else if (f)
@@ -159,17 +190,15 @@ __global__ void k_gaps(const int *__restrict__ ord, const u64 *__restrict__ keys
 // here and the rounds are skipped.  (The copies of a vertex usually carry the
 // same bits, so its segment is in order along every axis.)  unsettled: some
 // pair is out of order; flag2 is then ignored.
-__global__ void k_gc_settle(const int *__restrict__ ord, const double *__restrict__ x0,
-                            const double *__restrict__ x1, const double *__restrict__ x2,
-                            const double *__restrict__ dx, const int *__restrict__ flag, ll np,
-                            int ndim, double tol2, int *__restrict__ flag2,
-                            int *__restrict__ unsettled) {
+__global__ void k_gc_settle(const int *__restrict__ ord, const double4_32a *__restrict__ pt,
+                            const int *__restrict__ flag, ll np, int ndim, Tol2 tol2,
+                            int *__restrict__ flag2, int *__restrict__ unsettled) {
   const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   double v[4] = {0.0, 0.0, 0.0, 0.0}, l[4];
   auto load = [&](ll i, double *o) {
-    const int p = ord[i];
-    o[0] = x0[p], o[1] = x1[p], o[2] = ndim == 3 ? x2[p] : 0.0, o[3] = dx[p];
+    const double4_32a p = pt[ord[i]];
+    o[0] = p.x, o[1] = p.y, o[2] = p.z, o[3] = p.w;
   };
   if (j < np) load(j, v);
 #pragma unroll
@@ -185,7 +214,7 @@ __global__ void k_gc_settle(const int *__restrict__ ord, const double *__restric
         if (ordered_key(l[q]) > ordered_key(v[q])) bad = true;
         // (equal coordinates have no gap unless the distance is not a number)
         if (__double_as_longlong(l[q]) != __double_as_longlong(v[q]) || nan_bits(v[q]))
-          if (gap_between(dsq(v[q], l[q]), v[3], l[3], tol2)) f = 1;
+          if (gap_between(v[q], l[q], v[3], l[3], tol2)) f = 1;
       }
     }
     flag2[j] = f;
@@ -305,43 +334,72 @@ __global__ void k_element_check(const int *__restrict__ ids, ll nel, int nv,
 
 // face_check: an element e that contains exactly 3 of the 4 corners of a
 // face of element i is an error.  Candidates e are the elements sharing a
-// vertex with i (the points of i's vertex segments); e is examined once, at
-// the lowest corner of i that it contains.  A thread per element and corner
-// (32-bit ids, a sector per candidate): 1.17 -> 0.52 ms per million hexes
-// against a thread per element on 64-bit ids.
+// vertex with i (the points of i's vertex segments).  A thread takes a corner
+// of i and adds it to the corner sets of the elements around it, in a small
+// table of the element's; then its eight threads look at the sets.  Nothing of
+// the candidates is read but their numbers: 0.52 -> 0.31 ms per million hexes
+// against comparing their ids.  Elements with more neighbours than the table
+// has slots compare ids.
+constexpr int FC_SLOTS = 64;
+__device__ __forceinline__ bool split_face(unsigned mask) {
+  bool bad = false;
+#pragma unroll
+  for (int f = 0; f < 6; f++) bad = bad || __popc(mask & c_face_mask3[f]) == 3;
+  return bad;
+}
 __global__ void __launch_bounds__(256)
 k_face_check(const int *__restrict__ ids, const int *__restrict__ ord,
              const int *__restrict__ seg_start, int nseg, ll np, int *__restrict__ err) {
+  __shared__ int s_key[32][FC_SLOTS + 1];
+  __shared__ unsigned s_mask[32][FC_SLOTS + 1];
   const ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np) return;
-  const int k = (int)(p & 7);
-  int gi[8];
-  const int4 *row = reinterpret_cast<const int4 *>(ids + (p & ~7ll));
-  const int4 a = row[0], b = row[1];
-  gi[0] = a.x, gi[1] = a.y, gi[2] = a.z, gi[3] = a.w;
-  gi[4] = b.x, gi[5] = b.y, gi[6] = b.z, gi[7] = b.w;
-  const int s = ids[p];
-  const int q1 = s + 1 < nseg ? seg_start[s + 1] : (int)np;
-  for (int q = seg_start[s]; q < q1; q++) {
-    const ll el = ord[q] >> 3;
-    if (el == (p >> 3)) continue;  // (holds all four corners of every face)
-    const int4 *er = reinterpret_cast<const int4 *>(ids + el * 8);
-    const int4 c = er[0], d = er[1];
-    const int g[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
-    unsigned mask = 0;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      bool in = false;
-#pragma unroll
-      for (int v = 0; v < 8; v++) in = in || g[v] == gi[u];
-      mask |= in ? 1u << u : 0u;
+  const int k = threadIdx.x & 7, row = threadIdx.x >> 3;
+  const unsigned group = 0xFFu << (threadIdx.x & 24);
+  if (p >= np) return;  // (whole elements)
+  int *key = s_key[row];
+  unsigned *mask = s_mask[row];
+  for (int u = k; u < FC_SLOTS; u += 8) key[u] = -1, mask[u] = 0u;
+  __syncwarp(group);
+  const int me = (int)(p >> 3), s = ids[p];
+  const int q0 = seg_start[s], q1 = s + 1 < nseg ? seg_start[s + 1] : (int)np;
+  bool fits = true;
+  for (int q = q0; q < q1 && fits; q++) {
+    const int el = ord[q] >> 3;
+    if (el == me) continue;  // (holds all four corners of every face)
+    int u = (int)(((u32)el * 2654435761u) >> 26), tries = 0;
+    for (; tries < FC_SLOTS; tries++, u = (u + 1) & (FC_SLOTS - 1)) {
+      const int was = atomicCAS(&key[u], -1, el);
+      if (was == -1 || was == el) break;
     }
-    if ((__ffs(mask) - 1) != k) continue;  // seen at a lower corner
-    for (int f = 0; f < 6; f++)
-      if (__popc(mask & c_face_mask3[f]) == 3) {
-        atomicOr(err, 1);
-        return;
-      }
+    fits = tries < FC_SLOTS;
+    if (fits) atomicOr(&mask[u], 1u << k);
+  }
+  __syncwarp(group);
+  if (__all_sync(group, fits)) {
+    bool bad = false;
+    for (int u = k; u < FC_SLOTS; u += 8) {
+      const unsigned m = mask[u];
+      if (__popc(m) >= 3) bad = bad || split_face(m);
+    }
+    if (bad) atomicOr(err, 1);
+    return;
+  }
+  // e is examined once, at the lowest corner of i that it contains
+  int gi[8];
+  for (int u = 0; u < 8; u++) gi[u] = ids[(p & ~7ll) + u];
+  for (int q = q0; q < q1; q++) {
+    const int el = ord[q] >> 3;
+    if (el == me) continue;
+    unsigned m = 0;
+    for (int v = 0; v < 8; v++) {
+      const int g = ids[(ll)el * 8 + v];
+      for (int u = 0; u < 8; u++) m |= g == gi[u] ? 1u << u : 0u;
+    }
+    if ((__ffs(m) - 1) != k) continue;  // seen at a lower corner
+    if (split_face(m)) {
+      atomicOr(err, 1);
+      return;
+    }
   }
 }
 
@@ -382,8 +440,7 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     return PARRSB_OK;
   }
   if (np > 0x7FFFFFFFll) throw ArgError{PARRSB_ERR_UNSUPPORTED, "more than 2^31 corners"};
-  for (int d = 0; d < 3; d++) ws.x[d].ensure((size_t)np);
-  ws.dx.ensure((size_t)np);
+  ws.pt.ensure((size_t)np);
   ws.keys.ensure((size_t)np);
   ws.ord.ensure((size_t)np);
   ws.flag.ensure((size_t)np);
@@ -394,27 +451,24 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
   ws.ids.ensure((size_t)np);
   ws.ids32.ensure((size_t)np);
   {
-    const size_t smem = (size_t)GP_ELEMS * (nv * ndim + 1) * sizeof(double);
+    const size_t smem = (size_t)GP_ELEMS * (nv * ndim + 1 + nv + 1) * sizeof(double);
     const unsigned nb = grid_for(nel, GP_ELEMS);
     if (ndim == 2)
-      k_points<2><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.x[0].p, ws.x[1].p, ws.x[2].p,
-                                              ws.dx.p);
+      k_points<2><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.pt.p);
     else
-      k_points<3><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.x[0].p, ws.x[1].p, ws.x[2].p,
-                                              ws.dx.p);
+      k_points<3><<<nb, GP_ELEMS, smem, st>>>(d_coord, nel, ws.pt.p);
     CK_LAUNCH();
   }
   k_iota<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, np);
   CK_LAUNCH();
-  double tol2 = tol * tol;
+  const Tol2 tol2 = tol2_of(tol);
   ll nseg = 1, longest = np;
   DBuf<int> err(2);
   CK(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), st));
   for (int t = 0; t < ndim; t++) {
     if (t == 1) {
       // nothing left to sort: the later rounds' gaps at once
-      k_gc_settle<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[0].p, ws.x[1].p, ws.x[2].p,
-                                                     ws.dx.p, ws.flag.p, np, ndim, tol2,
+      k_gc_settle<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.pt.p, ws.flag.p, np, ndim, tol2,
                                                      ws.flag2.p, err.p + 1);
       CK_LAUNCH();
       int unsettled = 0;
@@ -429,10 +483,11 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     for (int d = 0; d < ndim; d++) {
       const bool first = t == 0 && d == 0;
       if (!first && longest <= 1) continue;  // no two points left to compare
-      k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.x[d].p, np, ws.keys.p);
+      k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(
+          ws.ord.p, reinterpret_cast<const double *>(ws.pt.p) + d, np, ws.keys.p);
       CK_LAUNCH();
       sort_by_value(ws.keys, ws.ord, np, first ? nullptr : ws.seg.p, nseg, longest, ws.sort);
-      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.keys.p, ws.dx.p, np, tol2,
+      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.keys.p, ws.pt.p, np, tol2,
                                                 first ? 1 : 0, ws.flag.p);
       CK_LAUNCH();
       segments_of(ws, ws.flag.p, np, &nseg, &longest);

@@ -7,7 +7,7 @@ namespace prsb {
 
 struct GenconWs {
   SortWs sort;
-  DBuf<double> x[3], dx;
+  DBuf<double4_32a> pt;  // points: coordinates, min squared neighbour distance
   DBuf<u64> keys;
   DBuf<int> ord, flag, flag2;
   DBuf<int> seg, seg_start, bsum;  // segment of every position, first position of each

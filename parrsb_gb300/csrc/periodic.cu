@@ -95,14 +95,12 @@ __device__ __forceinline__ double dsq(double a, double b) {
 
 // one thread per matched face pair: corner correspondence, (min, max) ids
 __global__ void k_pf_match(const int2 *__restrict__ pairs, int n, const ll *__restrict__ self,
-                           const ll *__restrict__ ids, const double *__restrict__ x0,
-                           const double *__restrict__ x1, const double *__restrict__ x2,
+                           const ll *__restrict__ ids, const double4_32a *__restrict__ pt,
                            int ndim, ll *__restrict__ pmin, ll *__restrict__ pmax,
                            int *__restrict__ mismatch) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int nv = ndim == 3 ? 8 : 4, nvf = nv / 2;
-  const double *xs[3] = {x0, x1, x2};
   double fx[4][3], gx[4][3];
   ll fid[4], gid[4];
   const ll sf = self[pairs[t].x], sg = self[pairs[t].y];
@@ -112,7 +110,9 @@ __global__ void k_pf_match(const int2 *__restrict__ pairs, int n, const ll *__re
     const ll pf = (sf >> 3) * nv + cf, pg = (sg >> 3) * nv + cg;
     fid[j] = ids[pf];
     gid[j] = ids[pg];
-    for (int d = 0; d < ndim; d++) fx[j][d] = xs[d][pf], gx[j][d] = xs[d][pg];
+    const double4_32a a = pt[pf], b = pt[pg];
+    fx[j][0] = a.x, fx[j][1] = a.y, fx[j][2] = a.z;
+    gx[j][0] = b.x, gx[j][1] = b.y, gx[j][2] = b.z;
   }
   double fmax = 0.0, gmax = 0.0;
   for (int d = 0; d < ndim; d++) {
@@ -213,9 +213,8 @@ void plus_one(const ll *d_ids, ll n, long long *d_out) {
   CK_LAUNCH();
 }
 
-int periodic_device(ll *d_ids, const double *d_x0, const double *d_x1, const double *d_x2,
-                    ll nel, int ndim, ll nseg, const long long *pinfo, int npf, SortWs &sws,
-                    ll *nseg_out) {
+int periodic_device(ll *d_ids, const double4_32a *d_pt, ll nel, int ndim, ll nseg,
+                    const long long *pinfo, int npf, SortWs &sws, ll *nseg_out) {
   cudaStream_t st = ctx().stream;
   const int nv = ndim == 3 ? 8 : 4, nvf = nv / 2, nfaces = ndim == 3 ? 6 : 4;
   const ll np = nel * nv;
@@ -264,7 +263,7 @@ int periodic_device(ll *d_ids, const double *d_x0, const double *d_x1, const dou
       pmin.ensure((size_t)npairs * nvf);
       pmax.ensure((size_t)npairs * nvf);
       k_pf_match<<<grid_for(npairs, 128), 128, 0, st>>>(pairs.p, (int)npairs, self.p, d_ids,
-                                                        d_x0, d_x1, d_x2, ndim, pmin.p,
+                                                        d_pt, ndim, pmin.p,
                                                         pmax.p, flags.p + 2);
       CK_LAUNCH();
       int mism = 0;
