@@ -524,71 +524,49 @@ __global__ void k_rank_write(const u64 *__restrict__ keys, const int *__restrict
 // elements sit in shared memory for the whole recursion; a thread keeps the
 // sub-range of each of its positions in registers and advances it by one
 // split per level.  Per level:
-//   boxes   - a warp-segmented min / max over every round of 32 positions;
-//             a sub-range inside one round takes its axis at once, a long one
-//             (more than SMALL_SHORT) goes through shared-memory atomics
-//             (table slot start / SMALL_SHORT: long sub-ranges are disjoint
-//             and longer than SMALL_SHORT, so their slots differ), and a
-//             short one crossing a round boundary is reduced sequentially;
-//   axis    - longest edge, uniq[max] - uniq[min] per axis;
-//   order   - stable sort of each sub-range by its axis rank.  When no
-//             sub-range exceeds SMALL_CMP elements, an element's new place
-//             is the number of elements of its sub-range before it in
-//             (rank, position) order; otherwise an LSD radix in shared memory
-//             over the varying bytes of the rank, then of the sub-range start
-//             (warp w ranks positions [SMALL_SPAN w, SMALL_SPAN (w + 1)) in order with
-//             __match_any_sync).
+//   starts  - the active sub-ranges, appended to a list by the threads that
+//             hold their first positions;
+//   boxes   - those longer than SMALL_SHORT by warp reductions and shared-
+//             memory atomics (table slot start / SMALL_SHORT: long sub-ranges
+//             are disjoint and longer than SMALL_SHORT, so their slots
+//             differ), the others by their thread of the list;
+//   axis    - longest edge, uniq[max] - uniq[min] per axis, by the threads of
+//             the list: a warp instruction in FP64 takes 64 cycles for one
+//             lane as for 32, so the lanes are filled;
+//   order   - stable sort of each sub-range by its axis rank: a bucket per
+//             position, by rank and then by position, and an element's new
+//             place is the number of elements before it in (rank, position)
+//             order inside its bucket.  Where a bucket holds too many, an LSD
+//             radix in shared memory over the varying bytes of the rank, then
+//             of the sub-range start (__match_any_sync).
+// The positions are dealt to the warps in rounds of 32, as many rounds each
+// as n asks for.  Bound by the barriers (about ten a level) and the shared-
+// memory accesses between them.  3315 elements into 6 parts (three levels):
+// 96 -> 43 us; radix passes and 64-bit divisions took most of it before.
 // Gives exactly the order of the level-by-level global path.
 // ---------------------------------------------------------------------------
 constexpr int SMALL_MAX = 8192;
 constexpr int SMALL_THREADS = 1024;
 constexpr int SMALL_WARPS = SMALL_THREADS / 32;
 constexpr int SMALL_ITEMS = SMALL_MAX / SMALL_THREADS;  // positions per thread
-constexpr int SMALL_SPAN = 32 * SMALL_ITEMS;            // positions per warp
-constexpr int SMALL_CMP = 64;     // comparison ranking up to this sub-range length
 constexpr int SMALL_SHORT = 32;   // sequential boxes up to this sub-range length
 constexpr int SMALL_NLONG = SMALL_MAX / SMALL_SHORT;  // box table slots
+// items of a bucket ranked by counting: 8192 items in buckets of 40 cost what
+// the four radix passes do, and the largest bucket is seldom the usual one
+constexpr int SMALL_BUCKET = 64;
 
-struct SubR {
-  int st, len, p, rank;
-};
-
-template <bool LOCAL>
-__device__ __forceinline__ SubR descend(int x, int n, int p0, int d) {
-  SubR r{0, n, p0, 0};
-  for (int k = 0; k < d; k++) {
-    int L, h;
-    if (r.p > 1) {
-      L = (int)lower_count(r.len, r.p);
-      h = (r.p + 1) / 2;
-    } else if (LOCAL && r.len >= 2) {
-      L = r.len / 2;
-      h = 0;
-    } else {
-      continue;  // finished sub-range keeps its place
-    }
-    if (x < r.st + L) {
-      r.len = L;
-      r.p = r.p > 1 ? h : r.p;
-    } else {
-      r.st += L;
-      r.len -= L;
-      r.rank += h;
-      r.p = r.p > 1 ? r.p - h : r.p;
-    }
-  }
-  return r;
-}
-
-template <bool LOCAL>
-__device__ __forceinline__ bool sub_active(const SubR &r) {
-  return r.p > 1 || (LOCAL && r.len >= 2);
-}
-
-// lower_count for the small segments (n <= SMALL_MAX): 32-bit arithmetic
+// lower_count for the small segments (n <= SMALL_MAX).  The quotient comes from
+// a single-precision one, which is off by one at most; every position takes
+// one per level, and the integer division is three times as long.
 __device__ __forceinline__ int lower_count_small(int n, int p) {
-  const int h = (p + 1) / 2;
-  const int nelt = n / p, nrem = n - p * nelt;
+  const int h = (int)((unsigned)(p + 1) / 2u);
+  int nelt = 0, nrem = n;
+  if (p <= n) {
+    nelt = (int)__fdividef((float)n, (float)p);
+    nrem = n - p * nelt;
+    if (nrem < 0) nelt--, nrem += p;
+    if (nrem >= p) nelt++, nrem -= p;
+  }
   if (nrem == 0) return h * nelt;
   const int s = p - nrem;
   return h * nelt + (h > s ? h - s : 0);
@@ -596,8 +574,8 @@ __device__ __forceinline__ int lower_count_small(int n, int p) {
 
 // Longest box edge from rank boxes: uniq[max] - uniq[min] per axis, the
 // first strictly longest wins.
-__device__ __forceinline__ unsigned char small_axis(const double *__restrict__ uniq, ll N,
-                                                    int ndim, const u32 *mn, const u32 *mx) {
+__device__ __forceinline__ int small_axis(const double *uniq, ll N, int ndim, const u32 *mn,
+                                          const u32 *mx) {
   double l[3];
 #pragma unroll
   for (int q = 0; q < 3; q++)
@@ -606,10 +584,57 @@ __device__ __forceinline__ unsigned char small_axis(const double *__restrict__ u
 #pragma unroll
   for (int q = 1; q < 3; q++)
     if (q < ndim && l[q] > l[ax]) ax = q;
-  return (unsigned char)ax;
+  return ax;
 }
 
-// Items of k_rcb_small: local id in bits 0-15, sub-range start in bits
+// Sub-ranges of a thread's positions in the CTA-resident recursions: start |
+// length << 16, virtual ranks and the first of them (not tracked for a
+// segment with one virtual rank).
+template <bool PONE>
+struct SmallPos {
+  u32 sl[SMALL_ITEMS];
+  int p[PONE ? 1 : SMALL_ITEMS], rk[PONE ? 1 : SMALL_ITEMS];
+};
+
+// Appends the active sub-ranges that start at one of the warp's positions to
+// list (start | length << 16).  Returns bit r for a position of round r in one
+// of them; alive: some sub-range is cut again (with more ranks than elements
+// it may be a single one, which has nothing to order).
+template <bool LOCAL, bool PONE>
+__device__ __forceinline__ u32 small_starts(const SmallPos<PONE> &pos, int x0, int R, int n,
+                                            u32 *list, int *count, bool *alive) {
+  const int lane = threadIdx.x & 31;
+  u32 act = 0, first = 0;
+  int total = 0;
+  *alive = false;
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    if (r >= R) break;
+    const int x = x0 + r * 32, ln = (int)(pos.sl[r] >> 16);
+    const bool cut = x < n && ((!PONE && pos.p[r] > 1) || (LOCAL && ln >= 2));
+    const bool a = cut && ln >= 2;
+    *alive = *alive || cut;
+    const bool f = a && (int)(pos.sl[r] & 0xFFFFu) == x;
+    if (a) act |= 1u << r;
+    if (f) first |= 1u << r;
+    total += __popc(__ballot_sync(0xffffffffu, f));
+  }
+  if (!total) return act;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(count, total);
+  at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    if (r >= R) break;
+    const bool f = (first >> r) & 1u;
+    const u32 b = __ballot_sync(0xffffffffu, f);
+    if (f) list[at + __popc(b & ((1u << lane) - 1u))] = pos.sl[r];
+    at += __popc(b);
+  }
+  return act;
+}
+
+// Items of the radix passes: local id in bits 0-15, sub-range start in bits
 // 16-30, bit 31 set while the sub-range is active.
 constexpr u32 ITEM_ACTIVE = 0x80000000u;
 __device__ __forceinline__ u32 item_st(u32 it) { return (it >> 16) & 0x7FFFu; }
@@ -619,356 +644,385 @@ __device__ __forceinline__ u32 kx_key(const u32 *rk, const unsigned char *sax, u
 }
 
 // shared memory of k_rcb_small
+struct SmallSmem {
+  u32 *rk;               // [3][SMALL_MAX] dense ranks by local id
+  u32 *item, *item2;     // local id by position; item2 also: bucket line by start / 2
+  u32 *cnt;              // buckets; also wcnt of the radix passes
+  u32 *box;              // [SMALL_NLONG][6] min0..2, max0..2
+  unsigned short *list;  // positions by bucket; also the start list
+  unsigned char *sax;    // axis by sub-range start
+};
 constexpr size_t small_smem_bytes() {
-  return (size_t)SMALL_MAX * (3 * 4 /*rk*/ + 4 + 4 /*item, item2*/ + 4 /*kx*/ + 1 /*sax*/) +
-         (size_t)SMALL_WARPS * 256 * 2 /*wcnt*/ + (size_t)SMALL_NLONG * 6 * 4 /*box*/;
+  return (size_t)SMALL_MAX * (3 * 4 + 4 + 4 + 4 + 2 + 1) + (size_t)SMALL_NLONG * 6 * 4;
+}
+__device__ __forceinline__ SmallSmem small_carve(u32 *s) {
+  SmallSmem m;
+  m.rk = s;
+  m.item = m.rk + 3 * SMALL_MAX;
+  m.item2 = m.item + SMALL_MAX;
+  m.cnt = m.item2 + SMALL_MAX;
+  m.box = m.cnt + SMALL_MAX;
+  m.list = reinterpret_cast<unsigned short *>(m.box + SMALL_NLONG * 6);
+  m.sax = reinterpret_cast<unsigned char *>(m.list + SMALL_MAX);
+  return m;
 }
 
-template <bool LOCAL>
-__global__ void __launch_bounds__(SMALL_THREADS)
-k_rcb_small(int *__restrict__ perm, const u32 *__restrict__ rank,
-            const double *__restrict__ uniq, ll N, int ndim,
-            const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
-            const int *__restrict__ seg_p, const int *__restrict__ seg_r0,
-            int *__restrict__ part) {
-  extern __shared__ u32 smem_u32[];
-  u32 *rk = smem_u32;                  // [3][SMALL_MAX] dense ranks by local id
-  u32 *item = rk + 3 * SMALL_MAX;      // (sub-range start << 16) | local id
-  u32 *item2 = item + SMALL_MAX;
-  u32 *kx = item2 + SMALL_MAX;         // axis rank per position
-  u32 *box = kx + SMALL_MAX;           // [SMALL_NLONG][6] min0..2, max0..2
-  unsigned short *wcnt = (unsigned short *)(box + SMALL_NLONG * 6);  // [SMALL_WARPS][256]
-  unsigned char *sax = (unsigned char *)(wcnt + SMALL_WARPS * 256);  // axis by sub-range start
+// Boxes of the long sub-ranges (slot start / SMALL_SHORT of the table).  A
+// lane folds its rounds while the warp stays in one sub-range; the warp
+// reduces when that changes.
+__device__ __forceinline__ void small_boxes(const SmallSmem &m, const u32 *item, const u32 *sl,
+                                            u32 act, int x0, int R, int ndim) {
+  const int lane = threadIdx.x & 31;
+  u32 mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
+  int cur = -1;  // start of the sub-range that the lanes fold
+  auto flush = [&]() {
+    if (cur < 0) return;
+    u32 *o = m.box + 6 * (cur / SMALL_SHORT);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      if (q >= ndim) break;
+      const u32 a = __reduce_min_sync(0xffffffffu, mn[q]), b = __reduce_max_sync(0xffffffffu, mx[q]);
+      if (lane == q) atomicMin(o + q, a), atomicMax(o + 3 + q, b);
+      mn[q] = 0xFFFFFFFFu, mx[q] = 0u;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    if (r >= R) break;
+    const bool lng = ((act >> r) & 1u) && (int)(sl[r] >> 16) > SMALL_SHORT;
+    const int st = (int)(sl[r] & 0xFFFFu);
+    u32 left = __ballot_sync(0xffffffffu, lng);
+    if (!left) continue;
+    const u32 id = item[x0 + r * 32] & 0xFFFFu;  // (of a long one: below n)
+    while (left) {  // usually one sub-range; a boundary makes it two
+      const int s = __shfl_sync(0xffffffffu, st, __ffs(left) - 1);
+      if (s != cur) flush(), cur = s;
+      const bool mine = lng && st == s;
+      if (mine)
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+          if (q < ndim) {
+            const u32 k = m.rk[q * SMALL_MAX + id];
+            mn[q] = min(mn[q], k), mx[q] = max(mx[q], k);
+          }
+      left &= ~__ballot_sync(0xffffffffu, mine);
+    }
+  }
+  flush();
+}
+
+// One level's order by LSD radix passes over the varying bytes of the rank,
+// then of the sub-range start; the result ends in item (swapped with item2).
+__device__ __forceinline__ void small_radix(const SmallSmem &m, u32 *&item, u32 *&item2,
+                                            const u32 *sl, u32 act, int x0, int R, int n) {
   __shared__ unsigned dbase[256];
   __shared__ u32 s_and, s_or, s_stand, s_stor;
-  __shared__ int s_maxlen;
+  unsigned short *wcnt = reinterpret_cast<unsigned short *>(m.cnt);  // [SMALL_WARPS][256]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  if (threadIdx.x == 0) s_and = 0xFFFFFFFFu, s_or = 0u, s_stand = 0xFFFFFFFFu, s_stor = 0u;
+  u32 kand = 0xFFFFFFFFu, kor = 0u, stand = 0xFFFFFFFFu, stor = 0u;
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    const int x = x0 + r * 32;
+    if (r >= R || x >= n) break;
+    const u32 st = sl[r] & 0xFFFFu;
+    const u32 it = (st << 16) | (item[x] & 0xFFFFu) | (((act >> r) & 1u) ? ITEM_ACTIVE : 0u);
+    const u32 k = kx_key(m.rk, m.sax, it);
+    item[x] = it;
+    kand &= k, kor |= k, stand &= st, stor |= st;
+  }
+  __syncthreads();
+  atomicAnd(&s_and, kand);
+  atomicOr(&s_or, kor);
+  atomicAnd(&s_stand, stand);
+  atomicOr(&s_stor, stor);
+  __syncthreads();
+  const u32 kdiff = s_and ^ s_or, sdiff = s_stand ^ s_stor;
+  for (int b = 0; b < 6; b++) {
+    const bool is_st = b >= 4;
+    const int shift = is_st ? 8 * (b - 4) : 8 * b;
+    if ((((is_st ? sdiff : kdiff) >> shift) & 255u) == 0) continue;
+    for (int i = threadIdx.x; i < SMALL_WARPS * 256; i += blockDim.x) wcnt[i] = 0;
+    __syncthreads();
+    unsigned rd[SMALL_ITEMS];  // digit << 16 | rank among the warp's equal digits
+    u32 itv[SMALL_ITEMS];
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      rd[r] = 256u << 16, itv[r] = 0;
+      if (r >= R) continue;
+      const int x = x0 + r * 32;
+      unsigned dgt = 256;
+      if (x < n) {
+        const u32 it = item[x];
+        itv[r] = it;
+        // inactive positions carry key 0 (their sub-range keeps its order)
+        const u32 k = is_st ? item_st(it) : kx_key(m.rk, m.sax, it);
+        dgt = (k >> shift) & 255u;
+      }
+      const unsigned peers = __match_any_sync(0xffffffffu, dgt);
+      unsigned before = 0;
+      if (dgt < 256) before = wcnt[warp * 256 + dgt];
+      __syncwarp();
+      if (dgt < 256) {
+        rd[r] = (dgt << 16) | (before + __popc(peers & lt_mask));
+        if (lane == __ffs(peers) - 1)
+          wcnt[warp * 256 + dgt] = (unsigned short)(before + __popc(peers));
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      unsigned run = 0;
+      for (int w = 0; w < SMALL_WARPS; w++) {
+        const unsigned t = wcnt[w * 256 + threadIdx.x];
+        wcnt[w * 256 + threadIdx.x] = (unsigned short)run;
+        run += t;
+      }
+      dbase[threadIdx.x] = run;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // exclusive scan of the 256 digit totals
+      unsigned v[8], s2 = 0;
+      for (int j = 0; j < 8; j++) v[j] = dbase[threadIdx.x * 8 + j], s2 += v[j];
+      unsigned incl = s2;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)threadIdx.x >= o) incl += y;
+      }
+      unsigned run = incl - s2;
+      for (int j = 0; j < 8; j++) dbase[threadIdx.x * 8 + j] = run, run += v[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      const unsigned dgr = rd[r] >> 16;
+      if (dgr < 256) item2[dbase[dgr] + wcnt[warp * 256 + dgr] + (rd[r] & 0xFFFFu)] = itv[r];
+    }
+    __syncthreads();
+    u32 *t = item;
+    item = item2;
+    item2 = t;
+  }
+}
+
+// The level loop; PONE: the segment has one virtual rank (only the local
+// halving: no rank counts to track, every part is r0).
+template <bool LOCAL, bool PONE>
+__device__ __forceinline__ void small_levels(const SmallSmem &m, int *__restrict__ perm,
+                                             const double *uniq, ll N, int ndim, ll start, int n,
+                                             int p0, int r0, int *__restrict__ part,
+                                             int *s_nst) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int R = (n + SMALL_THREADS - 1) / SMALL_THREADS;  // rounds per warp
+  const int x0 = warp * R * 32 + lane;                    // first position
+  u32 *item = m.item, *item2 = m.item2;
+  u32 *starts = reinterpret_cast<u32 *>(m.list);
+  SmallPos<PONE> pos;
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    pos.sl[r] = (u32)n << 16;
+    if (!PONE) pos.p[r] = p0, pos.rk[r] = 0;
+  }
+  for (int d = 0; d < 64; d++) {
+    if (d > 0) {  // advance every position's sub-range by the previous cut
+#pragma unroll
+      for (int r = 0; r < SMALL_ITEMS; r++) {
+        if (r >= R) break;
+        const int x = x0 + r * 32;
+        int st = (int)(pos.sl[r] & 0xFFFFu), ln = (int)(pos.sl[r] >> 16);
+        const int p = PONE ? 1 : pos.p[r];
+        int L, h;
+        if (p > 1) {
+          L = lower_count_small(ln, p);
+          h = (p + 1) / 2;
+        } else if (LOCAL && ln >= 2) {
+          L = ln / 2;
+          h = 0;
+        } else {
+          continue;  // finished sub-range keeps its place
+        }
+        const bool up = x >= st + L;
+        st += up ? L : 0;
+        ln = up ? ln - L : L;
+        pos.sl[r] = (u32)st | ((u32)ln << 16);
+        if (!PONE && p > 1) pos.p[r] = up ? p - h : h, pos.rk[r] += up ? h : 0;
+      }
+    }
+    bool alive;
+    const u32 act = small_starts<LOCAL, PONE>(pos, x0, R, n, starts, &s_nst[d & 1], &alive);
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      if (r >= R) break;
+      const int st = (int)(pos.sl[r] & 0xFFFFu);
+      if (st == x0 + r * 32 && (int)(pos.sl[r] >> 16) > SMALL_SHORT) {
+        u32 *o = m.box + 6 * (st / SMALL_SHORT);
+        o[0] = o[1] = o[2] = 0xFFFFFFFFu, o[3] = o[4] = o[5] = 0u;
+      }
+    }
+    if (!__syncthreads_or(alive)) break;
+    const int nst = s_nst[d & 1];
+    if (threadIdx.x == 0) s_nst[(d + 1) & 1] = 0;
+    small_boxes(m, item, pos.sl, act, x0, R, ndim);
+    for (int k = threadIdx.x; k < n; k += SMALL_THREADS) m.cnt[k] = 0u;
+    __syncthreads();
+    // axis, and the line that maps ranks to buckets: first rank and buckets
+    // per rank, in item2 (active sub-ranges have two positions or more)
+    for (int i = threadIdx.x; i < nst; i += SMALL_THREADS) {
+      const int st = (int)(starts[i] & 0xFFFFu), ln = (int)(starts[i] >> 16);
+      u32 mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
+      if (ln > SMALL_SHORT) {
+        const u32 *o = m.box + 6 * (st / SMALL_SHORT);
+#pragma unroll
+        for (int q = 0; q < 3; q++) mn[q] = o[q], mx[q] = o[3 + q];
+      } else {
+        for (int y = st; y < st + ln; y++) {
+          const u32 id = item[y] & 0xFFFFu;
+#pragma unroll
+          for (int q = 0; q < 3; q++)
+            if (q < ndim) {
+              const u32 k = m.rk[q * SMALL_MAX + id];
+              mn[q] = min(mn[q], k), mx[q] = max(mx[q], k);
+            }
+        }
+      }
+      const int ax = small_axis(uniq, N, ndim, mn, mx);
+      m.sax[st] = (unsigned char)ax;
+      const u32 lo = ax == 0 ? mn[0] : ax == 1 ? mn[1] : mn[2];
+      const u32 hi = ax == 0 ? mx[0] : ax == 1 ? mx[1] : mx[2];
+      reinterpret_cast<uint2 *>(item2)[st >> 1] =
+          make_uint2(lo, __float_as_uint((float)ln / ((float)(hi - lo) + 1.0f)));
+    }
+    __syncthreads();
+    // bucket of every position: (rank - first + (x - st) / len) x line.  The
+    // fraction spreads equal ranks over their buckets; every operation is
+    // monotonic and the fraction below one, so (rank, position) order is
+    // bucket order
+    u32 bk[SMALL_ITEMS];
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      const int x = x0 + r * 32;
+      if (r >= R || x >= n) break;
+      const int st = (int)(pos.sl[r] & 0xFFFFu), ln = (int)(pos.sl[r] >> 16);
+      bk[r] = (u32)x;
+      if ((act >> r) & 1u) {
+        const u32 k = m.rk[m.sax[st] * SMALL_MAX + (item[x] & 0xFFFFu)];
+        const uint2 line = reinterpret_cast<const uint2 *>(item2)[st >> 1];
+        const float f = (float)(k - line.x) + __fdividef((float)(x - st), (float)ln);
+        bk[r] = (u32)(st + min(ln - 1, (int)(f * __uint_as_float(line.y))));
+      }
+      atomicAdd(&m.cnt[bk[r]], 1u);
+    }
+    __syncthreads();
+    const u32 big = cta_scan<SMALL_MAX, SMALL_THREADS>(m.cnt, n);
+    if (big > SMALL_BUCKET) {
+      small_radix(m, item, item2, pos.sl, act, x0, R, n);
+      continue;
+    }
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      const int x = x0 + r * 32;
+      if (r >= R || x >= n) break;
+      m.list[atomicAdd(&m.cnt[bk[r]], 1u)] = (unsigned short)x;
+    }
+    __syncthreads();  // (cnt: now the end of every bucket)
+#pragma unroll
+    for (int r = 0; r < SMALL_ITEMS; r++) {
+      const int x = x0 + r * 32;
+      if (r >= R || x >= n) break;
+      const int b0 = bk[r] ? (int)m.cnt[bk[r] - 1] : 0, b1 = (int)m.cnt[bk[r]];
+      const u32 it = item[x] & 0xFFFFu;
+      int to = b0;
+      if (b1 - b0 > 1) {
+        const u32 *rk = m.rk + m.sax[pos.sl[r] & 0xFFFFu] * SMALL_MAX;
+        const u32 k = rk[it];
+        for (int j = b0; j < b1; j++) {
+          const int y = m.list[j];
+          const u32 k2 = rk[item[y] & 0xFFFFu];
+          to += (k2 < k) || (k2 == k && y < x);
+        }
+      }
+      item2[to] = it;
+    }
+    __syncthreads();
+    u32 *t = item;
+    item = item2;
+    item2 = t;
+  }
+  // ---- write the order (and ranks) back: read every old entry, then write
+  int ev[SMALL_ITEMS];
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    const int x = x0 + r * 32;
+    ev[r] = r < R && x < n ? perm[start + (item[x] & 0xFFFFu)] : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < SMALL_ITEMS; r++) {
+    const int x = x0 + r * 32;
+    if (r < R && x < n) {
+      perm[start + x] = ev[r];
+      if (part) part[ev[r]] = r0 + (PONE ? 0 : pos.rk[r]);
+    }
+  }
+}
+
+// sparse: null, or one segment of all N elements, whose ranks on axis q with
+// sparse[q] set are the numbers of elements strictly below (equal coordinates
+// leave numbers out); they are made dense first, in uniq too.
+template <bool LOCAL>
+__global__ void __launch_bounds__(SMALL_THREADS)
+k_rcb_small(int *__restrict__ perm, const u32 *__restrict__ rank, double *uniq, ll N, int ndim,
+            const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
+            const int *__restrict__ seg_p, const int *__restrict__ seg_r0,
+            int *__restrict__ part, const int *__restrict__ sparse) {
+  extern __shared__ __align__(16) u32 smem_u32[];
+  const SmallSmem m = small_carve(smem_u32);
+  __shared__ int s_nst[2];
   const ll sg = blockIdx.x;
   const ll start = seg_start[sg];
   const int n = (int)seg_n[sg], p0 = seg_p[sg], r0 = seg_r0[sg];
-  bool seg_act = p0 > 1 || (LOCAL && p0 == 1 && n >= 2);
+  const bool seg_act = p0 > 1 || (LOCAL && p0 == 1 && n >= 2);
   if (n <= 0 || p0 <= 0) return;
   if (!seg_act || n > SMALL_MAX) {
     if (part && n <= SMALL_MAX && p0 == 1)
       for (int x = threadIdx.x; x < n; x += blockDim.x) part[perm[start + x]] = r0;
     return;
   }
+  if (threadIdx.x == 0) s_nst[0] = s_nst[1] = 0;
   for (int x = threadIdx.x; x < n; x += blockDim.x) {
     const int e = perm[start + x];
-    for (int q = 0; q < ndim; q++) rk[q * SMALL_MAX + x] = rank[(ll)q * N + e];
-    item[x] = (u32)x;
+    for (int q = 0; q < ndim; q++) m.rk[q * SMALL_MAX + x] = rank[(ll)q * N + e];
+    m.item[x] = (u32)x;
   }
-  // The level loop, instantiated for segments with one virtual rank (only
-  // the local halving, no per-position rank counts) and for the general case.
-  auto levels = [&](auto pone) {
-    constexpr bool PONE = decltype(pone)::value;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    // Sub-range of each own position at the current depth, advanced by one
-    // split per level: start | length << 16, and its virtual-rank count.
-    u32 sl_r[SMALL_ITEMS];
-    int p_r[PONE ? 1 : SMALL_ITEMS];  // with one virtual rank (PONE) p stays 1
-  #pragma unroll
-    for (int r = 0; r < SMALL_ITEMS; r++) {
-      sl_r[r] = (u32)n << 16;
-      if (!PONE) p_r[r] = p0;
-    }
-    for (int d = 0; d < 64; d++) {
-      if (d > 0) {
-  #pragma unroll
-        for (int r = 0; r < SMALL_ITEMS; r++) {
-          const int x = warp * SMALL_SPAN + r * 32 + lane;
-          int st = (int)(sl_r[r] & 0xFFFFu), ln = (int)(sl_r[r] >> 16), p = PONE ? 1 : p_r[r];
-          int L, h;
-          if (p > 1) {
-            L = lower_count_small(ln, p);
-            h = (p + 1) / 2;
-          } else if (LOCAL && ln >= 2) {
-            L = ln / 2;
-            h = 0;
-          } else {
-            continue;  // finished sub-range keeps its place
-          }
-          if (x < st + L) {
-            ln = L;
-            p = p > 1 ? h : p;
-          } else {
-            st += L;
-            ln -= L;
-            p = p > 1 ? p - h : p;
-          }
-          sl_r[r] = (u32)st | ((u32)ln << 16);
-          if (!PONE) p_r[r] = p;
-        }
-      }
-      if (threadIdx.x == 0) s_maxlen = 0;
-      for (int t = threadIdx.x; t < SMALL_NLONG * 6; t += blockDim.x)
-        box[t] = (t % 6) < 3 ? 0xFFFFFFFFu : 0u;
+  if (sparse) {
+    for (int q = 0; q < ndim; q++) {
+      if (!sparse[q]) continue;
       __syncthreads();
-      u32 act_mask = 0;  // bit r: position r lies in an active sub-range
-      int mylen = 0;
-  #pragma unroll
-      for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
-        const int ln = (int)(sl_r[r] >> 16);
-        if (x < n && ((!PONE && p_r[r] > 1) || (LOCAL && ln >= 2)))
-          act_mask |= 1u << r, mylen = max(mylen, ln);
-      }
-      if (mylen) atomicMax(&s_maxlen, mylen);
-      if (!__syncthreads_or(act_mask != 0)) break;
-      const int maxlen = s_maxlen;
-      // ---- bounding boxes on dense ranks, axis of each sub-range.  A warp
-      // whose 256 positions all lie in one active sub-range folds them per
-      // lane and reduces once; other warps reduce each round of 32 positions
-      // with a segmented shuffle tree.
-      const int st0 = (int)(sl_r[0] & 0xFFFFu);
-      bool one = act_mask == (1u << SMALL_ITEMS) - 1u;
-#pragma unroll
-      for (int r = 1; r < SMALL_ITEMS; r++) one = one && (int)(sl_r[r] & 0xFFFFu) == st0;
-      const int st0_lane0 = __shfl_sync(0xffffffffu, st0, 0);  // every lane takes part
-      const bool warp_one = __all_sync(0xffffffffu, one && st0 == st0_lane0);
-      if (warp_one) {
-        u32 mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
-#pragma unroll
-        for (int r = 0; r < SMALL_ITEMS; r++) {
-          const u32 id = item[warp * SMALL_SPAN + r * 32 + lane] & 0xFFFFu;
-#pragma unroll
-          for (int q = 0; q < 3; q++)
-            if (q < ndim) {
-              const u32 k = rk[q * SMALL_MAX + id];
-              mn[q] = min(mn[q], k);
-              mx[q] = max(mx[q], k);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          mn[q] = __reduce_min_sync(0xffffffffu, mn[q]);
-          mx[q] = __reduce_max_sync(0xffffffffu, mx[q]);
-        }
-        const int ln0 = (int)(sl_r[0] >> 16);
-        if (lane == 0) {
-          if (st0 == warp * SMALL_SPAN && ln0 == SMALL_SPAN) {
-            sax[st0] = small_axis(uniq, N, ndim, mn, mx);  // the whole sub-range
-          } else {  // longer than SMALL_SHORT: box table slot
-            const int o = st0 / SMALL_SHORT;
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-              if (q < ndim) {
-                atomicMin(&box[6 * o + q], mn[q]);
-                atomicMax(&box[6 * o + 3 + q], mx[q]);
-              }
-          }
-        }
-      }
+      u32 *rk = m.rk + q * SMALL_MAX;
+      for (int x = threadIdx.x; x < n; x += blockDim.x) m.cnt[x] = 0u;
+      __syncthreads();
+      double v[SMALL_ITEMS];
 #pragma unroll
       for (int r = 0; r < SMALL_ITEMS; r++) {
-        const bool act = (act_mask >> r) & 1u;
-        if (warp_one || !__any_sync(0xffffffffu, act)) continue;  // warp-uniform
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
-        const int st = (int)(sl_r[r] & 0xFFFFu), ln = (int)(sl_r[r] >> 16);
-        const int segkey = act ? st : -1 - lane;
-        u32 mn[3], mx[3];
-        const u32 id = act ? (item[x] & 0xFFFFu) : 0u;
-  #pragma unroll
-        for (int q = 0; q < 3; q++) {
-          const u32 k = (act && q < ndim) ? rk[q * SMALL_MAX + id] : 0u;
-          mn[q] = act ? k : 0xFFFFFFFFu;
-          mx[q] = k;
-        }
-  #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const int ok = __shfl_down_sync(0xffffffffu, segkey, off);
-          const bool same = (lane + off < 32) && ok == segkey;
-  #pragma unroll
-          for (int q = 0; q < 3; q++) {
-            const u32 a2 = __shfl_down_sync(0xffffffffu, mn[q], off);
-            const u32 b2 = __shfl_down_sync(0xffffffffu, mx[q], off);
-            if (same) mn[q] = min(mn[q], a2), mx[q] = max(mx[q], b2);
-          }
-        }
-        const int prevkey = __shfl_up_sync(0xffffffffu, segkey, 1);
-        if (act && (lane == 0 || prevkey != segkey)) {  // first position of a run
-          const int rend = warp * SMALL_SPAN + r * 32 + 32;
-          if (x == st && st + ln <= rend) {
-            sax[st] = small_axis(uniq, N, ndim, mn, mx);  // whole sub-range in this round
-          } else if (ln > SMALL_SHORT) {
-            const int o = st / SMALL_SHORT;
-  #pragma unroll
-            for (int q = 0; q < 3; q++)
-              if (q < ndim) {
-                atomicMin(&box[6 * o + q], mn[q]);
-                atomicMax(&box[6 * o + 3 + q], mx[q]);
-              }
-          }
-        }
+        const int x = threadIdx.x + r * SMALL_THREADS;
+        if (x < n) m.cnt[rk[x]] = 1u, v[r] = uniq[(ll)q * N + rk[x]];
       }
       __syncthreads();
-      // sub-ranges spanning more than one round: long ones from the box table,
-      // short ones (crossing a round boundary) by a sequential loop
-  #pragma unroll
+      cta_scan<SMALL_MAX, SMALL_THREADS>(m.cnt, n);
+#pragma unroll
       for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
-        const int st = (int)(sl_r[r] & 0xFFFFu), ln = (int)(sl_r[r] >> 16);
-        const int rend = warp * SMALL_SPAN + r * 32 + 32;
-        const bool whole_warp = st == warp * SMALL_SPAN && ln == SMALL_SPAN;
-        if (((act_mask >> r) & 1u) && x == st && st + ln > rend && !(warp_one && whole_warp)) {
-          u32 mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
-          if (ln > SMALL_SHORT) {
-            const int o = st / SMALL_SHORT;
-  #pragma unroll
-            for (int q = 0; q < 3; q++) mn[q] = box[6 * o + q], mx[q] = box[6 * o + 3 + q];
-          } else {
-            for (int y = st; y < st + ln; y++) {
-              const u32 id = item[y] & 0xFFFFu;
-  #pragma unroll
-              for (int q = 0; q < 3; q++)
-                if (q < ndim) {
-                  const u32 k = rk[q * SMALL_MAX + id];
-                  mn[q] = min(mn[q], k);
-                  mx[q] = max(mx[q], k);
-                }
-            }
-          }
-          sax[st] = small_axis(uniq, N, ndim, mn, mx);
-        }
+        const int x = threadIdx.x + r * SMALL_THREADS;
+        if (x < n) rk[x] = m.cnt[rk[x]], uniq[(ll)q * N + rk[x]] = v[r];
       }
       __syncthreads();
-      // ---- keys: rank along the sub-range's axis
-      u32 kand = 0xFFFFFFFFu, kor = 0u, stand = 0xFFFFFFFFu, stor = 0u;
-  #pragma unroll
-      for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
-        if (x >= n) continue;
-        const u32 st = sl_r[r] & 0xFFFFu;
-        const bool act = (act_mask >> r) & 1u;
-        const u32 id = item[x] & 0xFFFFu;
-        const u32 k = act ? rk[sax[st] * SMALL_MAX + id] : 0u;
-        kx[x] = k;
-        item[x] = (st << 16) | id | (act ? ITEM_ACTIVE : 0u);
-        kand &= k, kor |= k, stand &= st, stor |= st;
-      }
-      __syncthreads();
-      if (maxlen <= SMALL_CMP) {
-        // ---- comparison ranking inside each sub-range
-  #pragma unroll
-        for (int r = 0; r < SMALL_ITEMS; r++) {
-          const int x = warp * SMALL_SPAN + r * 32 + lane;
-          if (x >= n) continue;
-          const int len = ((act_mask >> r) & 1u) ? (int)(sl_r[r] >> 16) : 0;
-          const int st = (int)(sl_r[r] & 0xFFFFu);
-          if (!len) {
-            item2[x] = item[x];
-            continue;
-          }
-          const u32 k = kx[x];
-          int c = 0;
-          for (int y = st; y < st + len; y++) {
-            const u32 k2 = kx[y];
-            c += (k2 < k) || (k2 == k && y < x);
-          }
-          item2[st + c] = item[x];
-        }
-        __syncthreads();
-        u32 *t = item;
-        item = item2;
-        item2 = t;
-      } else {
-        // ---- stable LSD passes over the varying bytes: rank, then start
-        if (threadIdx.x == 0) s_and = 0xFFFFFFFFu, s_or = 0u, s_stand = 0xFFFFFFFFu, s_stor = 0u;
-        __syncthreads();
-        atomicAnd(&s_and, kand);
-        atomicOr(&s_or, kor);
-        atomicAnd(&s_stand, stand);
-        atomicOr(&s_stor, stor);
-        __syncthreads();
-        const u32 kdiff = s_and ^ s_or, sdiff = s_stand ^ s_stor;
-        for (int b = 0; b < 6; b++) {
-          const bool is_st = b >= 4;
-          const int shift = is_st ? 8 * (b - 4) : 8 * b;
-          if ((((is_st ? sdiff : kdiff) >> shift) & 255u) == 0) continue;
-          for (int i = threadIdx.x; i < SMALL_WARPS * 256; i += blockDim.x) wcnt[i] = 0;
-          __syncthreads();
-          unsigned rd[SMALL_ITEMS];  // digit << 16 | rank among the warp's equal digits
-          u32 itv[SMALL_ITEMS];
-  #pragma unroll
-          for (int r = 0; r < SMALL_ITEMS; r++) {
-            const int x = warp * SMALL_SPAN + r * 32 + lane;
-            unsigned dgt = 256;
-            itv[r] = 0;
-            if (x < n) {
-              const u32 it = item[x];
-              itv[r] = it;
-              // inactive positions carry key 0 (their sub-range keeps its order)
-              const u32 k = is_st ? item_st(it) : kx_key(rk, sax, it);
-              dgt = (k >> shift) & 255u;
-            }
-            unsigned peers = __match_any_sync(0xffffffffu, dgt);
-            unsigned before = 0;
-            if (dgt < 256) before = wcnt[warp * 256 + dgt];
-            __syncwarp();
-            if (dgt < 256) {
-              rd[r] = (dgt << 16) | (before + __popc(peers & lt_mask));
-              if (lane == __ffs(peers) - 1)
-                wcnt[warp * 256 + dgt] = (unsigned short)(before + __popc(peers));
-            }
-            if (dgt >= 256) rd[r] = 256u << 16;
-            __syncwarp();
-          }
-          __syncthreads();
-          if (threadIdx.x < 256) {
-            unsigned run = 0;
-            for (int w = 0; w < SMALL_WARPS; w++) {
-              unsigned t = wcnt[w * 256 + threadIdx.x];
-              wcnt[w * 256 + threadIdx.x] = (unsigned short)run;
-              run += t;
-            }
-            dbase[threadIdx.x] = run;
-          }
-          __syncthreads();
-          if (threadIdx.x < 32) {  // exclusive scan of the 256 digit totals
-            unsigned v[8], s2 = 0;
-            for (int j = 0; j < 8; j++) v[j] = dbase[threadIdx.x * 8 + j], s2 += v[j];
-            unsigned incl = s2;
-            for (int o = 1; o < 32; o <<= 1) {
-              unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-              if (threadIdx.x >= o) incl += y;
-            }
-            unsigned run = incl - s2;
-            for (int j = 0; j < 8; j++) dbase[threadIdx.x * 8 + j] = run, run += v[j];
-          }
-          __syncthreads();
-  #pragma unroll
-          for (int r = 0; r < SMALL_ITEMS; r++) {
-            const unsigned dgr = rd[r] >> 16;
-            if (dgr < 256) item2[dbase[dgr] + wcnt[warp * 256 + dgr] + (rd[r] & 0xFFFFu)] = itv[r];
-          }
-          __syncthreads();
-          u32 *t = item;
-          item = item2;
-          item2 = t;
-        }
-      }
     }
-    // ---- write the order (and ranks) back: read every old entry, then write
-    int ev[SMALL_ITEMS];
-  #pragma unroll
-    for (int r = 0; r < SMALL_ITEMS; r++) {
-      const int x = warp * SMALL_SPAN + r * 32 + lane;
-      ev[r] = x < n ? perm[start + (item[x] & 0xFFFFu)] : 0;
-    }
-    __syncthreads();
-  #pragma unroll
-    for (int r = 0; r < SMALL_ITEMS; r++) {
-      const int x = warp * SMALL_SPAN + r * 32 + lane;
-      if (x < n) {
-        perm[start + x] = ev[r];
-        if (part) part[ev[r]] = r0 + descend<LOCAL>(x, n, p0, 64).rank;
-      }
-    }
-  };
+  }
+  __syncthreads();
   if (p0 == 1)
-    levels(std::true_type{});
+    small_levels<LOCAL, true>(m, perm, uniq, N, ndim, start, n, p0, r0, part, s_nst);
   else
-    levels(std::false_type{});
+    small_levels<LOCAL, false>(m, perm, uniq, N, ndim, start, n, p0, r0, part, s_nst);
 }
 
 // children of every segment; lc: active segments, those with more than one
@@ -1046,16 +1100,16 @@ cudaError_t rcb_small_prepare() {
                               (int)small_smem_bytes());
 }
 
-cudaError_t rcb_small_launch(int *perm, const u32 *rank, const double *uniq, ll N, int ndim,
+cudaError_t rcb_small_launch(int *perm, const u32 *rank, double *uniq, ll N, int ndim,
                              const ll *seg_start, const ll *seg_n, const int *seg_p,
-                             const int *seg_r0, ll nseg, bool local, int *part,
+                             const int *seg_r0, ll nseg, bool local, const int *sparse, int *part,
                              cudaStream_t stream) {
   if (local)
     k_rcb_small<true><<<(unsigned)nseg, SMALL_THREADS, small_smem_bytes(), stream>>>(
-        perm, rank, uniq, N, ndim, seg_start, seg_n, seg_p, seg_r0, part);
+        perm, rank, uniq, N, ndim, seg_start, seg_n, seg_p, seg_r0, part, sparse);
   else
     k_rcb_small<false><<<(unsigned)nseg, SMALL_THREADS, small_smem_bytes(), stream>>>(
-        perm, rank, uniq, N, ndim, seg_start, seg_n, seg_p, seg_r0, part);
+        perm, rank, uniq, N, ndim, seg_start, seg_n, seg_p, seg_r0, part, sparse);
   return cudaGetLastError();
 }
 
@@ -1351,15 +1405,17 @@ __global__ void k_ps_final(const int *__restrict__ lists, ll N, const int *__res
 constexpr int SMALL_ROUNDS = SMALL_MAX / 32;  // ballots per list
 constexpr size_t pss_smem_bytes() {
   // local id -> element (int); six list buffers and the lower child's size
-  // by sub-range start (u16); side and cut axis (u8); per list the ballots
-  // (u32) and the in-warp prefix of each round (u16)
-  return (size_t)SMALL_MAX * (sizeof(int) + 7 * sizeof(unsigned short) + 2) +
+  // by sub-range start (u16); side and cut axis (u8); the start list (u32 per
+  // two positions); per list the ballots (u32) and the in-warp prefix of each
+  // round (u16)
+  return (size_t)SMALL_MAX * (sizeof(int) + 7 * sizeof(unsigned short) + 2 + 2) +
          (size_t)3 * SMALL_ROUNDS * (sizeof(u32) + sizeof(unsigned short));
 }
 
 struct PssSmem {
   int *gl;               // local id -> element
   u32 *bal;              // [3][SMALL_ROUNDS] lower flags, one word per 32 positions
+  u32 *starts;           // active sub-ranges: start | length << 16
   unsigned short *buf;   // [6][SMALL_MAX]: three lists and three spares
   unsigned short *spl;   // lower child's size by sub-range start
   unsigned short *wpre;  // [3][SMALL_ROUNDS] lower flags before the round in its warp
@@ -1371,7 +1427,8 @@ __device__ __forceinline__ PssSmem pss_carve(unsigned char *s) {
   PssSmem m;
   m.gl = reinterpret_cast<int *>(s);
   m.bal = reinterpret_cast<u32 *>(m.gl + SMALL_MAX);
-  m.buf = reinterpret_cast<unsigned short *>(m.bal + 3 * SMALL_ROUNDS);
+  m.starts = m.bal + 3 * SMALL_ROUNDS;
+  m.buf = reinterpret_cast<unsigned short *>(m.starts + SMALL_MAX / 2);
   m.spl = m.buf + 6 * SMALL_MAX;
   m.wpre = m.spl + SMALL_MAX;
   m.side = reinterpret_cast<unsigned char *>(m.wpre + 3 * SMALL_ROUNDS);
@@ -1385,61 +1442,64 @@ template <bool LOCAL, bool PONE>
 __device__ __forceinline__ void pss_levels(int *__restrict__ perm, const double *__restrict__ cent,
                                            ll N, int ndim, ll start, int n, int p0, int r0,
                                            int *__restrict__ part, const PssSmem &m,
-                                           int (*wsum)[SMALL_WARPS]) {
+                                           int (*wsum)[SMALL_WARPS], int *s_nst) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const u32 lt = (1u << lane) - 1u;
-  // sub-range of each own position (start | length << 16), its virtual
-  // ranks, and the axis that cut it last
-  u32 sl_r[SMALL_ITEMS];
-  int p_r[PONE ? 1 : SMALL_ITEMS], rk_r[PONE ? 1 : SMALL_ITEMS];  // virtual ranks, first rank
+  const int R = (n + SMALL_THREADS - 1) / SMALL_THREADS;  // rounds per warp
+  const int inv_r = (65536 + R - 1) / R;                  // k / R for k < 256: k inv_r >> 16
+  const int x0 = warp * R * 32 + lane;                    // first position
+  // sub-range and virtual ranks of each own position, and the axis that cut
+  // it last
+  SmallPos<PONE> pos;
   signed char oax_r[SMALL_ITEMS];
 #pragma unroll
   for (int r = 0; r < SMALL_ITEMS; r++) {
-    sl_r[r] = (u32)n << 16, oax_r[r] = -1;
-    if (!PONE) p_r[r] = p0, rk_r[r] = 0;
+    pos.sl[r] = (u32)n << 16, oax_r[r] = -1;
+    if (!PONE) pos.p[r] = p0, pos.rk[r] = 0;
   }
   int cur = 0;  // the lists are in buffers 3 cur .. 3 cur + 2, the spares in the others
   for (int d = 0; d < 64; d++) {
     if (d > 0) {  // advance every position's sub-range by the previous cut
 #pragma unroll
       for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
-        int st = (int)(sl_r[r] & 0xFFFFu), ln = (int)(sl_r[r] >> 16), p = PONE ? 1 : p_r[r];
-        if (!(p > 1 || (LOCAL && ln >= 2))) continue;  // no longer cut
+        if (r >= R) break;
+        const int x = x0 + r * 32;
+        int st = (int)(pos.sl[r] & 0xFFFFu), ln = (int)(pos.sl[r] >> 16);
+        const int p = PONE ? 1 : pos.p[r];
+        if (x >= n || !(p > 1 || (LOCAL && ln >= 2))) continue;  // no longer cut
         const int L = m.spl[st], h = p > 1 ? (p + 1) / 2 : 0;
-        oax_r[r] = (signed char)m.sax[st];
-        if (x < st + L) {
-          ln = L;
-          p = p > 1 ? h : p;
-        } else {
-          st += L;
-          ln -= L;
-          p = p > 1 ? p - h : p;
-          if (!PONE) rk_r[r] += h;
-        }
-        sl_r[r] = (u32)st | ((u32)ln << 16);
-        if (!PONE) p_r[r] = p;
+        if (ln >= 2) oax_r[r] = (signed char)m.sax[st];
+        const bool up = x >= st + L;
+        st += up ? L : 0;
+        ln = up ? ln - L : L;
+        pos.sl[r] = (u32)st | ((u32)ln << 16);
+        if (!PONE && p > 1) pos.p[r] = up ? p - h : h, pos.rk[r] += up ? h : 0;
       }
     }
-    u32 act = 0;
-#pragma unroll
-    for (int r = 0; r < SMALL_ITEMS; r++) {
-      const int x = warp * SMALL_SPAN + r * 32 + lane;
-      const int ln = (int)(sl_r[r] >> 16);
-      if (x < n && ((!PONE && p_r[r] > 1) || (LOCAL && ln >= 2))) act |= 1u << r;
-    }
-    // barrier: the reads of sax and spl above and the previous level's
-    // partition are done before the cut axes are written and the lists read
-    if (!__syncthreads_or(act != 0)) break;
+    // the reads of sax and spl above and the previous level's partition are
+    // done at the barrier, before the cut axes are written and the lists read
+    bool alive;
+    const u32 act = small_starts<LOCAL, PONE>(pos, x0, R, n, m.starts, &s_nst[d & 1], &alive);
+    if (!__syncthreads_or(alive)) break;
+    const int nst = s_nst[d & 1];
+    if (threadIdx.x == 0) s_nst[(d + 1) & 1] = 0;
     const unsigned short *Lc = m.buf + 3 * cur * SMALL_MAX;   // current lists
     unsigned short *Ls = m.buf + 3 * (cur ^ 1) * SMALL_MAX;  // spares
-    // cut axis of each active sub-range: the coordinates of the first and
-    // last entry of each list
+    // lower child's size of each active sub-range
 #pragma unroll
     for (int r = 0; r < SMALL_ITEMS; r++) {
-      const int x = warp * SMALL_SPAN + r * 32 + lane;
-      const int st = (int)(sl_r[r] & 0xFFFFu), ln = (int)(sl_r[r] >> 16);
-      if (!((act >> r) & 1u) || x != st) continue;
+      if (r >= R) break;
+      const int st = (int)(pos.sl[r] & 0xFFFFu), ln = (int)(pos.sl[r] >> 16);
+      const int p = PONE ? 1 : pos.p[r];
+      if (x0 + r * 32 != st || st >= n || !(p > 1 || (LOCAL && ln >= 2))) continue;
+      m.spl[st] = (unsigned short)(p > 1 ? lower_count_small(ln, p) : ln / 2);
+    }
+    // and its cut axis: the coordinates of the first and last entry of each
+    // list.  By the threads of the start list: a warp instruction in FP64
+    // takes 64 cycles for one lane as for 32 (4096 elements to single ones:
+    // 190 -> 137 us, the rest is instruction issue of one SM)
+    for (int i = threadIdx.x; i < nst; i += SMALL_THREADS) {
+      const int st = (int)(m.starts[i] & 0xFFFFu), ln = (int)(m.starts[i] >> 16);
       double len[3] = {0.0, 0.0, 0.0};
 #pragma unroll
       for (int q = 0; q < 3; q++) {
@@ -1449,19 +1509,18 @@ __device__ __forceinline__ void pss_levels(int *__restrict__ perm, const double 
         len[q] = __dsub_rn(cent[(ll)q * N + hi], cent[(ll)q * N + lo]);
       }
       int ax = 0;
-      for (int q = 1; q < ndim; q++)
-        if (len[q] > len[ax]) ax = q;
+#pragma unroll
+      for (int q = 1; q < 3; q++)
+        if (q < ndim && len[q] > len[ax]) ax = q;
       m.sax[st] = (unsigned char)ax;
-      const int p = PONE ? 1 : p_r[r];
-      m.spl[st] = (unsigned short)(p > 1 ? lower_count_small(ln, p) : ln / 2);
     }
     __syncthreads();
     // side of every element of a cut sub-range, from the cut axis' list
 #pragma unroll
     for (int r = 0; r < SMALL_ITEMS; r++) {
-      if (!((act >> r) & 1u)) continue;
-      const int x = warp * SMALL_SPAN + r * 32 + lane;
-      const int st = (int)(sl_r[r] & 0xFFFFu);
+      if (r >= R || !((act >> r) & 1u)) continue;
+      const int x = x0 + r * 32;
+      const int st = (int)(pos.sl[r] & 0xFFFFu);
       m.side[Lc[m.sax[st] * SMALL_MAX + x]] = (x - st) >= (int)m.spl[st] ? 1 : 0;
     }
     __syncthreads();
@@ -1472,12 +1531,13 @@ __device__ __forceinline__ void pss_levels(int *__restrict__ perm, const double 
       int cnt = 0;
 #pragma unroll
       for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
+        if (r >= R) break;
+        const int x = x0 + r * 32;
         const bool f = ((act >> r) & 1u) && m.side[Lq[x]] == 0;  // act implies x < n
         const u32 b = __ballot_sync(0xffffffffu, f);
         if (lane == 0) {
-          m.bal[q * SMALL_ROUNDS + warp * SMALL_ITEMS + r] = b;
-          m.wpre[q * SMALL_ROUNDS + warp * SMALL_ITEMS + r] = (unsigned short)cnt;
+          m.bal[q * SMALL_ROUNDS + warp * R + r] = b;
+          m.wpre[q * SMALL_ROUNDS + warp * R + r] = (unsigned short)cnt;
         }
         cnt += __popc(b);
       }
@@ -1502,15 +1562,16 @@ __device__ __forceinline__ void pss_levels(int *__restrict__ perm, const double 
       const unsigned short *wq = m.wpre + q * SMALL_ROUNDS;
 #pragma unroll
       for (int r = 0; r < SMALL_ITEMS; r++) {
-        const int x = warp * SMALL_SPAN + r * 32 + lane;
+        if (r >= R) break;
+        const int x = x0 + r * 32;
         const bool a = (act >> r) & 1u;
-        const int st = a ? (int)(sl_r[r] & 0xFFFFu) : x;
-        const int base_st = __shfl_sync(0xffffffffu, exc, st / SMALL_SPAN);
+        const int st = a ? (int)(pos.sl[r] & 0xFFFFu) : x;
+        const int base_st = __shfl_sync(0xffffffffu, exc, ((st >> 5) * inv_r) >> 16);
         if (x >= n) continue;
         const unsigned short id = Lq[x];
         int dest = x;
         if (a) {
-          const int k = warp * SMALL_ITEMS + r, ks = st >> 5;
+          const int k = warp * R + r, ks = st >> 5;
           const u32 bx = bq[k];
           const int before = (base_x + (int)wq[k] + __popc(bx & lt)) -
                              (base_st + (int)wq[ks] + __popc(bq[ks] & ((1u << (st & 31)) - 1u)));
@@ -1526,12 +1587,12 @@ __device__ __forceinline__ void pss_levels(int *__restrict__ perm, const double 
   const unsigned short *Lc = m.buf + 3 * cur * SMALL_MAX;
 #pragma unroll
   for (int r = 0; r < SMALL_ITEMS; r++) {
-    const int x = warp * SMALL_SPAN + r * 32 + lane;
-    if (x < n) {
+    const int x = x0 + r * 32;
+    if (r < R && x < n) {
       const int a = oax_r[r] < 0 ? 0 : oax_r[r];
       const int e = m.gl[Lc[a * SMALL_MAX + x]];
       perm[start + x] = e;
-      if (part) part[e] = r0 + (PONE ? 0 : rk_r[r]);
+      if (part) part[e] = r0 + (PONE ? 0 : pos.rk[r]);
     }
   }
 }
@@ -1546,6 +1607,8 @@ k_rcb_small_ps(int *__restrict__ perm, const int *__restrict__ lists, int *__res
   extern __shared__ __align__(16) unsigned char pss_smem[];
   const PssSmem m = pss_carve(pss_smem);
   __shared__ int wsum[3][SMALL_WARPS];
+  __shared__ int s_nst[2];
+  if (threadIdx.x == 0) s_nst[0] = s_nst[1] = 0;
   const ll sg = blockIdx.x;
   const ll start = seg_start[sg];
   const int n = (int)seg_n[sg], p0 = seg_p[sg], r0 = seg_r0[sg];
@@ -1570,9 +1633,9 @@ k_rcb_small_ps(int *__restrict__ perm, const int *__restrict__ lists, int *__res
   }
   __syncthreads();
   if (p0 == 1)
-    pss_levels<LOCAL, true>(perm, cent, N, ndim, start, n, p0, r0, part, m, wsum);
+    pss_levels<LOCAL, true>(perm, cent, N, ndim, start, n, p0, r0, part, m, wsum, s_nst);
   else
-    pss_levels<LOCAL, false>(perm, cent, N, ndim, start, n, p0, r0, part, m, wsum);
+    pss_levels<LOCAL, false>(perm, cent, N, ndim, start, n, p0, r0, part, m, wsum, s_nst);
 }
 
 static void rcb_presorted(DBuf<int> &perm, SegTable &t, const double *cent, ll N, int ndim,
@@ -1848,13 +1911,13 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
                                 (int)small_smem));
         k_rcb_small<true><<<(unsigned)nseg, SMALL_THREADS, small_smem, st>>>(
             perm.p, ws.rank.p, ws.uniq.p, N, ndim, t.start.p, t.n.p, t.p.p, t.r0.p,
-            part_of_elem);
+            part_of_elem, nullptr);
       } else {
         CK(cudaFuncSetAttribute(k_rcb_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)small_smem));
         k_rcb_small<false><<<(unsigned)nseg, SMALL_THREADS, small_smem, st>>>(
             perm.p, ws.rank.p, ws.uniq.p, N, ndim, t.start.p, t.n.p, t.p.p, t.r0.p,
-            part_of_elem);
+            part_of_elem, nullptr);
       }
       CK_LAUNCH();
       if (level_log) {

@@ -16,13 +16,15 @@ enum BisectKind { BISECT_RCB = 0, BISECT_RIB = 1 };
 // every buffer themselves (no allocation, no library stream).  rank / uniq:
 // ndim x N order-preserving coordinate ranks (equal values -> equal rank)
 // and the coordinate value of each rank; segments of at most rcb_small_max()
-// elements.  rcb_small_prepare() sets the kernels' shared-memory limit on the
+// elements.  sparse (device, may be null): ndim flags, the axis' ranks are
+// numbers of elements strictly below in one segment of all N; they are made
+// dense, in uniq too.  rcb_small_prepare() sets the kernels' shared-memory limit on the
 // current device (once per device, before the first launch).
 int rcb_small_max();
 cudaError_t rcb_small_prepare();
-cudaError_t rcb_small_launch(int *perm, const u32 *rank, const double *uniq, ll N, int ndim,
+cudaError_t rcb_small_launch(int *perm, const u32 *rank, double *uniq, ll N, int ndim,
                              const ll *seg_start, const ll *seg_n, const int *seg_p,
-                             const int *seg_r0, ll nseg, bool local, int *part,
+                             const int *seg_r0, ll nseg, bool local, const int *sparse, int *part,
                              cudaStream_t stream);
 
 struct BisectWs {

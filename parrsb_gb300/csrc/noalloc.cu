@@ -22,13 +22,16 @@ namespace {
 
 constexpr int NA_MAX = 8192;  // elements (the CTA-resident recursion limit)
 constexpr int NA_MAXDEV = 64;
+constexpr int NA_THREADS = 1024, NA_SLICES = 8, NA_CROWD = 64;  // k_na_ranks
+constexpr int NA_RANKS_SMEM = NA_MAX * (8 + 4 + 2 + 4);         // keys, counts, list, values below
+static_assert(NA_SLICES * NA_THREADS >= NA_MAX, "an element per thread");
 
 constexpr size_t na_round(size_t b) { return (b + 255) & ~(size_t)255; }
 constexpr size_t NA_CENT = 0;                                           // double [3][NA_MAX]
 constexpr size_t NA_UNIQ = NA_CENT + na_round(3 * NA_MAX * sizeof(double));  // double [3][NA_MAX]
 constexpr size_t NA_RANK = NA_UNIQ + na_round(3 * NA_MAX * sizeof(double));  // u32 [3][NA_MAX]
 constexpr size_t NA_PERM = NA_RANK + na_round(3 * NA_MAX * sizeof(u32));     // int [NA_MAX]
-constexpr size_t NA_SEG = NA_PERM + na_round(NA_MAX * sizeof(int));          // 2 ll + 2 int
+constexpr size_t NA_SEG = NA_PERM + na_round(NA_MAX * sizeof(int));          // 2 ll + 5 int
 constexpr size_t NA_BYTES = NA_SEG + 256;                                    // 524,544 bytes
 
 // Nothing in it needs to start at zero: every word a kernel reads is written
@@ -43,7 +46,7 @@ NaDev na_dev[NA_MAXDEV];
 std::mutex na_mu;
 
 __global__ void k_na_ranks(const double *__restrict__ cent, int n, u32 *__restrict__ rank,
-                           double *__restrict__ uniq);
+                           double *__restrict__ uniq, int *__restrict__ sparse);
 
 // Once per device, with that device current: the scratch address and the
 // shared-memory limits of the rank and recursion kernels.
@@ -56,7 +59,7 @@ cudaError_t na_setup(int dev, unsigned char **out) {
     e = rcb_small_prepare();
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_na_ranks, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             NA_MAX * (int)sizeof(unsigned long long));
+                             NA_RANKS_SMEM);
     if (e != cudaSuccess) return e;
     na_dev[dev].ptr = static_cast<unsigned char *>(p);
     na_dev[dev].ready = true;
@@ -70,34 +73,131 @@ cudaError_t na_setup(int dev, unsigned char **out) {
 __global__ void k_na_init(const double *__restrict__ xyz, int n, int nv, int ndim, int nparts,
                           double *__restrict__ cent, int *__restrict__ perm,
                           ll *__restrict__ seg_ll, int *__restrict__ seg_int) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e == 0) seg_ll[0] = 0, seg_ll[1] = n, seg_int[0] = nparts, seg_int[1] = 0;
+  // a thread per element and axis: three times the chains in flight
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) seg_ll[0] = 0, seg_ll[1] = n, seg_int[0] = nparts, seg_int[1] = 0;
+  const int e = t / ndim, d = t - e * ndim;
   if (e >= n) return;
-  double c[3] = {0.0, 0.0, 0.0};
-  const double *x = xyz + (ll)e * nv * ndim;
-  for (int v = 0; v < nv; v++)
-    for (int d = 0; d < ndim; d++) c[d] = __dadd_rn(c[d], x[v * ndim + d]);
-  for (int d = 0; d < ndim; d++) c[d] = __ddiv_rn(c[d], (double)nv);
-  for (int d = 0; d < 3; d++) cent[(ll)d * n + e] = c[d];
-  perm[e] = e;
+  const double *x = xyz + (ll)e * nv * ndim + d;
+  double c = 0.0;
+  for (int v = 0; v < nv; v++) c = __dadd_rn(c, x[v * ndim]);
+  cent[(ll)d * n + e] = __ddiv_rn(c, (double)nv);
+  if (d == 0) perm[e] = e;
 }
 
-// rank = number of centroids strictly below on the axis (ties share a rank,
-// the order is that of the values); uniq[rank] = the value.  Block (x, a)
-// ranks 256 elements of axis a against all n keys held in shared memory.
-__global__ void __launch_bounds__(256)
+// rank = number of values below on the axis (ties share a rank, the order is
+// that of the values); uniq[rank] = the value.  Every block of axis blockIdx.y
+// puts all n centroids into buckets, one per element, linear in the value,
+// marks one item of every value, and ranks its share of the elements: the
+// values of the buckets below, and the smaller ones of its own bucket.  Where
+// more than NA_CROWD items with different values share a bucket, marking would
+// take too long: the rank is then the number of elements below (sparse[axis]).  Bound by the latency of about eight
+// barriers; counting against all n values took twice as long (31 -> 17
+// us at 3315 elements).  NA_SLICES blocks per axis keep values that crowd
+// into few buckets (ties, outliers) within the cost of that.
+__global__ void __launch_bounds__(NA_THREADS)
 k_na_ranks(const double *__restrict__ cent, int n, u32 *__restrict__ rank,
-           double *__restrict__ uniq) {
-  extern __shared__ unsigned long long na_keys[];
+           double *__restrict__ uniq, int *__restrict__ sparse) {
+  extern __shared__ __align__(16) unsigned long long na_keys[];
+  u32 *cnt = reinterpret_cast<u32 *>(na_keys + NA_MAX);
+  unsigned short *list = reinterpret_cast<unsigned short *>(cnt + NA_MAX);
+  u32 *below = reinterpret_cast<u32 *>(list + NA_MAX);  // values before a position of list
+  __shared__ unsigned long long s_min, s_max;
+  constexpr unsigned short FIRST = 0x8000;  // list: the marked item of a value
+  constexpr int PER = NA_MAX / NA_THREADS;
   const int a = blockIdx.y;
   const double *c = cent + (ll)a * n;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) na_keys[j] = ordered_key(c[j]);
+  if (threadIdx.x == 0) s_min = ~0ull, s_max = 0ull;
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  unsigned long long mn = ~0ull, mx = 0ull;
+  for (int j = threadIdx.x; j < n; j += NA_THREADS) {
+    const unsigned long long k = ordered_key(c[j]);
+    na_keys[j] = k;
+    cnt[j] = 0u;
+    mn = k < mn ? k : mn, mx = k > mx ? k : mx;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long p = __shfl_xor_sync(0xffffffffu, mn, o);
+    const unsigned long long q = __shfl_xor_sync(0xffffffffu, mx, o);
+    mn = p < mn ? p : mn, mx = q > mx ? q : mx;
+  }
+  if ((threadIdx.x & 31) == 0) atomicMin(&s_min, mn), atomicMax(&s_max, mx);
+  __syncthreads();
+  const int em = max(1, max(key_exp(s_min), key_exp(s_max)));
+  const ll f0 = key_fixed(s_min, em);
+  const unsigned long long range = (unsigned long long)(key_fixed(s_max, em) - f0);
+  const int sh = max(0, 32 - __clzll((ll)range));
+  const float line = (float)n / ((float)(u32)(range >> sh) + 1.0f);
+  auto bucket = [&](unsigned long long k) {
+    const u32 q = (u32)((unsigned long long)(key_fixed(k, em) - f0) >> sh);
+    return min(n - 1, (int)((float)q * line));
+  };
+  int bk[PER];
+#pragma unroll
+  for (int r = 0; r < PER; r++) {
+    const int j = threadIdx.x + r * NA_THREADS;
+    if (j >= n) break;
+    bk[r] = bucket(na_keys[j]);
+    atomicAdd(&cnt[bk[r]], 1u);
+  }
+  __syncthreads();
+  cta_scan<NA_MAX, NA_THREADS>(cnt, n);
+#pragma unroll
+  for (int r = 0; r < PER; r++) {
+    const int j = threadIdx.x + r * NA_THREADS;
+    if (j >= n) break;
+    const u32 p = atomicAdd(&cnt[bk[r]], 1u);
+    list[p] = (unsigned short)j;
+    below[p] = 0u;
+    bk[r] |= (int)p << 16;
+  }
+  __syncthreads();  // (cnt: now the end of every bucket)
+  // a bucket is crowded when it is long and some item differs from its first
+  bool crowd = false;
+#pragma unroll
+  for (int r = 0; r < PER; r++) {
+    const int j = threadIdx.x + r * NA_THREADS;
+    if (j >= n) break;
+    const int b = bk[r] & 0xFFFF, j0 = b ? (int)cnt[b - 1] : 0, j1 = (int)cnt[b];
+    crowd = crowd || (j1 - j0 > NA_CROWD && na_keys[list[j0]] != na_keys[j]);
+  }
+  const bool dense = !__syncthreads_or(crowd);
+  if (blockIdx.x == 0 && threadIdx.x == 0) sparse[a] = !dense;
+  if (dense) {
+    // marked: no item before it in the list of its bucket holds the same value
+    // (a long bucket holds a single value)
+    u32 first = 0;
+#pragma unroll
+    for (int r = 0; r < PER; r++) {
+      const int j = threadIdx.x + r * NA_THREADS;
+      if (j >= n) break;
+      const unsigned long long k = na_keys[j];
+      const int b = bk[r] & 0xFFFF, p = bk[r] >> 16;
+      bool f = true;
+      for (int q = b ? (int)cnt[b - 1] : 0; q < p && f; q++) f = na_keys[list[q]] != k;
+      first |= f ? 1u << r : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < PER; r++)
+      if ((first >> r) & 1u) {
+        const int p = bk[r] >> 16;
+        list[p] |= FIRST;
+        below[p] = 1u;
+      }
+    __syncthreads();
+    cta_scan<NA_MAX, NA_THREADS>(below, n);
+  }
+  const int share = (n + NA_SLICES - 1) / NA_SLICES, i = blockIdx.x * share + threadIdx.x;
+  if ((int)threadIdx.x >= share || i >= n) return;
   const unsigned long long k = na_keys[i];
-  u32 r = 0;
-  for (int j = 0; j < n; j++) r += na_keys[j] < k;
+  const int b = bucket(k), j0 = b ? (int)cnt[b - 1] : 0, j1 = (int)cnt[b];
+  u32 r = dense ? below[j0] : (u32)j0;
+  const int jn = dense && j1 - j0 > NA_CROWD ? j0 : j1;  // (a single value)
+  for (int j = j0; j < jn; j++) {
+    const unsigned l = list[j];
+    r += (!dense || (l & FIRST)) && na_keys[l & ~(unsigned)FIRST] < k;
+  }
   rank[(ll)a * n + i] = r;
   const double v = c[i];
   uniq[(ll)a * n + r] = v == 0.0 ? 0.0 : v;  // -0 and +0 share a rank
@@ -128,7 +228,7 @@ extern "C" PARRSB_API int parrsb_part_mesh_rcb_noalloc(int *d_part, const double
   int *perm = reinterpret_cast<int *>(base + NA_PERM);
   ll *seg_ll = reinterpret_cast<ll *>(base + NA_SEG);
   int *seg_int = reinterpret_cast<int *>(base + NA_SEG + 2 * sizeof(ll));
-  k_na_init<<<(nel + 255) / 256, 256, 0, st>>>(d_xyz, nel, nv, ndim, P, cent, perm, seg_ll,
+  k_na_init<<<(nel * ndim + 127) / 128, 128, 0, st>>>(d_xyz, nel, nv, ndim, P, cent, perm, seg_ll,
                                                seg_int);
   if (cudaGetLastError() != cudaSuccess) return PARRSB_ERR_CUDA;
   if (P == 1) {
@@ -136,11 +236,11 @@ extern "C" PARRSB_API int parrsb_part_mesh_rcb_noalloc(int *d_part, const double
       return PARRSB_ERR_CUDA;
     return PARRSB_OK;
   }
-  dim3 grid((nel + 255) / 256, ndim);
-  k_na_ranks<<<grid, 256, (size_t)nel * sizeof(unsigned long long), st>>>(cent, nel, rank, uniq);
+  k_na_ranks<<<dim3(NA_SLICES, ndim), NA_THREADS, NA_RANKS_SMEM, st>>>(cent, nel, rank, uniq,
+                                                                      seg_int + 2);
   if (cudaGetLastError() != cudaSuccess) return PARRSB_ERR_CUDA;
   if (rcb_small_launch(perm, rank, uniq, nel, ndim, seg_ll, seg_ll + 1, seg_int, seg_int + 1, 1,
-                       false, d_part, st) != cudaSuccess)
+                       false, seg_int + 2, d_part, st) != cudaSuccess)
     return PARRSB_ERR_CUDA;
   return PARRSB_OK;
 }

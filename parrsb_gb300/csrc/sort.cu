@@ -308,23 +308,6 @@ k_seg_rank(const u64 *__restrict__ keys, const int *__restrict__ vals,
   vout[to] = vals[i];
 }
 
-// 62-bit fixed point of the double behind an ordered key, the unit 2^(em - 1084)
-// (truncated towards zero: non-decreasing in the value)
-__device__ __forceinline__ int key_exp(u64 k) {
-  const u64 b = (k >> 63) ? (k ^ 0x8000000000000000ull) : ~k;
-  return (int)((b >> 52) & 0x7FF);
-}
-__device__ __forceinline__ ll key_fixed(u64 k, int em) {
-  const bool neg = (k >> 63) == 0;
-  const u64 b = neg ? ~k : k ^ 0x8000000000000000ull;
-  const int e = (int)((b >> 52) & 0x7FF);
-  u64 m = b & 0xFFFFFFFFFFFFFull;
-  if (e) m |= 1ull << 52;
-  const int sh = em - (e ? e : 1);  // >= 0
-  m = sh < 63 ? (m << 9) >> sh : 0ull;
-  return neg ? -(ll)m : (ll)m;
-}
-
 // (one item of padding per eight, against bank conflicts)
 __host__ __device__ constexpr int lo_at(int i) { return i + (i >> 3); }
 constexpr size_t local_smem(int w) { return (size_t)lo_at(w) * 12; }
@@ -398,46 +381,6 @@ __device__ __forceinline__ void local_store(const u64 *sk, const u32 *sp, int m,
     if (k < m) keys[k] = sk[lo_at(k)], vals[k] = v[r];
   }
 }
-// Exclusive scan of a[0..m) in place and its largest entry, by the CTA.
-template <int W, int THREADS>
-__device__ __forceinline__ u32 local_scan(u32 *a, int m) {
-  constexpr int PER = W / THREADS;
-  __shared__ u32 ws[THREADS / 32], wm[THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  u32 v[PER], sum = 0, big = 0;
-#pragma unroll
-  for (int r = 0; r < PER; r++) {
-    const int k = threadIdx.x * PER + r;
-    v[r] = k < m ? a[k] : 0u;
-    sum += v[r];
-    big = max(big, v[r]);
-  }
-  u32 x = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u32 y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  big = __reduce_max_sync(0xffffffffu, big);
-  if (lane == 31) ws[warp] = x, wm[warp] = big;
-  __syncthreads();
-  u32 run = x - sum;
-  big = 0;
-#pragma unroll
-  for (int w = 0; w < THREADS / 32; w++) {
-    if (w < warp) run += ws[w];
-    big = max(big, wm[w]);
-  }
-#pragma unroll
-  for (int r = 0; r < PER; r++) {
-    const int k = threadIdx.x * PER + r;
-    if (k < m) a[k] = run;
-    run += v[r];
-  }
-  __syncthreads();
-  return big;
-}
-
 // Segments of at most W / 2 items: CTA b sorts those that start in
 // [b W / 2, (b + 1) W / 2), in place.  Bound by its shared-memory accesses
 // (about 40 per item; the bitonic network took 1000 instructions): 8M points
@@ -546,7 +489,7 @@ k_seg_local(u64 *__restrict__ keys, int *__restrict__ vals, const int *__restric
   for (int r = 0; r < PER; r++)
     if (threadIdx.x + r * THREADS < m) atomicAdd(&A[q[r]], 1u);
   __syncthreads();
-  const u32 big = local_scan<W, THREADS>(A, m);
+  const u32 big = cta_scan<W, THREADS>(A, m);
   if (big > BUCKET_MAX) {
     // (A and B become the places; an item's segment is known by its first place)
     u32 *sp = A;
