@@ -478,48 +478,124 @@ __device__ __forceinline__ unsigned pack_bf16(bf16 lo, bf16 hi) {
   return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
 }
 
-// Weighted neighbour mean of DIN features: 8 features (one 16-byte load per
-// neighbour) of row i starting at column c8 * 8.
-template <int DIN>
-__device__ __forceinline__ void gather_mean(const bf16 *__restrict__ H, const unsigned *ep,
-                                            int wd, int c8, float inv, float acc[8]) {
-#pragma unroll
-  for (int q = 0; q < 8; q++) acc[q] = 0.f;
-  for (int k = 0; k < wd; k++) {
-    const unsigned x = ep[(ll)k * 32];
-    const unsigned w = x >> 28;
-    if (!w) continue;
-    const ll j = x & 0x0FFFFFFFu;
-    const uint4 hv = *reinterpret_cast<const uint4 *>(H + j * DIN + c8 * 8);
-    const bf16 *hb = reinterpret_cast<const bf16 *>(&hv);
-    const float fw = (float)w;
-#pragma unroll
-    for (int q = 0; q < 8; q++) acc[q] = fmaf(fw, __bfloat162float(hb[q]), acc[q]);
-  }
-#pragma unroll
-  for (int q = 0; q < 8; q++) acc[q] *= inv;
+// Four 8x8 matrices from shared memory, one row address per lane (lanes 0-7
+// the rows of the first); the second form transposes each.
+__device__ __forceinline__ void ldsm4(unsigned *r, const bf16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4_t(unsigned *r, const bf16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
 }
 
-// One layer, tiles of 64 rows (grid-stride):
-//   A = [h_prev | weighted neighbour mean of h_prev]   (64 x 2 DIN, BF16, smem)
+// 16 bytes from global to shared memory, asynchronously; zeros instead of
+// them where keep is false
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool keep = true) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(keep ? 16 : 0));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
+// all but the newest group have arrived
+__device__ __forceinline__ void cp_wait_older() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// c[n / 8] += A B over K: 16 rows of A at a (stride KP), N = 64 rows of B at
+// w (n-major, stride KP)
+template <int K, int KP>
+__device__ __forceinline__ void mma_rows(float c[8][4], const bf16 *a, const bf16 *w) {
+  const int l = threadIdx.x & 31;
+  const bf16 *pa = a + ((l & 7) + ((l >> 3) & 1) * 8) * KP + (l >> 4) * 8;
+  const bf16 *pw = w + ((l & 7) + (l >> 4) * 8) * KP + ((l >> 3) & 1) * 8;
+#pragma unroll
+  for (int ks = 0; ks < K / 16; ks++) {
+    unsigned fa[4];
+    ldsm4(fa, pa + ks * 16);
+#pragma unroll
+    for (int np = 0; np < 4; np++) {
+      unsigned fb[4];
+      ldsm4(fb, pw + np * 16 * KP + ks * 16);
+      mma_bf16(c[2 * np], fa[0], fa[1], fa[2], fa[3], fb[0], fb[1]);
+      mma_bf16(c[2 * np + 1], fa[0], fa[1], fa[2], fa[3], fb[2], fb[3]);
+    }
+  }
+}
+
+// Two rows of 64 BF16 values (h[nt][0]: row r0, h[nt][1]: row r1, as the
+// accumulators hold them) to memory.  Neighbouring lanes trade halves, so a
+// store covers whole 32-byte sectors.
+__device__ __forceinline__ void store_rows(bf16 *out, ll r0, ll r1, const unsigned h[8][2]) {
+  const int tig = threadIdx.x & 3;
+  const bool odd = tig & 1;
+#pragma unroll
+  for (int np = 0; np < 4; np++) {
+    const int n = np * 16 + (odd ? 8 + 2 * (tig - 1) : 2 * tig);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const unsigned keep = odd ? h[2 * np + 1][q] : h[2 * np][q];
+      const unsigned give = odd ? h[2 * np][q] : h[2 * np + 1][q];
+      const unsigned got = __shfl_xor_sync(0xffffffffu, give, 1);
+      *reinterpret_cast<uint2 *>(out + (q ? r1 : r0) * MP_HID + n) =
+          odd ? make_uint2(got, keep) : make_uint2(keep, got);
+    }
+  }
+}
+
+// a b + c with BF16 a and b (an exact product) in FP32
+__device__ __forceinline__ float fma_bf16(unsigned short a, unsigned short b, float c) {
+  float d;
+  asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
+  return d;
+}
+
+// Sum over the neighbours of row i, weight times feature, of the 16 features
+// from column c16 * 16 of 64: four neighbours' 32-byte loads in flight.  (A
+// slice's padding reads the row itself and counts nothing.)
+__device__ __forceinline__ void gather_sum(const bf16 *__restrict__ H, const unsigned *ep, int wd,
+                                           ll i, int c16, float acc[16]) {
+  const ulonglong4_32a *h4 = reinterpret_cast<const ulonglong4_32a *>(H) + c16;
+#pragma unroll
+  for (int q = 0; q < 16; q++) acc[q] = 0.f;
+  for (int k0 = 0; k0 < wd; k0 += 4) {
+    unsigned x[4];
+    ulonglong4_32a hv[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) x[u] = k0 + u < wd ? ep[(ll)(k0 + u) * 32] : 0u;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const ll j = x[u] >> 28 ? (ll)(x[u] & 0x0FFFFFFFu) : i;
+      hv[u] = h4[j * (MP_HID / 16)];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned w = x[u] >> 28;
+      const unsigned short bw = (unsigned short)(__float_as_uint((float)w) >> 16);
+      if (w == 0) continue;
+      const unsigned long long hw[4] = {hv[u].x, hv[u].y, hv[u].z, hv[u].w};
+#pragma unroll
+      for (int q = 0; q < 16; q++)
+        acc[q] = fma_bf16(bw, (unsigned short)(hw[q / 4] >> (16 * (q % 4))), acc[q]);
+    }
+  }
+}
+
+// First layer, tiles of 64 rows (grid-stride):
+//   A = [features | weighted neighbour mean of the features]  (FP32)
 //   Z = A W + b (tensor cores, FP32), h = relu(Z) -> Hout (BF16)
-// AG (optional): the neighbour means, kept for the backward pass.
-// HEAD: also y = h . wo + bo (FP32) per row.
-// F32IN (first layer): inputs and neighbour means in FP32, split into a
-// high and a low BF16 part; Z = A_hi W + A_lo W (two MMAs), AG in FP32.
-template <int DIN, bool HEAD, bool F32IN = false>
+// A is split into a high and a low BF16 part; Z = A_hi W + A_lo W (two MMAs).
+// AG (optional): the neighbour means, kept for the backward pass.  Two lanes
+// per row, four features each.
 __global__ void __launch_bounds__(MP_THREADS)
-k_mp_fwd(const void *__restrict__ Hin_, const unsigned *__restrict__ ell,
-         const ll *__restrict__ slice_off, const int *__restrict__ slice_w,
-         const float *__restrict__ wsum, ll N, ll Npad, const bf16 *__restrict__ Wf,
-         const float *__restrict__ bias, bf16 *__restrict__ Hout, void *__restrict__ AG_,
-         const float *__restrict__ wo, const float *__restrict__ bo, float *__restrict__ y,
-         const float *__restrict__ Xg) {
-  constexpr int K = 2 * DIN, KP = K + 8;
-  const bf16 *__restrict__ Hin = static_cast<const bf16 *>(Hin_);
-  bf16 *__restrict__ AG = static_cast<bf16 *>(AG_);
+k_mp_first(const float *__restrict__ X, const unsigned *__restrict__ ell,
+           const ll *__restrict__ slice_off, const int *__restrict__ slice_w,
+           const float *__restrict__ wsum, ll N, ll Npad, const bf16 *__restrict__ Wf,
+           const float *__restrict__ bias, bf16 *__restrict__ Hout, float *__restrict__ AG) {
+  constexpr int K = MP_K1, KP = K + 8;
+  static_assert(MP_FIN == 8 && MP_THREADS == 2 * MP_ROWS, "two lanes per row");
   __shared__ __align__(16) bf16 sA[MP_ROWS * KP];
-  __shared__ __align__(16) bf16 sAlo[F32IN ? MP_ROWS * KP : 8];
+  __shared__ __align__(16) bf16 sAlo[MP_ROWS * KP];
   __shared__ __align__(16) bf16 sW[MP_HID * KP];
   for (int q = threadIdx.x; q < MP_HID * (K / 8); q += blockDim.x) {
     const int n = q / (K / 8), k8 = q % (K / 8);
@@ -528,130 +604,185 @@ k_mp_fwd(const void *__restrict__ Hin_, const unsigned *__restrict__ ell,
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tig = lane & 3;
-  constexpr int LPR = DIN / 8;           // lanes per row in the gather
-  constexpr int RPP = MP_THREADS / LPR;  // rows per pass of the block
+  const int r = threadIdx.x >> 1, h4 = (threadIdx.x & 1) * 4;
   const ll ntiles = Npad / MP_ROWS;
   for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const ll base = tile * MP_ROWS;
+    const ll base = tile * MP_ROWS, i = base + r;
     __syncthreads();  // sA is free again (and sW is loaded)
-    if (F32IN) {  // one thread per row, 8 FP32 features
-      const float *Hf = static_cast<const float *>(Hin_);
-      float *AGf = static_cast<float *>(AG_);
-      for (int r = threadIdx.x; r < MP_ROWS; r += MP_THREADS) {
-        const ll i = base + r;
-        float sv[8] = {0, 0, 0, 0, 0, 0, 0, 0}, acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (i < N) {
-          const float4 a = reinterpret_cast<const float4 *>(Hf + i * 8)[0];
-          const float4 b = reinterpret_cast<const float4 *>(Hf + i * 8)[1];
-          sv[0] = a.x, sv[1] = a.y, sv[2] = a.z, sv[3] = a.w;
-          sv[4] = b.x, sv[5] = b.y, sv[6] = b.z, sv[7] = b.w;
-          const ll sl = i >> 5;
-          const unsigned *ep = ell + slice_off[sl] + (i & 31);
-          const int wd = slice_w[sl];
-          for (int k = 0; k < wd; k++) {
-            const unsigned x = ep[(ll)k * 32];
-            const unsigned w = x >> 28;
-            if (!w) continue;
-            const ll j = x & 0x0FFFFFFFu;
-            const float4 c = reinterpret_cast<const float4 *>(Hf + j * 8)[0];
-            const float4 d = reinterpret_cast<const float4 *>(Hf + j * 8)[1];
-            const float fw = (float)w;
-            acc[0] = fmaf(fw, c.x, acc[0]), acc[1] = fmaf(fw, c.y, acc[1]);
-            acc[2] = fmaf(fw, c.z, acc[2]), acc[3] = fmaf(fw, c.w, acc[3]);
-            acc[4] = fmaf(fw, d.x, acc[4]), acc[5] = fmaf(fw, d.y, acc[5]);
-            acc[6] = fmaf(fw, d.z, acc[6]), acc[7] = fmaf(fw, d.w, acc[7]);
-          }
-          const float ws = wsum[i];
-          const float inv = ws > 0.f ? 1.f / ws : 0.f;
-#pragma unroll
-          for (int q = 0; q < 8; q++) acc[q] *= inv;
-        }
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const bf16 h0 = __float2bfloat16_rn(sv[q]), h1 = __float2bfloat16_rn(acc[q]);
-          sA[r * KP + q] = h0;
-          sAlo[r * KP + q] = __float2bfloat16_rn(sv[q] - __bfloat162float(h0));
-          sA[r * KP + DIN + q] = h1;
-          sAlo[r * KP + DIN + q] = __float2bfloat16_rn(acc[q] - __bfloat162float(h1));
-        }
-        if (AGf && i < Npad) {
-          reinterpret_cast<float4 *>(AGf + i * 8)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-          reinterpret_cast<float4 *>(AGf + i * 8)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-        }
+    float4 self = make_float4(0.f, 0.f, 0.f, 0.f), acc = self;
+    if (i < N) {
+      self = *reinterpret_cast<const float4 *>(X + i * 8 + h4);
+      const ll sl = i >> 5;
+      const unsigned *ep = ell + slice_off[sl] + (i & 31);
+      const int wd = slice_w[sl];
+#pragma unroll 4
+      for (int k = 0; k < wd; k++) {
+        const unsigned x = ep[(ll)k * 32], w = x >> 28;
+        const ll j = w ? (ll)(x & 0x0FFFFFFFu) : i;
+        const float4 c = *reinterpret_cast<const float4 *>(X + j * 8 + h4);
+        const float fw = (float)w;
+        acc.x = w ? fmaf(fw, c.x, acc.x) : acc.x, acc.y = w ? fmaf(fw, c.y, acc.y) : acc.y;
+        acc.z = w ? fmaf(fw, c.z, acc.z) : acc.z, acc.w = w ? fmaf(fw, c.w, acc.w) : acc.w;
       }
-    } else
-    for (int r = threadIdx.x / LPR; r < MP_ROWS; r += RPP) {
-      const int c8 = threadIdx.x % LPR;
-      const ll i = base + r;
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      uint4 self = make_uint4(0u, 0u, 0u, 0u);
-      if (i < N) {
-        self = *reinterpret_cast<const uint4 *>(Hin + i * DIN + c8 * 8);
-        const ll sl = i >> 5;
-        const float ws = wsum[i];
-        gather_mean<DIN>(Hin, ell + slice_off[sl] + (i & 31), slice_w[sl], c8,
-                         ws > 0.f ? 1.f / ws : 0.f, acc);
-      }
-      __align__(16) bf16 ag[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) ag[q] = __float2bfloat16_rn(acc[q]);
-      *reinterpret_cast<uint4 *>(sA + r * KP + c8 * 8) = self;
-      *reinterpret_cast<uint4 *>(sA + r * KP + DIN + c8 * 8) = *reinterpret_cast<uint4 *>(ag);
-      if (AG) *reinterpret_cast<uint4 *>(AG + i * DIN + c8 * 8) = *reinterpret_cast<uint4 *>(ag);
+      const float ws = wsum[i];
+      const float inv = ws > 0.f ? 1.f / ws : 0.f;
+      acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
     }
+    const float sv[4] = {self.x, self.y, self.z, self.w}, av[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bf16 h0 = __float2bfloat16_rn(sv[q]), h1 = __float2bfloat16_rn(av[q]);
+      sA[r * KP + h4 + q] = h0;
+      sAlo[r * KP + h4 + q] = __float2bfloat16_rn(sv[q] - __bfloat162float(h0));
+      sA[r * KP + MP_FIN + h4 + q] = h1;
+      sAlo[r * KP + MP_FIN + h4 + q] = __float2bfloat16_rn(av[q] - __bfloat162float(h1));
+    }
+    if (AG) *reinterpret_cast<float4 *>(AG + i * 8 + h4) = acc;
     __syncthreads();
     float c[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-    const bf16 *ar0 = sA + (warp * 16 + g) * KP, *ar1 = ar0 + 8 * KP;
-#pragma unroll
-    for (int ks = 0; ks < K / 16; ks++) {
-      const int k0 = ks * 16 + 2 * tig;
-      const unsigned a0 = *reinterpret_cast<const unsigned *>(ar0 + k0);
-      const unsigned a1 = *reinterpret_cast<const unsigned *>(ar1 + k0);
-      const unsigned a2 = *reinterpret_cast<const unsigned *>(ar0 + k0 + 8);
-      const unsigned a3 = *reinterpret_cast<const unsigned *>(ar1 + k0 + 8);
-#pragma unroll
-      for (int nt = 0; nt < 8; nt++) {
-        const bf16 *bp = sW + (nt * 8 + g) * KP + k0;
-        mma_bf16(c[nt], a0, a1, a2, a3, *reinterpret_cast<const unsigned *>(bp),
-                 *reinterpret_cast<const unsigned *>(bp + 8));
-      }
-      if (F32IN) {  // the low parts of the inputs, same weights
-        const bf16 *lr0 = sAlo + (warp * 16 + g) * KP, *lr1 = lr0 + 8 * KP;
-        const unsigned l0 = *reinterpret_cast<const unsigned *>(lr0 + k0);
-        const unsigned l1 = *reinterpret_cast<const unsigned *>(lr1 + k0);
-        const unsigned l2 = *reinterpret_cast<const unsigned *>(lr0 + k0 + 8);
-        const unsigned l3 = *reinterpret_cast<const unsigned *>(lr1 + k0 + 8);
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-          const bf16 *bp = sW + (nt * 8 + g) * KP + k0;
-          mma_bf16(c[nt], l0, l1, l2, l3, *reinterpret_cast<const unsigned *>(bp),
-                   *reinterpret_cast<const unsigned *>(bp + 8));
-        }
-      }
-    }
-    const ll r0 = base + warp * 16 + g, r1 = r0 + 8;
-    float y0 = 0.f, y1 = 0.f;
+    mma_rows<K, KP>(c, sA + warp * 16 * KP, sW);
+    mma_rows<K, KP>(c, sAlo + warp * 16 * KP, sW);  // the low parts, same weights
+    unsigned h[8][2];
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
       const int n = nt * 8 + 2 * tig;
-      const float h00 = fmaxf(c[nt][0] + bias[n], 0.f), h01 = fmaxf(c[nt][1] + bias[n + 1], 0.f);
-      const float h10 = fmaxf(c[nt][2] + bias[n], 0.f), h11 = fmaxf(c[nt][3] + bias[n + 1], 0.f);
-      if (Hout) {
-        *reinterpret_cast<unsigned *>(Hout + r0 * MP_HID + n) =
-            pack_bf16(__float2bfloat16_rn(h00), __float2bfloat16_rn(h01));
-        *reinterpret_cast<unsigned *>(Hout + r1 * MP_HID + n) =
-            pack_bf16(__float2bfloat16_rn(h10), __float2bfloat16_rn(h11));
+      const float b0 = bias[n], b1 = bias[n + 1];
+      h[nt][0] = pack_bf16(__float2bfloat16_rn(fmaxf(c[nt][0] + b0, 0.f)),
+                           __float2bfloat16_rn(fmaxf(c[nt][1] + b1, 0.f)));
+      h[nt][1] = pack_bf16(__float2bfloat16_rn(fmaxf(c[nt][2] + b0, 0.f)),
+                           __float2bfloat16_rn(fmaxf(c[nt][3] + b1, 0.f)));
+    }
+    const ll r0 = base + warp * 16 + g;
+    store_rows(Hout, r0, r0 + 8, h);
+  }
+}
+
+// Neighbour sums of 64 BF16 features, 4 lanes per row, FP32 accumulation.
+//   forward:  AG = weighted mean of h over the neighbours (BF16)
+//   backward: dL/dh_prev = dH (self term) + sum_j w_ij U_j (neighbour terms),
+//             then the previous layer's ReLU: dZ_prev = dL/dh_prev *
+//             [h_prev > 0] (BF16); the graph is symmetric, so the scatter of
+//             the means' gradients is this gather.
+// Bound by the 128-byte rows that come from L2.  On its own, not in the layer
+// kernel, so that enough loads are in flight; and a block walks a contiguous
+// run of rows, whose neighbours overlap, so that most rows come from L1.
+// A lane takes 32 bytes and multiplies BF16 into FP32 without converting:
+// the conversions were half of the instructions.  330K rows of 26 neighbours:
+// 72 us forward, 82 us backward (132 us with 8 lanes a row, one row at a time).
+constexpr int MG_THREADS = 512;
+template <bool BWD>
+__global__ void __launch_bounds__(MG_THREADS, 2)
+k_mp_gather(const bf16 *__restrict__ H, const unsigned *__restrict__ ell,
+            const ll *__restrict__ slice_off, const int *__restrict__ slice_w,
+            const float *__restrict__ wsum, ll N, ll Npad, const float *__restrict__ dH,
+            const bf16 *__restrict__ Hprev, bf16 *__restrict__ out) {
+  constexpr int RPB = MG_THREADS / 4;  // rows per pass of the block
+  const ll passes = (Npad + RPB - 1) / RPB;
+  const ll per = (passes + gridDim.x - 1) / gridDim.x * RPB;
+  const ll i0 = blockIdx.x * per, i1 = i0 + per < Npad ? i0 + per : Npad;
+  const int c16 = threadIdx.x & 3;
+  for (ll i = i0 + (threadIdx.x >> 2); i < i1; i += RPB) {
+    float acc[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) acc[q] = 0.f;
+    if (i < N) {
+      const ll sl = i >> 5;
+      gather_sum(H, ell + slice_off[sl] + (i & 31), slice_w[sl], i, c16, acc);
+    }
+    const ll at = i * MP_HID + c16 * 16;
+    __align__(32) bf16 o[16];
+    if (BWD) {
+      __align__(32) bf16 hb[16];
+      *reinterpret_cast<ulonglong4_32a *>(hb) =
+          *reinterpret_cast<const ulonglong4_32a *>(Hprev + at);
+      const float4 *dp = reinterpret_cast<const float4 *>(dH + at);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float4 d = dp[q];
+        const float dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+          o[4 * q + t] = __float2bfloat16_rn(
+              __bfloat162float(hb[4 * q + t]) > 0.f ? dv[t] + acc[4 * q + t] : 0.f);
       }
+    } else {
+      const float ws = i < N ? wsum[i] : 0.f;
+      const float inv = ws > 0.f ? 1.f / ws : 0.f;
+#pragma unroll
+      for (int q = 0; q < 16; q++) o[q] = __float2bfloat16_rn(acc[q] * inv);
+    }
+    *reinterpret_cast<ulonglong4_32a *>(out + at) = *reinterpret_cast<const ulonglong4_32a *>(o);
+  }
+}
+
+// Second and third layer, tiles of 64 rows (grid-stride):
+//   A = [h_prev | AG]   (64 x 128, BF16), Z = A W + b (tensor cores, FP32),
+//   h = relu(Z) -> Hout (BF16, optional)
+// HEAD: also y = h . wo + bo (FP32) per row.
+// Bound by memory: 256 bytes of A and 128 of h a row, which the next tile's
+// asynchronous copies keep in flight (330K rows: 30 to 35 us, and 72 us
+// for the gather; 270 us as one kernel, whose gather had too few warps).
+template <bool HEAD>
+__global__ void __launch_bounds__(MP_THREADS, 4)
+k_mp_layer(const bf16 *__restrict__ Hin, const bf16 *__restrict__ AG, ll N, ll Npad,
+           const bf16 *__restrict__ Wf, const float *__restrict__ bias, bf16 *__restrict__ Hout,
+           const float *__restrict__ wo, const float *__restrict__ bo, float *__restrict__ y,
+           const float *__restrict__ Xg) {
+  constexpr int K = MP_K2, KP = K + 8, BUF = MP_ROWS * KP;
+  extern __shared__ __align__(16) unsigned char ml_smem[];
+  bf16 *sA = reinterpret_cast<bf16 *>(ml_smem), *sW = sA + 2 * BUF;
+  const ll ntiles = Npad / MP_ROWS;
+  auto load = [&](ll tile, int buf) {
+    for (int q = threadIdx.x; q < MP_ROWS * (K / 8); q += MP_THREADS) {
+      const int r = q / (K / 8), k8 = q % (K / 8);
+      const ll i = tile * MP_ROWS + r;  // (the rows from N on are zero)
+      const bf16 *src = k8 < MP_HID / 8 ? Hin + i * MP_HID + k8 * 8
+                                        : AG + i * MP_HID + (k8 - MP_HID / 8) * 8;
+      cp16(sA + buf * BUF + r * KP + k8 * 8, src, i < N);
+    }
+  };
+  if ((ll)blockIdx.x < ntiles) load(blockIdx.x, 0);
+  cp_commit();
+  for (int q = threadIdx.x; q < MP_HID * (K / 8); q += MP_THREADS) {
+    const int n = q / (K / 8), k8 = q % (K / 8);
+    *reinterpret_cast<uint4 *>(sW + n * KP + k8 * 8) =
+        *reinterpret_cast<const uint4 *>(Wf + n * K + k8 * 8);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, tig = lane & 3;
+  int buf = 0;
+  for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+    if (tile + gridDim.x < ntiles) load(tile + gridDim.x, buf ^ 1);
+    cp_commit();
+    cp_wait_older();
+    __syncthreads();
+    float c[8][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
+    mma_rows<K, KP>(c, sA + buf * BUF + warp * 16 * KP, sW);
+    const ll r0 = tile * MP_ROWS + warp * 16 + g, r1 = r0 + 8;
+    float y0 = 0.f, y1 = 0.f;
+    unsigned h[8][2];
+#pragma unroll
+    for (int nt = 0; nt < 8; nt++) {
+      const int n = nt * 8 + 2 * tig;
+      const float b0 = bias[n], b1 = bias[n + 1];
+      const bf16 h00 = __float2bfloat16_rn(fmaxf(c[nt][0] + b0, 0.f));
+      const bf16 h01 = __float2bfloat16_rn(fmaxf(c[nt][1] + b1, 0.f));
+      const bf16 h10 = __float2bfloat16_rn(fmaxf(c[nt][2] + b0, 0.f));
+      const bf16 h11 = __float2bfloat16_rn(fmaxf(c[nt][3] + b1, 0.f));
+      h[nt][0] = pack_bf16(h00, h01), h[nt][1] = pack_bf16(h10, h11);
       if (HEAD) {
         // the head reads the BF16-rounded activations, as the backward does
-        y0 = fmaf(__bfloat162float(__float2bfloat16_rn(h00)), wo[n], y0);
-        y0 = fmaf(__bfloat162float(__float2bfloat16_rn(h01)), wo[n + 1], y0);
-        y1 = fmaf(__bfloat162float(__float2bfloat16_rn(h10)), wo[n], y1);
-        y1 = fmaf(__bfloat162float(__float2bfloat16_rn(h11)), wo[n + 1], y1);
+        y0 = fmaf(__bfloat162float(h00), wo[n], y0);
+        y0 = fmaf(__bfloat162float(h01), wo[n + 1], y0);
+        y1 = fmaf(__bfloat162float(h10), wo[n], y1);
+        y1 = fmaf(__bfloat162float(h11), wo[n + 1], y1);
       }
     }
+    if (Hout) store_rows(Hout, r0, r1, h);
     if (HEAD) {
       y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
       y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
@@ -662,64 +793,117 @@ k_mp_fwd(const void *__restrict__ Hin_, const unsigned *__restrict__ ell,
         y[r1] = y1 + bo[0] + Xg[r1 * MP_FIN + 4];
       }
     }
+    __syncthreads();  // this buffer is free
   }
 }
+constexpr int ML_SMEM = (2 * MP_ROWS + MP_HID) * (MP_K2 + 8) * (int)sizeof(bf16);
 
 // ---------------------------------------------------------------------------
 // Loss and backward kernels (training)
 // ---------------------------------------------------------------------------
-// One block per group: sign-invariant cosine loss between the centred
-// prediction yc = y - mean(y) and the centred label fc:
+// Sign-invariant cosine loss between the centred prediction yc = y - mean(y)
+// and the centred label fc:
 //   loss_g = 1 - (yc . fc)^2 / (|yc|^2 |fc|^2)
 // and dloss_g / dy_i = (-2 c / (s ff) fc_i + 2 c^2 / (s^2 ff) yc_i) / G with
 // c = yc . fc, s = |yc|^2, ff = |fc|^2 (the centring adds nothing: both
 // vectors sum to zero).  G = number of groups (the loss is their mean).
-__global__ void __launch_bounds__(256)
-k_mp_loss(const float *__restrict__ y, const double *__restrict__ lab,
-          const ll *__restrict__ gstart, const ll *__restrict__ gn, int G,
-          float *__restrict__ dy, double *__restrict__ loss) {
-  const int g = blockIdx.x;
-  const ll b = gstart[g], n = gn[g];
+// Three launches: means and centred moments of tiles of ML_TILE rows, their
+// merge per group, the gradient.  (One block per group was bound by the
+// largest group: 331 -> 43 us on 24 meshes of 1000 to 64000 elements.)
+constexpr int ML_THREADS = 256, ML_ITEMS = 4, ML_TILE = ML_THREADS * ML_ITEMS;
+// n, means and centred moments of rows of y and f
+struct LossSum {
+  double n, my, mf, c, s, ff;
+};
+__global__ void __launch_bounds__(ML_THREADS)
+k_mp_loss_sums(const FTile *__restrict__ tiles, const float *__restrict__ y,
+               const double *__restrict__ lab, LossSum *__restrict__ part) {
+  const FTile t = tiles[blockIdx.x];
   __shared__ double sh[32];
-  __shared__ double bc[5];
-  double sy = 0.0, sl = 0.0;
-  for (ll i = b + threadIdx.x; i < b + n; i += blockDim.x) sy += y[i], sl += lab[i];
+  __shared__ double bc[2];
+  double vy[ML_ITEMS], vf[ML_ITEMS], sy = 0.0, sf = 0.0;
+#pragma unroll
+  for (int k = 0; k < ML_ITEMS; k++) {
+    const ll i = t.b + threadIdx.x + k * ML_THREADS;
+    vy[k] = i < t.e ? (double)y[i] : 0.0, vf[k] = i < t.e ? lab[i] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < ML_ITEMS; k++) sy += vy[k], sf += vf[k];
   sy = mp_block_sum(sy, sh);
-  sl = mp_block_sum(sl, sh);
-  if (threadIdx.x == 0) bc[0] = sy / (double)n, bc[1] = sl / (double)n;
+  sf = mp_block_sum(sf, sh);
+  const double n = (double)(t.e - t.b);
+  if (threadIdx.x == 0) bc[0] = sy / n, bc[1] = sf / n;
   __syncthreads();
-  const double my = bc[0], ml = bc[1];
+  const double my = bc[0], mf = bc[1];
   double c = 0.0, s = 0.0, ff = 0.0;
-  for (ll i = b + threadIdx.x; i < b + n; i += blockDim.x) {
-    const double yc = (double)y[i] - my, fc = lab[i] - ml;
+#pragma unroll
+  for (int k = 0; k < ML_ITEMS; k++) {
+    if (t.b + threadIdx.x + k * ML_THREADS >= t.e) break;
+    const double yc = vy[k] - my, fc = vf[k] - mf;
     c += yc * fc, s += yc * yc, ff += fc * fc;
   }
   c = mp_block_sum(c, sh);
   s = mp_block_sum(s, sh);
   ff = mp_block_sum(ff, sh);
-  if (threadIdx.x == 0) {
-    const bool ok = s > 1e-30 && ff > 1e-30;
-    bc[2] = ok ? -2.0 * c / (s * ff) / (double)G : 0.0;
-    bc[3] = ok ? 2.0 * c * c / (s * s * ff) / (double)G : 0.0;
-    loss[g] = ok ? 1.0 - c * c / (s * ff) : 1.0;
+  if (threadIdx.x == 0) part[blockIdx.x] = LossSum{n, my, mf, c, s, ff};
+}
+// a warp per group; coef: mean(y), mean(f), factors of fc and yc in dy
+__global__ void k_mp_loss_groups(const LossSum *__restrict__ part, const int *__restrict__ tile0,
+                                 int G, double4_32a *__restrict__ coef, double *__restrict__ loss) {
+  const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (g >= G) return;
+  auto sum = [](double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  // the group's means, then its moments about them: a tile's own plus those
+  // of its means
+  double n = 0.0, my = 0.0, mf = 0.0, c = 0.0, s = 0.0, ff = 0.0;
+  for (int t = tile0[g] + lane; t < tile0[g + 1]; t += 32)
+    n += part[t].n, my += part[t].n * part[t].my, mf += part[t].n * part[t].mf;
+  n = sum(n);
+  my = sum(my) / n, mf = sum(mf) / n;
+  for (int t = tile0[g] + lane; t < tile0[g + 1]; t += 32) {
+    const LossSum a = part[t];
+    const double dy = a.my - my, df = a.mf - mf;
+    c += a.c + a.n * dy * df, s += a.s + a.n * dy * dy, ff += a.ff + a.n * df * df;
   }
-  __syncthreads();
-  const double ka = bc[2], kb = bc[3];
-  for (ll i = b + threadIdx.x; i < b + n; i += blockDim.x)
-    dy[i] = (float)(ka * (lab[i] - ml) + kb * ((double)y[i] - my));
+  c = sum(c), s = sum(s), ff = sum(ff);
+  if (lane) return;
+  const bool ok = s > 1e-30 && ff > 1e-30;
+  coef[g] = make_double4_32a(my, mf, ok ? -2.0 * c / (s * ff) / (double)G : 0.0,
+                             ok ? 2.0 * c * c / (s * s * ff) / (double)G : 0.0);
+  loss[g] = ok ? 1.0 - c * c / (s * ff) : 1.0;
+}
+__global__ void __launch_bounds__(ML_THREADS)
+k_mp_loss_grad(const FTile *__restrict__ tiles, const float *__restrict__ y,
+               const double *__restrict__ lab, const double4_32a *__restrict__ coef,
+               float *__restrict__ dy) {
+  const FTile t = tiles[blockIdx.x];
+  const double4_32a k = coef[t.g];
+#pragma unroll
+  for (int q = 0; q < ML_ITEMS; q++) {
+    const ll i = t.b + threadIdx.x + q * ML_THREADS;
+    if (i < t.e) dy[i] = (float)(k.z * (lab[i] - k.y) + k.w * ((double)y[i] - k.x));
+  }
 }
 
-constexpr int MP_GB = 304;  // blocks of the backward kernels (fixed: partial sums in order)
+// blocks of the backward kernels (fixed: partial sums in order); three fit an
+// SM beside each other
+constexpr int MP_GB = 456;
 
 // Head and last ReLU: dZ3 = (dy wo) * [h3 > 0] (BF16); per block partial
 // sums of dwo = sum_i dy_i h3_i and dbo = sum_i dy_i -> part[block][65].
-__global__ void __launch_bounds__(MP_THREADS)
+constexpr int MH_THREADS = 512;
+__global__ void __launch_bounds__(MH_THREADS)
 k_mp_head_bwd(const float *__restrict__ dy, const bf16 *__restrict__ H3, ll Npad,
               const float *__restrict__ wo, bf16 *__restrict__ dZ, float *__restrict__ part) {
   const int c8 = threadIdx.x & 7;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, accb = 0.f;
-  for (ll i = (ll)blockIdx.x * (MP_THREADS / 8) + (threadIdx.x >> 3); i < Npad;
-       i += (ll)gridDim.x * (MP_THREADS / 8)) {
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, accb = 0.f, w[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) w[q] = wo[c8 * 8 + q];
+  for (ll i = (ll)blockIdx.x * (MH_THREADS / 8) + (threadIdx.x >> 3); i < Npad;
+       i += (ll)gridDim.x * (MH_THREADS / 8)) {
     const float d = dy[i];
     const uint4 hv = *reinterpret_cast<const uint4 *>(H3 + i * MP_HID + c8 * 8);
     const bf16 *hb = reinterpret_cast<const bf16 *>(&hv);
@@ -728,12 +912,12 @@ k_mp_head_bwd(const float *__restrict__ dy, const bf16 *__restrict__ H3, ll Npad
     for (int q = 0; q < 8; q++) {
       const float h = __bfloat162float(hb[q]);
       acc[q] = fmaf(d, h, acc[q]);
-      o[q] = __float2bfloat16_rn(h > 0.f ? d * wo[c8 * 8 + q] : 0.f);
+      o[q] = __float2bfloat16_rn(h > 0.f ? d * w[q] : 0.f);
     }
     if (c8 == 0) accb += d;
     *reinterpret_cast<uint4 *>(dZ + i * MP_HID + c8 * 8) = *reinterpret_cast<const uint4 *>(o);
   }
-  __shared__ float sh[MP_THREADS][9];
+  __shared__ float sh[MH_THREADS][9];
 #pragma unroll
   for (int q = 0; q < 8; q++) sh[threadIdx.x][q] = acc[q];
   sh[threadIdx.x][8] = accb;
@@ -742,9 +926,9 @@ k_mp_head_bwd(const float *__restrict__ dy, const bf16 *__restrict__ H3, ll Npad
     float s = 0.f;
     if (threadIdx.x < MP_HID) {
       const int n = threadIdx.x;
-      for (int t = n / 8; t < MP_THREADS; t += 8) s += sh[t][n % 8];
+      for (int t = n / 8; t < MH_THREADS; t += 8) s += sh[t][n % 8];
     } else {
-      for (int t = 0; t < MP_THREADS; t += 8) s += sh[t][8];
+      for (int t = 0; t < MH_THREADS; t += 8) s += sh[t][8];
     }
     part[(ll)blockIdx.x * (MP_HID + 1) + threadIdx.x] = s;
   }
@@ -754,198 +938,211 @@ k_mp_head_bwd(const float *__restrict__ dy, const bf16 *__restrict__ H3, ll Npad
 //   dA = dZ W^T (tensor cores): the first DIN columns are dL/dh_prev through
 //   the self term -> dH (FP32); the last DIN are dL/da, divided by the
 //   row's weight sum -> U (BF16), scattered to the neighbours by
-//   k_mp_gather_bwd (the graph is symmetric, so the scatter is a gather);
+//   k_mp_gather (the graph is symmetric, so the scatter is a gather);
 //   dW += A^T dZ, db += sum of dZ rows (per block, FP32) -> partials.
 // INPUT_GRAD = false for the first layer (its inputs are the features).
 // F32IN (first layer): Hprev (the features) and AG in FP32, split into high
 // and low BF16 parts for dW += A_hi^T dZ + A_lo^T dZ.
+// Bound by memory: 384 bytes in and 384 out a row.  The next tile is copied
+// while this one is multiplied, and transposing matrix loads give both
+// operands of A^T dZ; element-wise ones took most of the time before
+// (330K rows: 108 -> 61 us, first layer 84 -> 16 us).
+template <int DIN, bool INPUT_GRAD, bool F32IN>
+struct BwdSmem {
+  static constexpr int K = 2 * DIN, KP = K + 8, ZP = MP_HID + 8;
+  static constexpr int Z = MP_ROWS * ZP, A = MP_ROWS * KP;       // elements of one buffer
+  static constexpr int RAW = F32IN ? MP_ROWS * K : 0;            // FP32, two buffers
+  static constexpr int W = INPUT_GRAD ? K * ZP : 0;
+  static constexpr int BYTES = (2 * Z + 2 * A + W) * (int)sizeof(bf16) + 2 * RAW * 4;
+};
 template <int DIN, bool INPUT_GRAD, bool F32IN = false>
-__global__ void __launch_bounds__(MP_THREADS)
+__global__ void __launch_bounds__(MP_THREADS, 3)
 k_mp_bwd(const bf16 *__restrict__ dZ, const void *__restrict__ Hprev_,
          const void *__restrict__ AG_, const float *__restrict__ wsum, ll Npad,
          const bf16 *__restrict__ Wb, float *__restrict__ dH, bf16 *__restrict__ U,
          float *__restrict__ part_w, float *__restrict__ part_b) {
-  constexpr int K = 2 * DIN, KP = K + 8, ZP = MP_HID + 8;
-  constexpr int NPAIR = (K / 16) * 8;              // (m-tile, n-tile) pairs of dW
-  constexpr int PPW = NPAIR / (MP_THREADS / 32);  // per warp
-  const bf16 *__restrict__ Hprev = static_cast<const bf16 *>(Hprev_);
-  const bf16 *__restrict__ AG = static_cast<const bf16 *>(AG_);
-  __shared__ __align__(16) bf16 sZ[MP_ROWS * ZP];
-  __shared__ __align__(16) bf16 sA[MP_ROWS * KP];
-  __shared__ __align__(16) bf16 sAlo[F32IN ? MP_ROWS * KP : 8];
-  __shared__ __align__(16) bf16 sW[INPUT_GRAD ? K * ZP : 8];
+  typedef BwdSmem<DIN, INPUT_GRAD, F32IN> S;
+  constexpr int K = S::K, KP = S::KP, ZP = S::ZP, NWARP = MP_THREADS / 32;
+  // tiles of dW per warp: K / 16 by 8, whole rows of them where there are
+  // enough
+  constexpr int MT = K / 16 >= NWARP ? K / 16 / NWARP : 1;
+  constexpr int NT = K / 16 >= NWARP ? 8 : 8 / NWARP;
+  extern __shared__ __align__(16) unsigned char mb_smem[];
+  bf16 *sZ = reinterpret_cast<bf16 *>(mb_smem), *sA = sZ + 2 * S::Z, *sW = sA + 2 * S::A;
+  float *raw = reinterpret_cast<float *>(sW + S::W);
+  __shared__ float sb[NWARP][MP_HID];
+  const ll ntiles = Npad / MP_ROWS;
+  auto load = [&](ll tile, int buf) {
+    const ll base = tile * MP_ROWS;
+    for (int q = threadIdx.x; q < MP_ROWS * (MP_HID / 8); q += MP_THREADS) {
+      const int r = q / (MP_HID / 8), h8 = q % (MP_HID / 8);
+      cp16(sZ + buf * S::Z + r * ZP + h8 * 8, dZ + (base + r) * MP_HID + h8 * 8);
+    }
+    if (F32IN) {
+      const float *Hf = static_cast<const float *>(Hprev_), *Af = static_cast<const float *>(AG_);
+      for (int q = threadIdx.x; q < MP_ROWS * (K / 4); q += MP_THREADS) {
+        const int r = q / (K / 4), k4 = q % (K / 4) * 4;
+        cp16(raw + buf * S::RAW + r * K + k4,
+             k4 < DIN ? Hf + (base + r) * DIN + k4 : Af + (base + r) * DIN + k4 - DIN);
+      }
+    } else {
+      const bf16 *Hp = static_cast<const bf16 *>(Hprev_), *Ag = static_cast<const bf16 *>(AG_);
+      for (int q = threadIdx.x; q < MP_ROWS * (K / 8); q += MP_THREADS) {
+        const int r = q / (K / 8), k = q % (K / 8) * 8;
+        cp16(sA + buf * S::A + r * KP + k,
+             k < DIN ? Hp + (base + r) * DIN + k : Ag + (base + r) * DIN + k - DIN);
+      }
+    }
+  };
+  if ((ll)blockIdx.x < ntiles) load(blockIdx.x, 0);
+  cp_commit();
   if (INPUT_GRAD)
-    for (int q = threadIdx.x; q < K * (MP_HID / 8); q += blockDim.x) {
+    for (int q = threadIdx.x; q < K * (MP_HID / 8); q += MP_THREADS) {
       const int k = q / (MP_HID / 8), h8 = q % (MP_HID / 8);
       *reinterpret_cast<uint4 *>(sW + k * ZP + h8 * 8) =
           *reinterpret_cast<const uint4 *>(Wb + k * MP_HID + h8 * 8);
     }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tig = lane & 3;
-  float cw[PPW][4];
+  const int mt0 = K / 16 >= NWARP ? warp * MT : 0, nt0 = K / 16 >= NWARP ? 0 : warp * NT;
+  float cw[MT][NT][4];
 #pragma unroll
-  for (int j = 0; j < PPW; j++) cw[j][0] = cw[j][1] = cw[j][2] = cw[j][3] = 0.f;
-  float cb = 0.f;  // thread t: column t % 64, rows of half t / 64
-  const ll ntiles = Npad / MP_ROWS;
-  for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const ll base = tile * MP_ROWS;
+  for (int m = 0; m < MT; m++)
+#pragma unroll
+    for (int n = 0; n < NT; n++) cw[m][n][0] = cw[m][n][1] = cw[m][n][2] = cw[m][n][3] = 0.f;
+  float cb0 = 0.f, cb1 = 0.f;  // columns 2 lane, 2 lane + 1; 16 rows of each tile
+  int buf = 0;
+  for (ll tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+    if (tile + gridDim.x < ntiles) load(tile + gridDim.x, buf ^ 1);
+    cp_commit();
+    cp_wait_older();
     __syncthreads();
-    for (int q = threadIdx.x; q < MP_ROWS * (MP_HID / 8); q += blockDim.x) {
-      const int r = q / (MP_HID / 8), h8 = q % (MP_HID / 8);
-      *reinterpret_cast<uint4 *>(sZ + r * ZP + h8 * 8) =
-          *reinterpret_cast<const uint4 *>(dZ + (base + r) * MP_HID + h8 * 8);
-    }
+    const bf16 *z = sZ + buf * S::Z, *a = F32IN ? sA : sA + buf * S::A, *alo = sA + S::A;
     if (F32IN) {
-      const float *Hf = static_cast<const float *>(Hprev_), *Af = static_cast<const float *>(AG_);
-      for (int q = threadIdx.x; q < MP_ROWS * K; q += blockDim.x) {
+      for (int q = threadIdx.x; q < MP_ROWS * K; q += MP_THREADS) {
         const int r = q / K, k = q % K;
-        const float v = k < DIN ? Hf[(base + r) * DIN + k] : Af[(base + r) * DIN + k - DIN];
+        const float v = raw[buf * S::RAW + q];
         const bf16 h = __float2bfloat16_rn(v);
         sA[r * KP + k] = h;
-        sAlo[r * KP + k] = __float2bfloat16_rn(v - __bfloat162float(h));
+        sA[S::A + r * KP + k] = __float2bfloat16_rn(v - __bfloat162float(h));
       }
-    } else {
-      for (int q = threadIdx.x; q < MP_ROWS * (K / 8); q += blockDim.x) {
-        const int r = q / (K / 8), k8 = q % (K / 8);
-        const bf16 *src = k8 < DIN / 8 ? Hprev + (base + r) * DIN + k8 * 8
-                                       : AG + (base + r) * DIN + (k8 - DIN / 8) * 8;
-        *reinterpret_cast<uint4 *>(sA + r * KP + k8 * 8) = *reinterpret_cast<const uint4 *>(src);
-      }
+      __syncthreads();
     }
-    __syncthreads();
     if (INPUT_GRAD) {
-      constexpr int NT = K / 8;
-      float c[NT][4];
-#pragma unroll
-      for (int nt = 0; nt < NT; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-      const bf16 *ar0 = sZ + (warp * 16 + g) * ZP, *ar1 = ar0 + 8 * ZP;
-#pragma unroll
-      for (int ks = 0; ks < MP_HID / 16; ks++) {
-        const int k0 = ks * 16 + 2 * tig;
-        const unsigned a0 = *reinterpret_cast<const unsigned *>(ar0 + k0);
-        const unsigned a1 = *reinterpret_cast<const unsigned *>(ar1 + k0);
-        const unsigned a2 = *reinterpret_cast<const unsigned *>(ar0 + k0 + 8);
-        const unsigned a3 = *reinterpret_cast<const unsigned *>(ar1 + k0 + 8);
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
-          const bf16 *bp = sW + (nt * 8 + g) * ZP + k0;
-          mma_bf16(c[nt], a0, a1, a2, a3, *reinterpret_cast<const unsigned *>(bp),
-                   *reinterpret_cast<const unsigned *>(bp + 8));
-        }
-      }
-      const ll r0 = base + warp * 16 + g, r1 = r0 + 8;
+      const ll r0 = tile * MP_ROWS + warp * 16 + g, r1 = r0 + 8;
       const float w0 = wsum[r0], w1 = wsum[r1];
       const float i0 = w0 > 0.f ? 1.f / w0 : 0.f, i1 = w1 > 0.f ? 1.f / w1 : 0.f;
 #pragma unroll
-      for (int nt = 0; nt < NT; nt++) {
-        const int n = nt * 8 + 2 * tig;
-        if (n < DIN) {
-          *reinterpret_cast<float2 *>(dH + r0 * DIN + n) = make_float2(c[nt][0], c[nt][1]);
-          *reinterpret_cast<float2 *>(dH + r1 * DIN + n) = make_float2(c[nt][2], c[nt][3]);
+      for (int half = 0; half < 2; half++) {  // self columns, then neighbour columns
+        float c[8][4];
+#pragma unroll
+        for (int nt = 0; nt < 8; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
+        mma_rows<MP_HID, ZP>(c, z + warp * 16 * ZP, sW + half * MP_HID * ZP);
+        if (half == 0) {
+#pragma unroll
+          for (int nt = 0; nt < 8; nt++) {
+            const int n = nt * 8 + 2 * tig;
+            *reinterpret_cast<float2 *>(dH + r0 * DIN + n) = make_float2(c[nt][0], c[nt][1]);
+            *reinterpret_cast<float2 *>(dH + r1 * DIN + n) = make_float2(c[nt][2], c[nt][3]);
+          }
         } else {
-          *reinterpret_cast<unsigned *>(U + r0 * DIN + (n - DIN)) = pack_bf16(
-              __float2bfloat16_rn(c[nt][0] * i0), __float2bfloat16_rn(c[nt][1] * i0));
-          *reinterpret_cast<unsigned *>(U + r1 * DIN + (n - DIN)) = pack_bf16(
-              __float2bfloat16_rn(c[nt][2] * i1), __float2bfloat16_rn(c[nt][3] * i1));
+          unsigned h[8][2];
+#pragma unroll
+          for (int nt = 0; nt < 8; nt++) {
+            h[nt][0] = pack_bf16(__float2bfloat16_rn(c[nt][0] * i0),
+                                 __float2bfloat16_rn(c[nt][1] * i0));
+            h[nt][1] = pack_bf16(__float2bfloat16_rn(c[nt][2] * i1),
+                                 __float2bfloat16_rn(c[nt][3] * i1));
+          }
+          store_rows(U, r0, r1, h);
         }
       }
     }
     // dW += A^T dZ over this tile's 64 rows (k dimension of the MMA)
+    const int lr = (lane & 7), lq = lane >> 3;  // row and number of this lane's 8x8 matrix
 #pragma unroll
-    for (int j = 0; j < PPW; j++) {
-      const int pr = warp + j * (MP_THREADS / 32);
-      const int mt = pr / 8, nt = pr % 8;
+    for (int ks = 0; ks < MP_ROWS / 16; ks++) {
+      unsigned fb[NT / 2][4];
 #pragma unroll
-      for (int ks = 0; ks < MP_ROWS / 16; ks++) {
-        const int rk = ks * 16 + 2 * tig;
-        const bf16 *x0 = sA + rk * KP + mt * 16 + g;
-        const unsigned a0 = pack_bf16(x0[0], x0[KP]);
-        const unsigned a1 = pack_bf16(x0[8], x0[KP + 8]);
-        const unsigned a2 = pack_bf16(x0[8 * KP], x0[9 * KP]);
-        const unsigned a3 = pack_bf16(x0[8 * KP + 8], x0[9 * KP + 8]);
-        const bf16 *z0 = sZ + rk * ZP + nt * 8 + g;
-        const unsigned b0 = pack_bf16(z0[0], z0[ZP]);
-        const unsigned b1 = pack_bf16(z0[8 * ZP], z0[9 * ZP]);
-        mma_bf16(cw[j], a0, a1, a2, a3, b0, b1);
-        if (F32IN) {
-          const bf16 *y0 = sAlo + rk * KP + mt * 16 + g;
-          mma_bf16(cw[j], pack_bf16(y0[0], y0[KP]), pack_bf16(y0[8], y0[KP + 8]),
-                   pack_bf16(y0[8 * KP], y0[9 * KP]), pack_bf16(y0[8 * KP + 8], y0[9 * KP + 8]),
-                   b0, b1);
+      for (int np = 0; np < NT / 2; np++)
+        ldsm4_t(fb[np], z + (ks * 16 + (lq & 1) * 8 + lr) * ZP + (nt0 + 2 * np + (lq >> 1)) * 8);
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        const int at = (ks * 16 + (lq >> 1) * 8 + lr) * KP + (mt0 + m) * 16 + (lq & 1) * 8;
+#pragma unroll
+        for (int part = 0; part < (F32IN ? 2 : 1); part++) {
+          unsigned fa[4];
+          ldsm4_t(fa, (part ? alo : a) + at);
+#pragma unroll
+          for (int np = 0; np < NT / 2; np++) {
+            mma_bf16(cw[m][2 * np], fa[0], fa[1], fa[2], fa[3], fb[np][0], fb[np][1]);
+            mma_bf16(cw[m][2 * np + 1], fa[0], fa[1], fa[2], fa[3], fb[np][2], fb[np][3]);
+          }
         }
       }
     }
-    {
-      const int n = threadIdx.x % MP_HID, half = threadIdx.x / MP_HID;
-      for (int r = half * 32; r < half * 32 + 32; r++) cb += __bfloat162float(sZ[r * ZP + n]);
+#pragma unroll
+    for (int r = 0; r < MP_ROWS / NWARP; r++) {
+      const unsigned v = *reinterpret_cast<const unsigned *>(
+          z + (warp * (MP_ROWS / NWARP) + r) * ZP + 2 * lane);
+      cb0 += __uint_as_float(v << 16), cb1 += __uint_as_float(v & 0xFFFF0000u);
     }
+    __syncthreads();  // this buffer is free
   }
   // partials of this block
   float *pw = part_w + (ll)blockIdx.x * K * MP_HID;
 #pragma unroll
-  for (int j = 0; j < PPW; j++) {
-    const int pr = warp + j * (MP_THREADS / 32);
-    const int mt = pr / 8, nt = pr % 8;
-    const int m0 = mt * 16 + g, n0 = nt * 8 + 2 * tig;
-    pw[m0 * MP_HID + n0] = cw[j][0];
-    pw[m0 * MP_HID + n0 + 1] = cw[j][1];
-    pw[(m0 + 8) * MP_HID + n0] = cw[j][2];
-    pw[(m0 + 8) * MP_HID + n0 + 1] = cw[j][3];
-  }
-  __shared__ float sb[MP_THREADS];
-  sb[threadIdx.x] = cb;
-  __syncthreads();
-  if (threadIdx.x < MP_HID)
-    part_b[(ll)blockIdx.x * MP_HID + threadIdx.x] = sb[threadIdx.x] + sb[threadIdx.x + MP_HID];
-}
-
-// dL/dh_prev = dH (self term) + sum_j w_ij U_j (neighbour terms), then the
-// previous layer's ReLU: dZ_prev = dL/dh_prev * [h_prev > 0] (BF16).
-__global__ void __launch_bounds__(MP_THREADS)
-k_mp_gather_bwd(const float *__restrict__ dH, const bf16 *__restrict__ U,
-                const bf16 *__restrict__ Hprev, const unsigned *__restrict__ ell,
-                const ll *__restrict__ slice_off, const int *__restrict__ slice_w, ll N,
-                ll Npad, bf16 *__restrict__ dZ) {
-  const ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  const ll i = t >> 3;
-  const int c8 = (int)(t & 7);
-  if (i >= Npad) return;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (i < N) {
-    const ll sl = i >> 5;
-    gather_mean<MP_HID>(U, ell + slice_off[sl] + (i & 31), slice_w[sl], c8, 1.f, acc);
-  }
-  const uint4 hv = *reinterpret_cast<const uint4 *>(Hprev + i * MP_HID + c8 * 8);
-  const bf16 *hb = reinterpret_cast<const bf16 *>(&hv);
-  __align__(16) bf16 o[8];
+  for (int m = 0; m < MT; m++)
 #pragma unroll
-  for (int q = 0; q < 8; q++) {
-    const float d = dH[i * MP_HID + c8 * 8 + q] + acc[q];
-    o[q] = __float2bfloat16_rn(__bfloat162float(hb[q]) > 0.f ? d : 0.f);
+    for (int n = 0; n < NT; n++) {
+      const int m0 = (mt0 + m) * 16 + g, n0 = (nt0 + n) * 8 + 2 * tig;
+      *reinterpret_cast<float2 *>(pw + m0 * MP_HID + n0) = make_float2(cw[m][n][0], cw[m][n][1]);
+      *reinterpret_cast<float2 *>(pw + (m0 + 8) * MP_HID + n0) =
+          make_float2(cw[m][n][2], cw[m][n][3]);
+    }
+  sb[warp][2 * lane] = cb0, sb[warp][2 * lane + 1] = cb1;
+  __syncthreads();
+  if (threadIdx.x < MP_HID) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < NWARP; w++) t += sb[w][threadIdx.x];
+    part_b[(ll)blockIdx.x * MP_HID + threadIdx.x] = t;
   }
-  *reinterpret_cast<uint4 *>(dZ + i * MP_HID + c8 * 8) = *reinterpret_cast<const uint4 *>(o);
 }
 
-// Flat gradient from the per-block partials, summed in block order.
-__global__ void k_mp_grad_reduce(const float *__restrict__ pw0, const float *__restrict__ pb0,
-                                 const float *__restrict__ pw1, const float *__restrict__ pb1,
-                                 const float *__restrict__ pw2, const float *__restrict__ pb2,
-                                 const float *__restrict__ ph, int nblk, float *__restrict__ grad) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= MP_NPARAM) return;
-  const float *src;
-  ll stride;
-  int off;
-  if (q < MP_OFF_B1) src = pw0, stride = MP_K1 * MP_HID, off = q - MP_OFF_W1;
-  else if (q < MP_OFF_W2) src = pb0, stride = MP_HID, off = q - MP_OFF_B1;
-  else if (q < MP_OFF_B2) src = pw1, stride = MP_K2 * MP_HID, off = q - MP_OFF_W2;
-  else if (q < MP_OFF_W3) src = pb1, stride = MP_HID, off = q - MP_OFF_B2;
-  else if (q < MP_OFF_B3) src = pw2, stride = MP_K2 * MP_HID, off = q - MP_OFF_W3;
-  else if (q < MP_OFF_WO) src = pb2, stride = MP_HID, off = q - MP_OFF_B3;
-  else src = ph, stride = MP_HID + 1, off = q - MP_OFF_WO;
+// Flat gradient from the per-block partials: a block takes 32 parameters, a
+// warp every eighth partial of them, in a fixed order.
+__global__ void __launch_bounds__(256)
+k_mp_grad_reduce(const float *__restrict__ pw0, const float *__restrict__ pb0,
+                 const float *__restrict__ pw1, const float *__restrict__ pb1,
+                 const float *__restrict__ pw2, const float *__restrict__ pb2,
+                 const float *__restrict__ ph, int nblk, float *__restrict__ grad) {
+  __shared__ float sh[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int b = 0; b < nblk; b++) s += src[(ll)b * stride + off];
-  grad[q] = s;
+  if (q < MP_NPARAM) {
+    const float *src;
+    ll stride;
+    int off;
+    if (q < MP_OFF_B1) src = pw0, stride = MP_K1 * MP_HID, off = q - MP_OFF_W1;
+    else if (q < MP_OFF_W2) src = pb0, stride = MP_HID, off = q - MP_OFF_B1;
+    else if (q < MP_OFF_B2) src = pw1, stride = MP_K2 * MP_HID, off = q - MP_OFF_W2;
+    else if (q < MP_OFF_W3) src = pb1, stride = MP_HID, off = q - MP_OFF_B2;
+    else if (q < MP_OFF_B3) src = pw2, stride = MP_K2 * MP_HID, off = q - MP_OFF_W3;
+    else if (q < MP_OFF_WO) src = pb2, stride = MP_HID, off = q - MP_OFF_B3;
+    else src = ph, stride = MP_HID + 1, off = q - MP_OFF_WO;
+#pragma unroll 8
+    for (int b = warp; b < nblk; b += 8) s += src[(ll)b * stride + off];
+  }
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && q < MP_NPARAM) {
+    s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) s += sh[w][lane];
+    grad[q] = s;
+  }
 }
 
 // Adam (Kingma and Ba, 2015): m = b1 m + (1 - b1) g, v = b2 v + (1 - b2) g^2,
@@ -1032,12 +1229,24 @@ struct MpBuffers {
   DBuf<float> dy, dH, part_w[3], part_b[3], part_head, grad;
   DBuf<bf16> dZa, dZb, U;
   DBuf<double> loss, lab_pos;
-  DBuf<ll> d_gstart, d_gn;
+  DBuf<FTile> ltile;  // tiles of the loss, and the first of each group
+  DBuf<int> ltile0;
+  DBuf<LossSum> lpart;
+  DBuf<double4_32a> lcoef;
 };
 
 inline unsigned mp_grid(ll Npad) {
   const ll tiles = Npad / MP_ROWS;
-  return (unsigned)std::max<ll>(1, std::min<ll>(tiles, 152 * 8));
+  return (unsigned)std::max<ll>(1, std::min<ll>(tiles, 152 * 16));
+}
+
+// blocks that are on the chip at once, each with a run of rows or a tile at
+// a time
+inline unsigned mp_gather_grid(ll Npad) {
+  return (unsigned)std::max<ll>(1, std::min<ll>((Npad + 127) / 128, 152 * 2));
+}
+inline unsigned mp_layer_grid(ll Npad) {
+  return (unsigned)std::max<ll>(1, std::min<ll>(Npad / MP_ROWS, 152 * 4));
 }
 
 void mp_frames(const MpView &v, const double *cent, ll nel, int ndim, DBuf<double> &frame,
@@ -1114,25 +1323,36 @@ void mp_forward(const MpView &v, const NetDev &net, MpBuffers &B, bool keep) {
   cudaStream_t st = ctx().stream;
   const size_t nh = (size_t)v.Npad * MP_HID;
   B.H[0].ensure(nh), B.H[1].ensure(nh), B.y.ensure((size_t)v.Npad);
+  B.AG[1].ensure(nh);
   if (keep) {
     B.H[2].ensure(nh);
-    B.AG0.ensure((size_t)v.Npad * MP_FIN), B.AG[1].ensure(nh), B.AG[2].ensure(nh);
+    B.AG0.ensure((size_t)v.Npad * MP_FIN), B.AG[2].ensure(nh);
   }
   const Level &lv = *v.lv;
   const unsigned grid = mp_grid(v.Npad);
   const float *p = net.p;
-  k_mp_fwd<MP_FIN, false, true><<<grid, MP_THREADS, 0, st>>>(
-      B.X.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, net.Wf[0],
-      p + MP_OFF_B1, B.H[0].p, keep ? B.AG0.p : nullptr, nullptr, nullptr, nullptr, nullptr);
+  k_mp_first<<<grid, MP_THREADS, 0, st>>>(B.X.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p,
+                                          v.N, v.Npad, net.Wf[0], p + MP_OFF_B1, B.H[0].p,
+                                          keep ? B.AG0.p : nullptr);
   CK_LAUNCH();
-  k_mp_fwd<MP_HID, false><<<grid, MP_THREADS, 0, st>>>(
-      B.H[0].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, net.Wf[1],
-      p + MP_OFF_B2, B.H[1].p, keep ? B.AG[1].p : nullptr, nullptr, nullptr, nullptr, nullptr);
+  ensure_smem_limit(k_mp_layer<false>, ML_SMEM);
+  ensure_smem_limit(k_mp_layer<true>, ML_SMEM);
+  bf16 *ag2 = keep ? B.AG[2].p : B.AG[1].p;
+  k_mp_gather<false><<<mp_gather_grid(v.Npad), MG_THREADS, 0, st>>>(
+      B.H[0].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, nullptr, nullptr,
+      B.AG[1].p);
   CK_LAUNCH();
-  k_mp_fwd<MP_HID, true><<<grid, MP_THREADS, 0, st>>>(
-      B.H[1].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, net.Wf[2],
-      p + MP_OFF_B3, keep ? B.H[2].p : nullptr, keep ? B.AG[2].p : nullptr, p + MP_OFF_WO,
-      p + MP_OFF_BO, B.y.p, B.X.p);
+  k_mp_layer<false><<<mp_layer_grid(v.Npad), MP_THREADS, ML_SMEM, st>>>(
+      B.H[0].p, B.AG[1].p, v.N, v.Npad, net.Wf[1], p + MP_OFF_B2, B.H[1].p, nullptr, nullptr,
+      nullptr, nullptr);
+  CK_LAUNCH();
+  k_mp_gather<false><<<mp_gather_grid(v.Npad), MG_THREADS, 0, st>>>(
+      B.H[1].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, nullptr, nullptr,
+      ag2);
+  CK_LAUNCH();
+  k_mp_layer<true><<<mp_layer_grid(v.Npad), MP_THREADS, ML_SMEM, st>>>(
+      B.H[1].p, ag2, v.N, v.Npad, net.Wf[2], p + MP_OFF_B3, keep ? B.H[2].p : nullptr,
+      p + MP_OFF_WO, p + MP_OFF_BO, B.y.p, B.X.p);
   CK_LAUNCH();
 }
 
@@ -1150,39 +1370,62 @@ double mp_backward(const MpView &v, const NetDev &net, MpBuffers &B) {
   }
   B.part_head.ensure((size_t)MP_GB * (MP_HID + 1));
   B.grad.ensure(MP_NPARAM);
-  B.d_gstart.ensure((size_t)std::max(G, 1)), B.d_gn.ensure((size_t)std::max(G, 1));
-  h2d(B.d_gstart.p, v.gstart.data(), G);
-  h2d(B.d_gn.p, v.gn.data(), G);
   CK(cudaMemsetAsync(B.dy.p, 0, (size_t)v.Npad * sizeof(float), st));
+  std::vector<FTile> lt;  // (host memory of the copies: kept until the sync below)
+  std::vector<int> lt0(1, 0);
   if (G > 0) {
-    k_mp_loss<<<G, 256, 0, st>>>(B.y.p, B.lab_pos.p, B.d_gstart.p, B.d_gn.p, G, B.dy.p, B.loss.p);
+    for (int g = 0; g < G; g++) {
+      const ll e = v.gstart[g] + v.gn[g];
+      for (ll r = v.gstart[g]; r < e; r += ML_TILE)
+        lt.push_back({r, std::min<ll>(r + ML_TILE, e), g});
+      lt0.push_back((int)lt.size());
+    }
+    B.ltile.ensure(std::max<size_t>(lt.size(), 1)), B.ltile0.ensure(lt0.size());
+    B.lpart.ensure(std::max<size_t>(lt.size(), 1)), B.lcoef.ensure((size_t)G);
+    h2d(B.ltile0.p, lt0.data(), lt0.size());
+    if (!lt.empty()) {
+      h2d(B.ltile.p, lt.data(), lt.size());
+      k_mp_loss_sums<<<(unsigned)lt.size(), ML_THREADS, 0, st>>>(B.ltile.p, B.y.p, B.lab_pos.p,
+                                                                 B.lpart.p);
+      CK_LAUNCH();
+    }
+    k_mp_loss_groups<<<grid_for((ll)G * 32, 256), 256, 0, st>>>(B.lpart.p, B.ltile0.p, G,
+                                                                B.lcoef.p, B.loss.p);
     CK_LAUNCH();
+    if (!lt.empty()) {
+      k_mp_loss_grad<<<(unsigned)lt.size(), ML_THREADS, 0, st>>>(B.ltile.p, B.y.p, B.lab_pos.p,
+                                                                 B.lcoef.p, B.dy.p);
+      CK_LAUNCH();
+    }
   }
   const Level &lv = *v.lv;
   const float *p = net.p;
-  k_mp_head_bwd<<<MP_GB, MP_THREADS, 0, st>>>(B.dy.p, B.H[2].p, v.Npad, p + MP_OFF_WO, B.dZa.p,
+  k_mp_head_bwd<<<MP_GB, MH_THREADS, 0, st>>>(B.dy.p, B.H[2].p, v.Npad, p + MP_OFF_WO, B.dZa.p,
                                               B.part_head.p);
   CK_LAUNCH();
-  const unsigned gg = grid_for(v.Npad * 8, MP_THREADS);
-  k_mp_bwd<MP_HID, true><<<MP_GB, MP_THREADS, 0, st>>>(B.dZa.p, B.H[1].p, B.AG[2].p, B.wsum.p,
-                                                       v.Npad, net.Wb[2], B.dH.p, B.U.p,
-                                                       B.part_w[2].p, B.part_b[2].p);
+  constexpr int SM2 = BwdSmem<MP_HID, true, false>::BYTES, SM1 = BwdSmem<MP_FIN, false, true>::BYTES;
+  ensure_smem_limit(k_mp_bwd<MP_HID, true>, SM2);
+  ensure_smem_limit(k_mp_bwd<MP_FIN, false, true>, SM1);
+  const unsigned gg = mp_gather_grid(v.Npad);
+  k_mp_bwd<MP_HID, true><<<MP_GB, MP_THREADS, SM2, st>>>(B.dZa.p, B.H[1].p, B.AG[2].p, B.wsum.p,
+                                                         v.Npad, net.Wb[2], B.dH.p, B.U.p,
+                                                         B.part_w[2].p, B.part_b[2].p);
   CK_LAUNCH();
-  k_mp_gather_bwd<<<gg, MP_THREADS, 0, st>>>(B.dH.p, B.U.p, B.H[1].p, lv.ell.p, lv.slice_off.p,
-                                             lv.slice_w.p, v.N, v.Npad, B.dZb.p);
+  k_mp_gather<true><<<gg, MG_THREADS, 0, st>>>(B.U.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p,
+                                               nullptr, v.N, v.Npad, B.dH.p, B.H[1].p, B.dZb.p);
   CK_LAUNCH();
-  k_mp_bwd<MP_HID, true><<<MP_GB, MP_THREADS, 0, st>>>(B.dZb.p, B.H[0].p, B.AG[1].p, B.wsum.p,
-                                                       v.Npad, net.Wb[1], B.dH.p, B.U.p,
-                                                       B.part_w[1].p, B.part_b[1].p);
+  k_mp_bwd<MP_HID, true><<<MP_GB, MP_THREADS, SM2, st>>>(B.dZb.p, B.H[0].p, B.AG[1].p, B.wsum.p,
+                                                         v.Npad, net.Wb[1], B.dH.p, B.U.p,
+                                                         B.part_w[1].p, B.part_b[1].p);
   CK_LAUNCH();
-  k_mp_gather_bwd<<<gg, MP_THREADS, 0, st>>>(B.dH.p, B.U.p, B.H[0].p, lv.ell.p, lv.slice_off.p,
-                                             lv.slice_w.p, v.N, v.Npad, B.dZa.p);
+  k_mp_gather<true><<<gg, MG_THREADS, 0, st>>>(B.U.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p,
+                                               nullptr, v.N, v.Npad, B.dH.p, B.H[0].p, B.dZa.p);
   CK_LAUNCH();
-  k_mp_bwd<MP_FIN, false, true><<<MP_GB, MP_THREADS, 0, st>>>(
+  k_mp_bwd<MP_FIN, false, true><<<MP_GB, MP_THREADS, SM1, st>>>(
       B.dZa.p, B.X.p, B.AG0.p, B.wsum.p, v.Npad, nullptr, nullptr, nullptr, B.part_w[0].p,
       B.part_b[0].p);
   CK_LAUNCH();
-  k_mp_grad_reduce<<<grid_for(MP_NPARAM, 256), 256, 0, st>>>(
+  k_mp_grad_reduce<<<(MP_NPARAM + 31) / 32, 256, 0, st>>>(
       B.part_w[0].p, B.part_b[0].p, B.part_w[1].p, B.part_b[1].p, B.part_w[2].p, B.part_b[2].p,
       B.part_head.p, MP_GB, B.grad.p);
   CK_LAUNCH();
