@@ -2535,6 +2535,389 @@ __device__ __forceinline__ void row_words(RowSum<VT> &r, const unsigned *w, VT p
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP32 SpMV on rows staged in shared memory (levels too large for the team
+// kernel).  A block takes a run of tiles of one group (about SL_ROWS rows),
+// copies their p and that of their halo (the other rows their entries name)
+// into shared memory and gathers there.  Its rows are encoded once per level
+// (k_loc_encode): two 16-bit entries a word, each the byte offset of a place
+// (own row, or p_cap + place in the halo) with the weight code in the two low
+// bits.  Same arithmetic and reduction order as k_spmv.
+// k_spmv is bound by L1 lookups: the 32 gathers of a warp instruction touch
+// about eight lines.  Here an entry costs one shared-memory load and half the
+// bytes from HBM: 8M rows, 179 -> 131 us a step.
+// ---------------------------------------------------------------------------
+constexpr int SL_ROWS = (int)LZ_TILE;      // rows of a block, unless one tile is longer
+constexpr int SL_TILES = SL_ROWS / 512;    // its tiles at most
+constexpr int SL_HALO = 6144;              // halo rows at most
+constexpr int SL_HASH = 8192;              // slots of the encoder's table
+// rows of a level from which its encoding (8M rows: 0.63 ms) is worth it
+constexpr ll SL_MIN = 1ll << 20;
+constexpr int SL_CHUNKS = SL_ROWS / 32 + SL_TILES + 1;
+__host__ __device__ constexpr int sl_cap(int rows) { return (ts_place<float>(rows + 31) + 3) & ~3; }
+static_assert(sl_cap(SL_ROWS) + SL_HALO <= 1 << 14, "14-bit places");
+
+// One block per run: the halo list (sorted, so that neighbouring rows are
+// fetched together) and the encoded rows.  The halo is collected in a hash
+// table; the place of a halo row is looked up in it again.  bad[0]: a weight
+// other than 0, 1, 2, 4 or a halo of more than SL_HALO rows; bad[1]: the
+// longest halo.
+constexpr int LE_THREADS = 1024, LE_BATCH = 8;  // (loads in flight per lane)
+constexpr int LE_PROBES = 256;                 // of the table, then it counts as full
+constexpr int LE_SMEM = SL_HASH * (4 + 4 + 2);
+__global__ void __launch_bounds__(LE_THREADS)
+k_loc_encode(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
+             const int2 *__restrict__ runs, const unsigned *__restrict__ ell,
+             const ll *__restrict__ slice_off, const int *__restrict__ slice_w, int p_cap,
+             int max_w, unsigned *__restrict__ enc, int *__restrict__ halo,
+             int *__restrict__ nhalo, int *__restrict__ bad) {
+  extern __shared__ __align__(16) unsigned le_smem[];
+  unsigned *key = le_smem, *list = key + SL_HASH;
+  unsigned short *place = reinterpret_cast<unsigned short *>(list + SL_HASH);
+  __shared__ int wsum[LE_THREADS / 32];
+  constexpr unsigned EMPTY = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int2 run = runs[blockIdx.x];
+  const ll b0 = tbeg[run.x], e1 = tend[run.x + run.y - 1], B0 = b0 & ~31ll;
+  for (int k = threadIdx.x; k < SL_HASH; k += LE_THREADS) key[k] = EMPTY;
+  __syncthreads();
+  const ll sl0 = b0 >> 5;
+  const int ns = (int)(((e1 - 1) >> 5) - sl0) + 1;
+  const unsigned len = (unsigned)(e1 - b0);
+  auto slot = [](unsigned j) { return (j * 2654435761u) >> (32 - 13); };
+  bool over = false;
+  for (int q = warp; q < ns; q += LE_THREADS / 32) {
+    const ll i = (sl0 + q) * 32 + lane;
+    const unsigned *ep = ell + slice_off[sl0 + q] + lane;
+    const bool valid = i >= b0 && i < e1;
+    const int wd = slice_w[sl0 + q];
+    for (int k0 = 0; k0 < wd; k0 += LE_BATCH) {
+      unsigned x[LE_BATCH];
+#pragma unroll
+      for (int u = 0; u < LE_BATCH; u++) x[u] = k0 + u < wd ? ep[(ll)(k0 + u) * 32] : 0u;
+#pragma unroll
+      for (int u = 0; u < LE_BATCH; u++) {
+        const unsigned j = x[u] & 0x0FFFFFFFu;
+        const bool ext = valid && !over && x[u] >> 28 != 0 && j - (unsigned)b0 >= len;
+        if (!__any_sync(0xffffffffu, ext)) continue;
+        if (!ext) continue;
+        unsigned h = slot(j);
+        int tries = 0;
+        for (; tries < LE_PROBES; tries++) {
+          unsigned was = *reinterpret_cast<volatile unsigned *>(&key[h]);
+          if (was == EMPTY) was = atomicCAS(&key[h], EMPTY, j);
+          if (was == EMPTY || was == j) break;
+          h = (h + 1) & (SL_HASH - 1);
+        }
+        over = tries == LE_PROBES;
+      }
+    }
+  }
+  const bool full = __syncthreads_or(over);
+  // the keys, packed: eight slots a thread
+  int m = 0;
+  {
+    constexpr int PER = SL_HASH / LE_THREADS;
+    int c = 0;
+#pragma unroll
+    for (int u = 0; u < PER; u++) c += key[threadIdx.x + u * LE_THREADS] != EMPTY;
+    int x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    const int t = wsum[lane];  // LE_THREADS / 32 == 32
+    m = __reduce_add_sync(0xffffffffu, t);
+    int at = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0) + x - c;
+    if (full || m > SL_HALO) {  // block-uniform
+      if (threadIdx.x == 0) atomicOr(bad, 1);
+      return;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      const unsigned j = key[threadIdx.x + u * LE_THREADS];
+      if (j != EMPTY) list[at++] = j;
+    }
+  }
+  int p2 = 1;
+  while (p2 < m) p2 <<= 1;
+  __syncthreads();
+  for (int k = m + threadIdx.x; k < p2; k += LE_THREADS) list[k] = EMPTY;
+  __syncthreads();
+  for (int size = 2; size <= p2; size <<= 1)
+    for (int st = size >> 1; st > 0; st >>= 1) {
+      for (int u = threadIdx.x; u < p2 >> 1; u += LE_THREADS) {
+        const int a = ((u & ~(st - 1)) << 1) | (u & (st - 1)), b = a + st;
+        const unsigned x = list[a], y = list[b];
+        if ((x > y) == ((a & size) == 0)) list[a] = y, list[b] = x;
+      }
+      __syncthreads();
+    }
+  for (int k = threadIdx.x; k < m; k += LE_THREADS) {
+    const unsigned j = list[k];
+    halo[(ll)blockIdx.x * SL_HALO + k] = (int)j;
+    unsigned h = slot(j);
+    while (key[h] != j) h = (h + 1) & (SL_HASH - 1);
+    place[h] = (unsigned short)k;
+  }
+  if (threadIdx.x == 0) nhalo[blockIdx.x] = m, atomicMax(bad + 1, m);
+  __syncthreads();
+  unsigned *eo = enc + enc_base(slice_off[sl0], sl0, run.x, max_w);
+  unsigned mine = 0;
+  for (int q = warp; q < ns; q += LE_THREADS / 32) {
+    const ll i = (sl0 + q) * 32 + lane;
+    const ll so = slice_off[sl0 + q];
+    const unsigned *ep = ell + so + lane;
+    const int wd = slice_w[sl0 + q];
+    const bool valid = i >= b0 && i < e1;
+    const unsigned self = valid ? (unsigned)ts_place<float>((int)(i - B0)) : 0u;  // weight 0
+    unsigned *op = eo + ((so - slice_off[sl0]) >> 1) + 32 * q + lane;
+    for (int k0 = 0; k0 < wd; k0 += LE_BATCH) {
+      unsigned x[LE_BATCH];
+#pragma unroll
+      for (int u = 0; u < LE_BATCH; u++) x[u] = k0 + u < wd ? ep[(ll)(k0 + u) * 32] : 0u;
+#pragma unroll
+      for (int u = 0; u < LE_BATCH; u += 2) {
+        if (k0 + u >= wd) break;
+        unsigned w2 = 0;
+#pragma unroll
+        for (int h2 = 0; h2 < 2; h2++) {
+          const unsigned wt = x[u + h2] >> 28, j = x[u + h2] & 0x0FFFFFFFu;
+          const bool names = valid && wt != 0, ext = names && j - (unsigned)b0 >= len;
+          unsigned loc = names ? (unsigned)ts_place<float>((int)(j - (unsigned)B0)) : self;
+          const unsigned code = names ? wt - (wt >> 2) : 0u;
+          mine |= names ? 0xFFE8u >> wt & 1u : 0u;
+          if (__any_sync(0xffffffffu, ext)) {
+            if (ext) {
+              unsigned h = slot(j);
+              while (key[h] != j) h = (h + 1) & (SL_HASH - 1);
+              loc = (unsigned)p_cap + place[h];
+            }
+            __syncwarp();
+          }
+          w2 |= ((loc << 2 | (code & 3u)) & 0xFFFFu) << (16 * h2);
+        }
+        op[((k0 + u) >> 1) * 32] = w2;
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, mine) && lane == 0) atomicOr(bad, 1);
+}
+
+// two FP32 values in a register pair
+struct F2 {
+  unsigned long long v;
+  __device__ __forceinline__ static F2 of(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+  }
+  __device__ __forceinline__ float2 get() const {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+  }
+  // a b + c, each half rounded once
+  __device__ __forceinline__ static F2 fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+  }
+};
+// the weights of a word's two entries as BF16 bits, lower entry in the lower
+// half (codes 0 .. 3: 1/2, 1, 2, 4)
+__device__ __forceinline__ unsigned loc_weights(unsigned x) {
+  return (x & 0x00030003u) * 0x80u + 0x3F003F00u;
+}
+__device__ __forceinline__ float loc_lo(const float *sp, unsigned x) {
+  return sp[(x & 0xFFFFu) >> 2];
+}
+__device__ __forceinline__ float loc_hi(const float *sp, unsigned x) { return sp[x >> 18]; }
+
+// NW words of a row of each of two slices, on their way from HBM
+template <int NW>
+struct LocWords {
+  unsigned x[NW], y[NW];
+  __device__ __forceinline__ void load(const unsigned *oa, const unsigned *ob) {
+#pragma unroll
+    for (int u = 0; u < NW; u++) x[u] = __ldcs(oa + u * 32), y[u] = __ldcs(ob + u * 32);
+  }
+  // sum += w (p_i - p_j); of words u < na of the first row and u < nb of the
+  // second where MASK (the others name the row itself)
+  template <bool MASK>
+  __device__ __forceinline__ void add(F2 &sum, F2 pi, const float *sp, int na, int nb,
+                                      unsigned self_a, unsigned self_b) {
+    float xl[NW], xh[NW], yl[NW], yh[NW];
+    if (MASK)
+#pragma unroll
+      for (int u = 0; u < NW; u++) x[u] = u < na ? x[u] : self_a, y[u] = u < nb ? y[u] : self_b;
+#pragma unroll
+    for (int u = 0; u < NW; u++) {
+      xl[u] = loc_lo(sp, x[u]), xh[u] = loc_hi(sp, x[u]);
+      yl[u] = loc_lo(sp, y[u]), yh[u] = loc_hi(sp, y[u]);
+    }
+    const F2 neg = F2::of(-1.f, -1.f);
+#pragma unroll
+    for (int u = 0; u < NW; u++) {
+      const unsigned wx = loc_weights(x[u]), wy = loc_weights(y[u]);
+      const F2 dl = F2::fma(F2::of(xl[u], yl[u]), neg, pi);  // p_i - p_j
+      const F2 dh = F2::fma(F2::of(xh[u], yh[u]), neg, pi);
+      sum = F2::fma(F2::of(__uint_as_float(wx << 16), __uint_as_float(wy << 16)), dl, sum);
+      sum = F2::fma(
+          F2::of(__uint_as_float(wx & 0xFFFF0000u), __uint_as_float(wy & 0xFFFF0000u)), dh, sum);
+    }
+  }
+};
+// one word of one row
+__device__ __forceinline__ void loc_word(float &sum, unsigned x, float pi, const float *sp) {
+  const unsigned w = loc_weights(x);
+  sum = fmaf(__uint_as_float(w << 16), pi - loc_lo(sp, x), sum);
+  sum = fmaf(__uint_as_float(w & 0xFFFF0000u), pi - loc_hi(sp, x), sum);
+}
+
+__global__ void __launch_bounds__(512, 2)
+k_spmv_loc(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
+           const int *__restrict__ tgrp, const GState *__restrict__ gs,
+           const int2 *__restrict__ runs, const unsigned *__restrict__ enc,
+           const ll *__restrict__ slice_off, const int *__restrict__ slice_w,
+           const int *__restrict__ halo, const int *__restrict__ nhalo, int p_cap, int max_w,
+           const float *__restrict__ p, float *__restrict__ w, double *__restrict__ part,
+           int force) {
+  pdl_entry();
+  extern __shared__ __align__(16) float sl_p[];
+  __shared__ float2 cs[SL_CHUNKS];
+  __shared__ int tc[SL_TILES + 1];  // the tiles' first slices
+  // per slice: where its words start, its place among the block's slices, the
+  // words of a row, and the lanes whose rows belong to the tile
+  __shared__ __align__(16) uint4 s_sl[SL_CHUNKS + 3];
+  const int2 run = runs[blockIdx.x];
+  const int t0 = run.x, nt = run.y;
+  const GState &s = gs[tgrp[t0]];
+  if (!s.run && !force) return;
+  const float c = (float)s.c;
+  const ll b0 = tbeg[t0], e1 = tend[t0 + nt - 1], B0 = b0 & ~31ll;
+  const ll sl0 = b0 >> 5, so0 = slice_off[sl0];
+  const unsigned *eo = enc + enc_base(so0, sl0, t0, max_w);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (warp == 0) {  // (at most 32 tiles)
+    const ll b = lane < nt ? tbeg[t0 + lane] : 0, e = lane < nt ? tend[t0 + lane] : 1;
+    const int n = lane < nt ? (int)(((e - 1) >> 5) - (b >> 5)) + 1 : 0;
+    int x = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane <= nt) tc[lane] = x - n;
+  }
+  {
+    // whole slices, four rows a thread (rows beside the run's are not read)
+    const int rows = (int)(e1 - B0);
+    const float4 *p4 = reinterpret_cast<const float4 *>(p + B0);
+    for (int k = threadIdx.x; k < (rows + 3) >> 2; k += blockDim.x) {
+      const int r = 4 * k;
+      float4 v;
+      if (r + 4 <= rows)
+        v = p4[k];
+      else
+        v.x = p[B0 + r], v.y = r + 1 < rows ? p[B0 + r + 1] : 0.f,
+        v.z = r + 2 < rows ? p[B0 + r + 2] : 0.f, v.w = 0.f;
+      *reinterpret_cast<float4 *>(sl_p + ts_place<float>(r)) = v;
+    }
+  }
+  const int nh = nhalo[blockIdx.x];
+  const int *hl = halo + (ll)blockIdx.x * SL_HALO;
+#pragma unroll 4
+  for (int k = threadIdx.x; k < nh; k += blockDim.x) sl_p[p_cap + k] = p[hl[k]];
+  __syncthreads();
+  const int nc = tc[nt];
+  for (int q = threadIdx.x; q < nc + 3; q += blockDim.x) {
+    uint4 d = make_uint4(0u, 0u, 0u, 0u);  // (past the end: an empty slice)
+    if (q < nc) {
+      int t = 0;
+      while (q >= tc[t + 1]) t++;
+      const ll b = tbeg[t0 + t], e = tend[t0 + t], sl = (b >> 5) + (q - tc[t]);
+      d.x = (unsigned)((slice_off[sl] - so0) >> 1) + 32u * (unsigned)(sl - sl0);
+      d.y = (unsigned)(sl - sl0);
+      d.z = (unsigned)(slice_w[sl] + 1) >> 1;
+      const int lo = (int)max(b - sl * 32, 0ll), hi = (int)min(e - sl * 32, 32ll);
+      d.w = (hi < 32 ? (1u << hi) - 1u : 0xFFFFFFFFu) & ~((1u << lo) - 1u);
+    }
+    s_sl[q] = d;
+  }
+  __syncthreads();
+  const unsigned *el = eo + lane;
+  float *wp = w + B0 + lane;
+  // four consecutive slices per warp, two at a time: their chunk trees fold
+  // into one.  The first NB words of the next two slices, and the next NB of
+  // these, are on their way while the words at hand are added.
+  constexpr int NB = 7;  // (26 neighbours are 13 words)
+  LocWords<NB> first, next;
+  uint4 da = s_sl[min(4 * warp, nc)], db = s_sl[min(4 * warp, nc) + 1];
+  first.load(el + da.x, el + db.x);
+  for (int q0 = 4 * warp; q0 < nc; q0 += 4 * nw) {
+    Fold<float>::T two = Fold<float>::zero();  // the tree of the first two slices
+#pragma unroll 1
+    for (int j = 0; j < 4; j += 2) {
+      const unsigned *oa = el + da.x, *ob = el + db.x;
+      const bool va = (da.w >> lane) & 1u, vb = (db.w >> lane) & 1u;
+      const int ia = 36 * (int)da.y + lane, ib = 36 * (int)db.y + lane, ra = da.y, rb = db.y;
+      const float pa = va ? sl_p[ia] : 0.f, pb = vb ? sl_p[ib] : 0.f;
+      const F2 pi = F2::of(pa, pb);
+      const int na = da.z, nb = db.z;
+      // the row itself, twice, with weight 0 (place 0 on lanes without a row)
+      const unsigned sa = va ? (unsigned)ia * 0x40004u : 0u;
+      const unsigned sb = vb ? (unsigned)ib * 0x40004u : 0u;
+      F2 sum = F2::of(0.f, 0.f);
+      const bool more = max(na, nb) > NB;
+      if (more) next.load(oa + NB * 32, ob + NB * 32);
+      if (min(na, nb) >= NB)
+        first.add<false>(sum, pi, sl_p, na, nb, sa, sb);
+      else
+        first.add<true>(sum, pi, sl_p, na, nb, sa, sb);
+      {
+        const int qn = min(j == 0 ? q0 + 2 : q0 + 4 * nw, nc);
+        da = s_sl[qn], db = s_sl[qn + 1];
+        first.load(el + da.x, el + db.x);
+      }
+      if (more) next.add<true>(sum, pi, sl_p, na - NB, nb - NB, sa, sb);
+      float2 y = sum.get();
+      for (int r = 2 * NB; r < na; r++) loc_word(y.x, __ldcs(oa + r * 32), pa, sl_p);
+      for (int r = 2 * NB; r < nb; r++) loc_word(y.y, __ldcs(ob + r * 32), pb, sl_p);
+      Fold<float>::T a = Fold<float>::zero(), b = Fold<float>::zero();
+      if (va) {
+        wp[32 * ra] = y.x;
+        Fold<float>::first_prod(a, y.x, pa - c);
+      }
+      if (vb) {
+        wp[32 * rb] = y.y;
+        Fold<float>::first_prod(b, y.y, pb - c);
+      }
+      a = merge2<float>(a, b, 16);
+      if (j == 0) {
+        two = a;
+      } else {
+        a = merge2<float>(two, a, 8);
+        a = Fold<float>::join(a, Fold<float>::shfl_down(a, 4));
+        a = Fold<float>::join(a, Fold<float>::shfl_down(a, 2));
+        a = Fold<float>::join(a, Fold<float>::shfl_down(a, 1));
+        if ((lane & 7) == 0) {
+          const int m = (lane >> 4 & 1) | (lane >> 2 & 2);  // fold_lane's slice
+          if (q0 + m < nc) cs[q0 + m] = a;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int u = warp; u < nt; u += nw) {
+    const double v0 = tile_total_pair(cs + tc[u], tc[u + 1] - tc[u]);
+    if (lane == 0) part[t0 + u] = v0;
+  }
+}
+
 template <typename VT>
 __global__ void __launch_bounds__(TS_THREADS, 1) k_team_steps(TeamArgs a) {
   constexpr int NW = TS_NW, WT = NW * 32;
@@ -3011,7 +3394,7 @@ struct Lanczos {
   std::vector<cudaEvent_t> ev;  // SpMV start/stop events (timing mode)
   std::vector<cudaEvent_t> evk; // p / r per step, then init, eig, ritz (timing mode)
   int bd = 256;                  // threads per tile block (autotuned per level)
-  int sp_kind = 0;               // SpMV variant (autotuned): 0 k_spmv, 1 k_spmv_tma
+  int sp_kind = 0;               // SpMV variant (autotuned): 0 k_spmv, 1 k_spmv_tma, 2 k_spmv_loc
   DBuf<int> err;                 // [0]: a staged-SpMV wait gave up
   int pr_bd = 256;               // threads per block of k_pr
   int pr_u = 4;                  // chunks per warp in flight in k_pr
@@ -3037,6 +3420,10 @@ struct Lanczos {
   DBuf<int> d_list, d_item0, d_halo, d_nhalo, d_bad;
   DBuf<int2> d_items;
   DBuf<unsigned> d_enc;
+  // SpMV on staged rows (k_spmv_loc), FP32
+  std::vector<int2> sl_runs;     // first tile and tiles of each block
+  DBuf<int2> d_runs;
+  int sl_pcap = 0, sl_smem = 0;  // places of own rows, shared memory of a block
   DBuf<TeamSlot> slots;
   DBuf<unsigned long long> ts_epoch;
   DBuf<ll> fq;                   // fixed-point f of the residual check (FP32)
@@ -3624,7 +4011,12 @@ struct Lanczos {
   }
   void spmv(const Level &lv, int kind, int threads, const FinArgs &fa, int fuse, int force) {
     cudaStream_t st = ctx().stream;
-    if (kind == 1 && sizeof(VT) == 4) {
+    if (kind == 2 && sizeof(VT) == 4) {
+      launch_pdl(k_spmv_loc, (unsigned)sl_runs.size(), threads, (size_t)sl_smem, st, tbeg.p, tend.p,
+                 tgrp.p, gs.p, d_runs.p, d_enc.p, lv.slice_off.p, lv.slice_w.p, d_halo.p,
+                 d_nhalo.p, sl_pcap, lv.max_w, reinterpret_cast<const float *>(p.p),
+                 reinterpret_cast<float *>(w.p), part.p, force);
+    } else if (kind == 1 && sizeof(VT) == 4) {
       const size_t sb = sp_stage_bytes(lv, threads);
       launch_pdl(k_spmv_tma, T, threads, SP_NST * sb, st, tbeg.p, tend.p, tgrp.p, gs.p,
                  lv.ell.p, lv.slice_off.p, lv.slice_w.p, reinterpret_cast<const float *>(p.p),
@@ -3635,12 +4027,46 @@ struct Lanczos {
     }
   }
 
+  // Encodes the level for k_spmv_loc; false where it does not apply (a weight
+  // or a halo out of its range).
+  bool loc_prepare(const Level &lv) {
+    if (sizeof(VT) != 4 || sp_fused || T <= 0) return false;
+    cudaStream_t st = ctx().stream;
+    sl_runs.clear();
+    ll longest = 0;
+    for (const GState &s : hgs) {
+      const ll tr = tile_rows(s.n), k = std::max<ll>(1, SL_ROWS / tr);
+      for (int t = 0; t < s.ntiles; t += (int)k)
+        sl_runs.push_back(make_int2(s.tile0 + t, (int)std::min<ll>(k, s.ntiles - t)));
+      longest = std::max(longest, std::min(k * tr, s.n));
+    }
+    sl_pcap = sl_cap((int)longest);
+    const size_t nr = sl_runs.size();
+    d_runs.ensure(nr), d_nhalo.ensure(nr), d_halo.ensure(nr * SL_HALO), d_bad.ensure(2);
+    h2d(d_runs.p, sl_runs.data(), nr);
+    d_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
+                 (size_t)(T + 1) * (size_t)(lv.max_w + 1) * 32 + 1024);
+    CK(cudaMemsetAsync(d_bad.p, 0, 2 * sizeof(int), st));
+    ensure_smem_limit(k_loc_encode, LE_SMEM);
+    k_loc_encode<<<(unsigned)nr, LE_THREADS, LE_SMEM, st>>>(
+        tbeg.p, tend.p, d_runs.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, sl_pcap, lv.max_w,
+        d_enc.p, d_halo.p, d_nhalo.p, d_bad.p);
+    CK_LAUNCH();
+    int bad[2] = {0, 0};
+    d2h(bad, d_bad.p, 2);
+    sync();
+    sl_smem = (sl_pcap + bad[1]) * (int)sizeof(float);
+    ensure_smem_limit(k_spmv_loc, sl_smem);
+    return bad[0] == 0;
+  }
+
   // Autotuner: threads per tile block for this level.  Candidates are timed
   // on the level's own matrix (three forced SpMV launches each, CUDA
   // events); the tile reductions are canonical, so the choice never changes
   // a result.  Decisions are cached per (tiles, groups, rows) for the thread.
   void autotune(const Level &lv) {
-    // PARRSB_GPU_SPMV: 0 = k_spmv only, 1 = k_spmv_tma only, unset = time both
+    // PARRSB_GPU_SPMV: 0 = k_spmv only, 1 = k_spmv_tma only, 2 = k_spmv_loc only
+    // where it applies, unset = time them
     // per device (a later call may run on another device), before the cached
     // decision is used
     ensure_smem_limit(k_spmv_tma, 200 * 1024);
@@ -3655,6 +4081,8 @@ struct Lanczos {
       if (kv.first == key) {
         sp_kind = kv.second >> 16;
         bd = kv.second & 0xFFFF;
+        // (the same shape with other groups: the encoding may not fit them)
+        if (sp_kind == 2 && !loc_prepare(lv)) sp_kind = 0, bd = 256;
         return;
       }
     cudaStream_t st = ctx().stream;
@@ -3664,6 +4092,10 @@ struct Lanczos {
       if (force_kind < 0 || force_kind == 0) cand.push_back({0, th});
       if ((force_kind < 0 || force_kind == 1) && sp_tma_ok(lv, th)) cand.push_back({1, th});
     }
+    if (force_kind == 2 || (force_kind < 0 && N >= SL_MIN))
+      if (loc_prepare(lv))
+        for (int th : {256, 512})
+          if (!force_th || th == force_th) cand.push_back({2, th});
     if (cand.empty()) cand.push_back({0, 256});
     float best = 1e30f;
     std::pair<int, int> pick = cand[0];
@@ -3687,7 +4119,7 @@ struct Lanczos {
     cache.push_back({key, (pick.first << 16) | pick.second});
     if (getenv("PARRSB_GPU_AUTOTUNE_LOG"))
       fprintf(stderr, "parrsb_gb300: SpMV autotune tiles=%d groups=%d rows=%lld -> %s x %d\n", T,
-              A, (long long)N, pick.first ? "k_spmv_tma" : "k_spmv", pick.second);
+              A, (long long)N, pick.first == 2 ? "k_spmv_loc" : pick.first ? "k_spmv_tma" : "k_spmv", pick.second);
   }
 
   // Runs all passes; f holds the normalised Fiedler vectors afterwards.
