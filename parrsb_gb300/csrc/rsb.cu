@@ -73,9 +73,14 @@ __global__ void k_run_bounds(const int *__restrict__ flag, const ll *__restrict_
   if (i == ns - 1) run_start[nruns] = ns;
 }
 
-__global__ void k_scatter_inv(const int *__restrict__ vals, ll n, int *__restrict__ inv) {
+// run of every corner: first slot and length (they fit 32 bits)
+__global__ void k_scatter_run(const int *__restrict__ vals, const int *__restrict__ runid,
+                              const ll *__restrict__ run_start, ll n, int2 *__restrict__ run) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) inv[vals[i]] = (int)i;
+  if (i >= n) return;
+  const int r = runid[i];
+  const ll b = run_start[r];
+  run[vals[i]] = make_int2((int)b, (int)(run_start[r + 1] - b));
 }
 
 // Dual-graph rows, one warp per element a (src/con.c's element graph: two
@@ -84,12 +89,15 @@ __global__ void k_scatter_inv(const int *__restrict__ vals, ll n, int *__restric
 // its vertices, vertex by vertex, each run in slot order; an element b != a
 // occurs once per (vertex of a, equal vertex of b) pair, so its weight is its
 // number of occurrences, and the row lists every b at its first occurrence.
-// Up to GR_CAP candidates sit in shared memory, where a per-warp open-
-// addressing table (GR_HASH slots: element, count, first index) counts each
-// element's occurrences and keeps its first one in O(C) instead of
-// comparing every pair; a longer list is read from the runs again and
-// compared pairwise.  FILL = false: row lengths and the largest weight;
-// FILL = true: columns and weights at rowptr[a].
+// Up to GR_CAP candidates are taken 32 at a time: the lanes with the same
+// element find each other (__match_any_sync), their first one looks it up in a
+// per-warp open-addressing table (GR_HASH slots: element, count) and is its
+// first occurrence when it finds it missing.  So a candidate costs a 32nd of a
+// match and at most one atomic, and the table is emptied by those that filled
+// it.  A longer list is read from the runs again and compared pairwise.
+// FILL = false: row lengths and the largest weight; FILL = true: columns and
+// weights at rowptr[a].  Bound by instruction issue: 1.2M hexes, 0.79 -> 0.42 ms to count and 0.71 -> 0.54 ms to fill
+// (three atomics per candidate and a second search before).
 constexpr int GR_WARPS = 4;
 constexpr int GR_CAP = 256;
 constexpr int GR_HASH = 256;  // power of two >= GR_CAP: more slots than distinct keys
@@ -100,28 +108,27 @@ __device__ __forceinline__ int gr_slot0(int b) {
 
 template <bool FILL>
 __global__ void __launch_bounds__(GR_WARPS * 32)
-k_graph_rows(int nv, ll N, const int *__restrict__ sorted_slot, const int *__restrict__ inv,
-             const int *__restrict__ runid, const ll *__restrict__ run_start,
+k_graph_rows(int nv, ll N, const int *__restrict__ sorted_slot, const int2 *__restrict__ run,
              const ll *__restrict__ rowptr, int *__restrict__ col,
              unsigned char *__restrict__ wout, ll *__restrict__ rowlen, int *__restrict__ maxw) {
-  __shared__ __align__(16) int cand[GR_WARPS][GR_CAP + 4];
-  __shared__ int hkey[GR_WARPS][GR_HASH], hcnt[GR_WARPS][GR_HASH], hfirst[GR_WARPS][GR_HASH];
+  __shared__ int hkey[GR_WARPS][GR_HASH], hcnt[GR_WARPS][GR_HASH];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int h = lane; h < GR_HASH; h += 32)  // empty: key -1, count 0, first INT_MAX
-    hkey[wid][h] = -1, hcnt[wid][h] = 0, hfirst[wid][h] = 0x7fffffff;
+  const int lg = (nv & (nv - 1)) == 0 ? 31 - __clz(nv) : -1;  // nv = 2^lg
+  int *key = hkey[wid], *num = hcnt[wid];
+  for (int h = lane; h < GR_HASH; h += 32) key[h] = -1;  // empty
   __syncwarp();
   const unsigned lt = (1u << lane) - 1u;
-  const ll a = (ll)blockIdx.x * GR_WARPS + wid;
   int wmax = 0;
-  if (a < N) {  // warp-uniform
+  const ll step = (ll)gridDim.x * GR_WARPS;
+  ll a = (ll)blockIdx.x * GR_WARPS + wid;
+  int2 next = make_int2(0, 0);
+  if (a < N && lane < nv) next = run[a * nv + lane];
+  for (; a < N; a += step) {
     // run of each vertex of a (lane k < nv), then every lane holds all of them
-    // (slot positions and candidate counts fit 32 bits: N < 2^28, nv <= 8)
-    int rs = 0, rl = 0;
-    if (lane < nv) {
-      const int r = runid[inv[a * nv + lane]];
-      rs = (int)run_start[r];
-      rl = (int)(run_start[r + 1] - run_start[r]);
-    }
+    // (slot positions and candidate counts fit 32 bits: N < 2^28, nv <= 8);
+    // those of the warp's next element are on their way
+    const int rs = next.x, rl = next.y;
+    if (a + step < N && lane < nv) next = run[(a + step) * nv + lane];
     int RS[8], EX[8];
     int C = 0;
 #pragma unroll
@@ -131,43 +138,62 @@ k_graph_rows(int nv, ll N, const int *__restrict__ sorted_slot, const int *__res
       C += __shfl_sync(0xffffffffu, rl, k);  // lanes >= nv hold 0
     }
     auto cand_at = [&](int t) -> int {  // element of candidate t
-      int base = RS[0] - EX[0];
+      int base = RS[0];
 #pragma unroll
       for (int k = 1; k < 8; k++)
         if (k < nv && t >= EX[k]) base = RS[k] - EX[k];
-      return sorted_slot[base + t] / nv;
+      const int slot = sorted_slot[base + t];
+      return lg >= 0 ? slot >> lg : slot / nv;
     };
-    const bool staged = C <= GR_CAP;
-    if (staged) {
-      for (int t = lane; t < C; t += 32) {
-        const int b = cand_at(t);
-        cand[wid][t] = b;
-        if (b == (int)a) continue;
-        int h = gr_slot0(b);
-        for (;;) {  // fewer distinct keys than slots (a != b): a free or equal slot exists
-          const int prev = atomicCAS(&hkey[wid][h], -1, b);
-          if (prev == -1 || prev == b) break;
-          h = (h + 1) & (GR_HASH - 1);
+    const ll row = FILL ? rowptr[a] : 0;
+    int out = 0;
+    if (C <= GR_CAP) {
+      int b[GR_CAP / 32], slot[GR_CAP / 32];  // slot: of a first occurrence, else -1
+#pragma unroll
+      for (int r = 0; r < GR_CAP / 32; r++) {
+        if (32 * r >= C) break;
+        const int t = 32 * r + lane;
+        b[r] = t < C ? cand_at(t) : (int)a;
+        slot[r] = -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, b[r]);
+        if (b[r] != (int)a && (peers & lt) == 0) {
+          int h = gr_slot0(b[r]);
+          for (;;) {  // fewer distinct keys than slots (b != a): a free or equal slot exists
+            const int prev = atomicCAS(&key[h], -1, b[r]);
+            if (prev == -1) slot[r] = h, num[h] = 0;
+            if (prev == -1 || prev == b[r]) break;
+            h = (h + 1) & (GR_HASH - 1);
+          }
+          num[h] += __popc(peers);  // (one lane per element)
         }
-        atomicAdd(&hcnt[wid][h], 1);
-        atomicMin(&hfirst[wid][h], (int)t);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int r = 0; r < GR_CAP / 32; r++) {
+        if (32 * r >= C) break;
+        const bool first = slot[r] >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, first);
+        if (first) {
+          const int cnt = num[slot[r]];
+          key[slot[r]] = -1;
+          if (FILL) {
+            const ll pos = row + out + __popc(m & lt);
+            col[pos] = b[r];
+            wout[pos] = (unsigned char)(cnt > 255 ? 255 : cnt);
+          }
+          wmax = max(wmax, cnt);
+        }
+        out += __popc(m);
       }
       __syncwarp();
-    }
-    ll out = 0;
-    for (int t0 = 0; t0 < C; t0 += 32) {
-      const int t = t0 + lane;
-      bool first = false;
-      int b = -1, cnt = 0;
-      if (t < C) {
-        b = staged ? cand[wid][t] : cand_at(t);
-        if (b != (int)a) {
-          if (staged) {
-            int h = gr_slot0(b);
-            while (hkey[wid][h] != b) h = (h + 1) & (GR_HASH - 1);  // b was inserted
-            cnt = hcnt[wid][h];
-            first = hfirst[wid][h] == (int)t;
-          } else {
+    } else {
+      for (int t0 = 0; t0 < C; t0 += 32) {
+        const int t = t0 + lane;
+        bool first = false;
+        int b = -1, cnt = 0;
+        if (t < C) {
+          b = cand_at(t);
+          if (b != (int)a) {
             int before = 0;  // occurrences of b ahead of t
             for (int j = 0; j < C; j++) {
               const int m = cand_at(j) == b;
@@ -177,45 +203,22 @@ k_graph_rows(int nv, ll N, const int *__restrict__ sorted_slot, const int *__res
             first = before == 0;
           }
         }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, first);
-      if (first) {
-        if (FILL) {
-          const ll pos = rowptr[a] + out + __popc(m & lt);
-          col[pos] = b;
-          wout[pos] = (unsigned char)(cnt > 255 ? 255 : cnt);
+        const unsigned m = __ballot_sync(0xffffffffu, first);
+        if (first) {
+          if (FILL) {
+            const ll pos = row + out + __popc(m & lt);
+            col[pos] = b;
+            wout[pos] = (unsigned char)(cnt > 255 ? 255 : cnt);
+          }
+          wmax = max(wmax, cnt);
         }
-        wmax = max(wmax, cnt);
+        out += __popc(m);
       }
-      out += __popc(m);
     }
     if (!FILL && lane == 0) rowlen[a] = out;
-    if (staged) {  // empty the table again: find every used slot, then clear
-      __syncwarp();
-      int hs[GR_CAP / 32];
-#pragma unroll
-      for (int k = 0; k < GR_CAP / 32; k++) {
-        const int t = lane + 32 * k;
-        hs[k] = -1;
-        if (t < C) {
-          const int b = cand[wid][t];
-          if (b != (int)a) {
-            int h = gr_slot0(b);
-            while (hkey[wid][h] != b) h = (h + 1) & (GR_HASH - 1);
-            hs[k] = h;
-          }
-        }
-      }
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < GR_CAP / 32; k++)
-        if (hs[k] >= 0) hkey[wid][hs[k]] = -1, hcnt[wid][hs[k]] = 0, hfirst[wid][hs[k]] = 0x7fffffff;
-      __syncwarp();
-    }
   }
   if (!FILL) {  // one atomic per warp; every lane reaches the shuffles
-    for (int off = 16; off > 0; off >>= 1)
-      wmax = max(wmax, __shfl_xor_sync(0xffffffffu, wmax, off));
+    wmax = __reduce_max_sync(0xffffffffu, wmax);
     if (lane == 0 && wmax) atomicMax(maxw, wmax);
   }
 }
@@ -233,15 +236,17 @@ __global__ void k_max_ll(const ll *__restrict__ v, ll n, unsigned long long *__r
 // ----------------------------------------------------------------------------
 // Level restriction to sliced ELL (current order, same-group entries only)
 // ----------------------------------------------------------------------------
-__global__ void k_inv_perm(const int *__restrict__ perm, ll N, int *__restrict__ inv) {
+// The level-matrix kernels walk a dual-graph row per thread and gather the
+// position and the group of every entry, eight entries at a time.
+// position and group of every element, one record: a row's neighbours are then
+// one gather each
+__global__ void k_pos_grp(const int *__restrict__ perm, const int *__restrict__ grp, ll N,
+                          int2 *__restrict__ pg) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) inv[perm[i]] = (int)i;
+  if (i < N) pg[perm[i]] = make_int2((int)i, grp[i]);
 }
 
-// The level-matrix kernels walk a dual-graph row per thread through two
-// dependent gathers per entry (position inv[col], its group); eight entries
-// at a time keep eight of each in flight instead of one.
-__global__ void k_ell_count(const int *__restrict__ perm, const int *__restrict__ inv,
+__global__ void k_ell_count(const int *__restrict__ perm, const int2 *__restrict__ pg,
                             const int *__restrict__ grp, const ll *__restrict__ rowptr,
                             const int *__restrict__ col, ll N, int *__restrict__ rowlen) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
@@ -255,11 +260,11 @@ __global__ void k_ell_count(const int *__restrict__ perm, const int *__restrict_
     for (; q + 8 <= q1; q += 8) {
       int j[8];
 #pragma unroll
-      for (int u = 0; u < 8; u++) j[u] = inv[col[q + u]];
+      for (int u = 0; u < 8; u++) j[u] = col[q + u];
 #pragma unroll
-      for (int u = 0; u < 8; u++) cnt += grp[j[u]] == g;
+      for (int u = 0; u < 8; u++) cnt += pg[j[u]].y == g;
     }
-    for (; q < q1; q++) cnt += grp[inv[col[q]]] == g;
+    for (; q < q1; q++) cnt += pg[col[q]].y == g;
   }
   rowlen[i] = cnt;
 }
@@ -284,7 +289,7 @@ __global__ void k_slice_w(const int *__restrict__ rowlen, ll N, ll nslice,
   slots[s] = (ll)m * 32;
 }
 
-__global__ void k_ell_fill(const int *__restrict__ perm, const int *__restrict__ inv,
+__global__ void k_ell_fill(const int *__restrict__ perm, const int2 *__restrict__ pg,
                            const int *__restrict__ grp, const ll *__restrict__ rowptr,
                            const int *__restrict__ col, const unsigned char *__restrict__ w,
                            ll N, const ll *__restrict__ slice_off,
@@ -301,22 +306,23 @@ __global__ void k_ell_fill(const int *__restrict__ perm, const int *__restrict__
     const ll q0 = rowptr[a], q1 = rowptr[a + 1];
     ll q = q0;
     for (; q + 8 <= q1; q += 8) {  // same entries in the same order, eight gathers in flight
-      int j[8], gj[8];
+      int j[8];
+      int2 v[8];
 #pragma unroll
-      for (int u = 0; u < 8; u++) j[u] = inv[col[q + u]];
+      for (int u = 0; u < 8; u++) j[u] = col[q + u];
 #pragma unroll
-      for (int u = 0; u < 8; u++) gj[u] = grp[j[u]];
+      for (int u = 0; u < 8; u++) v[u] = pg[j[u]];
 #pragma unroll
       for (int u = 0; u < 8; u++)
-        if (gj[u] == g) {
-          out[(ll)k * 32] = (unsigned)j[u] | ((unsigned)w[q + u] << 28);
+        if (v[u].y == g) {
+          out[(ll)k * 32] = (unsigned)v[u].x | ((unsigned)w[q + u] << 28);
           k++;
         }
     }
     for (; q < q1; q++) {
-      int j = inv[col[q]];
-      if (grp[j] == g) {
-        out[(ll)k * 32] = (unsigned)j | ((unsigned)w[q] << 28);
+      const int2 v = pg[col[q]];
+      if (v.y == g) {
+        out[(ll)k * 32] = (unsigned)v.x | ((unsigned)w[q] << 28);
         k++;
       }
     }
@@ -4721,10 +4727,12 @@ __global__ void k_seq_rel(const int *__restrict__ perm, const int *__restrict__ 
 
 __global__ void k_fill_grp(const ll *__restrict__ gstart, const ll *__restrict__ gn,
                            const int *__restrict__ gid, int ng, int *__restrict__ grp) {
-  // one block per group, loop over its range
+  // gridDim.y blocks per group, looping over its range
   int g = blockIdx.x;
   if (g >= ng) return;
-  for (ll i = gstart[g] + threadIdx.x; i < gstart[g] + gn[g]; i += blockDim.x) grp[i] = gid[g];
+  for (ll i = gstart[g] + (ll)blockIdx.y * blockDim.x + threadIdx.x; i < gstart[g] + gn[g];
+       i += (ll)gridDim.y * blockDim.x)
+    grp[i] = gid[g];
 }
 
 // Fill pos -> id for host-described contiguous groups.
@@ -4737,16 +4745,20 @@ void fill_groups(const std::vector<ll> &st, const std::vector<ll> &n, const std:
   h2d(a.p, st.data(), ng);
   h2d(b.p, n.data(), ng);
   h2d(c.p, id.data(), ng);
-  k_fill_grp<<<ng, 256, 0, ctx().stream>>>(a.p, b.p, c.p, ng, d_out);
+  // a few thousand blocks in all, whatever the number of groups
+  const unsigned per = (unsigned)std::max(1, std::min(4096 / ng, (int)((N + 4095) / 4096)));
+  k_fill_grp<<<dim3((unsigned)ng, per), 256, 0, ctx().stream>>>(a.p, b.p, c.p, ng, d_out);
   CK_LAUNCH();
   sync();
 }
 
-void build_level(const Graph &g, const int *perm, const int *inv, const int *grp, ll N,
-                 Level &lv) {
+void build_level(const Graph &g, const int *perm, const int *grp, ll N, Level &lv) {
   cudaStream_t st = ctx().stream;
+  DBuf<int2> pg((size_t)N);
+  k_pos_grp<<<grid_for(N, 256), 256, 0, st>>>(perm, grp, N, pg.p);
+  CK_LAUNCH();
   DBuf<int> rowlen((size_t)N);
-  k_ell_count<<<grid_for(N, 256), 256, 0, st>>>(perm, inv, grp, g.rowptr.p, g.col.p, N,
+  k_ell_count<<<grid_for(N, 256), 256, 0, st>>>(perm, pg.p, grp, g.rowptr.p, g.col.p, N,
                                                 rowlen.p);
   CK_LAUNCH();
   ll nslice = (N + 31) / 32;
@@ -4759,7 +4771,7 @@ void build_level(const Graph &g, const int *perm, const int *inv, const int *grp
   h2d(lv.slice_off.p + nslice, &total, 1);  // end of the last slice
   lv.words = total;
   lv.ell.ensure((size_t)total + 32);
-  k_ell_fill<<<grid_for(N, 256), 256, 0, st>>>(perm, inv, grp, g.rowptr.p, g.col.p, g.w.p, N,
+  k_ell_fill<<<grid_for(N, 256), 256, 0, st>>>(perm, pg.p, grp, g.rowptr.p, g.col.p, g.w.p, N,
                                                lv.slice_off.p, lv.slice_w.p, lv.ell.p);
   CK_LAUNCH();
   // restricted nnz of active rows (for the algorithmic byte count)
@@ -5294,7 +5306,8 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   k_vid_keys<<<grid_for(ns, 256), 256, 0, st>>>(d_vtx, ns, keys.p, vals.p);
   CK_LAUNCH();
   seg_sort_pairs(keys, vals, ns, nullptr, 1, sws);
-  DBuf<int> flag((size_t)ns), runid((size_t)ns), inv((size_t)ns);
+  DBuf<int> flag((size_t)ns), runid((size_t)ns);
+  DBuf<int2> run((size_t)ns);
   DBuf<ll> excl((size_t)ns);
   k_run_flags<<<grid_for(ns, 256), 256, 0, st>>>(keys.p, ns, flag.p);
   CK_LAUNCH();
@@ -5303,7 +5316,7 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   k_run_bounds<<<grid_for(ns, 256), 256, 0, st>>>(flag.p, excl.p, ns, nruns, runid.p,
                                                   run_start.p);
   CK_LAUNCH();
-  k_scatter_inv<<<grid_for(ns, 256), 256, 0, st>>>(vals.p, ns, inv.p);
+  k_scatter_run<<<grid_for(ns, 256), 256, 0, st>>>(vals.p, runid.p, run_start.p, ns, run.p);
   CK_LAUNCH();
   keys.release();
   excl.release();
@@ -5312,9 +5325,9 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   DBuf<int> maxw(1);
   CK(cudaMemsetAsync(maxw.p, 0, sizeof(int), st));
   CK(cudaMemsetAsync(rowlen.p + nel, 0, sizeof(ll), st));
-  const unsigned gr_blocks = grid_for(nel, GR_WARPS);
+  const unsigned gr_blocks = std::min(grid_for(nel, GR_WARPS), 152u * 9u * 2u);  // two waves
   k_graph_rows<false><<<gr_blocks, GR_WARPS * 32, 0, st>>>(
-      nv, nel, vals.p, inv.p, runid.p, run_start.p, nullptr, nullptr, nullptr, rowlen.p, maxw.p);
+      nv, nel, vals.p, run.p, nullptr, nullptr, nullptr, rowlen.p, maxw.p);
   CK_LAUNCH();
   g.nnz = exclusive_scan_ll(rowlen.p, g.rowptr.p, nel + 1);
   DBuf<unsigned long long> mrow(1);
@@ -5331,8 +5344,7 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   g.col.ensure((size_t)g.nnz + 1);
   g.w.ensure((size_t)g.nnz + 1);
   k_graph_rows<true><<<gr_blocks, GR_WARPS * 32, 0, st>>>(
-      nv, nel, vals.p, inv.p, runid.p, run_start.p, g.rowptr.p, g.col.p, g.w.p, nullptr,
-      nullptr);
+      nv, nel, vals.p, run.p, g.rowptr.p, g.col.p, g.w.p, nullptr, nullptr);
   CK_LAUNCH();
 }
 
@@ -5352,7 +5364,7 @@ static void rsb_impl(const long long *d_vtx, const double *cent, ll N, int nv, i
   if (G.max_w >= 16 || N >= (1ll << 28))
     throw ArgError{PARRSB_ERR_UNSUPPORTED,
                    "dual-graph weight >= 16 or more than 2^28 elements"};
-  DBuf<int> perm((size_t)N), inv((size_t)N), grp((size_t)N), half((size_t)N),
+  DBuf<int> perm((size_t)N), grp((size_t)N), half((size_t)N),
       segpos((size_t)N), idx((size_t)N), moved((size_t)N), flag((size_t)N);
   DBuf<double> f_pos((size_t)N), f_tmp((size_t)N), y_pred;
   DBuf<float4> esp;  // element spacings (warm starts only)
@@ -5431,9 +5443,7 @@ static void rsb_impl(const long long *d_vtx, const double *cent, ll N, int nv, i
       StageTimer tm(PARRSB_STAGE_RESTRICT);
       fill_groups(all_st, all_n, all_active_id, grp.p, N);
       fill_groups(all_st, all_n, all_id, segpos.p, N);
-      k_inv_perm<<<grid_for(N, 256), 256, 0, st>>>(perm.p, N, inv.p);
-      CK_LAUNCH();
-      build_level(G, perm.p, inv.p, grp.p, N, lv);
+      build_level(G, perm.p, grp.p, N, lv);
     }
     // ---- learned warm start: predictions for the groups of this level
     // that are large enough (the judge in Lanczos::choose_start decides)
@@ -5691,14 +5701,22 @@ static void rsb_impl(const long long *d_vtx, const double *cent, ll N, int nv, i
   }
 }
 
+// cnt[g] += 1 for every lane with g >= 0: one atomic per group and warp (every
+// lane calls it; neighbouring elements usually share a group)
+__device__ __forceinline__ void count_groups(int g, int *__restrict__ cnt) {
+  const unsigned peers = __match_any_sync(0xffffffffu, g);
+  if (g >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[g], __popc(peers));
+}
+
 __global__ void k_group_keys(const int *__restrict__ group_of, ll N, u64 *__restrict__ keys,
                              int *__restrict__ vals, int *__restrict__ cnt) {
   ll e = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= N) return;
-  int g = group_of[e];
-  keys[e] = (u64)(unsigned)g;
-  vals[e] = (int)e;
-  atomicAdd(&cnt[g], 1);
+  const int g = e < N ? group_of[e] : -1;
+  if (e < N) {
+    keys[e] = (u64)(unsigned)g;
+    vals[e] = (int)e;
+  }
+  count_groups(g, cnt);
 }
 
 __global__ void k_scatter_f(const int *__restrict__ perm, const double *__restrict__ f_pos,
@@ -5722,7 +5740,7 @@ static void fiedler_groups_impl(const long long *d_vtx, ll N, int nv, const int 
     throw ArgError{PARRSB_ERR_UNSUPPORTED, "dual-graph weight >= 16 or more than 2^28 elements"};
   // order elements by group (stable: element order inside a group)
   DBuf<u64> keys((size_t)N);
-  DBuf<int> perm((size_t)N), cnt((size_t)ngroups), inv((size_t)N), grp((size_t)N);
+  DBuf<int> perm((size_t)N), cnt((size_t)ngroups), grp((size_t)N);
   CK(cudaMemsetAsync(cnt.p, 0, (size_t)ngroups * sizeof(int), st));
   k_group_keys<<<grid_for(N, 256), 256, 0, st>>>(d_group_of, N, keys.p, perm.p, cnt.p);
   CK_LAUNCH();
@@ -5745,12 +5763,10 @@ static void fiedler_groups_impl(const long long *d_vtx, ll N, int nv, const int 
     pos += hc[g];
   }
   fill_groups(all_st, all_n, act_id, grp.p, N);
-  k_inv_perm<<<grid_for(N, 256), 256, 0, st>>>(perm.p, N, inv.p);
-  CK_LAUNCH();
   Level lv;
   {
     StageTimer tm(PARRSB_STAGE_RESTRICT);
-    build_level(G, perm.p, inv.p, grp.p, N, lv);
+    build_level(G, perm.p, grp.p, N, lv);
   }
   DBuf<double> f_pos((size_t)N);
   CK(cudaMemsetAsync(f_pos.p, 0, (size_t)N * sizeof(double), st));
@@ -5809,11 +5825,12 @@ __global__ void k_group_keys_opt(const int *__restrict__ group_of, ll N, int ngr
                                  u64 *__restrict__ keys, int *__restrict__ vals,
                                  int *__restrict__ cnt) {
   ll e = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= N) return;
-  int g = group_of[e];
-  keys[e] = g >= 0 ? (u64)(unsigned)g : (u64)(unsigned)ngroups;
-  vals[e] = (int)e;
-  if (g >= 0) atomicAdd(&cnt[g], 1);
+  const int g = e < N ? group_of[e] : -1;
+  if (e < N) {
+    keys[e] = g >= 0 ? (u64)(unsigned)g : (u64)(unsigned)ngroups;
+    vals[e] = (int)e;
+  }
+  count_groups(g, cnt);
 }
 
 __global__ void k_iota(int *__restrict__ a, ll N) {
@@ -5840,7 +5857,7 @@ void build_group_level(const long long *d_vtx, ll N, int nv, const int *d_group_
   if (G.max_w >= 16 || N >= (1ll << 28))
     throw ArgError{PARRSB_ERR_UNSUPPORTED, "dual-graph weight >= 16 or more than 2^28 elements"};
   DBuf<u64> keys((size_t)N);
-  DBuf<int> cnt((size_t)ngroups), inv((size_t)N);
+  DBuf<int> cnt((size_t)ngroups);
   out.perm.ensure((size_t)N), out.grp.ensure((size_t)N);
   CK(cudaMemsetAsync(cnt.p, 0, (size_t)ngroups * sizeof(int), st));
   k_group_keys_opt<<<grid_for(N, 256), 256, 0, st>>>(d_group_of, N, ngroups, keys.p, out.perm.p,
@@ -5860,9 +5877,7 @@ void build_group_level(const long long *d_vtx, ll N, int nv, const int *d_group_
   }
   CK(cudaMemsetAsync(out.grp.p, 0xff, (size_t)N * sizeof(int), st));  // no group: -1
   fill_groups(st_, n_, id_, out.grp.p, N);
-  k_inv_perm<<<grid_for(N, 256), 256, 0, st>>>(out.perm.p, N, inv.p);
-  CK_LAUNCH();
-  build_level(G, out.perm.p, inv.p, out.grp.p, N, out.lv);
+  build_level(G, out.perm.p, out.grp.p, N, out.lv);
 }
 
 void components_device(const long long *d_vtx, ll N, int nv, const int *d_group_of, int ngroups,
