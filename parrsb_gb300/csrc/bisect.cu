@@ -24,8 +24,41 @@ namespace prsb {
 
 namespace {
 
-__global__ void k_centroids(const double *__restrict__ xyz, int nel, int nv,
-                            int ndim, double *__restrict__ cent) {
+// Bound by the FP64 pipe (64 cycles a warp instruction) and then by memory:
+// corners come through shared memory, the first one needs no addition, and a
+// division by 4 or 8 is an exact product.  8M hexes: 0.84 -> 0.44 ms.
+constexpr int CE_ELEMS = 128;
+__device__ __forceinline__ double no_minus_zero(double x) {  // 0.0 + x
+  return (__double_as_longlong(x) << 1) == 0 ? 0.0 : x;
+}
+template <int NV>
+__global__ void __launch_bounds__(CE_ELEMS)
+k_centroids(const double *__restrict__ xyz, int nel, double *__restrict__ cent) {
+  constexpr int ND = NV == 8 ? 3 : 2, ROW = NV * ND, PAD = ROW + 1;
+  extern __shared__ double ce_smem[];
+  const int e0 = blockIdx.x * CE_ELEMS, ne = min(CE_ELEMS, nel - e0);
+  const double *x = xyz + (ll)e0 * ROW;
+#pragma unroll 8
+  for (int k = threadIdx.x; k < ne * ROW; k += CE_ELEMS) ce_smem[k / ROW * PAD + k % ROW] = x[k];
+  __syncthreads();
+  if ((int)threadIdx.x >= ne) return;
+  const double *c = ce_smem + threadIdx.x * PAD;
+  const ll e = e0 + threadIdx.x;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    double s = 0.0;
+    if (d < ND) {
+      s = no_minus_zero(c[d]);
+#pragma unroll
+      for (int v = 1; v < NV; v++) s = __dadd_rn(s, c[v * ND + d]);
+      s = __dmul_rn(s, 1.0 / NV);
+    }
+    cent[d * (ll)nel + e] = s;
+  }
+}
+// without coordinates, or with another number of corners
+__global__ void k_centroids_any(const double *__restrict__ xyz, int nel, int nv, int ndim,
+                                double *__restrict__ cent) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   double c[3] = {0.0, 0.0, 0.0};
@@ -1115,7 +1148,13 @@ cudaError_t rcb_small_launch(int *perm, const u32 *rank, double *uniq, ll N, int
 
 void compute_centroids(const double *xyz, int nel, int nv, double *cent) {
   int ndim = (nv == 8) ? 3 : 2;
-  k_centroids<<<grid_for(nel, 256), 256, 0, ctx().stream>>>(xyz, nel, nv, ndim, cent);
+  const size_t smem = (size_t)CE_ELEMS * (nv * ndim + 1) * sizeof(double);
+  if (xyz && nv == 8)
+    k_centroids<8><<<grid_for(nel, CE_ELEMS), CE_ELEMS, smem, ctx().stream>>>(xyz, nel, cent);
+  else if (xyz && nv == 4)
+    k_centroids<4><<<grid_for(nel, CE_ELEMS), CE_ELEMS, smem, ctx().stream>>>(xyz, nel, cent);
+  else
+    k_centroids_any<<<grid_for(nel, 256), 256, 0, ctx().stream>>>(xyz, nel, nv, ndim, cent);
   CK_LAUNCH();
 }
 
@@ -1162,16 +1201,33 @@ __global__ void k_ps_axis(const int *__restrict__ lists, const u32 *__restrict__
   split[s] = p[s] > 1 ? lower_count(n[s], p[s]) : n[s] / 2;
 }
 
-// side of every element of a cut segment: 1 for the upper child
-__global__ void k_ps_side(const int *__restrict__ lists, ll N, const int *__restrict__ seg_of_pos,
-                          const ll *__restrict__ st, const int *__restrict__ axis,
-                          const ll *__restrict__ split, unsigned char *__restrict__ side) {
-  const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  const int s = seg_of_pos[j];
-  const int a = axis[s];
-  if (a < 0) return;
-  side[lists[(ll)a * N + j]] = (j - st[s]) >= split[s] ? 1 : 0;
+// The kernels over list positions below take PS_ITEMS rounds of 32 positions
+// per warp, the loads of all rounds first: each position is a chain of three
+// or four dependent loads, and their latency, not memory, bounded a thread per
+// position (8M elements: side 71 -> 52 us, flags 79 -> 59, scatter
+// 124 -> 58).
+
+// side of every element of a cut segment: 1 for the upper child (side is zero
+// before: half of the scattered stores)
+__global__ void __launch_bounds__(256)
+k_ps_side(const int *__restrict__ lists, ll N, const int *__restrict__ seg_of_pos,
+          const ll *__restrict__ st, const int *__restrict__ axis, const ll *__restrict__ split,
+          unsigned char *__restrict__ side) {
+  const ll j0 = ((ll)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * PS_ITEMS + (threadIdx.x & 31);
+  int s[PS_ITEMS], a[PS_ITEMS], e[PS_ITEMS];
+  ll cut[PS_ITEMS];
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) s[r] = j0 + 32 * r < N ? seg_of_pos[j0 + 32 * r] : -1;
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) {
+    a[r] = s[r] >= 0 ? axis[s[r]] : -1;
+    cut[r] = s[r] >= 0 ? st[s[r]] + split[s[r]] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) e[r] = a[r] >= 0 ? lists[(ll)a[r] * N + j0 + 32 * r] : 0;
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++)
+    if (a[r] >= 0 && j0 + 32 * r >= cut[r]) side[e[r]] = 1;
 }
 
 __device__ __forceinline__ int ps_block_excl(int v, int *total) {
@@ -1208,18 +1264,29 @@ __device__ __forceinline__ int ps_block_excl(int v, int *total) {
 constexpr int PS_WORDS = PS_TILE / 32;
 __global__ void __launch_bounds__(PS_THREADS)
 k_ps_flags(const int *__restrict__ lists, ll N, int ndim, const int *__restrict__ seg_of_pos,
-           const int *__restrict__ axis, const unsigned char *__restrict__ side,
+           const int *__restrict__ axis, int own, const unsigned char *__restrict__ side,
            u32 *__restrict__ bits, int *__restrict__ wpre, int *__restrict__ bsum, int nblk) {
   __shared__ int wtot[3][PS_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const ll nw = (N + 31) >> 5;
   const ll w0 = (ll)blockIdx.x * PS_WORDS + (ll)warp * PS_ITEMS;  // this warp's first word
-  bool cut[PS_ITEMS];
+  int e[3][PS_ITEMS], ax[PS_ITEMS];
 #pragma unroll
   for (int r = 0; r < PS_ITEMS; r++) {
     const ll j = (w0 + r) * 32 + lane;
-    cut[r] = j < N && axis[seg_of_pos[j]] >= 0;
+    ax[r] = j < N ? seg_of_pos[j] : -1;
+#pragma unroll
+    for (int b = 0; b < 3; b++) e[b][r] = b < ndim && j < N ? lists[(ll)b * N + j] : -1;
   }
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) ax[r] = ax[r] >= 0 ? axis[ax[r]] : -1;
+#pragma unroll
+  for (int b = 0; b < 3; b++)
+#pragma unroll
+    for (int r = 0; r < PS_ITEMS; r++) {
+      const bool look = e[b][r] >= 0 && ax[r] >= 0 && !(own && ax[r] == b);
+      e[b][r] = look ? side[e[b][r]] : 1;  // 0: goes to the lower child
+    }
   int pre[3][PS_ITEMS];
 #pragma unroll
   for (int b = 0; b < 3; b++) {
@@ -1227,9 +1294,7 @@ k_ps_flags(const int *__restrict__ lists, ll N, int ndim, const int *__restrict_
     int c = 0;
 #pragma unroll
     for (int r = 0; r < PS_ITEMS; r++) {
-      const ll j = (w0 + r) * 32 + lane;
-      const bool f = cut[r] && side[lists[(ll)b * N + j]] == 0;
-      const u32 bal = __ballot_sync(0xffffffffu, f);
+      const u32 bal = __ballot_sync(0xffffffffu, e[b][r] == 0);
       if (lane == 0 && w0 + r < nw) bits[(ll)b * nw + w0 + r] = bal;
       pre[b][r] = c;
       c += __popc(bal);
@@ -1278,42 +1343,61 @@ __global__ void __launch_bounds__(PS_THREADS) k_ps_bscan(int *__restrict__ bsum,
     }
 }
 
-// lower flags of list b before position x: the tiles before it, the words
-// before it in its tile, the bits below it in its word
-__device__ __forceinline__ ll ps_before(const u32 *__restrict__ bits,
-                                        const int *__restrict__ wpre,
-                                        const int *__restrict__ bsum, ll x) {
-  const ll w = x >> 5;
-  return (ll)bsum[w / PS_WORDS] + wpre[w] + __popc(bits[w] & ((1u << (x & 31)) - 1u));
-}
-
 // stable partition of every cut segment of each list by side, and the
 // segment of every position in the children's table (child_off: the first
 // child of each segment, the lower one of a cut)
-__global__ void k_ps_scatter(const int *__restrict__ lists, ll N, int ndim,
-                             const int *__restrict__ seg_of_pos, const ll *__restrict__ st,
-                             const int *__restrict__ axis, const ll *__restrict__ split,
-                             const u32 *__restrict__ bits, const int *__restrict__ wpre,
-                             const int *__restrict__ bsum, int nblk,
-                             const ll *__restrict__ child_off, int *__restrict__ lists2,
-                             int *__restrict__ seg_of_pos2) {
-  const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  const int s = seg_of_pos[j];
-  const ll s0 = st[s];
-  const bool cut = axis[s] >= 0;
-  seg_of_pos2[j] = (int)(child_off[s] + ((cut && j - s0 >= split[s]) ? 1 : 0));
+__global__ void __launch_bounds__(256)
+k_ps_scatter(const int *__restrict__ lists, ll N, int ndim, const int *__restrict__ seg_of_pos,
+             const ll *__restrict__ st, const int *__restrict__ axis, int own,
+             const ll *__restrict__ split, const u32 *__restrict__ bits,
+             const int *__restrict__ wpre, const int *__restrict__ bsum, int nblk,
+             const ll *__restrict__ child_off, int *__restrict__ lists2,
+             int *__restrict__ seg_of_pos2) {
+  const int lane = threadIdx.x & 31;
+  const ll j0 = ((ll)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * PS_ITEMS + lane;
   const ll nw = (N + 31) >> 5;
-  for (int b = 0; b < ndim; b++) {
-    const int e = lists[(ll)b * N + j];
-    ll dest = j;
-    if (cut) {
-      const u32 *bb = bits + (ll)b * nw;
-      const int *wp = wpre + (ll)b * nw, *bs = bsum + (ll)b * nblk;
-      const ll c = ps_before(bb, wp, bs, j) - ps_before(bb, wp, bs, s0);  // lower entries before j
-      dest = ((bb[j >> 5] >> (j & 31)) & 1u) ? s0 + c : s0 + split[s] + (j - s0 - c);
+  int s[PS_ITEMS], e[3][PS_ITEMS], ax[PS_ITEMS], s0[PS_ITEMS], up[PS_ITEMS], child[PS_ITEMS];
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) {
+    const ll j = j0 + 32 * r;
+    s[r] = j < N ? seg_of_pos[j] : -1;
+#pragma unroll
+    for (int b = 0; b < 3; b++) e[b][r] = b < ndim && j < N ? lists[(ll)b * N + j] : -1;
+  }
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++) {
+    const bool in = s[r] >= 0;
+    ax[r] = in ? axis[s[r]] : -1;
+    s0[r] = in ? (int)st[s[r]] : 0;
+    up[r] = in ? s0[r] + (int)split[s[r]] : 0;  // first position of the upper child
+    child[r] = in ? (int)child_off[s[r]] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < PS_ITEMS; r++)
+    if (s[r] >= 0)
+      seg_of_pos2[j0 + 32 * r] = child[r] + (ax[r] >= 0 && j0 + 32 * r >= up[r] ? 1 : 0);
+#pragma unroll
+  for (int b = 0; b < 3; b++) {
+    if (b >= ndim) break;
+    const u32 *bb = bits + (ll)b * nw;
+    const int *wp = wpre + (ll)b * nw, *bs = bsum + (ll)b * nblk;
+    int dest[PS_ITEMS];
+#pragma unroll
+    for (int r = 0; r < PS_ITEMS; r++) {
+      const int j = (int)(j0 + 32 * r);
+      dest[r] = j;
+      if (ax[r] >= 0 && !(own && ax[r] == b)) {
+        const u32 word = bb[j >> 5];
+        // lower entries of the segment before j
+        const int c = bs[j / PS_TILE] + wp[j >> 5] + __popc(word & ((1u << lane) - 1u)) -
+                      (bs[s0[r] / PS_TILE] + wp[s0[r] >> 5] +
+                       __popc(bb[s0[r] >> 5] & ((1u << (s0[r] & 31)) - 1u)));
+        dest[r] = (word >> lane & 1u) ? s0[r] + c : up[r] + (j - s0[r] - c);
+      }
     }
-    lists2[(ll)b * N + dest] = e;
+#pragma unroll
+    for (int r = 0; r < PS_ITEMS; r++)
+      if (s[r] >= 0) lists2[(ll)b * N + dest[r]] = e[b][r];
   }
 }
 
@@ -1681,13 +1765,13 @@ static void rcb_presorted(DBuf<int> &perm, SegTable &t, const double *cent, ll N
                                                        ws.child_off.p, ws.side.p);
       CK_LAUNCH();
       k_ps_flags<<<(unsigned)nblk, PS_THREADS, 0, st>>>(ws.glists.p, N, ndim, ws.oseg.p,
-                                                        ws.axis.p, ws.side.p, ws.pbits.p,
+                                                        ws.axis.p, 0, ws.side.p, ws.pbits.p,
                                                         ws.pwpre.p, ws.bsum.p, nblk);
       CK_LAUNCH();
       k_ps_bscan<<<(unsigned)ndim, PS_THREADS, 0, st>>>(ws.bsum.p, nblk);
       CK_LAUNCH();
-      k_ps_scatter<<<grid_for(N, 256), 256, 0, st>>>(
-          ws.glists.p, N, ndim, ws.oseg.p, ws.gt.start.p, ws.axis.p, ws.split.p, ws.pbits.p,
+      k_ps_scatter<<<grid_for(N, 256 * PS_ITEMS), 256, 0, st>>>(
+          ws.glists.p, N, ndim, ws.oseg.p, ws.gt.start.p, ws.axis.p, 0, ws.split.p, ws.pbits.p,
           ws.pwpre.p, ws.bsum.p, nblk, ws.child_off.p, ws.lists.p, ws.seg_of_pos2.p);
       CK_LAUNCH();
       built = true;
@@ -1767,11 +1851,12 @@ static void rcb_presorted(DBuf<int> &perm, SegTable &t, const double *cent, ll N
                                                    t.start.p, t.n.p, t.p.p, nseg, do_local,
                                                    ws.axis.p, ws.split.p);
     CK_LAUNCH();
-    k_ps_side<<<grid_for(N, 256), 256, 0, st>>>(ws.lists.p, N, ws.seg_of_pos.p, t.start.p,
+    CK(cudaMemsetAsync(ws.side.p, 0, (size_t)N, st));
+    k_ps_side<<<grid_for(N, 256 * PS_ITEMS), 256, 0, st>>>(ws.lists.p, N, ws.seg_of_pos.p, t.start.p,
                                                 ws.axis.p, ws.split.p, ws.side.p);
     CK_LAUNCH();
     k_ps_flags<<<(unsigned)nblk, PS_THREADS, 0, st>>>(ws.lists.p, N, ndim, ws.seg_of_pos.p,
-                                                      ws.axis.p, ws.side.p, ws.pbits.p,
+                                                      ws.axis.p, 1, ws.side.p, ws.pbits.p,
                                                       ws.pwpre.p, ws.bsum.p, nblk);
     CK_LAUNCH();
     k_ps_bscan<<<(unsigned)ndim, PS_THREADS, 0, st>>>(ws.bsum.p, nblk);
@@ -1780,8 +1865,8 @@ static void rcb_presorted(DBuf<int> &perm, SegTable &t, const double *cent, ll N
     ws.child_off.ensure((size_t)nseg + 1);
     exclusive_scan_int_to_ll_async(ws.child_cnt.p, ws.child_off.p, nseg);
     const ll nchild = nseg + nact;
-    k_ps_scatter<<<grid_for(N, 256), 256, 0, st>>>(
-        ws.lists.p, N, ndim, ws.seg_of_pos.p, t.start.p, ws.axis.p, ws.split.p, ws.pbits.p,
+    k_ps_scatter<<<grid_for(N, 256 * PS_ITEMS), 256, 0, st>>>(
+        ws.lists.p, N, ndim, ws.seg_of_pos.p, t.start.p, ws.axis.p, 1, ws.split.p, ws.pbits.p,
         ws.pwpre.p, ws.bsum.p, nblk, ws.child_off.p, ws.lists2.p, ws.seg_of_pos2.p);
     CK_LAUNCH();
     std::swap(ws.lists.p, ws.lists2.p);
