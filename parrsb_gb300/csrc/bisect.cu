@@ -534,14 +534,32 @@ __global__ void k_rank_flags(const u64 *__restrict__ keys, ll N, int *__restrict
   if (i < N) flag[i] = (i > 0 && keys[i] != keys[i - 1]) ? 1 : 0;
 }
 
+// cnt += positions whose key differs from the one before
+__global__ void __launch_bounds__(256)
+k_count_changes(const u64 *__restrict__ keys, ll N, unsigned long long *__restrict__ cnt) {
+  unsigned c = 0;
+  for (ll i = (ll)blockIdx.x * 256 + threadIdx.x; i < N; i += (ll)gridDim.x * 256)
+    c += i > 0 && keys[i] != keys[i - 1];
+  c = __reduce_add_sync(0xffffffffu, c);
+  __shared__ unsigned sh[8];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t = 0;
+    for (int w = 0; w < 8; w++) t += sh[w];
+    atomicAdd(cnt, t);
+  }
+}
+
+// flag null: every key differs from the one before
 __global__ void k_rank_write(const u64 *__restrict__ keys, const int *__restrict__ vals,
                              const int *__restrict__ flag, const ll *__restrict__ excl, ll N,
                              u32 *__restrict__ rank, double *__restrict__ uniq) {
   ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  ll r = excl[i] + flag[i];
+  ll r = flag ? excl[i] + flag[i] : i;
   rank[vals[i]] = (u32)r;
-  if (i == 0 || flag[i]) {
+  if (i == 0 || !flag || flag[i]) {
     u64 k = keys[i];
     u64 bits = (k >> 63) ? (k ^ 0x8000000000000000ull) : ~k;
     uniq[r] = __longlong_as_double((long long)bits);
@@ -1930,18 +1948,31 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
     ws.rank.ensure((size_t)3 * N);
     ws.uniq.ensure((size_t)3 * N);
     ws.sorted.ensure((size_t)ndim * N);
-    DBuf<int> flag((size_t)N);
-    DBuf<ll> excl((size_t)N);
+    DBuf<int> flag;
+    DBuf<ll> excl;
+    DBuf<unsigned long long> changes(1);
     ws.unique = true;
     for (int a = 0; a < ndim; a++) {
       k_axis_keys<<<grid_for(N, 256), 256, 0, st>>>(cent, N, a, ws.keys.p, ws.vals.p);
       CK_LAUNCH();
-      sort_by_value(ws.keys, ws.vals, N, nullptr, 1, N, ws.sort);
-      k_rank_flags<<<grid_for(N, 256), 256, 0, st>>>(ws.keys.p, N, flag.p);
+      sort_by_value(ws.keys, ws.vals, N, nullptr, 1, N, ws.sort, true);
+      CK(cudaMemsetAsync(changes.p, 0, sizeof(unsigned long long), st));
+      k_count_changes<<<std::min(grid_for(N, 256), 152u * 8u), 256, 0, st>>>(ws.keys.p, N,
+                                                                            changes.p);
       CK_LAUNCH();
-      const ll changes = exclusive_scan_int_to_ll(flag.p, excl.p, N);
-      if (changes != N - 1) ws.unique = false;  // two centroids share a coordinate
-      k_rank_write<<<grid_for(N, 256), 256, 0, st>>>(ws.keys.p, ws.vals.p, flag.p, excl.p, N,
+      unsigned long long h_changes = 0;
+      d2h(&h_changes, changes.p, 1);
+      sync();
+      const bool ties = (ll)h_changes != N - 1;  // two centroids share a coordinate
+      if (ties) {
+        ws.unique = false;
+        flag.ensure((size_t)N), excl.ensure((size_t)N);
+        k_rank_flags<<<grid_for(N, 256), 256, 0, st>>>(ws.keys.p, N, flag.p);
+        CK_LAUNCH();
+        exclusive_scan_int_to_ll_async(flag.p, excl.p, N);
+      }
+      k_rank_write<<<grid_for(N, 256), 256, 0, st>>>(ws.keys.p, ws.vals.p,
+                                                      ties ? flag.p : nullptr, excl.p, N,
                                                       ws.rank.p + (ll)a * N,
                                                       ws.uniq.p + (ll)a * N);
       CK_LAUNCH();

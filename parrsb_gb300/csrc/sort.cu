@@ -132,6 +132,19 @@ __global__ void k_tile_scan(u32 *__restrict__ counts, int ntiles,
   if (threadIdx.x == 0) totals[blockIdx.x] = carry_s;
 }
 
+// lanes with the same 8-bit digit (of the lanes in `valid`), by a ballot per
+// bit: __match_any_sync takes longer the more digits a warp holds
+__device__ __forceinline__ u32 digit_peers(u32 d, u32 valid) {
+  u32 peers = valid;
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const bool bit = (d >> b) & 1u;
+    const u32 bal = __ballot_sync(0xffffffffu, bit);
+    peers &= bit ? bal : ~bal;
+  }
+  return peers;
+}
+
 __global__ void __launch_bounds__(SORT_THREADS)
 k_scatter(const u64 *__restrict__ kin, const int *__restrict__ vin,
           u64 *__restrict__ kout, int *__restrict__ vout, ll n,
@@ -191,7 +204,7 @@ k_scatter(const u64 *__restrict__ kin, const int *__restrict__ vin,
   for (int r = 0; r < ITEMS_PER_THREAD; r++) {
     const u32 d = dig[r];
     const bool valid = d < 256;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned peers = digit_peers(d, __ballot_sync(0xffffffffu, valid));
     u32 before = 0;
     if (valid) before = wcnt[warp][d];
     __syncwarp();
@@ -567,19 +580,29 @@ __global__ void k_key_range(const u64 *__restrict__ keys, ll n, u64 *__restrict_
 }
 
 // q[i] = segment (top sb bits), value over the range (32 - sb bits)
-__global__ void k_quant(const u64 *__restrict__ keys, const int *__restrict__ seg, ll n, int sb,
-                        const u64 *__restrict__ range, u32 *__restrict__ q,
-                        int *__restrict__ idx) {
-  const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+constexpr int QU_THREADS = 256, QU_ITEMS = 4;  // (the range's shifts once per thread)
+__global__ void __launch_bounds__(QU_THREADS)
+k_quant(const u64 *__restrict__ keys, const int *__restrict__ seg, ll n, int sb,
+        const u64 *__restrict__ range, u32 *__restrict__ q) {
+  const ll i0 = (ll)blockIdx.x * (QU_THREADS * QU_ITEMS) + threadIdx.x;
   const u64 k0 = range[0], k1 = range[1];
   const int em = max(1, max(key_exp(k0), key_exp(k1)));
   const ll f0 = key_fixed(k0, em);
   const u64 r = (u64)(key_fixed(k1, em) - f0);
   const int s = max(0, 64 - __clzll((ll)r) - (32 - sb));
-  const u32 v = (u32)((u64)(key_fixed(keys[i], em) - f0) >> s);
-  q[i] = v | (seg && sb ? (u32)seg[i] << (32 - sb) : 0u);
-  idx[i] = (int)i;
+  u64 k[QU_ITEMS];
+  u32 g[QU_ITEMS];
+#pragma unroll
+  for (int u = 0; u < QU_ITEMS; u++) {
+    const ll i = i0 + u * QU_THREADS;
+    k[u] = i < n ? keys[i] : 0ull;
+    g[u] = seg && sb && i < n ? (u32)seg[i] << (32 - sb) : 0u;
+  }
+#pragma unroll
+  for (int u = 0; u < QU_ITEMS; u++) {
+    const ll i = i0 + u * QU_THREADS;
+    if (i < n) q[i] = (u32)((u64)(key_fixed(k[u], em) - f0) >> s) | g[u];
+  }
 }
 
 __global__ void __launch_bounds__(SORT_THREADS)
@@ -607,7 +630,9 @@ k_tile_hist32(const u32 *__restrict__ q, ll n, int shift, u32 *__restrict__ coun
   }
 }
 
-// k_scatter for 32-bit keys: a pair is one 8-byte word in shared memory
+// k_scatter for 32-bit keys: a pair is one 8-byte word in shared memory; vin
+// null: the positions.  The peers of all rounds are found before the counts,
+// which are a serial chain (8M random digits: 91 -> 56 us).
 __global__ void __launch_bounds__(SORT_THREADS)
 k_scatter32(const u32 *__restrict__ kin, const int *__restrict__ vin, u32 *__restrict__ kout,
             int *__restrict__ vout, ll n, int shift, const u32 *__restrict__ counts,
@@ -645,13 +670,17 @@ k_scatter32(const u32 *__restrict__ kin, const int *__restrict__ vin, u32 *__res
   for (int r = 0; r < ITEMS_PER_THREAD; r++) {
     const ll i = base + r * 32 + lane;
     key[r] = i < n ? kin[i] : 0u;
-    val[r] = i < n ? vin[i] : 0;
+    val[r] = i < n ? (vin ? vin[i] : (int)i) : 0;
   }
+#pragma unroll
+  for (int r = 0; r < ITEMS_PER_THREAD; r++)
+    rank[r] = digit_peers(key[r] >> shift,
+                          __ballot_sync(0xffffffffu, base + r * 32 + lane < n));
 #pragma unroll
   for (int r = 0; r < ITEMS_PER_THREAD; r++) {
     const bool valid = base + r * 32 + lane < n;
     const u32 d = valid ? (key[r] >> shift) & 255u : 256u;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned peers = rank[r];
     u32 before = 0;
     if (valid) before = wcnt[warp][d];
     __syncwarp();
@@ -712,7 +741,7 @@ __global__ void k_gather_kv(const int *__restrict__ idx, const u64 *__restrict__
   if (i >= n) return;
   const int j = idx[i];
   kout[i] = keys[j];
-  vout[i] = vals[j];
+  vout[i] = vals ? vals[j] : j;
 }
 
 __global__ void k_gather_val(const int *__restrict__ idx, const int *__restrict__ in, ll n,
@@ -874,7 +903,7 @@ void seg_sort_pairs(DBuf<u64> &keys, DBuf<int> &vals, ll n,
 }
 
 void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos, ll nseg,
-                   ll max_len, SortWs &ws) {
+                   ll max_len, SortWs &ws, bool iota) {
   if (n <= 1 || max_len <= 1) return;
   cudaStream_t st = ctx().stream;
   if (!seg_of_pos) nseg = 1;
@@ -918,8 +947,8 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
     k_key_range<<<(unsigned)std::min<ll>((n + 1023) / 1024, 152 * 4), 256, 0, st>>>(keys.p, n,
                                                                                   ws.range.p);
     CK_LAUNCH();
-    k_quant<<<grid_for(n, 256), 256, 0, st>>>(keys.p, seg_of_pos, n, sb, ws.range.p, ws.q.p,
-                                              ws.idx.p);
+    k_quant<<<grid_for(n, QU_THREADS * QU_ITEMS), QU_THREADS, 0, st>>>(keys.p, seg_of_pos, n, sb,
+                                                                       ws.range.p, ws.q.p);
     CK_LAUNCH();
     ensure_smem_limit(k_scatter32, (int)(TILE * sizeof(uint2)));  // with the tables over 48 KB
     for (int shift = 0; shift < 32; shift += 8) {
@@ -927,14 +956,15 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
       CK_LAUNCH();
       k_tile_scan<<<256, 1024, 0, st>>>(ws.counts.p, ntiles, ws.totals.p);
       CK_LAUNCH();
-      k_scatter32<<<ntiles, SORT_THREADS, TILE * sizeof(uint2), st>>>(ws.q.p, ws.idx.p, ws.qtmp.p, ws.idxtmp.p, n,
-                                                   shift, ws.counts.p, ws.totals.p, ntiles);
+      k_scatter32<<<ntiles, SORT_THREADS, TILE * sizeof(uint2), st>>>(
+          ws.q.p, shift ? ws.idx.p : nullptr, ws.qtmp.p, ws.idxtmp.p, n, shift, ws.counts.p,
+          ws.totals.p, ntiles);
       CK_LAUNCH();
       std::swap(ws.q, ws.qtmp);
       std::swap(ws.idx, ws.idxtmp);
     }
-    k_gather_kv<<<grid_for(n, 256), 256, 0, st>>>(ws.idx.p, keys.p, vals.p, n, ws.ktmp.p,
-                                                  ws.vtmp.p);
+    k_gather_kv<<<grid_for(n, 256), 256, 0, st>>>(ws.idx.p, keys.p, iota ? nullptr : vals.p, n,
+                                                  ws.ktmp.p, ws.vtmp.p);
     CK_LAUNCH();
     CK(cudaMemsetAsync(ws.idxtmp.p, 0, (size_t)n * sizeof(int), st));
     k_fix_runs<<<grid_for(n, 256), 256, 0, st>>>(ws.q.p, n, ws.ktmp.p, ws.vtmp.p, ws.range.p,

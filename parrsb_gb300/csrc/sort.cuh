@@ -95,9 +95,9 @@ void seg_sort_pairs(DBuf<u64> &keys, DBuf<int> &vals, ll n,
 // Sort (keys[i], vals[i]), i < n, stably by key inside each segment, for keys
 // that order doubles (ordered_key).  seg_of_pos[i] (may be null: one segment)
 // is the segment of position i, non-decreasing in [0, nseg); no segment is
-// longer than max_len.  Same result as seg_sort_pairs with the segment of
+// longer than max_len; iota: vals[i] is i.  Same result as seg_sort_pairs with the segment of
 // every value; keys / vals point at the sorted arrays on return.
 void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos, ll nseg,
-                   ll max_len, SortWs &ws);
+                   ll max_len, SortWs &ws, bool iota = false);
 
 }  // namespace prsb
