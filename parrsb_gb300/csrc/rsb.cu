@@ -1678,36 +1678,84 @@ k_rupd(const ll *__restrict__ tbeg, const ll *__restrict__ tend, const int *__re
 // The vector's sign is fixed later, on the final Fiedler vector (canonical
 // orientation).  Writes coef[j] = y_j / |r_j|.
 
+// x == 0, on 32-bit halves
+__device__ __forceinline__ bool zero_bits(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
 // number of eigenvalues of T below x (Sturm sequence of the leading
 // principal minors).  Only the two multiplies and the subtraction of each
 // step use the FP64 pipe (GB300 runs FP64 at 1/64 of the FP32 rate): signs,
 // zero tests and the range check read the bit pattern with integer
 // instructions, and the rescaling multiplies by exact powers of two.
-__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x) {
+// (Tests of a double's 64 bits against zero compile to FP64 comparisons again;
+// tests of its halves do not, and a rescaling in line is computed for every
+// row: 408 -> 274 cycles a row without them.)
+// FED: the differences d[i] - x come from another warp through shared memory
+// (dx[32 i], this lane's column; feed_rows), which leaves two instructions a
+// row (217 cycles).  Rows arrive in chunks that end at 4, 12, 28, 60, 124:
+// the feeder takes half as long per row, so each chunk is there when the last
+// one is used up.  Chunk k is announced on the named barrier FEED_BAR + k.
+constexpr int FEED_BAR = 2;
+__device__ __forceinline__ void feed_wait(int k) {
+  asm volatile("barrier.sync %0, 64;" ::"r"(FEED_BAR + k) : "memory");
+}
+__device__ __forceinline__ void feed_done(int k) {
+  asm volatile("barrier.arrive %0, 64;" ::"r"(FEED_BAR + k) : "memory");
+}
+__device__ __forceinline__ void feed_rows(const double *d, int n, double x, double *dx) {
+  for (int k = 0, i = 0; k == 0 || i < n; k++) {
+    const int end = min(n, (8 << k) - 4);
+    for (; i < end; i++) dx[32 * i] = __dsub_rn(d[i], x);
+    feed_done(k);
+  }
+}
+template <bool FED = false>
+__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x,
+                                           const double *dx = nullptr) {
+  int chunk = 0, bound = 0;  // next chunk to wait for and its first row
+  auto row = [&](int i) -> double {
+    if (!FED) return __dsub_rn(d[i], x);
+    if (i == bound) {
+      feed_wait(chunk);
+      bound = (8 << chunk) - 4;
+      chunk++;
+    }
+    return dx[32 * i];
+  };
   const double TINY = 1e-300;
-  double pm = 1.0, p = __dsub_rn(d[0], x);
-  long long pb = __double_as_longlong(p);
-  if ((pb << 1) == 0) p = -TINY, pb = __double_as_longlong(p);
-  int cnt = pb < 0;
+  double p = row(0);
+  if (zero_bits(p)) p = -TINY;
+  int hb = __double2hiint(p);
+  int cnt = (int)((unsigned)hb >> 31);
+  // a row ahead: d[i] - x, e2[i - 1] and its product with p two rows back (1
+  // at first), so that the product is under way beside the FMA
+  double s = n > 1 ? row(1) : 0.0, m = n > 1 ? e2[0] : 0.0, e = n > 2 ? e2[1] : 0.0;
   for (int i = 1; i < n; i++) {
-    double pn = fma(__dsub_rn(d[i], x), p, -__dmul_rn(e2[i - 1], pm));
-    long long nb = __double_as_longlong(pn);
-    if ((nb << 1) == 0) {  // exact zero: sign opposite to p
-      pn = pb < 0 ? TINY : -TINY;
-      nb = __double_as_longlong(pn);
+    double pn = fma(s, p, -m);
+    const double ei = e;
+    m = __dmul_rn(ei, p);
+    if (i + 1 < n) s = row(i + 1);
+    if (i + 2 < n) e = e2[i + 1];
+    int h = __double2hiint(pn);
+    // a binary exponent outside [423, 1623], zero among them
+    const bool odd = (unsigned)(h & 0x7FF00000) - 0x1A700000u > 0x4B000000u;
+    if (!odd) {
+      cnt += (int)((unsigned)(h ^ hb) >> 31);
+    } else {
+      asm volatile("");  // a branch, or every row pays for the three products
+      if (zero_bits(pn)) {  // exact zero: sign opposite to p
+        pn = hb < 0 ? TINY : -TINY;
+        h = __double2hiint(pn);
+      }
+      cnt += (int)((unsigned)(h ^ hb) >> 31);
+      const double scale = ((h >> 20) & 0x7FF) > 1023 + 600 ? 0x1p-600 : 0x1p600;
+      pn = __dmul_rn(pn, scale);
+      m = __dmul_rn(ei, __dmul_rn(p, scale));
+      h = __double2hiint(pn);
     }
-    cnt += (nb ^ pb) < 0;
-    pm = p;
     p = pn;
-    pb = nb;
-    const int ex = (int)((nb >> 52) & 0x7FF);
-    if (ex > 1023 + 600) {
-      p = __dmul_rn(p, 0x1p-600), pm = __dmul_rn(pm, 0x1p-600);
-      pb = __double_as_longlong(p);
-    } else if (ex < 1023 - 600) {
-      p = __dmul_rn(p, 0x1p600), pm = __dmul_rn(pm, 0x1p600);
-      pb = __double_as_longlong(p);
-    }
+    hb = h;
   }
   return cnt;
 }
@@ -1741,17 +1789,18 @@ __device__ __forceinline__ double fast_div(double y, double x) {
 
 // T - lam I = P L U with U having two super-diagonals (dgttrf), by lane 0 of
 // the warp: a, c, c2 the diagonals of U, b the multipliers.  L^-1 P is applied
-// to x (all ones) in the same loop.
-__device__ void tri_factor(int n, const double *a0, const double *e, double lam, double *x,
+// to x (all ones) in the same loop.  c2 holds the diagonal of T - lam I on
+// entry (its row i + 1 is read before its place i + 1 is written).
+__device__ void tri_factor(int n, const double *e, double *x,
                            double *a, double *b, double *c, double *c2, int *piv, double tiny) {
   // the rows of T - lam I enter one ahead of the elimination
-  double ai = __dsub_rn(a0[0], lam), ci = n > 1 ? e[0] : 0.0, xi = 1.0;
+  double ai = c2[0], ci = n > 1 ? e[0] : 0.0, xi = 1.0;
   for (int i = 0; i < n - 1; i++) {
-    const double bi = e[i], an = __dsub_rn(a0[i + 1], lam);  // row i + 1
+    const double bi = e[i], an = c2[i + 1];  // row i + 1
     const double cn = i < n - 2 ? e[i + 1] : 0.0;
     if (mag_bits(ai) >= mag_bits(bi)) {
       piv[i] = 0;
-      if (mag_bits(ai) == 0) ai = tiny;
+      if (zero_bits(ai)) ai = tiny;
       const double fact = fast_div(bi, ai);
       a[i] = ai, b[i] = fact, c[i] = ci, c2[i] = 0.0;
       ai = fma(-fact, ci, an);
@@ -1769,7 +1818,7 @@ __device__ void tri_factor(int n, const double *a0, const double *e, double lam,
       xi = fma(-fact, 1.0, xi);
     }
   }
-  if (mag_bits(ai) == 0) ai = tiny;
+  if (zero_bits(ai)) ai = tiny;
   a[n - 1] = ai;
   x[n - 1] = xi;
 }
@@ -1795,7 +1844,7 @@ __device__ double tri_back(int n, const double *a, const double *r, const double
   for (int i = n - 1; i >= 0; i--) {
     double v = x[i];
     if (i + 1 < n) v = fma(-c[i], x1, v);
-    if (i + 2 < n) v = fma(-c2[i], x2, v);
+    if (i + 2 < n && !zero_bits(c2[i])) v = fma(-c2[i], x2, v);  // (0 without a pivot)
     x2 = x1;
     x1 = div_rcp(v, a[i], r[i]);
     x[i] = x1;
@@ -1817,16 +1866,18 @@ __device__ __forceinline__ double warp_max_d(double v) {
 }
 
 // k-th smallest eigenvalue (0-based) by multisection inside [lo, hi], to a
-// bracket of relative width rel
-__device__ double eig_index(const double *d, const double *e2, int n, int k, double lo,
-                            double hi, double rel = 2.2e-16) {
+// bracket of relative width rel; count(x): eigenvalues below x
+template <typename F>
+__device__ __forceinline__ double eig_index(F &&count, int k, double lo, double hi,
+                                            double rel = 2.2e-16) {
   const int lane = threadIdx.x & 31;
+  const double frac = (double)(lane + 1) / 33.0;
   double a = lo, b = hi;
   for (int round = 0; round < 24; round++) {
     double w = __dsub_rn(b, a);
     if (!(w > rel * fmax(fabs(a), fabs(b)) + 1e-300)) break;
-    double x = fma(w, (double)(lane + 1) / 33.0, a);
-    int cnt = sturm_count(d, e2, n, x);
+    double x = fma(w, frac, a);
+    int cnt = count(x);
     unsigned ball = __ballot_sync(0xffffffffu, cnt > k);
     int first = ball ? __ffs(ball) - 1 : 32;
     double xl = __shfl_sync(0xffffffffu, x, first > 0 ? first - 1 : 0);
@@ -1844,14 +1895,29 @@ __global__ void k_tri_eig(GState *__restrict__ gs, int ngroups,
                           const double *__restrict__ vnorm, int MI, double *__restrict__ coef) {
   pdl_entry();
   extern __shared__ double eig_sm[];
-  const int g = blockIdx.x, lane = threadIdx.x;
+  const int g = blockIdx.x, lane = threadIdx.x & 31;
   if (g >= ngroups) return;
   GState &st = gs[g];
   if (!st.active) return;
   const int n = st.iters;
   double *D0 = eig_sm, *E0 = D0 + MI, *e2 = E0 + MI;
   double *a = e2 + MI, *b = a + MI, *c = b + MI, *c2 = c + MI, *x = c2 + MI;
-  int *piv = (int *)(x + MI);
+  double *xs = x + MI, *dx = xs + 32 + lane;  // shifts of a round, rows of D0 - shift
+  int *piv = (int *)(xs + 32 + 32 * MI);
+  __shared__ int s_go;
+  if (threadIdx.x >= 32) {  // the second warp feeds the Sturm counts
+    for (;;) {
+      asm volatile("barrier.sync 1, 64;" ::: "memory");
+      if (!s_go) return;
+      feed_rows(D0, n, xs[lane], dx);
+    }
+  }
+  auto count = [&](double at) {
+    xs[lane] = at;
+    if (lane == 0) s_go = 1;
+    asm volatile("barrier.sync 1, 64;" ::: "memory");
+    return sturm_count<true>(D0, e2, n, at, dx);
+  };
   for (int i = lane; i < n; i += 32) {
     D0[i] = diagT[(ll)g * MI + i];
     if (i < n - 1) {
@@ -1874,23 +1940,27 @@ __global__ void k_tri_eig(GState *__restrict__ gs, int ngroups,
   glo -= pad, ghi += pad;
   // eigenvalue of least modulus: the negative one closest to 0 or the
   // smallest non-negative one
-  int c0 = sturm_count(D0, e2, n, 0.0);  // eigenvalues below 0 (all lanes agree)
+  int c0 = count(0.0);  // eigenvalues below 0 (all lanes agree)
   double lam;
   if (c0 == 0) {
-    lam = eig_index(D0, e2, n, 0, glo, ghi);
+    lam = eig_index(count, 0, glo, ghi);
   } else if (c0 >= n) {
-    lam = eig_index(D0, e2, n, n - 1, glo, ghi);
+    lam = eig_index(count, n - 1, glo, ghi);
   } else {
-    double ln = eig_index(D0, e2, n, c0 - 1, glo, ghi);
-    double lp = eig_index(D0, e2, n, c0, glo, ghi);
+    double ln = eig_index(count, c0 - 1, glo, ghi);
+    double lp = eig_index(count, c0, glo, ghi);
     lam = fabs(lp) < fabs(ln) ? lp : ln;
   }
+  if (lane == 0) s_go = 0;  // the feeder is done
+  asm volatile("barrier.sync 1, 64;" ::: "memory");
   // inverse iteration: the factors of T - lam I serve both sweeps, and lane 0
   // has its chains of dependent FP64 instructions to itself (the reciprocals
   // of U's diagonal and the scaling run on all lanes)
   const double tnorm = fmax(fabs(glo), fabs(ghi));
   const double tiny = fmax(tnorm, 1e-300) * 1e-16;
-  if (lane == 0) tri_factor(n, D0, E0, lam, x, a, b, c, c2, piv, tiny);
+  for (int i = lane; i < n; i += 32) c2[i] = __dsub_rn(D0[i], lam);
+  __syncwarp();
+  if (lane == 0) tri_factor(n, E0, x, a, b, c, c2, piv, tiny);
   __syncwarp();
   for (int i = lane; i < n; i += 32) e2[i] = fast_rcp(a[i]);
   __syncwarp();
@@ -1947,10 +2017,11 @@ __device__ __noinline__ double ritz_bound_warp(const double *D0, const double *E
   const int c0 = __shfl_sync(0xffffffffu, cq, 0), clo = __shfl_sync(0xffffffffu, cq, 1),
             chi = __shfl_sync(0xffffffffu, cq, 2);
   const bool pd = c0 == 0;
+  auto count = [&](double x) { return sturm_count(D0, e2, n, x); };
   const bool warm = th0 > 0.0 && clo == 0 && chi >= 1;
   const double theta =
-      pd ? (warm ? eig_index(D0, e2, n, 0, 0.99 * th0, th0, 1e-10)
-                 : eig_index(D0, e2, n, 0, glo, ghi, 1e-10))
+      pd ? (warm ? eig_index(count, 0, 0.99 * th0, th0, 1e-10)
+                 : eig_index(count, 0, glo, ghi, 1e-10))
          : 0.0;
   double bound = 1e300;
   if (pd) {
@@ -3534,9 +3605,10 @@ struct Lanczos {
     return c * (early > 0.0 ? 2 : 1);
   }
 
-  // shared memory of k_tri_eig: 8 arrays of MI doubles and MI ints
+  // shared memory of k_tri_eig: 8 arrays of MI doubles, the feeder's shifts and
+  // rows, and MI ints
   size_t eig_smem() const {
-    return (size_t)8 * MI * sizeof(double) + (size_t)(MI + 2) * sizeof(int) + 16;
+    return (size_t)(8 * MI + 32 + 32 * MI) * sizeof(double) + (size_t)(MI + 2) * sizeof(int) + 16;
   }
 
   FinArgs fargs(int it, double tol, int mpass) {
@@ -3731,7 +3803,7 @@ struct Lanczos {
       mark(4 * it + 3);
     }
     mark(4 * MI + 2);
-    launch_pdl(k_tri_eig, A, 32, eig_smem(), st, gs.p, A, diagT.p, upperT.p, vnorm.p, MI, coef.p);
+    launch_pdl(k_tri_eig, A, 64, eig_smem(), st, gs.p, A, diagT.p, upperT.p, vnorm.p, MI, coef.p);
     mark(4 * MI + 3);
     mark(4 * MI + 4);
     launch_pdl(k_ritz<VT>, T, ritz_bd, 0, st, tbeg.p, tend.p, tgrp.p, gs.p, V.p, VS, coef.p, MI,
