@@ -29,7 +29,7 @@ namespace {
 // division by 4 or 8 is an exact product.  8M hexes: 0.84 -> 0.44 ms.
 constexpr int CE_ELEMS = 128;
 __device__ __forceinline__ double no_minus_zero(double x) {  // 0.0 + x
-  return (__double_as_longlong(x) << 1) == 0 ? 0.0 : x;
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u ? 0.0 : x;
 }
 template <int NV>
 __global__ void __launch_bounds__(CE_ELEMS)

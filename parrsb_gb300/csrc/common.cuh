@@ -206,7 +206,8 @@ inline unsigned grid_for(ll n, int threads) {
 // +0.0 map to the same key, matching a '<' comparison sort).
 __device__ __forceinline__ unsigned long long ordered_key(double x) {
   unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  if (x == 0.0) b = 0ull;  // -0.0 -> +0.0
+  // -0.0 -> +0.0, tested by halves: an FP64 comparison takes 64 cycles
+  if ((((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u) b = 0ull;
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 

@@ -117,10 +117,6 @@ __global__ void k_iota(int *__restrict__ a, ll n) {
   if (i < n) a[i] = (int)i;
 }
 
-__device__ __forceinline__ double key_value(u64 k) {
-  return __longlong_as_double((ll)((k >> 63) ? (k ^ 0x8000000000000000ull) : ~k));
-}
-
 // |x| to 23 bits, truncated, without the FP64 pipe (a conversion would use it);
 // below the normal range 0, above it infinity, not a number as it is
 __device__ __forceinline__ float rough(double x) {
@@ -151,7 +147,7 @@ Tol2 tol2_of(double tol) {
 // distances da, db: (x - xl)^2 > min(da, db) tol^2.  In FP64 that is five
 // instructions of 64 cycles on a sub-partition's pipe; only the difference is
 // taken there, and single precision with error bounds decides unless the two
-// sides agree to 2^-17 (settling 8M points: 321 -> 103 us)
+// sides agree to 2^-17 (settling 8M points: 321 -> 84 us)
 __device__ __forceinline__ bool gap_between(double x, double xl, double da, double db,
                                             const Tol2 &tol) {
   const double d = __dsub_rn(x, xl), m = min_sq(da, db);
@@ -163,19 +159,29 @@ __device__ __forceinline__ bool gap_between(double x, double xl, double da, doub
   return __dmul_rn(d, d) > __dmul_rn(m, tol.x);
 }
 
-// flag[j] |= gap between sorted neighbours j-1, j along the coordinate that
-// was sorted last (its values are the keys).  A warp's lane takes its left
-// neighbour's point from the lane beside it, so dx is gathered once.
-__global__ void k_gaps(const int *__restrict__ ord, const u64 *__restrict__ keys,
-                       const double4_32a *__restrict__ pt, ll np, Tol2 tol2,
-                       int first_pass, int *__restrict__ flag) {
+// flag[j] |= gap between sorted neighbours j-1, j along axis d, which was
+// sorted last.  A warp's lane takes its left neighbour's point from the lane
+// beside it, so a point is gathered once; and its coordinate along axis next
+// goes out as the next sort's key (next >= 0), which saves another gather of
+// the same points (65 us per 8M).
+__global__ void k_gaps(const int *__restrict__ ord, const double4_32a *__restrict__ pt, ll np,
+                       Tol2 tol2, int first_pass, int d, int next, u64 *__restrict__ keys,
+                       int *__restrict__ flag) {
   const ll j = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
+  auto along = [](const double4_32a &p, int q) { return q == 0 ? p.x : q == 1 ? p.y : p.z; };
   double x = 0.0, w = 0.0;
-  if (j < np) x = key_value(keys[j]), w = pt[ord[j]].w;
+  if (j < np) {
+    const double4_32a p = pt[ord[j]];
+    x = along(p, d), w = p.w;
+    if (next >= 0) keys[j] = ordered_key(along(p, next));
+  }
   double xl = __shfl_up_sync(0xffffffffu, x, 1), wl = __shfl_up_sync(0xffffffffu, w, 1);
   if (j >= np) return;
-  if (lane == 0 && j > 0) xl = key_value(keys[j - 1]), wl = pt[ord[j - 1]].w;
+  if (lane == 0 && j > 0) {
+    const double4_32a p = pt[ord[j - 1]];
+    xl = along(p, d), wl = p.w;
+  }
   if (j == 0) {
     flag[0] = 1;
     return;
@@ -468,6 +474,7 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
   ll nseg = 1, longest = np;
   DBuf<int> err(2);
   CK(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), st));
+  int keys_of = -1;  // axis whose coordinates ws.keys holds, in the current order
   for (int t = 0; t < ndim; t++) {
     if (t == 1) {
       // nothing left to sort: the later rounds' gaps at once
@@ -486,12 +493,16 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     for (int d = 0; d < ndim; d++) {
       const bool first = t == 0 && d == 0;
       if (!first && longest <= 1) continue;  // no two points left to compare
-      k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(
-          ws.ord.p, reinterpret_cast<const double *>(ws.pt.p) + d, np, ws.keys.p);
-      CK_LAUNCH();
-      sort_by_value(ws.keys, ws.ord, np, first ? nullptr : ws.seg.p, nseg, longest, ws.sort);
-      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.keys.p, ws.pt.p, np, tol2,
-                                                first ? 1 : 0, ws.flag.p);
+      if (keys_of != d) {
+        k_gc_keys<<<grid_for(np, 256), 256, 0, st>>>(
+            ws.ord.p, reinterpret_cast<const double *>(ws.pt.p) + d, np, ws.keys.p);
+        CK_LAUNCH();
+      }
+      sort_by_value(ws.keys, ws.ord, np, first ? nullptr : ws.seg.p, nseg, longest, ws.sort, first);
+      // (after the first round the points are usually settled)
+      keys_of = t == 0 && d == ndim - 1 ? -1 : (d + 1) % ndim;
+      k_gaps<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.pt.p, np, tol2, first ? 1 : 0, d,
+                                                keys_of, ws.keys.p, ws.flag.p);
       CK_LAUNCH();
       segments_of(ws, ws.flag.p, np, &nseg, &longest);
     }
