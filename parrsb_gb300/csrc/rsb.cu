@@ -696,6 +696,13 @@ __device__ __forceinline__ double tile_total_pair(const float2 *cs, int nc) {
   return (double)t.x + (double)t.y;
 }
 
+// small non-negative integer (< 2^20) as a double, by integer instructions
+__device__ __forceinline__ double small_u2d(unsigned d) {
+  const int e = 31 - __clz((int)d);
+  const unsigned hi = d ? ((unsigned)(1023 + e) << 20) | ((d << (20 - e)) & 0xFFFFFu) : 0u;
+  return __hiloint2double((int)hi, 0);
+}
+
 template <typename VT, int MODE, int GATE, int FUSE>
 __global__ void __launch_bounds__(512)
 k_tile(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
@@ -758,11 +765,27 @@ k_tile(const ll *__restrict__ tbeg, const ll *__restrict__ tend,
         ll sl = i >> 5;
         const unsigned *ep = ell + slice_off[sl] + (i & 31);
         int wd = slice_w[sl];
+        // eight gathers in flight; the product with 0, 1, 2, 4 or 8 is exact, so
+        // it may enter the sum in one instruction (two on the FP64 pipe per
+        // entry instead of four)
         double yv = 0.0;
-        for (int k = 0; k < wd; k++) {
-          unsigned x = ep[(ll)k * 32];
-          yv = __dadd_rn(yv, __dmul_rn((double)(x >> 28),
-                                       __dsub_rn(fi, (double)f[x & 0x0FFFFFFFu])));
+        for (int k = 0; k < wd; k += 8) {
+          unsigned x[8];
+          double fj[8];
+#pragma unroll
+          for (int u = 0; u < 8; u++) x[u] = k + u < wd ? ep[(ll)(k + u) * 32] : (unsigned)i;
+#pragma unroll
+          for (int u = 0; u < 8; u++) fj[u] = (double)f[x[u] & 0x0FFFFFFFu];
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            if (k + u >= wd) break;
+            const unsigned wt = x[u] >> 28;
+            const double d = __dsub_rn(fi, fj[u]), wv = small_u2d(wt);
+            if ((wt & (wt - 1)) == 0)
+              yv = fma(wv, d, yv);
+            else
+              yv = __dadd_rn(yv, __dmul_rn(wv, d));
+          }
         }
         y64[i] = yv;
         d1 = __dmul_rn(fi, yv);
@@ -2433,13 +2456,6 @@ __device__ __forceinline__ void team_publish(bool solo, double *own, TeamSlot *s
       if (lane < TS_REP) slot_put(slot + (ll)lane * T + t, v, tag, rel);
     }
   }
-}
-
-// small non-negative integer (< 2^20) as a double, by integer instructions
-__device__ __forceinline__ double small_u2d(unsigned d) {
-  const int e = 31 - __clz((int)d);
-  const unsigned hi = d ? ((unsigned)(1023 + e) << 20) | ((d << (20 - e)) & 0xFFFFFu) : 0u;
-  return __hiloint2double((int)hi, 0);
 }
 
 // Where the encoded rows of a block start that owns the slices from sl on
