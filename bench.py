@@ -136,7 +136,7 @@ def load_traffic():
     """DRAM bytes per algorithmic byte of one SpMV launch, from the committed
     ncu summary of a smaller case (the benchmark's launches are scaled by
     their own algorithmic bytes: traffic grows with the matrix)."""
-    path = os.path.join(ROOT, "profiles", "k_spmv_rsb_hex_128x128x64_level0.md")
+    path = os.path.join(ROOT, "profiles", "k_spmv_loc_rsb_hex_128x128x64_level0.md")
     try:
         with open(path) as f:
             for line in f:
@@ -694,7 +694,7 @@ def main():
                 "link": link},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
-                     "traffic": tr_val, "kernel": "k_spmv (sliced-ELL Laplacian)",
+                     "traffic": tr_val, "kernel": "k_spmv_loc or k_spmv, as autotuned (Laplacian)",
                      "traffic_note": ("DRAM bytes per launch: ncu dram bytes / algorithmic "
                                       "bytes of one level-0 launch on the 1M-element box "
                                       f"({traffic['dram_bytes_per_algorithmic_byte']:.3f}, "

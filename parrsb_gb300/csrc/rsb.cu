@@ -3513,9 +3513,12 @@ struct Lanczos {
   DBuf<int> d_list, d_item0, d_halo, d_nhalo, d_bad;
   DBuf<int2> d_items;
   DBuf<unsigned> d_enc;
-  // SpMV on staged rows (k_spmv_loc), FP32
+  // SpMV on staged rows (k_spmv_loc), FP32; buffers of its own: the team kernel
+  // may encode the level too and then not run
   std::vector<int2> sl_runs;     // first tile and tiles of each block
   DBuf<int2> d_runs;
+  DBuf<unsigned> sl_enc;
+  DBuf<int> sl_halo, sl_nhalo, sl_bad;
   int sl_pcap = 0, sl_smem = 0;  // places of own rows, shared memory of a block
   DBuf<TeamSlot> slots;
   DBuf<unsigned long long> ts_epoch;
@@ -4107,8 +4110,8 @@ struct Lanczos {
     cudaStream_t st = ctx().stream;
     if (kind == 2 && sizeof(VT) == 4) {
       launch_pdl(k_spmv_loc, (unsigned)sl_runs.size(), threads, (size_t)sl_smem, st, tbeg.p, tend.p,
-                 tgrp.p, gs.p, d_runs.p, d_enc.p, lv.slice_off.p, lv.slice_w.p, d_halo.p,
-                 d_nhalo.p, sl_pcap, lv.max_w, reinterpret_cast<const float *>(p.p),
+                 tgrp.p, gs.p, d_runs.p, sl_enc.p, lv.slice_off.p, lv.slice_w.p, sl_halo.p,
+                 sl_nhalo.p, sl_pcap, lv.max_w, reinterpret_cast<const float *>(p.p),
                  reinterpret_cast<float *>(w.p), part.p, force);
     } else if (kind == 1 && sizeof(VT) == 4) {
       const size_t sb = sp_stage_bytes(lv, threads);
@@ -4136,18 +4139,18 @@ struct Lanczos {
     }
     sl_pcap = sl_cap((int)longest);
     const size_t nr = sl_runs.size();
-    d_runs.ensure(nr), d_nhalo.ensure(nr), d_halo.ensure(nr * SL_HALO), d_bad.ensure(2);
+    d_runs.ensure(nr), sl_nhalo.ensure(nr), sl_halo.ensure(nr * SL_HALO), sl_bad.ensure(2);
     h2d(d_runs.p, sl_runs.data(), nr);
-    d_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
+    sl_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
                  (size_t)(T + 1) * (size_t)(lv.max_w + 1) * 32 + 1024);
-    CK(cudaMemsetAsync(d_bad.p, 0, 2 * sizeof(int), st));
+    CK(cudaMemsetAsync(sl_bad.p, 0, 2 * sizeof(int), st));
     ensure_smem_limit(k_loc_encode, LE_SMEM);
     k_loc_encode<<<(unsigned)nr, LE_THREADS, LE_SMEM, st>>>(
         tbeg.p, tend.p, d_runs.p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, sl_pcap, lv.max_w,
-        d_enc.p, d_halo.p, d_nhalo.p, d_bad.p);
+        sl_enc.p, sl_halo.p, sl_nhalo.p, sl_bad.p);
     CK_LAUNCH();
     int bad[2] = {0, 0};
-    d2h(bad, d_bad.p, 2);
+    d2h(bad, sl_bad.p, 2);
     sync();
     sl_smem = (sl_pcap + bad[1]) * (int)sizeof(float);
     ensure_smem_limit(k_spmv_loc, sl_smem);
@@ -5602,11 +5605,13 @@ static void rsb_impl(const long long *d_vtx, const double *cent, ll N, int nv, i
       if (res[g].resid > S.max_fiedler_resid) S.max_fiedler_resid = res[g].resid;
     }
     // algorithmic bytes of the SpMV launches of this level: per row and
-    // step 4 B per stored nonzero plus the row's own p read and w write
+    // step 4 B per stored nonzero (2 B in k_spmv_loc) plus the row's own p read
+    // and w write
     {
+      const double entry = !lz.team && lz.sp_kind == 2 ? 2.0 : 4.0;
       long long row_iters = 0;
       for (int g = 0; g < na; g++) row_iters += res[g].total_iters * res[g].n;
-      double per_row = rows > 0 ? 4.0 * (double)lv.nnz / (double)rows + 2.0 * sizeof(VT) : 0.0;
+      double per_row = rows > 0 ? entry * (double)lv.nnz / (double)rows + 2.0 * sizeof(VT) : 0.0;
       S.spmv_bytes += (long long)(per_row * (double)row_iters);
     }
     // ---- sort by Fiedler value (src/rsb.c:307-309)
