@@ -2174,9 +2174,13 @@ __global__ void k_apply_stop(GState *__restrict__ gs, int ngroups) {
 //
 // The early pass exit's Ritz residual bound runs on an extra warp of the
 // team's first block beside the next steps; its stop request travels in the
-// tag of that block's first |r|^2 slot of the step before it takes effect.
-// Every wait gives up after about one second, sets err and returns; a block
-// that sees err set returns at its next wait, so the kernel always ends.
+// tag of that block's first |r|^2 slot of the step before it takes effect.  So
+// a request has to wait for a step after its check (2 <= e_delay <= e_stride):
+// the check's reply is then taken exactly once, and before the next check is
+// sent, which the two-warp barriers between the workers and the checker rely
+// on; with a delay of one step the level keeps the launch-per-kernel steps.
+// Every wait for another block gives up after about one second, sets err and
+// returns; a block that sees err set returns at its next wait.
 //
 // Bound by the FP64 pipe with FP64 vectors (59k of 110k cycles of a step at
 // 4096 rows per block are the SpMV's DFMAs) and by instruction issue with
@@ -4044,6 +4048,8 @@ struct Lanczos {
     if (e && atoi(e) == 0) return false;
     const bool force = e && atoi(e) != 0;
     if (reorth || pr_fused || sp_fused || bound_log || !ev.empty() || T <= 0) return false;
+    // (a stop request travels with the step after its check at the earliest)
+    if (early > 0.0 && early_delay < 2) return false;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -4236,11 +4242,11 @@ struct Lanczos {
       const char *v = getenv("PARRSB_GPU_PASS_LOG");
       return v ? atoi(v) : 0;
     }();
-    // early pass exit (residual-stop mode only): after steps 3, 6, 9, ... a group whose Ritz residual
-    // bound is below 0.7 rsb_tol ends its pass three steps later (the check
-    // runs beside the next two); the FP64 residual of its Ritz vector still
-    // decides whether it restarts.
-    // PARRSB_GPU_EARLY=<factor> (0: off), _MIN, _STRIDE (at least 2)
+    // early pass exit (residual-stop mode only): after steps 3, 6, 9, ... a
+    // group whose Ritz residual bound is below 0.7 rsb_tol ends its pass three
+    // steps later (the check runs beside the next two); the FP64 residual of
+    // its Ritz vector still decides whether it restarts.
+    // PARRSB_GPU_EARLY=<factor> (0: off), _MIN, _STRIDE, _DELAY (1 to the stride)
     early = 0.0;
     if (resid_stop) {
       early = 0.7, early_min = 3, early_stride = 3;
