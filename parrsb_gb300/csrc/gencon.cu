@@ -348,7 +348,9 @@ __global__ void k_element_check(const int *__restrict__ ids, ll nel, int nv,
 // table of the element's; then its eight threads look at the sets.  Nothing of
 // the candidates is read but their numbers: 0.52 -> 0.31 ms per million hexes
 // against comparing their ids.  Elements with more neighbours than the table
-// has slots compare ids.
+// has slots compare ids.  Nothing is done when the element check has failed
+// (*err): points that ran together make vertices that any number of elements
+// share, and the work grows with its square (a call on 8M graded points: 64 -> 7 ms).
 constexpr int FC_SLOTS = 64;
 __device__ __forceinline__ bool split_face(unsigned mask) {
   bool bad = false;
@@ -361,10 +363,13 @@ k_face_check(const int *__restrict__ ids, const int *__restrict__ ord,
              const int *__restrict__ seg_start, int nseg, ll np, int *__restrict__ err) {
   __shared__ int s_key[32][FC_SLOTS + 1];
   __shared__ unsigned s_mask[32][FC_SLOTS + 1];
+  __shared__ int s_failed;
+  if (threadIdx.x == 0) s_failed = *(volatile int *)err;
+  __syncthreads();
   const ll p = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = threadIdx.x & 7, row = threadIdx.x >> 3;
   const unsigned group = 0xFFu << (threadIdx.x & 24);
-  if (p >= np) return;  // (whole elements)
+  if (p >= np || s_failed) return;  // (whole elements)
   int *key = s_key[row];
   unsigned *mask = s_mask[row];
   for (int u = k; u < FC_SLOTS; u += 8) key[u] = -1, mask[u] = 0u;
