@@ -34,6 +34,11 @@ namespace prsb {
 static thread_local Ctx g_ctx;
 Ctx &ctx() { return g_ctx; }
 
+bool fault_injected(const char *what) {
+  const char *f = getenv("PARRSB_FAULT");
+  return f && strcmp(f, what) == 0;
+}
+
 void *dev_alloc(size_t bytes) {
   void *p = nullptr;
   CK(cudaMallocAsync(&p, bytes, ctx().stream));
@@ -425,8 +430,7 @@ int guarded(F &&fn) {
 // Host-side fault injection for tests: PARRSB_FAULT=<stage> makes that stage
 // fail with PARRSB_ERR_CHECK after everything before it ran.
 void maybe_fault(const char *stage) {
-  const char *f = getenv("PARRSB_FAULT");
-  if (f && strcmp(f, stage) == 0) throw ArgError{PARRSB_ERR_CHECK, "injected fault"};
+  if (fault_injected(stage)) throw ArgError{PARRSB_ERR_CHECK, "injected fault"};
 }
 
 }  // namespace

@@ -43,6 +43,9 @@ struct ArgError {
   const char *msg;
 };
 
+// whether a test asks for this failure (PARRSB_FAULT=<what>)
+bool fault_injected(const char *what);
+
 // --------------------------------------------------------------------------
 // Device buffer (RAII) and a per-thread context that owns the stream, event
 // pool and statistics of the current call.

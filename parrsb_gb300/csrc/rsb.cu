@@ -2180,7 +2180,9 @@ __global__ void k_apply_stop(GState *__restrict__ gs, int ngroups) {
 // sent, which the two-warp barriers between the workers and the checker rely
 // on; with a delay of one step the level keeps the launch-per-kernel steps.
 // Every wait for another block gives up after about one second, sets err and
-// returns; a block that sees err set returns at its next wait.
+// returns; a block that sees err set returns at its next wait.  The host then
+// repeats the level with the launch-per-kernel steps, which need no blocks
+// side by side (Lanczos::run).
 //
 // Bound by the FP64 pipe with FP64 vectors (59k of 110k cycles of a step at
 // 4096 rows per block are the SpMV's DFMAs) and by instruction issue with
@@ -3526,6 +3528,9 @@ struct Lanczos {
   int sl_pcap = 0, sl_smem = 0;  // places of own rows, shared memory of a block
   DBuf<TeamSlot> slots;
   DBuf<unsigned long long> ts_epoch;
+  bool team_off = false;         // it failed once: no more in this call
+  DBuf<GState> gs0;              // where a level starts, should it have to be repeated
+  DBuf<VT> f0;
   DBuf<ll> fq;                   // fixed-point f of the residual check (FP32)
   DBuf<unsigned> gmax, tmax;     //   each group's and tile's largest |f| (IEEE bits)
   bool resid_stop = false;       // restarts decided by the FP64 eigen-residual
@@ -3885,6 +3890,8 @@ struct Lanczos {
     attr.val.cooperative = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    if (fault_injected("team_launch"))
+      throw CudaError{cudaErrorCooperativeLaunchTooLarge, __FILE__, __LINE__};
     ctx().kernel_launches++;
     CK(cudaLaunchKernelEx(&cfg, k_team_steps<VT>, ta));
   }
@@ -4047,7 +4054,7 @@ struct Lanczos {
     const char *e = getenv("PARRSB_GPU_PERSIST");
     if (e && atoi(e) == 0) return false;
     const bool force = e && atoi(e) != 0;
-    if (reorth || pr_fused || sp_fused || bound_log || !ev.empty() || T <= 0) return false;
+    if (reorth || pr_fused || sp_fused || bound_log || ctx().timing || T <= 0) return false;
     // (a stop request travels with the step after its check at the earliest)
     if (early > 0.0 && early_delay < 2) return false;
     int dev = 0, sms = 0, per_sm = 0;
@@ -4277,17 +4284,93 @@ struct Lanczos {
       CK(cudaFuncSetAttribute(k_tri_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)eig_smem()));
     autotune(lv);
-    k_set_active<<<grid_for(A, 128), 128, 0, st>>>(gs.p, A);
-    CK_LAUNCH();
-    if (!warm) {
-      if (start_kind == 1)
-        random_vector();
-      else
-        initial_vector();
+    team = !team_off && want_team(lv);
+    if (team) {  // (what the passes overwrite)
+      gs0.ensure(A);
+      CK(cudaMemcpyAsync(gs0.p, gs.p, (size_t)A * sizeof(GState), cudaMemcpyDeviceToDevice, st));
+      if (warm) {
+        f0.ensure(N);
+        CK(cudaMemcpyAsync(f0.p, f.p, (size_t)N * sizeof(VT), cudaMemcpyDeviceToDevice, st));
+      }
     }
-    long long launches = 0;
-    cudaGraphExec_t exec = nullptr;
+    auto start = [&] {
+      k_set_active<<<grid_for(A, 128), 128, 0, st>>>(gs.p, A);
+      CK_LAUNCH();
+      if (!warm) {
+        if (start_kind == 1)
+          random_vector();
+        else
+          initial_vector();
+      }
+    };
+    start();
+    const parrsb_stats before = ctx().stats;
+    cudaError_t why = cudaErrorLaunchTimeout;  // a wait gave up
+    try {
+      // (a test's failure: the flag that a wait would set)
+      if (team && fault_injected("team_wait"))
+        CK(cudaMemsetAsync(err.p, 2, sizeof(int), st));
+      passes(lv, tol, mpass, use_graph, pass_log);
+      if (!wait_gave_up()) {
+        normalise();
+        return;
+      }
+      if (!team) throw CudaError{why, __FILE__, __LINE__};  // (the staged SpMV's)
+    } catch (const CudaError &e) {
+      if (!team) throw;
+      why = e.err;
+    }
+    // the team kernel could not be built into a graph or launched (an error
+    // that sticks shows at the next call), or its blocks waited in vain for
+    // each other: the level again from its start, one launch per kernel
+    end_capture(true);
+    cudaGetLastError();
+    team_off = true;
+    team = false;
+    fprintf(stderr, "parrsb_gb300: team step kernel not available (%s); steps as single launches\n",
+            cudaGetErrorString(why));
+    sync();
+    ctx().stats = before;
+    CK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+    CK(cudaMemcpyAsync(gs.p, gs0.p, (size_t)A * sizeof(GState), cudaMemcpyDeviceToDevice, st));
+    if (warm)
+      CK(cudaMemcpyAsync(f.p, f0.p, (size_t)N * sizeof(VT), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemsetAsync(p.p, 0, (size_t)N * sizeof(VT), st));
+    start();
+    passes(lv, tol, mpass, use_graph, pass_log);
+    if (wait_gave_up()) throw CudaError{cudaErrorLaunchTimeout, __FILE__, __LINE__};
+    normalise();
+  }
+
+  // ends a capture that an error interrupted; own: into a graph of its own
+  void end_capture(bool own) {
+    cudaStream_t st = ctx().stream;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
+      cudaGraph_t g = nullptr;
+      cudaStreamEndCapture(st, &g);
+      if (own && g) cudaGraphDestroy(g);
+    }
+  }
+
+  struct PassGraph {
     cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    void drop() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (graph) cudaGraphDestroy(graph);
+      exec = nullptr, graph = nullptr;
+    }
+    ~PassGraph() { drop(); }
+  };
+
+  // all passes (restarts) of the level
+  void passes(const Level &lv, double tol, int mpass, bool use_graph, int pass_log) {
+    cudaStream_t st = ctx().stream;
+    long long launches = 0;
+    PassGraph pg;
+    cudaGraphExec_t &exec = pg.exec;
+    cudaGraph_t &graph = pg.graph;
     if (ctx().timing) {
       ev.assign(2 * MI, nullptr);
       for (auto &e : ev) CK(cudaEventCreate(&e));
@@ -4301,13 +4384,9 @@ struct Lanczos {
       const char *e = getenv("PARRSB_GPU_DEVICE_LOOP");
       return !(e && atoi(e) == 0);
     }();
-    // sticky fallbacks after a graph could not be built (any thread, any device)
+    // sticky fallback after a graph could not be built (any thread, any device)
     static std::atomic<bool> device_loop_broken{false};
-    static std::atomic<bool> team_broken{false};  // a graph with k_team_steps failed once
-    team = !team_broken && want_team(lv);
-    for (int attempt = 0;
-         attempt < 2 && !exec && use_graph && ev.empty() && device_loop_env && !device_loop_broken;
-         attempt++) try {
+    if (use_graph && ev.empty() && device_loop_env && !device_loop_broken) try {
       const auto h0 = std::chrono::steady_clock::now();
       CK(cudaGraphCreate(&graph, 0));
       cudaGraphConditionalHandle hnd;
@@ -4337,23 +4416,10 @@ struct Lanczos {
     } catch (const CudaError &e) {
       // the graph could not be built or instantiated here: end any capture,
       // report once, and run the restarts from the host from now on
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(st, &g2);
-        if (g2) cudaGraphDestroy(g2);
-      }
+      end_capture(false);
+      if (team) throw;  // (the launch-per-kernel steps are tried first)
       cudaGetLastError();
-      if (exec) cudaGraphExecDestroy(exec);
-      if (graph) cudaGraphDestroy(graph);
-      exec = nullptr, graph = nullptr;
-      if (team) {  // try again with the launch-per-kernel steps
-        team_broken = true;
-        team = false;
-        fprintf(stderr, "parrsb_gb300: team step kernel unavailable in graphs (%s)\n",
-                cudaGetErrorString(e.err));
-        continue;
-      }
+      pg.drop();
       device_loop_broken = true;
       fprintf(stderr, "parrsb_gb300: device restart loop unavailable (%s); host loop used\n",
               cudaGetErrorString(e.err));
@@ -4372,13 +4438,9 @@ struct Lanczos {
       ctx().stats.lanczos_host_ms[2] +=
           std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h1)
               .count();
-      cudaGraphExecDestroy(exec);
-      cudaGraphDestroy(graph);
-      exec = nullptr, graph = nullptr;
-      finish_run();
       return;
     }
-    for (int attempt = 0; attempt < 2 && use_graph && !exec; attempt++) try {
+    if (use_graph) {
       const auto h0 = std::chrono::steady_clock::now();
       CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       long long kl = ctx().kernel_launches;
@@ -4388,22 +4450,6 @@ struct Lanczos {
       CK(cudaGraphInstantiate(&exec, graph, 0));
       ctx().stats.lanczos_host_ms[1] +=
           std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
-    } catch (const CudaError &e) {
-      if (!team) throw;
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(st, &g2);
-        if (g2) cudaGraphDestroy(g2);
-      }
-      cudaGetLastError();
-      if (exec) cudaGraphExecDestroy(exec);
-      if (graph) cudaGraphDestroy(graph);
-      exec = nullptr, graph = nullptr;
-      team_broken = true;
-      team = false;
-      fprintf(stderr, "parrsb_gb300: team step kernel unavailable in graphs (%s)\n",
-              cudaGetErrorString(e.err));
     }
     const long long per_pass_kernels =
         4 + step_kernels() + 5 + (resid_stop ? 3 + resid1_launches(lv) : 0);
@@ -4465,9 +4511,6 @@ struct Lanczos {
     for (auto &e : evk) cudaEventDestroy(e);
     evk.clear();
     ctx().stats.spmv_launches += launches;
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    finish_run();
   }
 
   // one stderr line per group (the first four) after a pass of the host loop
@@ -4499,16 +4542,17 @@ struct Lanczos {
     }
   }
 
-  // after the restarts: the staged SpMV's error flag, then normalise
-  // (src/fiedler.c:606-613) and fix the sign canonically: sum_i s_i f_i >= 0
-  // with s = +1 on the first half of the group's order
-  void finish_run() {
-    {
-      int h_err = 0;
-      d2h(&h_err, err.p, 1);
-      sync();
-      if (h_err) throw CudaError{cudaErrorLaunchTimeout, __FILE__, __LINE__};  // a stage wait gave up
-    }
+  // after the restarts: whether a wait in the staged SpMV or the team kernel
+  // gave up
+  bool wait_gave_up() {
+    int h_err = 0;
+    d2h(&h_err, err.p, 1);
+    sync();
+    return h_err != 0;
+  }
+  // normalises (src/fiedler.c:606-613) and fixes the sign canonically:
+  // sum_i s_i f_i >= 0 with s = +1 on the first half of the group's order
+  void normalise() {
     tile<TM_SQ_F, GATE_ALL>();
     fin<FIN_NORM, GATE_ALL>();
     tile<TM_ORIENT, GATE_ALL>();
