@@ -4174,6 +4174,8 @@ struct Lanczos {
   // on the level's own matrix (three forced SpMV launches each, CUDA
   // events); the tile reductions are canonical, so the choice never changes
   // a result.  Decisions are cached per (tiles, groups, rows) for the thread.
+  // Where the team kernel runs the steps, only the block size of the other
+  // tile kernels comes from here: the level is not encoded for k_spmv_loc.
   void autotune(const Level &lv) {
     // PARRSB_GPU_SPMV: 0 = k_spmv only, 1 = k_spmv_tma only, 2 = k_spmv_loc only
     // where it applies, unset = time them
@@ -4182,11 +4184,12 @@ struct Lanczos {
     ensure_smem_limit(k_spmv_tma, 200 * 1024);
     const char *force_env = getenv("PARRSB_GPU_SPMV");
     const int force_kind = force_env ? atoi(force_env) : -1;
-    static thread_local std::vector<std::pair<std::array<ll, 5>, int>> cache;
+    static thread_local std::vector<std::pair<std::array<ll, 6>, int>> cache;
     // PARRSB_GPU_SPMV_THREADS: only this block size (128, 256 or 512)
     const char *th_env = getenv("PARRSB_GPU_SPMV_THREADS");
     const int force_th = th_env ? atoi(th_env) : 0;
-    std::array<ll, 5> key = {(ll)T, (ll)A, N, (ll)lv.max_w, (ll)force_kind * 1024 + force_th};
+    std::array<ll, 6> key = {(ll)T, (ll)A, N, (ll)lv.max_w, (ll)force_kind * 1024 + force_th,
+                             (ll)team};
     for (auto &kv : cache)
       if (kv.first == key) {
         sp_kind = kv.second >> 16;
@@ -4202,7 +4205,7 @@ struct Lanczos {
       if (force_kind < 0 || force_kind == 0) cand.push_back({0, th});
       if ((force_kind < 0 || force_kind == 1) && sp_tma_ok(lv, th)) cand.push_back({1, th});
     }
-    if (force_kind == 2 || (force_kind < 0 && N >= SL_MIN))
+    if (!team && (force_kind == 2 || (force_kind < 0 && N >= SL_MIN)))
       if (loc_prepare(lv))
         for (int th : {256, 512})
           if (!force_th || th == force_th) cand.push_back({2, th});
@@ -4283,8 +4286,8 @@ struct Lanczos {
     if (eig_smem() > 48 * 1024)
       CK(cudaFuncSetAttribute(k_tri_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)eig_smem()));
-    autotune(lv);
     team = !team_off && want_team(lv);
+    autotune(lv);
     if (team) {  // (what the passes overwrite)
       gs0.ensure(A);
       CK(cudaMemcpyAsync(gs0.p, gs.p, (size_t)A * sizeof(GState), cudaMemcpyDeviceToDevice, st));
@@ -4333,6 +4336,7 @@ struct Lanczos {
     ctx().stats = before;
     CK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
     CK(cudaMemcpyAsync(gs.p, gs0.p, (size_t)A * sizeof(GState), cudaMemcpyDeviceToDevice, st));
+    autotune(lv);
     if (warm)
       CK(cudaMemcpyAsync(f.p, f0.p, (size_t)N * sizeof(VT), cudaMemcpyDeviceToDevice, st));
     CK(cudaMemsetAsync(p.p, 0, (size_t)N * sizeof(VT), st));

@@ -1,0 +1,30 @@
+"""The level encodings of the team step kernel and of the staged SpMV: which
+of them a level makes, and what runs where one does not apply."""
+import numpy as np
+import pytest
+
+import parrsb_gb300 as P
+from parrsb_gb300 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+def _launches(vtx, grp):
+    P.fiedler_groups(vtx, grp, 1, rsb_max_passes=2)  # (decides the block size)
+    f, it, _ = P.fiedler_groups(vtx, grp, 1, rsb_max_passes=2)
+    return P.last_stats().kernel_launches, f, it
+
+
+def test_one_encoding_per_level(monkeypatch):
+    """A level of the team kernel is not encoded for the staged SpMV too."""
+    monkeypatch.setenv("PARRSB_GPU_FP32", "1")
+    monkeypatch.setenv("PARRSB_GPU_PERSIST", "1")
+    vtx, _ = meshgen.box_hex(24, 20, 16, jitter=0.1, seed=4)
+    grp = np.zeros(len(vtx), np.int32)
+    monkeypatch.setenv("PARRSB_GPU_SPMV", "0")
+    plain, f0, i0 = _launches(vtx, grp)
+    monkeypatch.setenv("PARRSB_GPU_SPMV", "2")
+    staged, f2, i2 = _launches(vtx, grp)
+    assert staged == plain
+    np.testing.assert_array_equal(f0, f2)
+    np.testing.assert_array_equal(i0, i2)
