@@ -2469,8 +2469,16 @@ __device__ __forceinline__ void team_publish(bool solo, double *own, TeamSlot *s
 // a slice of width w takes (w + 1) / 2 rows of 32 words, slice q of the block
 // starting at half its ELL offset plus 32 q.  A slice that two blocks share
 // is encoded by both, so every tile leaves room for one widest slice more.
+// (Blocks start at whole rows of 32 words: the half offset rounded up, at most
+// 16 words more, which the 32 per slice and the room per tile hold.)
+__host__ __device__ __forceinline__ ll enc_room(int max_w) { return ((max_w + 1) / 2 + 1) * 32ll; }
 __device__ __forceinline__ ll enc_base(ll word, ll sl, int tile, int max_w) {
-  return word + 32 * sl + (ll)tile * (max_w + 1) * 32;
+  return (((word >> 1) + 31) & ~31ll) + 32 * sl + (ll)tile * enc_room(max_w);
+}
+// words of a level's encoding: `words` of the matrix, N rows in T tiles, and
+// what the kernels fetch ahead past the last slice (16 rows of 32 at most)
+inline size_t enc_words(ll words, ll N, int T, int max_w) {
+  return (size_t)((words >> 1) + 32 + (N / 32 + 2) * 32 + (T + 1) * enc_room(max_w) + 1024);
 }
 
 // One block per item: the halo list and the encoded rows.  The halo is marked
@@ -3900,6 +3908,33 @@ struct Lanczos {
            (size_t)ts_halo * sizeof(int) + (size_t)ts_enc * sizeof(unsigned);
   }
 
+  // The buffers of a level's encoding.  No other form of the steps needs them, so
+  // where the device has no room for them the level does without (false).
+  template <typename F>
+  bool room(F &&alloc) {
+    try {
+      if (fault_injected("encoding"))
+        throw CudaError{cudaErrorMemoryAllocation, __FILE__, __LINE__};
+      alloc();
+      return true;
+    } catch (const CudaError &e) {
+      if (e.err != cudaErrorMemoryAllocation) throw;
+      cudaGetLastError();
+      drop_encodings(0);
+      return false;
+    }
+  }
+  // gives encodings of more than `keep` words back: the sorts and balancing
+  // between two levels use the memory, and the next level is encoded anew
+  void drop_encodings(size_t keep) {
+    if (d_enc.n > keep) d_enc.release(), d_halo.release();
+    if (sl_enc.n > keep) sl_enc.release(), sl_halo.release();
+  }
+  struct EncodingScope {  // of one level's run
+    Lanczos *l;
+    ~EncodingScope() { l->drop_encodings(4u << 20); }  // (16 MB)
+  };
+
   // Assigns the level's groups to teams of blocks (G in all, one per SM).  A
   // group whose rows fit the share of one block goes to a single block, which
   // takes such groups one after the other (largest first, to the least loaded
@@ -4081,17 +4116,20 @@ struct Lanczos {
     const size_t bm = halos ? (size_t)((biggest + 127) / 128) * (16 + 2) + 64 : 64;
     if (bm > (size_t)TS_SMEM) return false;
     cudaStream_t st = ctx().stream;
-    d_blk.ensure(ts_blk.size()), d_list.ensure(ts_list.size());
-    d_item0.ensure(ts_item0.size()), d_items.ensure(ts_items.size());
+    if (!room([&] {
+          d_blk.ensure(ts_blk.size()), d_list.ensure(ts_list.size());
+          d_item0.ensure(ts_item0.size()), d_items.ensure(ts_items.size());
+          d_nhalo.ensure(ts_items.size());
+          d_halo.ensure((size_t)std::max(multi, 1) * TS_HALO);
+          d_enc.ensure(enc_words(lv.words, N, T, lv.max_w));
+          d_bad.ensure(1);
+          slots.ensure((size_t)3 * TS_REP * T);
+        }))
+      return false;
     h2d(d_blk.p, ts_blk.data(), ts_blk.size());
     h2d(d_list.p, ts_list.data(), ts_list.size());
     h2d(d_item0.p, ts_item0.data(), ts_item0.size());
     h2d(d_items.p, ts_items.data(), ts_items.size());
-    d_nhalo.ensure(ts_items.size());
-    d_halo.ensure((size_t)std::max(multi, 1) * TS_HALO);
-    d_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
-                 (size_t)(T + 1) * (size_t)(lv.max_w + 1) * 32 + 128);
-    d_bad.ensure(1);
     CK(cudaMemsetAsync(d_bad.p, 0, sizeof(int), st));
     ensure_smem_limit(k_team_encode<VT>, TS_SMEM);
     k_team_encode<VT><<<(unsigned)ts_items.size(), TE_THREADS, bm, st>>>(
@@ -4103,7 +4141,6 @@ struct Lanczos {
     d2h(&bad, d_bad.p, 1);
     sync();
     if (bad) return false;
-    slots.ensure((size_t)3 * TS_REP * T);
     CK(cudaMemsetAsync(slots.p, 0, (size_t)3 * TS_REP * T * sizeof(TeamSlot), ctx().stream));
     if (!ts_epoch.p) {
       ts_epoch.alloc(1);
@@ -4152,10 +4189,12 @@ struct Lanczos {
     }
     sl_pcap = sl_cap((int)longest);
     const size_t nr = sl_runs.size();
-    d_runs.ensure(nr), sl_nhalo.ensure(nr), sl_halo.ensure(nr * SL_HALO), sl_bad.ensure(2);
+    if (!room([&] {
+          d_runs.ensure(nr), sl_nhalo.ensure(nr), sl_halo.ensure(nr * SL_HALO), sl_bad.ensure(2);
+          sl_enc.ensure(enc_words(lv.words, N, T, lv.max_w));
+        }))
+      return false;
     h2d(d_runs.p, sl_runs.data(), nr);
-    sl_enc.ensure((size_t)lv.words + (size_t)(N / 32 + 2) * 32 +
-                 (size_t)(T + 1) * (size_t)(lv.max_w + 1) * 32 + 1024);
     CK(cudaMemsetAsync(sl_bad.p, 0, 2 * sizeof(int), st));
     ensure_smem_limit(k_loc_encode, LE_SMEM);
     k_loc_encode<<<(unsigned)nr, LE_THREADS, LE_SMEM, st>>>(
@@ -4286,15 +4325,17 @@ struct Lanczos {
     if (eig_smem() > 48 * 1024)
       CK(cudaFuncSetAttribute(k_tri_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)eig_smem()));
-    team = !team_off && want_team(lv);
-    autotune(lv);
-    if (team) {  // (what the passes overwrite)
+    const EncodingScope scope{this};
+    // (gs0, f0: what the passes overwrite)
+    team = !team_off && want_team(lv) && room([&] {
       gs0.ensure(A);
+      if (warm) f0.ensure(N);
+    });
+    autotune(lv);
+    if (team) {
       CK(cudaMemcpyAsync(gs0.p, gs.p, (size_t)A * sizeof(GState), cudaMemcpyDeviceToDevice, st));
-      if (warm) {
-        f0.ensure(N);
+      if (warm)
         CK(cudaMemcpyAsync(f0.p, f.p, (size_t)N * sizeof(VT), cudaMemcpyDeviceToDevice, st));
-      }
     }
     auto start = [&] {
       k_set_active<<<grid_for(A, 128), 128, 0, st>>>(gs.p, A);

@@ -28,3 +28,22 @@ def test_one_encoding_per_level(monkeypatch):
     assert staged == plain
     np.testing.assert_array_equal(f0, f2)
     np.testing.assert_array_equal(i0, i2)
+
+
+@pytest.mark.parametrize("persist,spmv", [("1", "0"), ("0", "2"), ("1", "2")])
+def test_no_memory_for_an_encoding(monkeypatch, persist, spmv):
+    """An encoding that does not fit the device's memory (injected on the
+    host) leaves the level to the form that needs none."""
+    monkeypatch.setenv("PARRSB_GPU_FP32", "1")
+    vtx, _ = meshgen.box_hex(24, 20, 16, jitter=0.1, seed=4)
+    grp = np.zeros(len(vtx), np.int32)
+    monkeypatch.setenv("PARRSB_GPU_PERSIST", "0")
+    monkeypatch.setenv("PARRSB_GPU_SPMV", "0")
+    plain, f0, i0 = _launches(vtx, grp)
+    monkeypatch.setenv("PARRSB_GPU_PERSIST", persist)
+    monkeypatch.setenv("PARRSB_GPU_SPMV", spmv)
+    monkeypatch.setenv("PARRSB_FAULT", "encoding")
+    got, f1, i1 = _launches(vtx, grp)
+    assert got == plain
+    np.testing.assert_array_equal(f0, f1)
+    np.testing.assert_array_equal(i0, i1)
