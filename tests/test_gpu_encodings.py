@@ -47,3 +47,21 @@ def test_no_memory_for_an_encoding(monkeypatch, persist, spmv):
     assert got == plain
     np.testing.assert_array_equal(f0, f1)
     np.testing.assert_array_equal(i0, i1)
+
+
+def test_staged_spmv_after_the_team_encoder_refuses(monkeypatch):
+    """Planes of seven lines of 300 elements: the rows beside a block of 512 are
+    more than the team kernel holds, those beside a staged run of 8192 are not.
+    The team encoder has written its own buffers by then."""
+    monkeypatch.setenv("PARRSB_GPU_FP32", "1")
+    vtx, _ = meshgen.box_hex(300, 7, 14, jitter=0.1, seed=4)
+    grp = np.zeros(len(vtx), np.int32)
+    monkeypatch.setenv("PARRSB_GPU_PERSIST", "0")
+    monkeypatch.setenv("PARRSB_GPU_SPMV", "0")
+    plain, f0, i0 = _launches(vtx, grp)
+    monkeypatch.setenv("PARRSB_GPU_PERSIST", "1")
+    monkeypatch.setenv("PARRSB_GPU_SPMV", "2")
+    got, f1, i1 = _launches(vtx, grp)
+    assert got == plain + 2  # both encoders, then a launch per kernel
+    np.testing.assert_array_equal(f0, f1)
+    np.testing.assert_array_equal(i0, i1)
