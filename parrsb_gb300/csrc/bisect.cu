@@ -1981,6 +1981,7 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
     }
     ws.rank_of = cent;
     ws.g_ok = false;  // lists of other centroids
+    ws.sort.trim(1ll << 18);  // (with unique ranks nothing more is sorted)
   }
   // PARRSB_GPU_RCB_PRESORT=0: the sort-per-level path even for unique ranks
   if (kind == BISECT_RCB && ws.unique) {

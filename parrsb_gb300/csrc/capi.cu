@@ -605,14 +605,14 @@ extern "C" int parrsb_conn_mesh(long long *vtx, double *coord, unsigned int nel,
       // periodic faces (src/con.c:261-264); without any, the consecutive
       // renumbering leaves the ids as they are
       StageTimer tm(PARRSB_STAGE_GENCON);
-      r = periodic_device(W.gc.ids.p, W.gc.pt.p, nel, (int)nDim,
+      r = periodic_device(W.gc.ids(), W.gc.pt.p, nel, (int)nDim,
                           nseg, periodicInfo, nPeriodicFaces, W.gc.sort, &nseg);
       ctx().stats.gencon_segments = nseg;
       if (r != PARRSB_OK) {
         print_if(1, "\t%s:%d periodic faces did not match.", __FILE__, __LINE__);
         return r;
       }
-      plus_one(W.gc.ids.p, np, W.ids.p);
+      plus_one(W.gc.ids(), np, W.ids.p);
     }
     {
       StageTimer tm(PARRSB_STAGE_DOWNLOAD);

@@ -458,12 +458,9 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
   ws.keys.ensure((size_t)np);
   ws.ord.ensure((size_t)np);
   ws.flag.ensure((size_t)np);
-  ws.flag2.ensure((size_t)np);
   ws.seg.ensure((size_t)np);
   ws.seg_start.ensure((size_t)np);
   ws.nseg_max.ensure(2);
-  ws.ids.ensure((size_t)np);
-  ws.ids32.ensure((size_t)np);
   {
     const size_t smem = (size_t)GP_ELEMS * (nv * ndim + 1 + nv + 1) * sizeof(double);
     const unsigned nb = grid_for(nel, GP_ELEMS);
@@ -484,14 +481,14 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     if (t == 1) {
       // nothing left to sort: the later rounds' gaps at once
       k_gc_settle<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.pt.p, ws.flag.p, np, ndim, tol2,
-                                                     ws.flag2.p, err.p + 1);
+                                                     ws.flag2(), err.p + 1);
       CK_LAUNCH();
+      keys_of = -1;
       int unsettled = 0;
       d2h(&unsettled, err.p + 1, 1);
       sync();
       if (!unsettled) {
-        std::swap(ws.flag, ws.flag2);
-        segments_of(ws, ws.flag.p, np, &nseg, &longest);
+        segments_of(ws, ws.flag2(), np, &nseg, &longest);
         break;
       }
     }
@@ -513,16 +510,16 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     }
   }
   if (nseg_out) *nseg_out = nseg;
-  k_ids<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.seg.p, np, ws.ids.p, ws.ids32.p);
+  k_ids<<<grid_for(np, 256), 256, 0, st>>>(ws.ord.p, ws.seg.p, np, ws.ids(), ws.ids32());
   CK_LAUNCH();
   if (d_ids_out)
-    CK(cudaMemcpyAsync(d_ids_out, ws.ids.p, np * sizeof(ll), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemcpyAsync(d_ids_out, ws.ids(), np * sizeof(ll), cudaMemcpyDeviceToDevice, st));
   {
     StageTimer tm(PARRSB_STAGE_CHECK);
-    k_element_check<<<grid_for(nel, 256), 256, 0, st>>>(ws.ids32.p, nel, nv, err.p);
+    k_element_check<<<grid_for(nel, 256), 256, 0, st>>>(ws.ids32(), nel, nv, err.p);
     CK_LAUNCH();
     if (ndim == 3) {  // in 2D an edge has two corners: a count of 3 is impossible
-      k_face_check<<<grid_for(np, 256), 256, 0, st>>>(ws.ids32.p, ws.ord.p, ws.seg_start.p,
+      k_face_check<<<grid_for(np, 256), 256, 0, st>>>(ws.ids32(), ws.ord.p, ws.seg_start.p,
                                                       (int)nseg, np, err.p);
       CK_LAUNCH();
     }
@@ -532,7 +529,7 @@ int gencon_device(long long *d_vtx, const double *d_coord, ll nel, int ndim,
     if (h_err) return 1;
   }
   if (d_vtx) {
-    k_plus_one<<<grid_for(np, 256), 256, 0, st>>>(ws.ids.p, np, d_vtx);
+    k_plus_one<<<grid_for(np, 256), 256, 0, st>>>(ws.ids(), np, d_vtx);
     CK_LAUNCH();
   }
   return PARRSB_OK;

@@ -9,11 +9,15 @@ struct GenconWs {
   SortWs sort;
   DBuf<double4_32a> pt;  // points: coordinates, min squared neighbour distance
   DBuf<u64> keys;
-  DBuf<int> ord, flag, flag2;
+  DBuf<int> ord, flag;
   DBuf<int> seg, seg_start, bsum;  // segment of every position, first position of each
   DBuf<int> nseg_max;              // number of segments, longest one
-  DBuf<ll> ids;
-  DBuf<int> ids32;
+  // buffers whose first contents are no longer needed by then: the flags of the
+  // later rounds at once in place of the keys, then the ids (all segments found)
+  // in place of the keys, and in 32 bits of the flags
+  int *flag2() const { return reinterpret_cast<int *>(keys.p); }
+  ll *ids() const { return reinterpret_cast<ll *>(keys.p); }
+  int *ids32() const { return flag.p; }
 };
 
 // Device-resident gencon.  d_coord: nel*nv*ndim corner coordinates in

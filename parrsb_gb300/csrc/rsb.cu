@@ -5493,7 +5493,6 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   CK_LAUNCH();
   seg_sort_pairs(keys, vals, ns, nullptr, 1, sws);
   DBuf<int> flag((size_t)ns), runid((size_t)ns);
-  DBuf<int2> run((size_t)ns);
   DBuf<ll> excl((size_t)ns);
   k_run_flags<<<grid_for(ns, 256), 256, 0, st>>>(keys.p, ns, flag.p);
   CK_LAUNCH();
@@ -5502,18 +5501,20 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   k_run_bounds<<<grid_for(ns, 256), 256, 0, st>>>(flag.p, excl.p, ns, nruns, runid.p,
                                                   run_start.p);
   CK_LAUNCH();
-  k_scatter_run<<<grid_for(ns, 256), 256, 0, st>>>(vals.p, runid.p, run_start.p, ns, run.p);
+  int2 *run = reinterpret_cast<int2 *>(keys.p);  // (the keys have done their work)
+  k_scatter_run<<<grid_for(ns, 256), 256, 0, st>>>(vals.p, runid.p, run_start.p, ns, run);
   CK_LAUNCH();
-  keys.release();
   excl.release();
   flag.release();
+  runid.release();
+  sws.trim(1ll << 22);  // (a corner's share; what follows sorts elements)
   DBuf<ll> rowlen((size_t)nel + 1);
   DBuf<int> maxw(1);
   CK(cudaMemsetAsync(maxw.p, 0, sizeof(int), st));
   CK(cudaMemsetAsync(rowlen.p + nel, 0, sizeof(ll), st));
   const unsigned gr_blocks = std::min(grid_for(nel, GR_WARPS), 152u * 9u * 2u);  // two waves
   k_graph_rows<false><<<gr_blocks, GR_WARPS * 32, 0, st>>>(
-      nv, nel, vals.p, run.p, nullptr, nullptr, nullptr, rowlen.p, maxw.p);
+      nv, nel, vals.p, run, nullptr, nullptr, nullptr, rowlen.p, maxw.p);
   CK_LAUNCH();
   g.nnz = exclusive_scan_ll(rowlen.p, g.rowptr.p, nel + 1);
   DBuf<unsigned long long> mrow(1);
@@ -5530,7 +5531,7 @@ void build_dual_graph(const long long *d_vtx, ll nel, int nv, Graph &g, SortWs &
   g.col.ensure((size_t)g.nnz + 1);
   g.w.ensure((size_t)g.nnz + 1);
   k_graph_rows<true><<<gr_blocks, GR_WARPS * 32, 0, st>>>(
-      nv, nel, vals.p, run.p, g.rowptr.p, g.col.p, g.w.p, nullptr, nullptr);
+      nv, nel, vals.p, run, g.rowptr.p, g.col.p, g.w.p, nullptr, nullptr);
   CK_LAUNCH();
 }
 

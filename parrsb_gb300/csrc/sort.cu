@@ -998,7 +998,8 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
     return;
   }
   // the full radix sort of (key, position), the segments by position
-  DBuf<int> pos((size_t)n);
+  DBuf<int> &pos = ws.idxtmp;
+  pos.ensure((size_t)n);
   k_iota_pos<<<grid_for(n, 256), 256, 0, st>>>(pos.p, n);
   CK_LAUNCH();
   seg_sort_pairs(keys, pos, n, seg_of_pos, nseg, ws);

@@ -81,6 +81,13 @@ struct SortWs {
   DBuf<int> idx, idxtmp;
   DBuf<u64> range;      // smallest and largest key, runs that cannot be listed, runs listed
   DBuf<int2> runs;      // long runs out of order: start, length
+  // gives the buffers of more than `keep` items back to the pool
+  void trim(ll keep) {
+    auto drop = [keep](auto &b) {
+      if ((ll)b.n > keep) b.release();
+    };
+    drop(ktmp), drop(vtmp), drop(q), drop(qtmp), drop(idx), drop(idxtmp);
+  }
 };
 
 // Sort pairs (keys[i], vals[i]), i < n, stably by (seg_of_val[vals[i]], key).
