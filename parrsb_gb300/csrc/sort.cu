@@ -745,14 +745,14 @@ k_scatter32(const u32 *__restrict__ kin, const int *__restrict__ vin, u32 *__res
   }
 }
 
-__global__ void k_gather_kv(const int *__restrict__ idx, const u64 *__restrict__ keys,
-                            const int *__restrict__ vals, ll n, u64 *__restrict__ kout,
-                            int *__restrict__ vout) {
+// idx: positions in, values out (null vals: the positions)
+__global__ void k_gather_kv(int *__restrict__ idx, const u64 *__restrict__ keys,
+                            const int *__restrict__ vals, ll n, u64 *__restrict__ kout) {
   const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int j = idx[i];
   kout[i] = keys[j];
-  vout[i] = vals ? vals[j] : j;
+  if (vals) idx[i] = vals[j];
 }
 
 __global__ void k_gather_val(const int *__restrict__ idx, const int *__restrict__ in, ll n,
@@ -768,7 +768,8 @@ __global__ void k_iota_pos(int *__restrict__ a, ll n) {
 // Runs of equal 32-bit keys into the order of their full keys: the thread of a
 // run's first item sorts a run of at most FIX_MAX by insertion (stable); of a
 // longer one every pair of neighbours is checked, and a run that is not in
-// order is listed once (mark, zero before the launch) for k_sort_run.
+// order is listed once (mark, a bit per item, zero before the launch) for
+// k_sort_run.
 // range[2]: a run cannot be listed; range[3]: runs listed.
 __device__ __forceinline__ ll run_bound(const u32 *__restrict__ q, ll n, u64 v) {
   ll lo = 0, hi = n;  // first position with q >= v
@@ -782,11 +783,12 @@ __device__ __forceinline__ ll run_bound(const u32 *__restrict__ q, ll n, u64 v) 
   return lo;
 }
 __device__ __forceinline__ void list_run(const u32 *__restrict__ q, ll n, u32 qi,
-                                         u64 *__restrict__ range, int *__restrict__ mark,
+                                         u64 *__restrict__ range, u32 *__restrict__ mark,
                                          int2 *__restrict__ runs) {
   if (*(volatile u64 *)&range[2]) return;
   const ll b = run_bound(q, n, qi);
-  if (atomicExch(&mark[b], 1)) return;
+  const u32 bit = 1u << (b & 31);
+  if (atomicOr(&mark[b >> 5], bit) & bit) return;
   const ll e = run_bound(q, n, (u64)qi + 1);
   const u64 at = e - b <= LOCAL_MAX ? atomicAdd(&range[3], 1ull) : (u64)RUN_LIST;
   if (at < RUN_LIST)
@@ -796,7 +798,7 @@ __device__ __forceinline__ void list_run(const u32 *__restrict__ q, ll n, u32 qi
 }
 __global__ void k_fix_runs(const u32 *__restrict__ q, ll n, u64 *__restrict__ keys,
                            int *__restrict__ vals, u64 *__restrict__ range,
-                           int *__restrict__ mark, int2 *__restrict__ runs) {
+                           u32 *__restrict__ mark, int2 *__restrict__ runs) {
   const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const u32 qi = q[i];
@@ -947,9 +949,12 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
   if (!full) {
     ws.range.ensure(4);
     ws.runs.ensure(RUN_LIST);
-    ws.q.ensure((size_t)n), ws.qtmp.ensure((size_t)n);
-    ws.idx.ensure((size_t)n), ws.idxtmp.ensure((size_t)n);
+    ws.q.ensure((size_t)n), ws.mark.ensure((size_t)(n + 31) / 32);
     ws.ktmp.ensure((size_t)n), ws.vtmp.ensure((size_t)n);
+    // the passes go from (qa, ia) to (qb, ib) and back; ktmp holds the second
+    // pair until it takes the sorted keys
+    u32 *qa = ws.q.p, *qb = reinterpret_cast<u32 *>(ws.ktmp.p);
+    int *ia = ws.vtmp.p, *ib = reinterpret_cast<int *>(qb + n);
     const int ntiles = (int)((n + TILE - 1) / TILE);
     ws.counts.ensure((size_t)256 * ntiles);
     ws.totals.ensure(256);
@@ -962,24 +967,23 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
                                                                        ws.range.p, ws.q.p);
     CK_LAUNCH();
     ensure_smem_limit(k_scatter32, (int)(TILE * sizeof(uint2)));  // with the tables over 48 KB
-    for (int shift = 0; shift < 32; shift += 8) {
-      k_tile_hist32<<<ntiles, SORT_THREADS, 0, st>>>(ws.q.p, n, shift, ws.counts.p, ntiles);
+    for (int shift = 0; shift < 32; shift += 8) {  // (an even number: back in qa, ia)
+      k_tile_hist32<<<ntiles, SORT_THREADS, 0, st>>>(qa, n, shift, ws.counts.p, ntiles);
       CK_LAUNCH();
       k_tile_scan<<<256, 1024, 0, st>>>(ws.counts.p, ntiles, ws.totals.p);
       CK_LAUNCH();
       k_scatter32<<<ntiles, SORT_THREADS, TILE * sizeof(uint2), st>>>(
-          ws.q.p, shift ? ws.idx.p : nullptr, ws.qtmp.p, ws.idxtmp.p, n, shift, ws.counts.p,
-          ws.totals.p, ntiles);
+          qa, shift ? ia : nullptr, qb, ib, n, shift, ws.counts.p, ws.totals.p, ntiles);
       CK_LAUNCH();
-      std::swap(ws.q, ws.qtmp);
-      std::swap(ws.idx, ws.idxtmp);
+      std::swap(qa, qb);
+      std::swap(ia, ib);
     }
-    k_gather_kv<<<grid_for(n, 256), 256, 0, st>>>(ws.idx.p, keys.p, iota ? nullptr : vals.p, n,
-                                                  ws.ktmp.p, ws.vtmp.p);
+    k_gather_kv<<<grid_for(n, 256), 256, 0, st>>>(ws.vtmp.p, keys.p, iota ? nullptr : vals.p, n,
+                                                  ws.ktmp.p);
     CK_LAUNCH();
-    CK(cudaMemsetAsync(ws.idxtmp.p, 0, (size_t)n * sizeof(int), st));
+    CK(cudaMemsetAsync(ws.mark.p, 0, (size_t)(n + 31) / 32 * sizeof(u32), st));
     k_fix_runs<<<grid_for(n, 256), 256, 0, st>>>(ws.q.p, n, ws.ktmp.p, ws.vtmp.p, ws.range.p,
-                                                 ws.idxtmp.p, ws.runs.p);
+                                                 ws.mark.p, ws.runs.p);
     CK_LAUNCH();
     u64 said[2] = {0, 0};
     d2h(said, ws.range.p + 2, 2);
@@ -998,15 +1002,15 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
     return;
   }
   // the full radix sort of (key, position), the segments by position
-  DBuf<int> &pos = ws.idxtmp;
-  pos.ensure((size_t)n);
-  k_iota_pos<<<grid_for(n, 256), 256, 0, st>>>(pos.p, n);
+  ws.q.release();
+  ws.pos.ensure((size_t)n);
+  k_iota_pos<<<grid_for(n, 256), 256, 0, st>>>(ws.pos.p, n);
   CK_LAUNCH();
-  seg_sort_pairs(keys, pos, n, seg_of_pos, nseg, ws);
-  ws.idx.ensure((size_t)n);
-  k_gather_val<<<grid_for(n, 256), 256, 0, st>>>(pos.p, vals.p, n, ws.idx.p);
+  seg_sort_pairs(keys, ws.pos, n, seg_of_pos, nseg, ws);
+  ws.vtmp.ensure((size_t)n);
+  k_gather_val<<<grid_for(n, 256), 256, 0, st>>>(ws.pos.p, vals.p, n, ws.vtmp.p);
   CK_LAUNCH();
-  std::swap(vals, ws.idx);
+  std::swap(vals, ws.vtmp);
 }
 
 }  // namespace prsb

@@ -77,8 +77,9 @@ struct SortWs {
   DBuf<u32> totals;     // [256]
   DBuf<u32> hist_all;   // [npass][256]
   // sort_by_value
-  DBuf<u32> q, qtmp;
-  DBuf<int> idx, idxtmp;
+  DBuf<u32> q;          // 32-bit keys (their other buffer: ktmp)
+  DBuf<u32> mark;       // a bit per item
+  DBuf<int> pos;        // positions, where the full keys are sorted
   DBuf<u64> range;      // smallest and largest key, runs that cannot be listed, runs listed
   DBuf<int2> runs;      // long runs out of order: start, length
   // gives the buffers of more than `keep` items back to the pool
@@ -86,7 +87,7 @@ struct SortWs {
     auto drop = [keep](auto &b) {
       if ((ll)b.n > keep) b.release();
     };
-    drop(ktmp), drop(vtmp), drop(q), drop(qtmp), drop(idx), drop(idxtmp);
+    drop(ktmp), drop(vtmp), drop(q), drop(pos);
   }
 };
 
