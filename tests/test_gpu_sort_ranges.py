@@ -1,0 +1,58 @@
+"""Sorts of values that a linear map over their range does not separate (one far
+point, clumps, geometric grading), on both sides of the sample's decision: RIB
+orders and RCB parts against the oracle, gencon ids against those of the same
+mesh without its far element."""
+import numpy as np
+import pytest
+
+import parrsb_gb300 as P
+from parrsb_gb300 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+def _line(values):
+    n = len(values)
+    xyz = np.zeros((n, 4, 2))
+    xyz[..., 0] = values[:, None]
+    return np.arange(n * 4, dtype=np.int64).reshape(n, 4) + 1, xyz
+
+
+def _values(kind, n):
+    rng = np.random.Generator(np.random.PCG64(5))
+    x = rng.random(n)
+    if kind == "far":
+        x[n // 3] = 1e9
+    elif kind == "clumps":  # half of them within 1e-7, 1e-9, 1e-12 of the range
+        x[: n // 2] *= 1e-7
+    elif kind == "tight_clumps":
+        x[: n // 2] *= 1e-9
+    elif kind == "points":
+        x[: n // 2] = 0.5 + x[: n // 2] * 1e-12
+    elif kind == "graded":
+        x = np.expm1(np.log(1e12) * x)
+    elif kind == "planes":  # 30 values, in their last bits apart
+        x = np.floor(30.0 * x) / 30.0 * (1.0 + 2.0 ** -52 * rng.integers(-2, 3, n))
+    return x
+
+
+@pytest.mark.parametrize("n", [4097, 20000, 262144, 300001])
+@pytest.mark.parametrize("kind", ["far", "clumps", "tight_clumps", "points", "graded", "planes"])
+def test_ranges(oracle, kind, n):
+    vtx, xyz = _line(_values(kind, n))
+    for partitioner in (1, 2):
+        part, seq = P.part_mesh_seq(vtx, xyz, 2, partitioner=partitioner)
+        rc, ref, order, _, _ = oracle.part_mesh(vtx, xyz, 2, want_order=True,
+                                                partitioner=partitioner)
+        assert rc == 0
+        np.testing.assert_array_equal(part, ref)
+        np.testing.assert_array_equal(np.lexsort((seq, part)), order)
+
+
+def test_gencon_far_element():
+    _, xyz = meshgen.box_hex(40, 20, 20, jitter=0.1, seed=2)
+    want = P.conn_mesh(xyz, 3)
+    far = xyz[:1] + 1e9 * np.ones(3)
+    got = P.conn_mesh(np.concatenate([xyz, far]), 3)
+    np.testing.assert_array_equal(got[:-1], want)
+    assert len(np.unique(got[-1])) == 8 and got[-1].min() > want.max()
