@@ -94,6 +94,24 @@ __device__ __forceinline__ double tree_pair(double a, double b) {
   return v;
 }
 
+// the V values whose sums a segment takes, of element e (avg: the segment's means)
+template <int V, int GEN>
+__device__ __forceinline__ void seg_values(const double *__restrict__ cent, ll N, int e,
+                                           const double *__restrict__ avg, double *v) {
+  const double c0 = cent[e], c1 = cent[N + e], c2 = cent[2 * N + e];
+  if (GEN == GEN_MEAN) {
+    v[0] = c0, v[1] = c1, v[2] = c2;
+  } else {  // inertia products (00, 01, 02, 11, 12, 22)
+    const double x = __dsub_rn(c0, avg[0]), y = __dsub_rn(c1, avg[1]), z = __dsub_rn(c2, avg[2]);
+    v[0] = __dmul_rn(x, x);
+    v[1] = __dmul_rn(x, y);
+    v[2] = __dmul_rn(x, z);
+    v[3] = __dmul_rn(y, y);
+    v[V - 2] = __dmul_rn(y, z);
+    v[V - 1] = __dmul_rn(z, z);
+  }
+}
+
 // V sums per segment (even V): one block per 1024 consecutive items of a
 // segment takes two levels of the canonical 32-wide tree at once (a warp per
 // 32-item tile, then the first warp over the tiles); a segment's count shrinks
@@ -135,20 +153,7 @@ k_seg_tree(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
 #pragma unroll
       for (int q = 0; q < V; q++) v[q] = in[src + q];
     } else {
-      const int e = perm[seg_start[s] + i];
-      const double c0 = cent[e], c1 = cent[N + e], c2 = cent[2 * N + e];
-      if (GEN == GEN_MEAN) {
-        v[0] = c0, v[1] = c1, v[2] = c2;
-      } else {  // inertia products (00, 01, 02, 11, 12, 22)
-        const double *a = avg + 3 * s;
-        const double x = __dsub_rn(c0, a[0]), y = __dsub_rn(c1, a[1]), z = __dsub_rn(c2, a[2]);
-        v[0] = __dmul_rn(x, x);
-        v[1] = __dmul_rn(x, y);
-        v[2] = __dmul_rn(x, z);
-        v[3] = __dmul_rn(y, y);
-        v[V - 2] = __dmul_rn(y, z);
-        v[V - 1] = __dmul_rn(z, z);
-      }
+      seg_values<V, GEN>(cent, N, perm[seg_start[s] + i], avg + 3 * s, v);
     }
   }
   const int tiles = (m + 31) / 32;
@@ -177,6 +182,66 @@ k_seg_tree(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
       if (lane == 0) out[(ll)blockIdx.x * V + q] = t;
       if (lane == 16) out[(ll)blockIdx.x * V + q + 1] = t;
     }
+  }
+}
+
+// The same sums where no segment has more than 1024 items: the whole tree of a
+// segment in one block of as many threads as the largest asks for, or in a warp
+// up to 32 items; sums of segment s at s V.  With a block of 1024 threads for
+// every segment a level of 262144 segments of four elements took 14.0 ms for its
+// two sums and their tables; these take 0.56.
+template <int V, int GEN>
+__global__ void __launch_bounds__(1024)
+k_seg_block(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
+            const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
+            const int *__restrict__ p, const double *__restrict__ avg, double *__restrict__ out) {
+  __shared__ double sv[V][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const ll s = blockIdx.x;
+  if (p[s] <= 1) return;
+  const int m = (int)seg_n[s], tiles = (m + 31) / 32;
+  double v[V];
+#pragma unroll
+  for (int q = 0; q < V; q++) v[q] = 0.0;
+  if ((int)threadIdx.x < m)
+    seg_values<V, GEN>(cent, N, perm[seg_start[s] + threadIdx.x], avg + 3 * s, v);
+#pragma unroll
+  for (int q = 0; q < V; q += 2) {
+    const double t = tree_pair(v[q], v[q + 1]);
+    if (lane == 0) sv[q][warp] = t;
+    if (lane == 16) sv[q + 1][warp] = t;
+  }
+  __syncthreads();
+  if (warp > 0) return;
+#pragma unroll
+  for (int q = 0; q < V; q += 2) {
+    double a = lane < tiles ? sv[q][lane] : 0.0, b = lane < tiles ? sv[q + 1][lane] : 0.0;
+    if (tiles > 1) {  // (one value after the first level is the sum)
+      const double t = tree_pair(a, b);
+      a = t, b = __shfl_sync(0xffffffffu, t, 16);
+    }
+    if (lane == 0) out[s * V + q] = a, out[s * V + q + 1] = b;
+  }
+}
+template <int V, int GEN>
+__global__ void __launch_bounds__(256)
+k_seg_warp(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
+           const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
+           const int *__restrict__ p, ll nseg, const double *__restrict__ avg,
+           double *__restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const ll s = ((ll)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (s >= nseg || p[s] <= 1) return;  // (whole warps)
+  double v[V];
+#pragma unroll
+  for (int q = 0; q < V; q++) v[q] = 0.0;
+  if (lane < (int)seg_n[s])
+    seg_values<V, GEN>(cent, N, perm[seg_start[s] + lane], avg + 3 * s, v);
+#pragma unroll
+  for (int q = 0; q < V; q += 2) {
+    const double t = tree_pair(v[q], v[q + 1]);
+    if (lane == 0) out[s * V + q] = t;
+    if (lane == 16) out[s * V + q + 1] = t;
   }
 }
 
@@ -364,6 +429,34 @@ __device__ double power_quad(bool active, int N, const double *A) {
   return y;
 }
 
+// The same iteration by one thread, for more than RIB_QUADS segments: a quad
+// costs the pipe twice as much per segment, which counts once the quads' warps
+// fill it (quads against threads at 4096 segments 125 and 222 us, 8192: 188 and
+// 222, 16384: 347 and 224, 262144: 5086 and 2521).
+constexpr ll RIB_QUADS = 8192;
+__device__ void power_serial(double *y, int N, const double *A) {
+  const double start[3] = {31.0 / 50.0, 17.0 / 50.0, 43.0 / 50.0};
+  double norm = 0.0;
+  for (int i = 0; i < N; i++) norm = __dadd_rn(norm, __dmul_rn(start[i], start[i]));
+  const double scale = __ddiv_rn(1.0, __dsqrt_rn(norm));
+  for (int i = 0; i < N; i++) y[i] = __dmul_rn(start[i], scale);
+  double ay[3], lambda = 0.0;
+  for (int i = 0; i < 100; i++) {
+    norm = 0.0;
+    for (int j = 0; j < N; j++) {
+      ay[j] = 0.0;
+      for (int k = 0; k < N; k++) ay[j] = __dadd_rn(ay[j], __dmul_rn(A[j * N + k], y[k]));
+      norm = __dadd_rn(norm, __dmul_rn(ay[j], ay[j]));
+    }
+    const double sn = __dsqrt_rn(norm);
+    const double err = i > 0 ? __ddiv_rn(__dsub_rn(sn, lambda), lambda) : 1.0;
+    lambda = sn;
+    const double inv = __ddiv_rn(1.0, sn);
+    for (int j = 0; j < N; j++) y[j] = __dmul_rn(ay[j], inv);
+    if (fabs(err) < 1e-12) break;
+  }
+}
+
 // RIB axis per segment.  Group segments (p > 1) use the tree sums in
 // sums/isums; rank-local segments (p == 1) sum sequentially over their
 // elements in order, as get_rib_axis does with c == NULL.
@@ -398,24 +491,25 @@ __global__ void k_rib_mean_group(const double *__restrict__ sums, const int *__r
   if (s >= nseg || p[s] <= 1) return;
   double dn = (double)seg_n[s];
   for (int d = 0; d < 3; d++)  // (the sums of 4, the last one unused)
-    avg[3 * s + d] = __ddiv_rn(sums[4 * (ll)off[s] + d], dn);
+    avg[3 * s + d] = __ddiv_rn(sums[4 * (off ? (ll)off[s] : s) + d], dn);
 }
 
+template <bool QUAD>
 __global__ void __launch_bounds__(128)
 k_rib_axis(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
            const ll *__restrict__ seg_start, const ll *__restrict__ seg_n,
            const int *__restrict__ p, ll nseg, int ndim, int do_local,
            const double *__restrict__ avg, const double *__restrict__ isums,
            const int *__restrict__ off, double *__restrict__ ev, int *__restrict__ act) {
-  const ll s = ((ll)blockIdx.x * blockDim.x + threadIdx.x) >> 2;  // a quad per segment
-  const int j = threadIdx.x & 3;
+  const ll s = ((ll)blockIdx.x * blockDim.x + threadIdx.x) >> (QUAD ? 2 : 0);
+  const int j = QUAD ? threadIdx.x & 3 : 0;
   const bool in = s < nseg;
   const bool active = in && seg_active(p[in ? s : 0], seg_n[in ? s : 0], do_local);
   if (in && j == 0) act[s] = active;
   double I6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (active) {
     if (p[s] > 1) {
-      for (int q = 0; q < 6; q++) I6[q] = isums[6 * (ll)off[s] + q];
+      for (int q = 0; q < 6; q++) I6[q] = isums[6 * (off ? (ll)off[s] : s) + q];
     } else {
       const double *a = avg + 3 * s;
       ll st = seg_start[s], n = seg_n[s];
@@ -433,8 +527,14 @@ k_rib_axis(const int *__restrict__ perm, const double *__restrict__ cent, ll N,
     }
   }
   const double I[9] = {I6[0], I6[1], I6[2], I6[1], I6[3], I6[4], I6[2], I6[4], I6[5]};
-  const double y = power_quad(active, ndim, I);
-  if (active && j < 3) ev[3 * s + j] = j < ndim ? y : 0.0;
+  if (QUAD) {
+    const double y = power_quad(active, ndim, I);
+    if (active && j < 3) ev[3 * s + j] = j < ndim ? y : 0.0;
+  } else if (active) {
+    double y[3] = {0.0, 0.0, 0.0};
+    power_serial(y, ndim, I);
+    ev[3 * s] = y[0], ev[3 * s + 1] = y[1], ev[3 * s + 2] = ndim == 3 ? y[2] : 0.0;
+  }
 }
 
 template <int KIND>
@@ -1108,15 +1208,29 @@ inline int tree_launches(ll maxn) {
   return l;
 }
 
-// Sums of V values over every segment with more than one rank (tables of
-// k_tree_offsets), in the canonical tree; the sums of segment s are at
-// off[s] V of the returned buffer.  No host wait: the launches cover the
-// largest possible number of blocks.
+// Sums of V values over every segment with more than one rank, in the
+// canonical tree; the sums of segment s are at off[s] V of the returned buffer
+// (off null: s V; the tables of k_tree_offsets are for segments of more than
+// 1024 items, maxn the largest).  No host wait: the launches cover the largest
+// possible number of blocks.
 template <int V, int GEN0>
 const double *seg_tree_reduce(const int *perm, const double *cent, ll N, SegTable &t,
-                              const double *avg, int launches, BisectWs &ws, const int **off_out) {
+                              const double *avg, ll maxn, int launches, BisectWs &ws,
+                              const int **off_out) {
   cudaStream_t st = ctx().stream;
   const ll nseg = t.count;
+  if (maxn <= 1024) {
+    *off_out = nullptr;
+    ws.red_a.ensure((size_t)nseg * V);
+    if (maxn <= 32)
+      k_seg_warp<V, GEN0><<<grid_for(nseg * 32, 256), 256, 0, st>>>(
+          perm, cent, N, t.start.p, t.n.p, t.p.p, nseg, avg, ws.red_a.p);
+    else
+      k_seg_block<V, GEN0><<<(unsigned)nseg, (unsigned)((maxn + 31) / 32 * 32), 0, st>>>(
+          perm, cent, N, t.start.p, t.n.p, t.p.p, avg, ws.red_a.p);
+    CK_LAUNCH();
+    return ws.red_a.p;
+  }
   DBuf<double> *bufs[2] = {&ws.red_a, &ws.red_b};
   ll items = N;
   for (int l = 0; l < launches; l++) {
@@ -2077,11 +2191,13 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
       const double *isums = nullptr;
       const int launches = tree_launches((ll)maxn);
       if (ngroup) {
-        ws.tree_tab.ensure((size_t)2 * launches * (nseg + 1));
-        k_tree_offsets<<<launches, 1024, 0, st>>>(t.n.p, t.p.p, nseg, launches, ws.tree_tab.p);
-        CK_LAUNCH();
-        const double *sums = seg_tree_reduce<4, GEN_MEAN>(perm.p, cent, N, t, nullptr, launches,
-                                                          ws, &off);
+        if (maxn > 1024) {
+          ws.tree_tab.ensure((size_t)2 * launches * (nseg + 1));
+          k_tree_offsets<<<launches, 1024, 0, st>>>(t.n.p, t.p.p, nseg, launches, ws.tree_tab.p);
+          CK_LAUNCH();
+        }
+        const double *sums = seg_tree_reduce<4, GEN_MEAN>(perm.p, cent, N, t, nullptr, (ll)maxn,
+                                                          launches, ws, &off);
         k_rib_mean_group<<<grid_for(nseg, 256), 256, 0, st>>>(sums, off, t.n.p, t.p.p, nseg,
                                                               avg.p);
         CK_LAUNCH();
@@ -2092,10 +2208,16 @@ void bisect_segments(BisectKind kind, DBuf<int> &perm, SegTable &t,
         CK_LAUNCH();
       }
       if (ngroup)
-        isums = seg_tree_reduce<6, GEN_INERTIA>(perm.p, cent, N, t, avg.p, launches, ws, &off);
-      k_rib_axis<<<grid_for(4 * nseg, 128), 128, 0, st>>>(
-          perm.p, cent, N, t.start.p, t.n.p, t.p.p, nseg, ndim, do_local ? 1 : 0,
-          avg.p, isums, off, ws.ev.p, ws.axis.p);
+        isums = seg_tree_reduce<6, GEN_INERTIA>(perm.p, cent, N, t, avg.p, (ll)maxn, launches, ws,
+                                                &off);
+      if (nseg <= RIB_QUADS)
+        k_rib_axis<true><<<grid_for(4 * nseg, 128), 128, 0, st>>>(
+            perm.p, cent, N, t.start.p, t.n.p, t.p.p, nseg, ndim, do_local ? 1 : 0,
+            avg.p, isums, off, ws.ev.p, ws.axis.p);
+      else
+        k_rib_axis<false><<<grid_for(nseg, 128), 128, 0, st>>>(
+            perm.p, cent, N, t.start.p, t.n.p, t.p.p, nseg, ndim, do_local ? 1 : 0,
+            avg.p, isums, off, ws.ev.p, ws.axis.p);
       CK_LAUNCH();
       k_keys<BISECT_RIB><<<grid_for(N, 256), 256, 0, st>>>(
           perm.p, cent, nullptr, N, ws.seg_of_pos.p, ws.axis.p, avg.p, ws.ev.p, ws.keys.p,
