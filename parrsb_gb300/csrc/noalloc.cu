@@ -22,9 +22,9 @@ namespace {
 
 constexpr int NA_MAX = 8192;  // elements (the CTA-resident recursion limit)
 constexpr int NA_MAXDEV = 64;
-constexpr int NA_THREADS = 1024, NA_SLICES = 8, NA_CROWD = 64;  // k_na_ranks
+constexpr int NA_THREADS = 1024, NA_CROWD = 64;  // k_na_ranks
+constexpr int NA_SHARE = NA_THREADS / 4;         // elements that a block ranks
 constexpr int NA_RANKS_SMEM = NA_MAX * (8 + 4 + 2 + 4);         // keys, counts, list, values below
-static_assert(NA_SLICES * NA_THREADS >= NA_MAX, "an element per thread");
 
 constexpr size_t na_round(size_t b) { return (b + 255) & ~(size_t)255; }
 constexpr size_t NA_CENT = 0;                                           // double [3][NA_MAX]
@@ -91,10 +91,13 @@ __global__ void k_na_init(const double *__restrict__ xyz, int n, int nv, int ndi
 // marks one item of every value, and ranks its share of the elements: the
 // values of the buckets below, and the smaller ones of its own bucket.  Where
 // more than NA_CROWD items with different values share a bucket, marking would
-// take too long: the rank is then the number of elements below (sparse[axis]).  Bound by the latency of about eight
-// barriers; counting against all n values took twice as long (31 -> 17
-// us at 3315 elements).  NA_SLICES blocks per axis keep values that crowd
-// into few buckets (ties, outliers) within the cost of that.
+// take too long: the rank is then the number of elements below (sparse[axis]).
+// Bound by the latency of about eight barriers; counting against all n values
+// took twice as long (31 -> 17 us at 3315 elements).  Four threads rank an
+// element, so that values that crowd into few buckets (outliers, graded
+// meshes) stay within the cost of that; where one bucket holds most of them,
+// against all values in order, which takes a third of the list's instructions
+// (8000 elements into 16 parts, one of them far: 0.54 -> 0.21 ms, 0.26 by counting alone).
 __global__ void __launch_bounds__(NA_THREADS)
 k_na_ranks(const double *__restrict__ cent, int n, u32 *__restrict__ rank,
            double *__restrict__ uniq, int *__restrict__ sparse) {
@@ -188,16 +191,29 @@ k_na_ranks(const double *__restrict__ cent, int n, u32 *__restrict__ rank,
     __syncthreads();
     cta_scan<NA_MAX, NA_THREADS>(below, n);
   }
-  const int share = (n + NA_SLICES - 1) / NA_SLICES, i = blockIdx.x * share + threadIdx.x;
-  if ((int)threadIdx.x >= share || i >= n) return;
-  const unsigned long long k = na_keys[i];
+  const int i = blockIdx.x * NA_SHARE + (threadIdx.x >> 2), sub = threadIdx.x & 3;
+  const bool in = i < n;
+  const unsigned long long k = na_keys[in ? i : 0];
   const int b = bucket(k), j0 = b ? (int)cnt[b - 1] : 0, j1 = (int)cnt[b];
-  u32 r = dense ? below[j0] : (u32)j0;
-  const int jn = dense && j1 - j0 > NA_CROWD ? j0 : j1;  // (a single value)
-  for (int j = j0; j < jn; j++) {
-    const unsigned l = list[j];
-    r += (!dense || (l & FIRST)) && na_keys[l & ~(unsigned)FIRST] < k;
+  u32 r = 0;
+  if (!in || (dense && j1 - j0 > NA_CROWD)) {
+    // nothing to rank, or a single value
+  } else if (!dense && 2 * (j1 - j0) > n) {
+#pragma unroll 8
+    for (int j = sub; j < n; j += 4) r += na_keys[j] < k;
+  } else {
+    for (int j = j0 + sub; j < j1; j += 4) {
+      const unsigned l = list[j];
+      r += (!dense || (l & FIRST)) && na_keys[l & ~(unsigned)FIRST] < k;
+    }
   }
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  if (!in || sub) return;
+  if (dense)
+    r += below[j0];
+  else if (2 * (j1 - j0) <= n)
+    r += (u32)j0;
   rank[(ll)a * n + i] = r;
   const double v = c[i];
   uniq[(ll)a * n + r] = v == 0.0 ? 0.0 : v;  // -0 and +0 share a rank
@@ -229,15 +245,15 @@ extern "C" PARRSB_API int parrsb_part_mesh_rcb_noalloc(int *d_part, const double
   ll *seg_ll = reinterpret_cast<ll *>(base + NA_SEG);
   int *seg_int = reinterpret_cast<int *>(base + NA_SEG + 2 * sizeof(ll));
   k_na_init<<<(nel * ndim + 127) / 128, 128, 0, st>>>(d_xyz, nel, nv, ndim, P, cent, perm, seg_ll,
-                                               seg_int);
+                                                      seg_int);
   if (cudaGetLastError() != cudaSuccess) return PARRSB_ERR_CUDA;
   if (P == 1) {
     if (cudaMemsetAsync(d_part, 0, (size_t)nel * sizeof(int), st) != cudaSuccess)
       return PARRSB_ERR_CUDA;
     return PARRSB_OK;
   }
-  k_na_ranks<<<dim3(NA_SLICES, ndim), NA_THREADS, NA_RANKS_SMEM, st>>>(cent, nel, rank, uniq,
-                                                                      seg_int + 2);
+  k_na_ranks<<<dim3((nel + NA_SHARE - 1) / NA_SHARE, ndim), NA_THREADS, NA_RANKS_SMEM, st>>>(
+      cent, nel, rank, uniq, seg_int + 2);
   if (cudaGetLastError() != cudaSuccess) return PARRSB_ERR_CUDA;
   if (rcb_small_launch(perm, rank, uniq, nel, ndim, seg_ll, seg_ll + 1, seg_int, seg_int + 1, 1,
                        false, seg_int + 2, d_part, st) != cudaSuccess)
