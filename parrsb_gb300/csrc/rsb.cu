@@ -4066,21 +4066,35 @@ struct Lanczos {
   // group 118 / 141; FP32: 65K 12 / 23, 524K 24 / 44, 1M in 16 groups 35 / 52;
   // 1M in one group 54 / 52 and 8M in 512 groups 230 / 255 (lists of 7 groups
   // a team) are not worth it, hence the margin.
-  bool team_pays() const {
-    const bool f64 = sizeof(VT) == 8;
-    double worst = 0.0, rows = 0.0;
+  static constexpr double TS_US_GROUP = 7.3, TS_US_ROW = sizeof(VT) == 8 ? 0.0106 : 0.00266;
+  double launches_us(double rows) const {
+    return sizeof(VT) == 8 ? 24.0 + 112e-6 * rows : 22.0 + 29e-6 * rows;
+  }
+  double level_rows() const {
+    double rows = 0.0;
     for (const GState &s : hgs) rows += (double)s.n;
+    return rows;
+  }
+  bool team_pays() const {
+    double worst = 0.0;
     for (const int4 &b : ts_blk) {
       double t = 0.0;
       for (int q = 0; q < b.y; q++) {
         const GState &s = hgs[ts_list[b.x + q]];
         const ll k = ((ll)s.ntiles + b.w - 1) / b.w;
-        t += 7.3 + (f64 ? 0.0106 : 0.00266) * (double)std::min(k * tile_rows(s.n), s.n) +
+        t += TS_US_GROUP + TS_US_ROW * (double)std::min(k * tile_rows(s.n), s.n) +
              (b.w > 1 ? 0.03 * s.ntiles : 0.0);
       }
       worst = std::max(worst, t * (b.y > 1 && b.w > 1 ? 1.35 : 1.2));
     }
-    return worst < (f64 ? 24.0 + 112e-6 * rows : 22.0 + 29e-6 * rows);
+    return worst < launches_us(level_rows());
+  }
+  // false where the average of G blocks, which the busiest cannot be below, does
+  // not pay already: planning teams for thousands of groups takes the host
+  // longer than a step (4000 groups: 0.7 ms)
+  bool team_may_pay(int G) const {
+    const double rows = level_rows();
+    return 1.2 * (TS_US_GROUP * A + TS_US_ROW * rows) / G < launches_us(rows);
   }
 
   // whether this level runs its steps in k_team_steps (PARRSB_GPU_PERSIST=0:
@@ -4098,7 +4112,8 @@ struct Lanczos {
     ensure_smem_limit(k_team_steps<VT>, TS_SMEM);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_team_steps<VT>, TS_THREADS,
                                                      TS_SMEM));
-    if (per_sm < 1 || !plan_teams(sms) || !(force || team_pays())) return false;
+    if (per_sm < 1 || !(force || team_may_pay(sms))) return false;
+    if (!plan_teams(sms) || !(force || team_pays())) return false;
     // shared memory: p and w, the halo, then the encoded rows, then r as they fit
     const bool halos = ts_blk[0].w > 1;  // (teams of several blocks come first)
     // (a compact run of r rows of a 3D mesh has about 1.5 r^(2/3) x 6 halo rows)
