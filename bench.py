@@ -19,9 +19,11 @@ not installed) on the host cores.
 import argparse
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
+import tempfile
 import threading
 import time
 
@@ -132,11 +134,39 @@ def load_peaks():
         return 6800.0, "fallback"
 
 
-def load_traffic():
+class StderrCapture:
+    """What the process writes to file descriptor 2 inside the block (.text),
+    passed on afterwards."""
+
+    def __enter__(self):
+        sys.stderr.flush()
+        self.text, self.saved, self.file = "", os.dup(2), tempfile.TemporaryFile()
+        os.dup2(self.file.fileno(), 2)
+        return self
+
+    def __exit__(self, *exc):
+        sys.stderr.flush()
+        os.dup2(self.saved, 2)
+        os.close(self.saved)
+        self.file.seek(0)
+        self.text = self.file.read().decode(errors="replace")
+        self.file.close()
+        sys.stderr.write(self.text)
+
+
+def spmv_kernels(log):
+    """The SpMV kernels that the autotuner's log names, sorted."""
+    return sorted(set(re.findall(r"SpMV autotune .*-> (\w+) x", log)))
+
+
+def load_traffic(kernels):
     """DRAM bytes per algorithmic byte of one SpMV launch, from the committed
     ncu summary of a smaller case (the benchmark's launches are scaled by
-    their own algorithmic bytes: traffic grows with the matrix)."""
-    path = os.path.join(ROOT, "profiles", "k_spmv_loc_rsb_hex_128x128x64_level0.md")
+    their own algorithmic bytes: traffic grows with the matrix).  None where
+    the levels ran several kernels, or one without a summary."""
+    if len(kernels) != 1:
+        return None
+    path = os.path.join(ROOT, "profiles", f"{kernels[0]}_rsb_hex_128x128x64_level0.md")
     try:
         with open(path) as f:
             for line in f:
@@ -493,9 +523,11 @@ def main():
     t_dev = max_over_ranks(ev0.elapsed_time(ev1) / 1e3 / args.steps)
     # ---- one more step with CUDA events around every SpMV and vector update
     # of the Lanczos graphs (per-kernel times for the roofline and breakdown)
-    os.environ["PARRSB_GPU_TIMING"] = "1"
-    stats = [step_device()]
+    os.environ["PARRSB_GPU_TIMING"] = os.environ["PARRSB_GPU_AUTOTUNE_LOG"] = "1"
+    with StderrCapture() as log:
+        stats = [step_device()]
     os.environ["PARRSB_GPU_TIMING"] = "0"
+    del os.environ["PARRSB_GPU_AUTOTUNE_LOG"]
     # ---- end to end (host buffers, copies inside the timed region)
     t_e2e = None
     e2e_stages = None
@@ -635,7 +667,8 @@ def main():
     spmv_launches = sum(x.spmv_launches for x in stats)
     achieved = spmv_bytes / (spmv_ms / 1e3) / 1e9 if spmv_ms > 0 else None
     peak, peak_kind = load_peaks()
-    traffic = load_traffic()
+    kernels = spmv_kernels(log.text)
+    traffic = load_traffic(kernels)
     per_launch_bytes = spmv_bytes / spmv_launches if spmv_launches else None
     # the whole pass graph: SpMV bytes plus the vector updates' 3 x 4 B per
     # row and step each (FP32), over the pass graphs' device time
@@ -694,7 +727,7 @@ def main():
                 "link": link},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
-                     "traffic": tr_val, "kernel": "k_spmv_loc or k_spmv, as autotuned (Laplacian)",
+                     "traffic": tr_val, "kernel": " and ".join(kernels) + " (Laplacian)",
                      "traffic_note": ("DRAM bytes per launch: ncu dram bytes / algorithmic "
                                       "bytes of one level-0 launch on the 1M-element box "
                                       f"({traffic['dram_bytes_per_algorithmic_byte']:.3f}, "

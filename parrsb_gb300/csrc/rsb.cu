@@ -4244,12 +4244,19 @@ struct Lanczos {
     const int force_th = th_env ? atoi(th_env) : 0;
     std::array<ll, 6> key = {(ll)T, (ll)A, N, (ll)lv.max_w, (ll)force_kind * 1024 + force_th,
                              (ll)team};
+    auto log = [&] {
+      if (getenv("PARRSB_GPU_AUTOTUNE_LOG"))
+        fprintf(stderr, "parrsb_gb300: SpMV autotune tiles=%d groups=%d rows=%lld -> %s x %d\n", T,
+                A, (long long)N,
+                sp_kind == 2 ? "k_spmv_loc" : sp_kind == 1 ? "k_spmv_tma" : "k_spmv", bd);
+    };
     for (auto &kv : cache)
       if (kv.first == key) {
         sp_kind = kv.second >> 16;
         bd = kv.second & 0xFFFF;
         // (the same shape with other groups: the encoding may not fit them)
         if (sp_kind == 2 && !loc_prepare(lv)) sp_kind = 0, bd = 256;
+        log();
         return;
       }
     cudaStream_t st = ctx().stream;
@@ -4284,9 +4291,7 @@ struct Lanczos {
     sp_kind = pick.first;
     bd = pick.second;
     cache.push_back({key, (pick.first << 16) | pick.second});
-    if (getenv("PARRSB_GPU_AUTOTUNE_LOG"))
-      fprintf(stderr, "parrsb_gb300: SpMV autotune tiles=%d groups=%d rows=%lld -> %s x %d\n", T,
-              A, (long long)N, pick.first == 2 ? "k_spmv_loc" : pick.first ? "k_spmv_tma" : "k_spmv", pick.second);
+    log();
   }
 
   // Runs all passes; f holds the normalised Fiedler vectors afterwards.
