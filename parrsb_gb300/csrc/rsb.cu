@@ -96,8 +96,9 @@ __global__ void k_scatter_run(const int *__restrict__ vals, const int *__restric
 // match and at most one atomic, and the table is emptied by those that filled
 // it.  A longer list is read from the runs again and compared pairwise.
 // FILL = false: row lengths and the largest weight; FILL = true: columns and
-// weights at rowptr[a].  Bound by instruction issue: 1.2M hexes, 0.79 -> 0.42 ms to count and 0.71 -> 0.54 ms to fill
-// (three atomics per candidate and a second search before).
+// weights at rowptr[a].  Bound by instruction issue: 1.2M hexes, 0.79 -> 0.42 ms
+// to count and 0.71 -> 0.54 ms to fill (three atomics per candidate and a second
+// search before).
 constexpr int GR_WARPS = 4;
 constexpr int GR_CAP = 256;
 constexpr int GR_HASH = 256;  // power of two >= GR_CAP: more slots than distinct keys

@@ -8,10 +8,10 @@
 //
 // Per pass: a tile histogram kernel (4096 items per 512-thread CTA), a
 // per-digit exclusive scan over tiles, and a scatter kernel that loads its
-// 8 items per thread up front, ranks them stably inside the CTA with
-// __match_any_sync (warp w owns items [w*256, w*256+256) of the tile,
-// processed 32 at a time in order), stages the tile in shared memory in
-// digit order and writes each digit's run with consecutive addresses.  One
+// 8 items per thread up front, ranks them stably inside the CTA (warp w owns
+// items [w*256, w*256+256) of the tile, processed 32 at a time in order; the
+// lanes with the same digit by a ballot per bit), stages the tile in shared
+// memory in digit order and writes each digit's run with consecutive addresses.  One
 // up-front kernel builds the global digit histograms of every pass; passes
 // whose digit is constant over all items are skipped.
 #include <algorithm>
@@ -280,9 +280,9 @@ k_scatter(const u64 *__restrict__ kin, const int *__restrict__ vin,
 //                       the few items that share a 32-bit key are then put
 //                       right by their full keys (k_fix_runs), long runs (a
 //                       value that many items share, and one beside it) by a
-//                       CTA each.  Runs too long or too many for that (many
-//                       values that differ in their last bits only, or one far
-//                       outside the range of the others) take the full radix
+//                       CTA each.  Runs too long for that (many values that
+//                       differ in their last bits only, or one far outside the
+//                       range of the others) or too many take the full radix
 //                       sort, after the passes: RCB of 1M hexes 1.50 ms, with
 //                       one far element 2.22, by the full sort alone 2.05 (8M:
 //                       5.0, 7.6 and 8.2).  Asking a sample of 1024 keys first
@@ -294,7 +294,12 @@ constexpr int RANK_THREADS = 512;
 constexpr int LOCAL_MAX = 4096;
 constexpr int BUCKET_MAX = 128;  // items of a bucket that are ranked by counting
 constexpr int FIX_MAX = 32;  // items of a run that one thread puts right
-constexpr int RUN_LIST = 1024;  // longer runs that CTAs put right
+// Longer runs that CTAs put right.  A pipe of 96 x 72 x 106 without jitter has
+// 3500 of 212 (two last-bit forms of a value, 106 times each): RCB of it takes
+// 2.02 ms with them sorted by CTAs of 128 threads, 2.48 with the full sort, 2.37
+// by the full sort alone.
+constexpr int RUN_LIST = 1 << 16;
+constexpr int RUN_SHORT = 512;  // items of a run that 128 threads sort
 
 // keys[i], vals[i] of the segments of at most RANK_MAX items, out of place.
 // The CTA sees its positions and RANK_MAX more on both sides.
@@ -567,7 +572,7 @@ k_seg_local(u64 *__restrict__ keys, int *__restrict__ vals, const int *__restric
 }
 
 __global__ void k_range_init(u64 *__restrict__ range) {
-  range[0] = ~0ull, range[1] = 0ull, range[2] = 0ull, range[3] = 0ull;
+  range[0] = ~0ull, range[1] = 0ull, range[2] = 0ull, range[3] = 0ull, range[4] = 0ull;
 }
 __global__ void k_key_range(const u64 *__restrict__ keys, ll n, u64 *__restrict__ range) {
   u64 mn = ~0ull, mx = 0ull;
@@ -796,22 +801,28 @@ __device__ __forceinline__ void list_run(const u32 *__restrict__ q, ll n, u32 qi
   if (atomicOr(&mark[b >> 5], bit) & bit) return;
   const ll e = run_bound(q, n, (u64)qi + 1);
   const u64 at = e - b <= LOCAL_MAX ? atomicAdd(&range[3], 1ull) : (u64)RUN_LIST;
-  if (at < RUN_LIST)
+  if (at < RUN_LIST) {
     runs[at] = make_int2((int)b, (int)(e - b));
-  else
+    if (range[4] < (u64)(e - b)) atomicMax(&range[4], (u64)(e - b));
+  } else
     range[2] = 1ull;
 }
 __global__ void k_fix_runs(const u32 *__restrict__ q, ll n, u64 *__restrict__ keys,
                            int *__restrict__ vals, u64 *__restrict__ range,
                            u32 *__restrict__ mark, int2 *__restrict__ runs) {
   const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const u32 qi = q[i];
-  if (i > 0 && q[i - 1] == qi) {
-    if (i >= FIX_MAX && q[i - FIX_MAX] == qi && keys[i] < keys[i - 1])
-      list_run(q, n, qi, range, mark, runs);
-    return;
+  const bool in = i < n;
+  const u32 qi = in ? q[i] : 0u;
+  const bool first = in && !(i > 0 && q[i - 1] == qi);
+  const bool list = in && !first && i >= FIX_MAX && q[i - FIX_MAX] == qi && keys[i] < keys[i - 1];
+  const unsigned lists = __ballot_sync(0xffffffffu, list);
+  if (lists) {  // (the first of a run's lanes: the run is looked up once a warp)
+    const int lane = threadIdx.x & 31;
+    const unsigned before = lists & ((1u << lane) - 1u);
+    const u32 qb = __shfl_sync(0xffffffffu, qi, before ? 31 - __clz((int)before) : lane);
+    if (list && (!before || qb != qi)) list_run(q, n, qi, range, mark, runs);
   }
+  if (!first) return;
   int len = 1;
   bool sorted = true;
   u64 prev = keys[i];
@@ -839,22 +850,24 @@ __global__ void k_fix_runs(const u32 *__restrict__ q, ll n, u64 *__restrict__ ke
     vals[i + b] = v;
   }
 }
-// one CTA per listed run
-__global__ void __launch_bounds__(1024)
+// one CTA per listed run of more than MIN and at most MAX items
+template <int MIN, int MAX, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 k_sort_run(const int2 *__restrict__ runs, u64 *__restrict__ keys, int *__restrict__ vals) {
   extern __shared__ __align__(16) unsigned char lo_smem[];
   u64 *sk = reinterpret_cast<u64 *>(lo_smem);
-  u32 *sp = reinterpret_cast<u32 *>(sk + lo_at(LOCAL_MAX));
+  u32 *sp = reinterpret_cast<u32 *>(sk + lo_at(MAX));
   const int2 r = runs[blockIdx.x];
+  if (r.y <= MIN || r.y > MAX) return;
   int p2 = 2;
   while (p2 < r.y) p2 <<= 1;
-  for (int k = threadIdx.x; k < p2; k += 1024) {
+  for (int k = threadIdx.x; k < p2; k += THREADS) {
     sk[lo_at(k)] = k < r.y ? keys[r.x + k] : ~0ull;
     sp[lo_at(k)] = k < r.y ? (u32)k : 0xFFFF0000u | (u32)k;
   }
   __syncthreads();
-  bitonic_sort<1024>(sk, sp, p2);
-  local_store<LOCAL_MAX, 1024>(sk, sp, r.y, keys + r.x, vals + r.x);
+  bitonic_sort<THREADS>(sk, sp, p2);
+  local_store<MAX, THREADS>(sk, sp, r.y, keys + r.x, vals + r.x);
 }
 
 int bits_for(ll nseg) {
@@ -952,8 +965,8 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
   const int sb = bits_for(nseg);
   bool full = sb > 16;  // too few bits left for the values
   if (!full) {
-    ws.range.ensure(4);
-    ws.runs.ensure(RUN_LIST);
+    ws.range.ensure(5);
+    ws.runs.ensure((size_t)std::min<ll>(RUN_LIST, n / FIX_MAX + 1));
     ws.q.ensure((size_t)n), ws.mark.ensure((size_t)(n + 31) / 32);
     ws.ktmp.ensure((size_t)n), ws.vtmp.ensure((size_t)n);
     // the passes go from (qa, ia) to (qb, ib) and back; ktmp holds the second
@@ -990,14 +1003,20 @@ void sort_by_value(DBuf<u64> &keys, DBuf<int> &vals, ll n, const int *seg_of_pos
     k_fix_runs<<<grid_for(n, 256), 256, 0, st>>>(ws.q.p, n, ws.ktmp.p, ws.vtmp.p, ws.range.p,
                                                  ws.mark.p, ws.runs.p);
     CK_LAUNCH();
-    u64 said[2] = {0, 0};
-    d2h(said, ws.range.p + 2, 2);
+    u64 said[3] = {0, 0, 0};
+    d2h(said, ws.range.p + 2, 3);
     sync();
     full = said[0] != 0;
     if (!full && said[1] > 0) {
-      ensure_smem_limit(k_sort_run, (int)local_smem(LOCAL_MAX));
-      k_sort_run<<<(unsigned)said[1], 1024, local_smem(LOCAL_MAX), st>>>(ws.runs.p, ws.ktmp.p,
-                                                                         ws.vtmp.p);
+      k_sort_run<0, RUN_SHORT, 128><<<(unsigned)said[1], 128, local_smem(RUN_SHORT), st>>>(
+          ws.runs.p, ws.ktmp.p, ws.vtmp.p);
+      CK_LAUNCH();
+    }
+    if (!full && said[2] > RUN_SHORT) {
+      auto kern = k_sort_run<RUN_SHORT, LOCAL_MAX, 1024>;
+      ensure_smem_limit(kern, (int)local_smem(LOCAL_MAX));
+      kern<<<(unsigned)said[1], 1024, local_smem(LOCAL_MAX), st>>>(ws.runs.p, ws.ktmp.p,
+                                                                   ws.vtmp.p);
       CK_LAUNCH();
     }
   }

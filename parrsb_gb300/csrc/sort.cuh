@@ -80,7 +80,8 @@ struct SortWs {
   DBuf<u32> q;          // 32-bit keys (their other buffer: ktmp)
   DBuf<u32> mark;       // a bit per item
   DBuf<int> pos;        // positions, where the full keys are sorted
-  DBuf<u64> range;      // smallest and largest key, runs that cannot be listed, runs listed
+  DBuf<u64> range;      // smallest and largest key, runs that cannot be listed, runs listed,
+                        // the longest of these
   DBuf<int2> runs;      // long runs out of order: start, length
   // gives the buffers of more than `keep` items back to the pool
   void trim(ll keep) {

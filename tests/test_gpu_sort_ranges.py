@@ -1,7 +1,7 @@
 """Sorts of values that a linear map over their range does not separate (one far
-point, clumps, geometric grading), on both sides of the sample's decision: RIB
-orders and RCB parts against the oracle, gencon ids against those of the same
-mesh without its far element."""
+point, clumps, geometric grading, last-bit forms of a value): RIB orders and RCB
+parts against the oracle, gencon ids against those of the same mesh without its
+far element."""
 import numpy as np
 import pytest
 
@@ -31,13 +31,16 @@ def _values(kind, n):
         x[: n // 2] = 0.5 + x[: n // 2] * 1e-12
     elif kind == "graded":
         x = np.expm1(np.log(1e12) * x)
+    elif kind == "twins":  # many values, each in two forms
+        x = (np.floor(n / 100.0 * x) + 1.0) * (1.0 + 2.0 ** -52 * rng.integers(0, 2, n))
     elif kind == "planes":  # 30 values, in their last bits apart
         x = np.floor(30.0 * x) / 30.0 * (1.0 + 2.0 ** -52 * rng.integers(-2, 3, n))
     return x
 
 
 @pytest.mark.parametrize("n", [4097, 20000, 262144, 300001])
-@pytest.mark.parametrize("kind", ["far", "clumps", "tight_clumps", "points", "graded", "planes"])
+@pytest.mark.parametrize("kind", ["far", "clumps", "tight_clumps", "points", "graded", "twins",
+                                  "planes"])
 def test_ranges(oracle, kind, n):
     vtx, xyz = _line(_values(kind, n))
     for partitioner in (1, 2):
