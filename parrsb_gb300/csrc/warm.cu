@@ -721,13 +721,15 @@ k_mp_gather(const bf16 *__restrict__ H, const unsigned *__restrict__ ell,
 //   A = [h_prev | AG]   (64 x 128, BF16), Z = A W + b (tensor cores, FP32),
 //   h = relu(Z) -> Hout (BF16, optional)
 // HEAD: also y = h . wo + bo (FP32) per row.
+// Hout may be AG's buffer: a block has read a tile when it writes it, and what
+// it is reading by then are other rows.
 // Bound by memory: 256 bytes of A and 128 of h a row, which the next tile's
 // asynchronous copies keep in flight (330K rows: 30 to 35 us, and 72 us
 // for the gather; 270 us as one kernel, whose gather had too few warps).
 template <bool HEAD>
 __global__ void __launch_bounds__(MP_THREADS, 4)
-k_mp_layer(const bf16 *__restrict__ Hin, const bf16 *__restrict__ AG, ll N, ll Npad,
-           const bf16 *__restrict__ Wf, const float *__restrict__ bias, bf16 *__restrict__ Hout,
+k_mp_layer(const bf16 *__restrict__ Hin, const bf16 *AG, ll N, ll Npad,
+           const bf16 *__restrict__ Wf, const float *__restrict__ bias, bf16 *Hout,
            const float *__restrict__ wo, const float *__restrict__ bo, float *__restrict__ y,
            const float *__restrict__ Xg) {
   constexpr int K = MP_K2, KP = K + 8, BUF = MP_ROWS * KP;
@@ -1323,11 +1325,13 @@ void mp_forward(const MpView &v, const NetDev &net, MpBuffers &B, bool keep) {
   cudaStream_t st = ctx().stream;
   const size_t nh = (size_t)v.Npad * MP_HID;
   B.H[0].ensure(nh), B.H[1].ensure(nh), B.y.ensure((size_t)v.Npad);
-  B.AG[1].ensure(nh);
   if (keep) {
     B.H[2].ensure(nh);
-    B.AG0.ensure((size_t)v.Npad * MP_FIN), B.AG[2].ensure(nh);
+    B.AG0.ensure((size_t)v.Npad * MP_FIN), B.AG[1].ensure(nh), B.AG[2].ensure(nh);
   }
+  // the neighbour means of a forward pass alone: the second layer's where its
+  // output goes, the third's where the first layer's output was
+  bf16 *ag1 = keep ? B.AG[1].p : B.H[1].p, *ag2 = keep ? B.AG[2].p : B.H[0].p;
   const Level &lv = *v.lv;
   const unsigned grid = mp_grid(v.Npad);
   const float *p = net.p;
@@ -1337,14 +1341,13 @@ void mp_forward(const MpView &v, const NetDev &net, MpBuffers &B, bool keep) {
   CK_LAUNCH();
   ensure_smem_limit(k_mp_layer<false>, ML_SMEM);
   ensure_smem_limit(k_mp_layer<true>, ML_SMEM);
-  bf16 *ag2 = keep ? B.AG[2].p : B.AG[1].p;
   k_mp_gather<false><<<mp_gather_grid(v.Npad), MG_THREADS, 0, st>>>(
       B.H[0].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, nullptr, nullptr,
-      B.AG[1].p);
+      ag1);
   CK_LAUNCH();
   k_mp_layer<false><<<mp_layer_grid(v.Npad), MP_THREADS, ML_SMEM, st>>>(
-      B.H[0].p, B.AG[1].p, v.N, v.Npad, net.Wf[1], p + MP_OFF_B2, B.H[1].p, nullptr, nullptr,
-      nullptr, nullptr);
+      B.H[0].p, ag1, v.N, v.Npad, net.Wf[1], p + MP_OFF_B2, B.H[1].p, nullptr, nullptr, nullptr,
+      nullptr);
   CK_LAUNCH();
   k_mp_gather<false><<<mp_gather_grid(v.Npad), MG_THREADS, 0, st>>>(
       B.H[1].p, lv.ell.p, lv.slice_off.p, lv.slice_w.p, B.wsum.p, v.N, v.Npad, nullptr, nullptr,
